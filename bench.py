@@ -47,7 +47,7 @@ CONFIG_BASE = {"workload": "bulk stream-mode digest generation", "files": 4096, 
                "mode": "stream (-b 0)", "l2": "inputs larger than L2 (no flush needed)"}
 
 
-KERNELS = ("k_stream_ranks", "k_stream_tiles", "k_stream_fails", "k_stream_fix_list", "k_stream_check", "k_stream_fix",
+KERNELS = ("k_stream_ranks", "k_stream_tiles", "k_stream_fails", "k_stream_fix_list", "k_stream_fix",
            "k_stream_commit", "k_pack_filters", "k_scan_offsets")
 
 
@@ -1065,7 +1065,7 @@ def main_index(args):
 
 
 IB_METRIC = "index build input GB/s"
-IB_KERNELS = ("k_stream_tiles", "k_stream_check", "k_stream_fix", "k_stream_commit_round", "k_stream_index_pred", "k_pred_dirty",
+IB_KERNELS = ("k_stream_tiles", "k_stream_fix", "k_stream_commit_round", "k_stream_index_pred", "k_pred_dirty",
               "k_index_first_init", "k_stream_index_first", "k_stream_index_mark", "k_stream_commit_index",
               "k_scan_offsets", "k_pack_filters", "k_block_digest", "k_index_first", "k_index_mark")
 

@@ -54,7 +54,7 @@ uint64_t sdbfg_ctx_launch_count(const sdbfg_ctx *ctx);
 /* Per-kernel timing with CUDA events recorded on the launch stream around
  * every launch (off by default; enabling clears previous totals).
  * sdbfg_ctx_kernel_time reports the accumulated milliseconds and launch
- * count of one kernel ("k_stream_tiles", "k_stream_check", "k_stream_fix",
+ * count of one kernel ("k_stream_tiles", "k_stream_fix",
  * "k_stream_commit", "k_pack_filters", "k_block_digest", "k_compare_pairs",
  * "k_scan_offsets").  While profiling, the stream kernels also count SM
  * cycles per phase; the names "k_stream_tiles.{load,ranks,fres,walk,link,

@@ -9,12 +9,10 @@
 //                   (gen_chunk_scores :50-89, parallelised below) ->
 //                   selection score > 16 -> SHA-1 of every selected 64-byte
 //                   feature.  Writes the ordered feature digests of the tile.
-//  k_stream_check   one warp per chunk: finds the first tile whose
-//                   speculative entry state differs from its predecessor's
-//                   exit state.
-//  k_stream_fix     one CTA per chunk with such a tile (others exit at
-//                   once): recomputes tiles in place from the true state.
-//  k_stream_commit  one warp per file: the ordered filter fill of
+//  k_stream_fix     one CTA per chunk: finds tiles whose speculative entry
+//                   state differs from their predecessor's exit state and
+//                   recomputes them in place from the true state.
+//  k_stream_commit  one CTA per file: the ordered filter fill of
 //                   gen_chunk_hash (:93-136) -- 256-byte filter insert with
 //                   zero-new-bit suppression, the 16 KiB "big filter"
 //                   dedupe (bloom_filter.cc:333-359), roll-over at 160
@@ -34,7 +32,7 @@
 // with the state its left neighbour reaches at the same step.  Equal states
 // prove the segment exact (induction from step 0, which is always a full
 // rescan); a mismatch is re-walked from the neighbour's state.  The same
-// check links consecutive tiles of a chunk (k_stream_check / k_stream_fix).
+// check links consecutive tiles of a chunk (k_stream_fails / k_stream_fix).
 #include <cstdint>
 #include <cuda_runtime.h>
 
@@ -852,6 +850,10 @@ __device__ inline TileGeom stream_geom(uint32_t n, uint32_t t0) {
     return g;
 }
 
+// A tile's features in GenParams::features: words 0..3 of each feature as one
+// uint4, then the fifth words.
+__device__ __forceinline__ uint32_t feat_word(uint32_t f, int k) { return k < 4 ? 4 * f + k : 4 * kTileCap + f; }
+
 // kPre: ranks precomputed in P.ranks (tile_smem_bytes_pre layout); the
 // SHA-1 phase then reads the feature bytes from global memory.
 template <bool kPre>
@@ -897,8 +899,9 @@ __device__ void stream_tile_body(const GenParams& P, uint32_t tile, const uint64
         else
             load_be16(s.bytes32, p, w);
         sha1_feature(w, h);
-#pragma unroll
-        for (int k = 0; k < 5; k++) feat[k * kTileCap + f] = h[k];
+        static_assert(5 * kTileCap % 4 == 0, "a tile's features start 16-byte aligned");
+        reinterpret_cast<uint4*>(feat)[f] = make_uint4(h[0], h[1], h[2], h[3]);
+        feat[4 * kTileCap + f] = h[4];
     }
     if (threadIdx.x == 0) {
         out->count = nf;
@@ -933,36 +936,20 @@ __global__ void __launch_bounds__(kGenThreads, 5) k_stream_tiles_pre(GenParams P
 
 // Link tiles of a chunk: a tile's speculative entry state must equal its
 // predecessor's exit state (tiles whose lead-in reaches step 0 are exact).
-// k_stream_check (one warp per chunk, no shared memory) finds the first
-// tile of each chunk whose link fails; k_stream_fix (one CTA per chunk,
-// normally exiting at once) recomputes that tile from the true entry state
-// and moves on through the chunk: its threads check the links of the next
-// kGenThreads tiles at once, and the first failing one (a later tile whose
-// entry no longer matches, or an unrelated mis-speculation) is recomputed
-// next.
+// k_stream_fix (one CTA per chunk) first checks all links of its chunk, with
+// no exit from the loop so that the loads overlap (a 32 MiB chunk has 4,229;
+// a warp per chunk that left at the first failing link spent 84 us on the
+// six full chunks of a 200 MiB file), and normally ends there; else it recomputes the first failing tile from
+// the true entry state and moves on through the chunk: its threads check
+// the links of the next kGenThreads tiles at once, and the first failing
+// one (a later tile whose entry no longer matches, or an unrelated
+// mis-speculation) is recomputed next.
 __device__ __forceinline__ bool link_fails(const GenParams& P, const GenChunk& C, uint32_t tile) {
     const TileGeom g = stream_geom(C.n, P.tiles[tile].t0);
     return g.S0 > P.lead && P.tile_out[tile - 1].tau_out != P.tile_out[tile].sig_in;
 }
 
-__global__ void __launch_bounds__(128) k_stream_check(GenParams P) {
-    const uint32_t lane = threadIdx.x & 31;
-    const uint32_t warp = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5);
-    const uint32_t nwarps = gridDim.x * (blockDim.x / 32);
-    for (uint32_t c = warp; c < P.nchunks; c += nwarps) {
-        const GenChunk C = P.chunks[c];
-        uint32_t first = 0xFFFFFFFFu;
-        for (uint32_t j0 = 1; j0 < C.ntiles && first == 0xFFFFFFFFu; j0 += 32) {
-            const uint32_t j = j0 + lane;
-            const bool bad = j < C.ntiles && link_fails(P, C, C.first_tile + j);
-            const uint32_t m = __ballot_sync(0xffffffffu, bad);
-            if (m) first = j0 + __ffs(m) - 1;
-        }
-        if (lane == 0) P.chunk_redo[c] = first;
-    }
-}
-
-// Before k_stream_check / k_stream_fix: every tile whose link fails goes
+// Before k_stream_fix: every tile whose link fails goes
 // to P.fix_list (fix_list[0] = their number, zeroed by the host), and
 // k_stream_fix_list recomputes them all at once, one CTA each, from their
 // predecessors' exit states as they stand.  A tile whose predecessor is
@@ -996,11 +983,19 @@ __global__ void __launch_bounds__(kGenThreads) k_stream_fix(GenParams P) {
     __shared__ uint64_t entry;
     __shared__ uint32_t bad_first;
     for (uint32_t c = blockIdx.x; c < P.nchunks; c += gridDim.x) {
-        const uint32_t first = P.chunk_redo[c];
-        if (first == 0xFFFFFFFFu) continue;
         const GenChunk C = P.chunks[c];
-        uint32_t j = first;
-        while (j < C.ntiles) {
+        __syncthreads();  // the previous chunk is done with bad_first
+        if (threadIdx.x == 0) bad_first = 0xFFFFFFFFu;
+        __syncthreads();
+        uint32_t mine = 0xFFFFFFFFu;
+#pragma unroll 4
+        for (uint32_t jj = 1 + threadIdx.x; jj < C.ntiles; jj += blockDim.x)
+            if (link_fails(P, C, C.first_tile + jj)) mine = min(mine, jj);
+        if (mine != 0xFFFFFFFFu) atomicMin(&bad_first, mine);
+        __syncthreads();
+        uint32_t j = bad_first;
+        __syncthreads();
+        while (j < C.ntiles) {  // ~0: every link holds
             // the first failing link among tiles [j, j + blockDim.x); tiles
             // recomputed before it are visible here (same CTA, after a barrier)
             if (threadIdx.x == 0) bad_first = 0xFFFFFFFFu;
@@ -1094,13 +1089,92 @@ __global__ void __launch_bounds__(kRkThreads, 3) k_stream_ranks(GenParams P) {
 }
 
 // ------------------------------------------------------- ordered commit
-// Per-warp shared state for the stream commit.
+// The ordered filter fill (gen_chunk_hash, sdbf_core.cc:93-136): a feature
+// is counted iff it sets a new bit in the 256-byte filter F (bf_sha1_insert)
+// and a new bit in the 16 KiB big filter G (query_and_set); F keeps the bits
+// of features that fail G.  F rolls over at 160 counted features, G at 8,738
+// counted per chunk (the counter is local to a chunk, sdbf_core.cc:100; G
+// itself continues).
+//
+// One CTA per file takes a window of up to kCmWin consecutive features per
+// pass, one per thread; the order inside the window is recovered without a
+// serial step:
+//  * every hash word puts its feature's number into a table of the smallest
+//    feature number per 12-bit index (atomicMin; the pass number, counting
+//    down, is the key's high part, so a pass overrides its predecessors and
+//    the table is never cleared).  The 11-bit filter index of a word is new
+//    in F iff it is unset before the window and neither of its two 12-bit
+//    entries names an earlier feature;
+//  * a big-filter bit whose 12-bit entry names this very feature has no
+//    earlier holder in the window, so it is new in G iff it was unset.  A
+//    feature whose unset big-filter bits all have an earlier 12-bit holder
+//    is compared with the 17-bit values of the earlier F-passing features
+//    (slow path; 0.3 features per pass on mixture content);
+//  * a prefix count of the counted flags cuts the window behind the feature
+//    at which F or G rolls over: exactly the features with fewer counted
+//    predecessors than that are applied, the rest start the next pass.
+// A filter takes ~163 features, so a pass is normally one whole filter.
+// Three barriers per pass: (1) table filled and the last window's bits
+// applied, (2) flags known, (3) the window's end known; (2) and (3) are the
+// window's threads' only.  A separate warp streams the
+// tiles' features into a ring; it meets the others once a pass, at (1), and
+// what it publishes there counts from the next pass on, so that its copies
+// and its own instructions have a whole pass.
+//
+// What bounds it: the chain of passes of the largest file -- about 1,000
+// cycles of shared-memory work (random words: four cycles per warp
+// instruction) and the latency of the barriers.  One 200 MiB file (2.7 M
+// features, 16,720 passes of 1,885 cycles) commits in 15.2 ms, 64 files of
+// 1 MiB in 0.107 ms; one warp per file taking 32 features per pass took 87.2
+// and 0.543 ms.  Measured beside it: a lane per (feature, hash word), 30
+// warps: 3,225 cycles per pass; the loading warp taking part in barrier (2):
+// 2,740; the window's end found by every warp instead of at barrier (3), and
+// F read when it is known to be empty: 2,270.
+//
+// With an index being built (sdhash --index: sdbf_core.cc:108-114), a
+// feature whose filter insert set a new bit is inserted into the index and
+// is skipped unless that set a new index bit -- so each file depends on
+// every earlier file's features.  Two ways to get that order:
+// * k_stream_commit_index: one warp commits all files in input order, one
+//   feature at a time, the index in global memory;
+// * k_stream_commit_round: one round of a fixed point.  Files commit in
+//   parallel; a feature is taken as setting a new index bit iff no feature
+//   inserted in the previous round precedes it as the first setter of one of
+//   its bits (GenParams::index_pred, one bit per feature), and the inserted
+//   features are recorded (GenParams::index_seen).  A file's commit depends
+//   only on its own features and their predicate bits, so later rounds
+//   re-commit only the files whose bits changed (GenParams::commit_dirty),
+//   after clearing their seen bits, from the last checkpoint before the
+//   first change.  A round that inserts the same features as the previous
+//   one reproduces the sequential result: by induction over the input order,
+//   every decision then depends only on earlier decisions that already agree.
+constexpr uint32_t kCmWarps = kCmWin / 32;
+constexpr uint32_t kCmRing = 1024;  // features staged ahead (a tile has at most kTileCap)
+constexpr uint32_t kCmTiles = 4;    // tiles the loading warp starts per pass
+static_assert(kCmWin % 32 == 0 && kCmWin <= 256 && kCmThreads == (int)kCmWin + 32, "one thread per window feature");
+static_assert(kCmWarps == 6, "the warps' flags are read as a uint4 and a uint2");
+static_assert(kCmRing >= kTileCap + 2 * kCmWin, "a tile fits the ring beside two windows");
+
+template <bool kRound>
 struct CommitSmem {
-    uint32_t F[64];                  // current 256-byte filter
-    uint32_t own[2048];              // lanes of the group holding each filter index
-    uint32_t G[kBigBytes / 4];       // current 16 KiB big filter
-    uint32_t feat[2][5][kTileCap];   // double-buffered features of a tile
+    uint4 feat4[kCmRing];                   // hash words 0..3 of the staged features
+    uint32_t feat1[kCmRing];                // hash word 4
+    alignas(16) uint32_t G[kBigBytes / 4];  // current big filter (cleared and copied in 16-byte words)
+    uint32_t tab[4096];                     // (pass key << 8 | feature) of each 12-bit index
+    uint32_t F[2][64];                      // current filter (the other one is being written out)
+    uint32_t match[kCmWin];                 // slow path: big-filter values held by an earlier feature
+    alignas(16) uint32_t counted[8], ambig[8];  // per warp
+    uint32_t end;                           // features the pass consumes, when F or G rolls over
+    // published before barrier (1) of a pass, by pass parity (a reader may be
+    // late by the time until the next barrier (1)):
+    uint32_t pos[2];     // the window's start, for the loading warp
+    uint32_t avail[2];   // features of the file in the ring so far (end position)
+    uint32_t final_[2];  // avail is the end of the segment
+    uint32_t seg_pos;    // the segment's end position, once it is through
+    uint32_t ord[kRound ? kCmRing : 1];     // index rounds: the feature's ordinal
 };
+// barrier of the window's threads (the loading warp does not take part)
+__device__ __forceinline__ void commit_sync() { asm volatile("bar.sync 1, %0;" ::"n"(kCmWin) : "memory"); }
 
 __device__ inline uint32_t lanemask_le() {
     uint32_t m;
@@ -1112,65 +1186,33 @@ __device__ inline uint32_t lanemask_lt() {
     asm("mov.u32 %0, %%lanemask_lt;" : "=r"(m));
     return m;
 }
+__device__ __forceinline__ void cp_async4(void* smem, const void* gmem) {
+    const uint32_t s = static_cast<uint32_t>(__cvta_generic_to_shared(smem));
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(s), "l"(gmem));
+}
+__device__ __forceinline__ void cp_async_wait_2() { asm volatile("cp.async.wait_group 2;\n" ::); }
 
-
-// Stage the first `nf` features of a tile (5 rows of kTileCap words) into buf.
-__device__ __forceinline__ void stage_tile(uint32_t (*buf)[kTileCap], const uint32_t* feat, uint32_t nf,
-                                           uint32_t lane) {
-    const uint32_t n4 = (nf + 3) / 4;
-    for (uint32_t q = lane; q < 5 * n4; q += 32) {
-        const uint32_t k = q / n4, j = q - k * n4;
-        cp_async16(&buf[k][4 * j], feat + (size_t)k * kTileCap + 4 * j);
+// The last filter is out; the chop of sdbf_core.cc:235-238 and the file's result.
+__device__ __forceinline__ void commit_result(const GenParams& P, uint32_t file, uint32_t bf_count, uint32_t last_count) {
+    if (bf_count > 1 && last_count < (uint32_t)kMaxElem / 8) {
+        bf_count--;
+        last_count = kMaxElem;
     }
-    cp_async_commit();
+    P.out_info[file].bf_count = bf_count;
+    P.out_info[file].last_count = last_count;
 }
 
-// The ordered filter fill for one group of up to 32 features (lane l holds
-// feature l), in feature order, with the semantics of gen_chunk_hash
-// (sdbf_core.cc:103-130): a feature is counted iff it sets a new bit in the
-// 256-byte filter F (bf_sha1_insert) and a new bit in the big filter G
-// (query_and_set); F keeps the bits of features that fail G.
-//
-// "New" means unset before this feature, i.e. unset in the state before the
-// group and not held by an earlier lane of the group.  Earlier holders of a
-// filter index come from an owner mask (bit l set for every lane holding the
-// 11-bit index).  Two big-filter indices can only be equal if their low 11
-// bits -- the filter index -- are, so the same mask names the only lanes
-// whose 17-bit values need an exact comparison (register shuffles).  Bits
-// are written only for lanes up to the first roll-over, which is found
-// before anything is written; later lanes are re-run against the new state.
-//
-// With an index being built (sdhash --index: sdbf_core.cc:108-114), a
-// feature whose filter insert set a new bit is inserted into the index and
-// is skipped unless that set a new index bit -- so each file depends on
-// every earlier file's features.  Two ways to get that order:
-// * kCommitSeq: one warp commits all files in input order, one feature at
-//   a time (lane 0), the index in global memory;
-// * kCommitRound: one round of a fixed point.  Files commit in parallel; a
-//   feature is taken as setting a new index bit iff no feature inserted in
-//   the previous round precedes it as the first setter of one of its bits
-//   (GenParams::index_pred, one bit per feature, read with the tile), and
-//   the inserted features are recorded (GenParams::index_seen).  A file's
-//   commit depends only on its own features and their predicate bits, so
-//   later rounds re-commit only the files whose bits changed
-//   (GenParams::commit_dirty), after clearing their seen bits.  A round that inserts the same features as
-//   the previous one reproduces the sequential result: by induction over
-//   the input order, every decision then depends only on earlier decisions
-//   that already agree.
-enum : int { kCommitPlain = 0, kCommitSeq = 1, kCommitRound = 2 };
-
-template <int kMode>
+template <bool kRound>
 __device__ __forceinline__ void commit_files(const GenParams& P, uint8_t* smem) {
-    constexpr bool kIdx = kMode == kCommitSeq;
-    const uint32_t wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    if (kIdx && (blockIdx.x != 0 || wid != 0)) return;
-    CommitSmem& S = reinterpret_cast<CommitSmem*>(smem)[wid];
-    for (uint32_t i = lane; i < 2048; i += 32) S.own[i] = 0;
-    const uint32_t fstep = kIdx ? 1u : gridDim.x * kCommitWarps;
-    constexpr uint32_t kGroup = kIdx ? 1u : 32u;
-    for (uint32_t fi = kIdx ? 0u : blockIdx.x * kCommitWarps + wid; fi < P.nfiles; fi += fstep) {
+    CommitSmem<kRound>& S = *reinterpret_cast<CommitSmem<kRound>*>(smem);
+    const uint32_t tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    const bool loader = wid == kCmWarps;
+    for (uint32_t i = tid; i < 4096; i += kCmThreads) S.tab[i] = 0xFFFFFFFFu;
+    for (uint32_t i = tid; i < kCmWin; i += kCmThreads) S.match[i] = 0;
+    uint32_t epoch = 0xFFFFFFu;  // counts down: a later pass has smaller keys
+    for (uint32_t fi = blockIdx.x; fi < P.nfiles; fi += gridDim.x) {
         const uint32_t file = P.file_order[fi];
-        if (kMode == kCommitRound && P.commit_dirty && !P.commit_dirty[file]) continue;
+        if (kRound && P.commit_dirty && !P.commit_dirty[file]) continue;
         const GenFile Fd = P.files[file];
         if (Fd.nchunks == 0) continue;
         uint32_t* out = P.out_filters + (size_t)Fd.filter_base * 64;
@@ -1178,6 +1220,7 @@ __device__ __forceinline__ void commit_files(const GenParams& P, uint8_t* smem) 
         const GenChunk c0 = P.chunks[Fd.first_chunk];
         const GenChunk cl = P.chunks[Fd.first_chunk + Fd.nchunks - 1];
         const uint32_t t_first = c0.first_tile, t_end = cl.first_tile + cl.ntiles;
+        const uint32_t chunk_end = Fd.first_chunk + Fd.nchunks;
         uint32_t chunk = Fd.first_chunk;
         uint32_t next_chunk_tile = (Fd.nchunks > 1) ? P.chunks[chunk + 1].first_tile : 0xFFFFFFFFu;
         uint32_t bf_count = 1, last_count = 0, bigfi = 0;
@@ -1185,290 +1228,415 @@ __device__ __forceinline__ void commit_files(const GenParams& P, uint8_t* smem) 
         // last checkpoint at or before the first changed predicate (nothing
         // before it changed, so the state there is the one recorded)
         uint32_t ts = t_first;
-        if (kMode == kCommitRound && P.commit_dirty) {
+        if (kRound && P.commit_dirty) {
             const uint32_t from = P.commit_from[file];
             const uint32_t tc = from == 0xFFFFFFFFu ? 0u : from / kTileCap / kCkptTiles * kCkptTiles;
             if (tc > t_first && tc < t_end) ts = tc;
-            if (P.phase && lane == 0 && ts > t_first) atomicAdd(P.phase + kPhCkptRestarts, 1ull);
+            if (P.phase && tid == 0 && ts > t_first) atomicAdd(P.phase + kPhCkptRestarts, 1ull);
         }
+        __syncthreads();  // the previous file is done with the shared state
         if (ts > t_first) {
             const uint32_t* ck = P.commit_ckpt + (size_t)(ts / kCkptTiles) * kCkptWords;
-            for (uint32_t i = lane; i < 64; i += 32) S.F[i] = ck[i];
+            for (uint32_t i = tid; i < 64; i += kCmThreads) {
+                S.F[0][i] = ck[i];
+                S.F[1][i] = 0;
+            }
             const uint4* g4 = reinterpret_cast<const uint4*>(ck + 64);
-            for (uint32_t i = lane; i < kBigBytes / 16; i += 32) reinterpret_cast<uint4*>(S.G)[i] = g4[i];
+            for (uint32_t i = tid; i < kBigBytes / 16; i += kCmThreads) reinterpret_cast<uint4*>(S.G)[i] = g4[i];
             bf_count = ck[64 + 4096];
             last_count = ck[64 + 4096 + 1];
             bigfi = ck[64 + 4096 + 2];
-            // the chunk holding tile ts - 1, as the loop leaves it
+            // the chunk holding tile ts - 1, as the segment loop leaves it
             while (next_chunk_tile < ts) {
                 chunk++;
-                next_chunk_tile = (chunk + 1 < Fd.first_chunk + Fd.nchunks) ? P.chunks[chunk + 1].first_tile
-                                                                             : 0xFFFFFFFFu;
+                next_chunk_tile = chunk + 1 < chunk_end ? P.chunks[chunk + 1].first_tile : 0xFFFFFFFFu;
             }
         } else {
-            for (uint32_t i = lane; i < 64; i += 32) S.F[i] = 0;
-            for (uint32_t i = lane; i < kBigBytes / 4; i += 32) S.G[i] = 0;
+            for (uint32_t i = tid; i < 128; i += kCmThreads) S.F[0][i] = 0;
+            for (uint32_t i = tid; i < kBigBytes / 16; i += kCmThreads)
+                reinterpret_cast<uint4*>(S.G)[i] = make_uint4(0, 0, 0, 0);
         }
-        if (kMode == kCommitRound && P.commit_dirty && ts < t_end) {
+        if (kRound && P.commit_dirty && ts < t_end) {
             // clear the file's seen bits, ordinals [ts, t_end) * kTileCap;
             // inner words are the file's alone, edge words shared with neighbours
             const uint32_t o0 = ts * kTileCap, o1 = t_end * kTileCap - 1;
-            for (uint32_t w = (o0 >> 5) + lane; w <= (o1 >> 5); w += 32) {
+            for (uint32_t w = (o0 >> 5) + tid; w <= (o1 >> 5); w += kCmThreads) {
                 const uint32_t lo = w == (o0 >> 5) ? (o0 & 31u) : 0u, hi = w == (o1 >> 5) ? (o1 & 31u) : 31u;
                 const uint32_t m = (0xffffffffu >> (31u - hi)) & (0xffffffffu << lo);
                 if (m == 0xffffffffu) P.index_seen[w] = 0;
                 else atomicAnd(P.index_seen + w, ~m);
             }
-            __syncwarp();
         }
-        uint32_t nf_cur = ts < t_end ? P.tile_out[ts].count : 0;
-        uint32_t nf_next = ts + 1 < t_end ? P.tile_out[ts + 1].count : 0;
-        if (ts < t_end) stage_tile(S.feat[0], P.features + (size_t)ts * 5 * kTileCap, nf_cur, lane);
-        // kCommitRound: the tile's predicate words (its <= 472 ordinals span
-        // at most 16 words), lane q holding word q; the next tile's in flight
-        uint32_t pw_cur = 0, pw_next = 0;
-        if (kMode == kCommitRound) {
-            if (ts < t_end && lane < 16) pw_cur = __ldg(P.index_pred + ((ts * kTileCap) >> 5) + lane);
-            if (ts + 1 < t_end && lane < 16) pw_next = __ldg(P.index_pred + (((ts + 1) * kTileCap) >> 5) + lane);
-        }
-        __syncwarp();
-        long long t_file = clock64(), t_wait = 0;
-        uint32_t n_groups = 0, n_loops = 0;
-        for (uint32_t t = ts; t < t_end; t++) {
-            const uint32_t cur = (t - ts) & 1u;
-            if (kMode == kCommitRound && t > ts && t % kCkptTiles == 0) {
-                // checkpoint of the state entering tile t
-                uint32_t* ck = P.commit_ckpt + (size_t)(t / kCkptTiles) * kCkptWords;
-                for (uint32_t i = lane; i < 64; i += 32) ck[i] = S.F[i];
+        __syncthreads();
+        long long t_file = P.phase ? clock64() : 0, t_wait = 0;
+        uint32_t n_pass = 0, n_ambig = 0;
+        uint32_t cur = 0;            // F[cur] fills
+        bool fresh = ts == t_first;  // F[cur] holds no bit
+        bool flush = false;          // F[cur ^ 1] is complete: filter bf_count - 2 goes out
+        uint32_t pos = 0, avail = 0; // window start, end of the staged features (positions in the file)
+        // segments of tiles: a chunk (the big-filter counter restarts behind
+        // it), in index rounds also cut at checkpoints
+        uint32_t t_seg = ts;
+        while (t_seg < t_end) {
+            if (kRound && t_seg > ts && t_seg % kCkptTiles == 0) {
+                // checkpoint of the state entering tile t_seg
+                uint32_t* ck = P.commit_ckpt + (size_t)(t_seg / kCkptTiles) * kCkptWords;
+                __syncthreads();  // the last pass's bits are applied
+                for (uint32_t i = tid; i < 64; i += kCmThreads) ck[i] = S.F[cur][i];
                 uint4* g4 = reinterpret_cast<uint4*>(ck + 64);
-                for (uint32_t i = lane; i < kBigBytes / 16; i += 32) g4[i] = reinterpret_cast<const uint4*>(S.G)[i];
-                if (lane == 0) {
+                for (uint32_t i = tid; i < kBigBytes / 16; i += kCmThreads) g4[i] = reinterpret_cast<const uint4*>(S.G)[i];
+                if (tid == 0) {
                     ck[64 + 4096] = bf_count;
                     ck[64 + 4096 + 1] = last_count;
                     ck[64 + 4096 + 2] = bigfi;
                 }
             }
-            // chunk boundary: the big-filter counter is local to each chunk
-            // (sdbf_core.cc:100); the big filter itself continues
-            while (t >= next_chunk_tile) {
+            while (t_seg >= next_chunk_tile) {
                 bigfi = 0;
                 chunk++;
-                next_chunk_tile = (chunk + 1 < Fd.first_chunk + Fd.nchunks) ? P.chunks[chunk + 1].first_tile
-                                                                             : 0xFFFFFFFFu;
+                next_chunk_tile = chunk + 1 < chunk_end ? P.chunks[chunk + 1].first_tile : 0xFFFFFFFFu;
             }
-            const long long w0 = clock64();
-            cp_async_wait_all();
-            __syncwarp();
-            t_wait += clock64() - w0;
-            const uint32_t nf = nf_cur;
-            if (t + 1 < t_end)
-                stage_tile(S.feat[cur ^ 1u], P.features + (size_t)(t + 1) * 5 * kTileCap, nf_next, lane);
-            const uint32_t pw = pw_cur;
-            if (kMode == kCommitRound) {
-                pw_cur = pw_next;
-                pw_next = (t + 2 < t_end && lane < 16) ? __ldg(P.index_pred + (((t + 2) * kTileCap) >> 5) + lane) : 0u;
-            }
-            nf_cur = nf_next;
-            nf_next = t + 2 < t_end ? P.tile_out[t + 2].count : 0;
-            for (uint32_t g0 = 0; g0 < nf; g0 += kGroup) {
-                const uint32_t gi = g0 + (kIdx ? 0u : lane);
-                const bool have = gi < nf && (!kIdx || lane == 0);
-                uint32_t a[5], b[5], hw[5];
-#pragma unroll
-                for (int k = 0; k < 5; k++) {
-                    const uint32_t h = have ? S.feat[cur][k][gi] : 0u;
-                    hw[k] = h;
-                    a[k] = h & kBfMask;
-                    b[k] = h & kBigMask;
-                }
-                bool ipred = false;
-                if (kMode == kCommitRound) {
-                    const uint32_t o = t * kTileCap + gi;
-                    const uint32_t w = __shfl_sync(0xffffffffu, pw, ((o >> 5) - ((t * kTileCap) >> 5)) & 31u);
-                    ipred = have && ((w >> (o & 31u)) & 1u);
-                }
-                uint32_t start = 0;
-                n_groups++;
+            uint32_t seg_end = min(next_chunk_tile, t_end);
+            if (kRound) seg_end = min(seg_end, (t_seg / kCkptTiles + 1) * kCkptTiles);
+            // the loading warp and the window's threads run the same number of
+            // passes: both see what was published before barrier (1)
+            if (loader) {
+                // tiles [tn, seg_end) to come, their counts 32 at a time (lane
+                // l: tile cb + l), e0 >= e1 >= e2 the staged ends after this
+                // pass's copies, the last pass's, the one's before
+                uint32_t tn = t_seg, cb = t_seg, cnt = 0, cnt_next = 0, e0 = pos, e1 = pos, e2 = pos, par = 0;
+                if (cb + lane < seg_end) cnt = P.tile_out[cb + lane].count;
+                if (cb + 32 + lane < seg_end) cnt_next = P.tile_out[cb + 32 + lane].count;
                 while (true) {
-                    const bool act = have && lane >= start;
-                    if (!__any_sync(0xffffffffu, act)) break;
-                    n_loops++;
-                    // pass 1: state before the group, publish holders
-                    uint32_t fpre = 0, gpre = 0;
-                    if (act) {
-#pragma unroll
-                        for (int k = 0; k < 5; k++) {
-                            fpre |= ((S.F[a[k] >> 5] >> (a[k] & 31)) & 1u) << k;
-                            gpre |= ((S.G[b[k] >> 5] >> (b[k] & 31)) & 1u) << k;
-                            atomicOr(&S.own[a[k]], 1u << lane);
+                    // stage the next tiles that fit (positions below the last
+                    // window's start are free), then publish the end of what
+                    // has arrived: copies started two passes ago, or all of
+                    // them when the next windows would run short
+                    uint32_t started = 0;
+                    while (tn < seg_end && started < kCmTiles) {
+                        const uint32_t c = min(__shfl_sync(0xffffffffu, cnt, tn - cb), kTileCap);
+                        if (e0 - pos + c > kCmRing) break;
+                        const uint32_t* src = P.features + (size_t)tn * 5 * kTileCap;
+                        for (uint32_t q = lane; q < c; q += 32) {
+                            const uint32_t d = (e0 + q) & (kCmRing - 1);
+                            cp_async16(&S.feat4[d], src + 4 * q);
+                            cp_async4(&S.feat1[d], src + 4 * kTileCap + q);
+                            if (kRound) S.ord[d] = tn * kTileCap + q;
+                        }
+                        e0 += c;
+                        tn++;
+                        started += c != 0;
+                        if (tn - cb == 32) {
+                            cb += 32;
+                            cnt = cnt_next;
+                            cnt_next = cb + 32 + lane < seg_end ? P.tile_out[cb + 32 + lane].count : 0;
                         }
                     }
+                    cp_async_commit();
+                    const long long w0 = P.phase ? clock64() : 0;
+                    const bool all = e2 - pos < 3 * kCmWin;
+                    if (all) cp_async_wait_all();
+                    else cp_async_wait_2();
+                    if (P.phase) t_wait += clock64() - w0;
+                    const uint32_t got = all ? e0 : e2;
+                    e2 = all ? e0 : e1;
+                    e1 = e0;
+                    const bool fin = tn == seg_end && got == e0;
                     __syncwarp();
-                    // pass 2: holders of each index
-                    uint32_t m[5];
-#pragma unroll
-                    for (int k = 0; k < 5; k++) m[k] = act ? S.own[a[k]] : 0u;
-                    __syncwarp();
-                    if (act) {
-#pragma unroll
-                        for (int k = 0; k < 5; k++) S.own[a[k]] = 0;
+                    if (lane == 0) {
+                        S.avail[par] = got;
+                        S.final_[par] = fin;
                     }
-                    // 256-byte filter: new iff unset before the group and this
-                    // lane is the first holder
-                    bool fpass = false;
+                    __syncthreads();  // (1)
+                    pos = S.pos[par];
+                    par ^= 1u;
+                    if (fin) break;
+                }
+            }
+            // window's threads: after a pass whose barrier (1) carried
+            // final_, the rest of the segment runs without the loading warp
+            bool final_ = false;
+            uint32_t par = 0;
+            while (!loader && (!final_ || pos != avail)) {
+                if (epoch == 0) {  // once in 2^24 passes
+                    commit_sync();
+                    for (uint32_t i = tid; i < 4096; i += kCmWin) S.tab[i] = 0xFFFFFFFFu;
+                    epoch = 0xFFFFFFu;
+                    commit_sync();
+                }
+                epoch--;
+                n_pass++;
+                const uint32_t W = min((uint32_t)kCmWin, avail - pos);
+                const bool have = tid < W;
+                const uint32_t key = (epoch << 8) | tid;
+                const uint32_t slot = (pos + tid) & (kCmRing - 1);
+                uint32_t h[5] = {0, 0, 0, 0, 0};
+                uint32_t ord = 0;
+                bool ipred = true;
+                if (have) {
+                    const uint4 v = S.feat4[slot];
+                    h[0] = v.x;
+                    h[1] = v.y;
+                    h[2] = v.z;
+                    h[3] = v.w;
+                    h[4] = S.feat1[slot];
 #pragma unroll
-                    for (int k = 0; k < 5; k++)
-                        if (act && !((fpre >> k) & 1u) && (uint32_t)(__ffs(m[k]) - 1) == lane) fpass = true;
-                    const uint32_t fmask = __ballot_sync(0xffffffffu, fpass);
-                    // index: insert_sha1 of the filter-passing feature; it goes
-                    // on only if that set a new index bit
-                    bool inew = true;
-                    if (kMode == kCommitRound) inew = fpass && ipred;
-                    if (kIdx) {
-                        inew = false;
-                        if (fpass) {
-#pragma unroll
-                            for (int k = 0; k < 5; k++) {
-                                const uint32_t pos = hw[k] & P.index_mask, bit = 1u << (pos & 31);
-                                if (!(atomicOr(P.index_bits + (pos >> 5), bit) & bit)) inew = true;
-                            }
-                            if (inew) atomicAdd(P.index_new, 1ull);
-                        }
+                    for (int k = 0; k < 5; k++) atomicMin(&S.tab[h[k] & 0xFFFu], key);
+                    if (kRound) {
+                        ord = S.ord[slot];
+                        ipred = (__ldg(P.index_pred + (ord >> 5)) >> (ord & 31u)) & 1u;
                     }
-                    // big filter: new iff unset before the group and no earlier
-                    // filter-passing lane holds the same 17-bit value
-                    uint32_t gnew = 0, pend = 0;
-                    uint32_t cand[5];
-                    const uint32_t imask = kMode == kCommitRound ? __ballot_sync(0xffffffffu, fpass && inew) : fmask;
+                }
+                if (tid == 0) S.pos[par] = pos;
+                uint32_t avail_next = avail;
+                if (final_) {
+                    commit_sync();  // (1)
+                } else {
+                    __syncthreads();  // (1)
+                    avail_next = S.avail[par];
+                    final_ = S.final_[par] != 0;
+                    par ^= 1u;
+                }
+                if (flush) {
+                    if (tid < 64) {
+                        if (bf_count - 1 <= Fd.filter_cap) out[(size_t)(bf_count - 2) * 64 + tid] = S.F[cur ^ 1u][tid];
+                        else if (tid == 0) atomicAdd(P.counters + 1, 1u);
+                        S.F[cur ^ 1u][tid] = 0;
+                    }
+                    flush = false;
+                }
+                bool fnew = false, gate = false, cnt_def = false, amb = false;
+                uint32_t gun = 0;  // big-filter bits unset before the window
+                if (have) {
+                    bool gnew = false;
 #pragma unroll
                     for (int k = 0; k < 5; k++) {
-                        cand[k] = m[k] & imask & lanemask_lt();
-                        if (fpass && inew && !((gpre >> k) & 1u)) {
-                            if (cand[k]) pend |= 1u << k;
-                            else gnew |= 1u << k;
-                        }
+                        const uint32_t i12 = h[k] & 0xFFFu, a = h[k] & kBfMask, b = h[k] & kBigMask;
+                        const uint32_t t0 = S.tab[i12], t1 = S.tab[i12 ^ 0x800u];
+                        const uint32_t fw = fresh ? 0u : S.F[cur][a >> 5] >> (a & 31), gw = S.G[b >> 5] >> (b & 31);
+                        fnew |= t0 == key && t1 >= key && !(fw & 1u);
+                        gnew |= t0 == key && !(gw & 1u);
+                        gun |= (~gw & 1u) << k;
                     }
-                    while (__any_sync(0xffffffffu, pend != 0)) {
-                        // each pending lane checks one candidate lane per pass
-                        int kk = pend ? __ffs(pend) - 1 : 0;
-                        uint32_t ck = 0, vk = 0;
-#pragma unroll
-                        for (int k = 0; k < 5; k++)
-                            if (k == kk) {
-                                ck = cand[k];
-                                vk = b[k];
-                            }
-                        const uint32_t j = pend ? (uint32_t)(__ffs(ck) - 1) : lane;
-                        bool same = false;
-#pragma unroll
-                        for (int q = 0; q < 5; q++) same |= (__shfl_sync(0xffffffffu, b[q], j) == vk);
-                        if (pend) {
-                            ck &= ck - 1u;
-#pragma unroll
-                            for (int k = 0; k < 5; k++)
-                                if (k == kk) cand[k] = ck;
-                            if (same) pend &= ~(1u << kk);
-                            else if (ck == 0) {
-                                pend &= ~(1u << kk);
-                                gnew |= 1u << kk;
-                            }
-                        }
-                    }
-                    const bool counted = fpass && inew && gnew != 0;
-                    const uint32_t cm = __ballot_sync(0xffffffffu, counted);
-                    const uint32_t before = __popc(cm & lanemask_le());
-                    const bool hit_small = counted && (last_count + before == (uint32_t)kMaxElem);
-                    const bool hit_big = counted && (bigfi + before == (uint32_t)kBigElem);
-                    const uint32_t hm = __ballot_sync(0xffffffffu, hit_small || hit_big);
-                    const uint32_t r = hm ? (uint32_t)(__ffs(hm) - 1) : 31u;
-                    if (kMode == kCommitRound) {
-                        // the inserted features of this pass: filter-passing lanes up to r
-                        const uint32_t sm = __ballot_sync(0xffffffffu, act && lane <= r && fpass);
-                        if (lane == 0 && sm) {
-                            const uint32_t base = t * kTileCap + g0, sh = base & 31u;
-                            atomicOr(P.index_seen + (base >> 5), sm << sh);
-                            if (sh && (sm >> (32u - sh))) atomicOr(P.index_seen + (base >> 5) + 1, sm >> (32u - sh));
-                        }
-                    }
-                    // write the bits of lanes up to r (all of them without a roll-over)
-                    if (act && lane <= r) {
-#pragma unroll
-                        for (int k = 0; k < 5; k++) {
-                            atomicOr(&S.F[a[k] >> 5], 1u << (a[k] & 31));
-                            if (fpass && inew) atomicOr(&S.G[b[k] >> 5], 1u << (b[k] & 31));
-                        }
-                    }
-                    __syncwarp();
-                    if (!hm) {
-                        last_count += __popc(cm);
-                        bigfi += __popc(cm);
-                        break;
-                    }
-                    const bool roll_small = __shfl_sync(0xffffffffu, hit_small, r);
-                    const bool roll_big = __shfl_sync(0xffffffffu, hit_big, r);
-                    const uint32_t ncnt = __popc(cm & ((2u << r) - 1u));
-                    last_count += ncnt;
-                    bigfi += ncnt;
-                    if (roll_small) {
-                        const bool fits = bf_count <= Fd.filter_cap;
-                        for (uint32_t i = lane; i < 64; i += 32) {
-                            if (fits) out[(size_t)(bf_count - 1) * 64 + i] = S.F[i];
-                            S.F[i] = 0;
-                        }
-                        if (!fits && lane == 0) atomicAdd(P.counters + 1, 1u);
-                        bf_count++;
-                        last_count = 0;
-                    }
-                    if (roll_big) {
-                        for (uint32_t i = lane; i < kBigBytes / 4; i += 32) S.G[i] = 0;
-                        bigfi = 0;
-                    }
-                    __syncwarp();
-                    start = r + 1;
+                    gate = fnew && ipred;
+                    cnt_def = gate && gnew;
+                    amb = gate && !gnew && gun;
                 }
+                {
+                    const uint32_t mc = __ballot_sync(0xffffffffu, cnt_def), ma = __ballot_sync(0xffffffffu, amb);
+                    if (lane == 0) {
+                        S.counted[wid] = mc;
+                        S.ambig[wid] = ma;
+                    }
+                }
+                commit_sync();  // (2)
+                uint32_t m[kCmWarps], am_[kCmWarps];
+                auto read_flags = [&](const uint32_t* src, uint32_t (&v)[kCmWarps]) {
+                    const uint4 x = *reinterpret_cast<const uint4*>(src);
+                    const uint2 y = *reinterpret_cast<const uint2*>(src + 4);
+                    v[0] = x.x;
+                    v[1] = x.y;
+                    v[2] = x.z;
+                    v[3] = x.w;
+                    v[4] = y.x;
+                    v[5] = y.y;
+                };
+                read_flags(S.counted, m);
+                read_flags(S.ambig, am_);
+                if (am_[0] | am_[1] | am_[2] | am_[3] | am_[4] | am_[5]) {
+                    // an ambiguous feature's value k is held by an earlier
+                    // F-passing feature of the window?
+#pragma unroll
+                    for (uint32_t w = 0; w < kCmWarps; w++) {
+                        for (uint32_t am = am_[w]; am; am &= am - 1u) {
+                            const uint32_t j = 32 * w + (uint32_t)(__ffs(am) - 1);
+                            n_ambig++;
+                            if (wid > w) continue;  // later features only
+                            uint32_t mm = 0;
+                            if (gate && tid < j) {
+                                const uint32_t js = (pos + j) & (kCmRing - 1);
+                                const uint4 v4 = S.feat4[js];
+                                const uint32_t v[5] = {v4.x, v4.y, v4.z, v4.w, S.feat1[js]};
+#pragma unroll
+                                for (int k = 0; k < 5; k++)
+#pragma unroll
+                                    for (int q = 0; q < 5; q++) mm |= (uint32_t)(((h[q] ^ v[k]) & kBigMask) == 0) << k;
+                            }
+                            mm = __reduce_or_sync(0xffffffffu, mm);
+                            if (lane == 0 && mm) atomicOr(&S.match[j], mm);
+                        }
+                    }
+                    commit_sync();
+                    if (amb) {
+                        cnt_def = (gun & ~S.match[tid]) != 0;
+                        S.match[tid] = 0;
+                    }
+                    const uint32_t mc = __ballot_sync(0xffffffffu, cnt_def);
+                    if (lane == 0) S.counted[wid] = mc;
+                    commit_sync();
+                    read_flags(S.counted, m);
+                }
+                // counted features before this one and in all
+                uint32_t before = 0, total = 0;
+#pragma unroll
+                for (uint32_t w = 0; w < kCmWarps; w++) {
+                    const uint32_t c = __popc(m[w]);
+                    before += w < wid ? c : w == wid ? __popc(m[w] & lanemask_lt()) : 0u;
+                    total += c;
+                }
+                const uint32_t need_s = (uint32_t)kMaxElem - last_count, need_b = (uint32_t)kBigElem - bigfi;
+                const uint32_t need = min(need_s, need_b);
+                const bool roll = total >= need;  // the need-th counted feature ends the pass
+                if (roll && cnt_def && before + 1 == need) S.end = tid + 1;
+                commit_sync();  // (3)
+                const uint32_t n = roll ? S.end : W;
+                const bool roll_small = roll && need == need_s, roll_big = roll && need == need_b;
+                if (have && before < need) {
+#pragma unroll
+                    for (int k = 0; k < 5; k++) {
+                        const uint32_t a = h[k] & kBfMask, b = h[k] & kBigMask;
+                        atomicOr(&S.F[cur][a >> 5], 1u << (a & 31));
+                        if (gate && !roll_big) atomicOr(&S.G[b >> 5], 1u << (b & 31));
+                    }
+                    // the inserted features of this pass
+                    if (kRound && fnew) atomicOr(P.index_seen + (ord >> 5), 1u << (ord & 31u));
+                }
+                if (roll_big)
+                    for (uint32_t i = tid; i < kBigBytes / 16; i += kCmWin)
+                        reinterpret_cast<uint4*>(S.G)[i] = make_uint4(0, 0, 0, 0);
+                fresh = roll_small || (fresh && n == 0);
+                last_count += min(total, need);
+                bigfi += min(total, need);
+                if (roll_small) {
+                    bf_count++;
+                    last_count = 0;
+                    cur ^= 1u;
+                    flush = true;
+                }
+                if (roll_big) bigfi = 0;
+                pos += n;
+                avail = avail_next;
             }
+            if (tid == 0) S.seg_pos = pos;
+            __syncthreads();  // the segment's last bits are applied
+            pos = avail = S.seg_pos;
+            t_seg = seg_end;
         }
-        cp_async_wait_all();
-        __syncwarp();
-        // emit the current (last) filter, then the chop of sdbf_core.cc:235-238
+        __syncthreads();
+        if (flush && tid < 64) {
+            if (bf_count - 1 <= Fd.filter_cap) out[(size_t)(bf_count - 2) * 64 + tid] = S.F[cur ^ 1u][tid];
+            else if (tid == 0) atomicAdd(P.counters + 1, 1u);
+        }
+        // emit the current (last) filter
         if (bf_count <= Fd.filter_cap) {
-            for (uint32_t i = lane; i < 64; i += 32) out[(size_t)(bf_count - 1) * 64 + i] = S.F[i];
-        } else if (lane == 0) {
+            if (tid < 64) out[(size_t)(bf_count - 1) * 64 + tid] = S.F[cur][tid];
+        } else if (tid == 0) {
             atomicAdd(P.counters + 1, 1u);
         }
-        if (bf_count > 1 && last_count < (uint32_t)kMaxElem / 8) {
-            bf_count--;
-            last_count = kMaxElem;
-        }
-        if (lane == 0) {
-            P.out_info[file].bf_count = bf_count;
-            P.out_info[file].last_count = last_count;
+        if (tid == 0) {
+            commit_result(P, file, bf_count, last_count);
             if (P.phase) {
                 const long long busy = clock64() - t_file;
-                atomicAdd(P.phase + kPhCommitWait, (unsigned long long)t_wait);
                 atomicAdd(P.phase + kPhCommitBusy, (unsigned long long)busy);
-                atomicAdd(P.phase + kPhCommitGroups, (unsigned long long)n_groups);
-                atomicAdd(P.phase + kPhCommitLoops, (unsigned long long)n_loops);
+                atomicAdd(P.phase + kPhCommitGroups, (unsigned long long)n_pass);
+                atomicAdd(P.phase + kPhCommitLoops, (unsigned long long)n_ambig);
                 atomicMax(P.phase + kPhCommitMaxFile, (unsigned long long)busy);
             }
         }
-        __syncwarp();
+        if (P.phase && loader && lane == 0) atomicAdd(P.phase + kPhCommitWait, (unsigned long long)t_wait);
     }
 }
 
-__global__ void __launch_bounds__(kCommitWarps * 32) k_stream_commit(GenParams P) {
+__global__ void __launch_bounds__(kCmThreads) k_stream_commit(GenParams P) {
     extern __shared__ __align__(16) uint8_t smem[];
-    commit_files<kCommitPlain>(P, smem);
+    commit_files<false>(P, smem);
 }
 
-__global__ void __launch_bounds__(kCommitWarps * 32) k_stream_commit_index(GenParams P) {
+__global__ void __launch_bounds__(kCmThreads) k_stream_commit_round(GenParams P) {
     extern __shared__ __align__(16) uint8_t smem[];
-    commit_files<kCommitSeq>(P, smem);
+    commit_files<true>(P, smem);
 }
 
-__global__ void __launch_bounds__(kCommitWarps * 32) k_stream_commit_round(GenParams P) {
-    extern __shared__ __align__(16) uint8_t smem[];
-    commit_files<kCommitRound>(P, smem);
+// The sequential commit of an index build: one warp, files in input order,
+// one feature at a time, lane k (< 5) holding its k-th hash word.  Setting a
+// bit and learning whether it was new is one atomic each on the filter, the
+// index and the big filter.
+__global__ void __launch_bounds__(32) k_stream_commit_index(GenParams P) {
+    __shared__ uint32_t F[64], G[kBigBytes / 4];
+    __shared__ __align__(16) uint32_t feat[2][5 * kTileCap];  // double-buffered features of a tile
+    const uint32_t lane = threadIdx.x;
+    const uint32_t k = min(lane, 4u);
+    auto stage = [&](uint32_t buf, uint32_t t, uint32_t nf) {
+        const uint32_t* src = P.features + (size_t)t * 5 * kTileCap;
+        for (uint32_t q = lane; q < nf; q += 32) cp_async16(&feat[buf][4 * q], src + 4 * q);
+        for (uint32_t q = lane; q < (nf + 3) / 4; q += 32)
+            cp_async16(&feat[buf][4 * (kTileCap + q)], src + 4 * (kTileCap + q));
+        cp_async_commit();
+    };
+    for (uint32_t fi = 0; fi < P.nfiles; fi++) {
+        const uint32_t file = P.file_order[fi];
+        const GenFile Fd = P.files[file];
+        if (Fd.nchunks == 0) continue;
+        uint32_t* out = P.out_filters + (size_t)Fd.filter_base * 64;
+        for (uint32_t i = lane; i < 64; i += 32) F[i] = 0;
+        for (uint32_t i = lane; i < kBigBytes / 4; i += 32) G[i] = 0;
+        __syncwarp();
+        uint32_t bf_count = 1, last_count = 0;
+        auto emit = [&]() {
+            __syncwarp();
+            const bool fits = bf_count <= Fd.filter_cap;
+            for (uint32_t i = lane; i < 64; i += 32) {
+                if (fits) out[(size_t)(bf_count - 1) * 64 + i] = F[i];
+                F[i] = 0;
+            }
+            if (!fits && lane == 0) atomicAdd(P.counters + 1, 1u);
+            __syncwarp();
+        };
+        for (uint32_t c = Fd.first_chunk; c < Fd.first_chunk + Fd.nchunks; c++) {
+            const uint32_t ta = P.chunks[c].first_tile, tb = ta + P.chunks[c].ntiles;
+            uint32_t bigfi = 0;  // local to the chunk
+            uint32_t nf = ta < tb ? P.tile_out[ta].count : 0;
+            if (ta < tb) stage(0, ta, nf);
+            for (uint32_t t = ta; t < tb; t++) {
+                const uint32_t cur = (t - ta) & 1u;
+                cp_async_wait_all();
+                __syncwarp();
+                const uint32_t nf_next = t + 1 < tb ? P.tile_out[t + 1].count : 0;
+                if (t + 1 < tb) stage(cur ^ 1u, t + 1, nf_next);
+                for (uint32_t g = 0; g < nf; g++) {
+                    const uint32_t h = feat[cur][feat_word(g, k)];
+                    const uint32_t a = h & kBfMask, b = h & kBigMask, pos = h & P.index_mask;
+                    bool nw = false;
+                    if (lane < 5) nw = !((atomicOr(&F[a >> 5], 1u << (a & 31)) >> (a & 31)) & 1u);
+                    if (!__any_sync(0xffffffffu, nw)) continue;
+                    nw = false;
+                    if (lane < 5) nw = !((atomicOr(P.index_bits + (pos >> 5), 1u << (pos & 31)) >> (pos & 31)) & 1u);
+                    if (!__any_sync(0xffffffffu, nw)) continue;
+                    if (lane == 0) atomicAdd(P.index_new, 1ull);
+                    nw = false;
+                    if (lane < 5) nw = !((atomicOr(&G[b >> 5], 1u << (b & 31)) >> (b & 31)) & 1u);
+                    if (!__any_sync(0xffffffffu, nw)) continue;
+                    last_count++;
+                    bigfi++;
+                    if (last_count == (uint32_t)kMaxElem) {
+                        emit();
+                        bf_count++;
+                        last_count = 0;
+                    }
+                    if (bigfi == (uint32_t)kBigElem) {
+                        __syncwarp();
+                        for (uint32_t i = lane; i < kBigBytes / 4; i += 32) G[i] = 0;
+                        __syncwarp();
+                        bigfi = 0;
+                    }
+                }
+                nf = nf_next;
+            }
+        }
+        emit();
+        if (lane == 0) commit_result(P, file, bf_count, last_count);
+        __syncwarp();
+    }
 }
 
 // Features of a stream launch recorded in a seen bitmap (ordinal = tile *
@@ -1485,9 +1653,9 @@ __global__ void k_stream_index_pred(const uint32_t* __restrict__ feats, const Ti
         if (i < n) {
             const uint32_t t = (uint32_t)(i / kTileCap), g = (uint32_t)(i - (uint64_t)t * kTileCap);
             if (g < tile_out[t].count) {
-                const uint32_t* w = feats + (size_t)t * 5 * kTileCap + g;
+                const uint32_t* w = feats + (size_t)t * 5 * kTileCap;
 #pragma unroll
-                for (int k = 0; k < 5; k++) p |= __ldg(first + (w[(size_t)k * kTileCap] & mask)) >= (uint32_t)i + 1u;
+                for (int k = 0; k < 5; k++) p |= __ldg(first + (w[feat_word(g, k)] & mask)) >= (uint32_t)i + 1u;
             }
         }
         const uint32_t word = __ballot_sync(0xffffffffu, p);
@@ -1503,9 +1671,9 @@ __global__ void k_stream_index_first(const uint32_t* __restrict__ feats, const T
         if (!((seen[i >> 5] >> (i & 31)) & 1u)) continue;
         const uint32_t t = (uint32_t)(i / kTileCap), g = (uint32_t)(i - (uint64_t)t * kTileCap);
         if (g >= tile_out[t].count) continue;
-        const uint32_t* w = feats + (size_t)t * 5 * kTileCap + g;
+        const uint32_t* w = feats + (size_t)t * 5 * kTileCap;
 #pragma unroll
-        for (int k = 0; k < 5; k++) atomicMin(first + (w[(size_t)k * kTileCap] & mask), (uint32_t)i + 1u);
+        for (int k = 0; k < 5; k++) atomicMin(first + (w[feat_word(g, k)] & mask), (uint32_t)i + 1u);
     }
 }
 
@@ -1519,11 +1687,11 @@ __global__ void k_stream_index_mark(const uint32_t* __restrict__ feats, const Ti
         if (!((seen[i >> 5] >> (i & 31)) & 1u)) continue;
         const uint32_t t = (uint32_t)(i / kTileCap), g = (uint32_t)(i - (uint64_t)t * kTileCap);
         if (g >= tile_out[t].count) continue;
-        const uint32_t* w = feats + (size_t)t * 5 * kTileCap + g;
+        const uint32_t* w = feats + (size_t)t * 5 * kTileCap;
         bool fresh = false;
 #pragma unroll
         for (int k = 0; k < 5; k++) {
-            const uint32_t pos = w[(size_t)k * kTileCap] & mask;
+            const uint32_t pos = w[feat_word(g, k)] & mask;
             fresh |= first[pos] == (uint32_t)i + 1u;
             atomicOr(bits + (pos >> 5), 1u << (pos & 31));
         }
@@ -1753,14 +1921,15 @@ static void set_stream_attrs() {
     cudaFuncSetAttribute(k_stream_fix_list<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
     cudaFuncSetAttribute(k_stream_fix_list<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smp);
     cudaFuncSetAttribute(k_stream_ranks, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRkSmem);
-    cudaFuncSetAttribute(k_stream_commit, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)(sizeof(CommitSmem) * kCommitWarps));
+    cudaFuncSetAttribute(k_stream_commit, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(CommitSmem<false>));
+    cudaFuncSetAttribute(k_stream_commit_round, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)sizeof(CommitSmem<true>));
     // one shared-memory / L1 split for every kernel of the stream pipeline
     // (the largest shared memory): CTAs of different kernels can then share
     // an SM
     for (const void* f : {(const void*)k_stream_ranks, (const void*)k_stream_tiles, (const void*)k_stream_tiles_pre,
                           (const void*)k_stream_fails, (const void*)k_stream_fix_list<false>,
-                          (const void*)k_stream_fix_list<true>, (const void*)k_stream_check,
+                          (const void*)k_stream_fix_list<true>,
                           (const void*)k_stream_fix<false>, (const void*)k_stream_fix<true>,
                           (const void*)k_stream_commit, (const void*)k_stream_commit_round,
                           (const void*)k_stream_commit_index})
@@ -1797,11 +1966,6 @@ cudaError_t launch_stream_fix_list(const GenParams& P, uint32_t grid, cudaStream
     return cudaGetLastError();
 }
 
-cudaError_t launch_stream_check(const GenParams& P, uint32_t grid, cudaStream_t st) {
-    k_stream_check<<<grid, 128, 0, st>>>(P);
-    return cudaGetLastError();
-}
-
 cudaError_t launch_stream_fix(const GenParams& P, uint32_t grid, cudaStream_t st) {
     set_stream_attrs();
     if (P.ranks)
@@ -1812,16 +1976,13 @@ cudaError_t launch_stream_fix(const GenParams& P, uint32_t grid, cudaStream_t st
 }
 
 cudaError_t launch_stream_commit_index(const GenParams& P, cudaStream_t st) {
-    cudaFuncSetAttribute(k_stream_commit_index, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)(sizeof(CommitSmem) * kCommitWarps));
-    k_stream_commit_index<<<1, kCommitWarps * 32, sizeof(CommitSmem) * kCommitWarps, st>>>(P);
+    k_stream_commit_index<<<1, 32, 0, st>>>(P);
     return cudaGetLastError();
 }
 
 cudaError_t launch_stream_commit_round(const GenParams& P, uint32_t grid, cudaStream_t st) {
-    cudaFuncSetAttribute(k_stream_commit_round, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)(sizeof(CommitSmem) * kCommitWarps));
-    k_stream_commit_round<<<grid, kCommitWarps * 32, sizeof(CommitSmem) * kCommitWarps, st>>>(P);
+    set_stream_attrs();
+    k_stream_commit_round<<<grid, kCmThreads, sizeof(CommitSmem<true>), st>>>(P);
     return cudaGetLastError();
 }
 
@@ -1852,7 +2013,7 @@ cudaError_t launch_pred_dirty(const GenParams& P, const uint32_t* a, const uint3
 
 cudaError_t launch_stream_commit(const GenParams& P, uint32_t grid, cudaStream_t st) {
     set_stream_attrs();
-    k_stream_commit<<<grid, kCommitWarps * 32, sizeof(CommitSmem) * kCommitWarps, st>>>(P);
+    k_stream_commit<<<grid, kCmThreads, sizeof(CommitSmem<false>), st>>>(P);
     return cudaGetLastError();
 }
 

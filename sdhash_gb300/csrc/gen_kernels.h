@@ -22,8 +22,8 @@ constexpr uint32_t kTileL = 7936;
 // at most one selected feature per 17 credited steps (score > 16), and a
 // tile's positions are credited by kTileL + 64 steps
 constexpr uint32_t kTileCap = ((kTileL + 64) / 17 + 2 + 3) / 4 * 4;  // rows 16-byte aligned
-constexpr int kCommitWarps = 1;      // files per commit CTA (one: its 44 KB of shared memory then
-                                     // displaces a single tile CTA on its SM)
+constexpr uint32_t kCmWin = 192;     // stream commit: features per pass (a filter takes ~163)
+constexpr int kCmThreads = kCmWin + 32;  // one thread per feature and a loading warp
 constexpr uint32_t kMaxBlockBytes = 16384;  // dd block size limit (sdhash.cc:215-219)
 constexpr uint64_t kChunkBytes = 32ull << 20;  // stream chunk (sdbf_class.cc:43)
 
@@ -82,7 +82,7 @@ struct GenParams {
     const uint32_t* file_order;  // commit order (largest first)
     uint32_t nfiles;
     TileOut* tile_out;
-    uint32_t* features;          // [tile][5][kTileCap]
+    uint32_t* features;          // [tile][5 * kTileCap]: kTileCap uint4 (hash words 0..3), then the fifth words
     uint32_t* out_filters;       // 64 words per filter
     uint16_t* out_counts;        // block mode: elements per filter
     FileInfoDev* out_info;       // stream mode: per file
@@ -92,7 +92,6 @@ struct GenParams {
     uint32_t block_lmax;         // block mode: max window steps per block
     uint32_t lead;               // speculative lead-in steps (<= kLead)
     unsigned long long* phase;   // optional phase cycle counters (kPhase*), null = off
-    uint32_t* chunk_redo;        // per chunk: first tile whose link failed (stream)
     uint32_t* fix_list;          // stream: [0] = n, then the n tiles whose link failed
     // block mode with index search: SHA-1 words of every fourth counted
     // feature of each block ([slot][kProbeWords]) and their number per slot;
@@ -150,10 +149,9 @@ cudaError_t launch_stream_ranks(const GenParams& P, uint32_t grid, cudaStream_t 
 // feature bytes from the input in global memory), else they compute ranks.
 cudaError_t launch_stream_tiles(const GenParams& P, uint32_t grid, cudaStream_t st);
 // Tiles whose link fails into P.fix_list (zeroed count first), then all of
-// them recomputed in parallel; k_stream_check / k_stream_fix finish the job.
+// them recomputed in parallel; k_stream_fix finishes the job.
 cudaError_t launch_stream_fails(const GenParams& P, uint32_t grid, cudaStream_t st);
 cudaError_t launch_stream_fix_list(const GenParams& P, uint32_t grid, cudaStream_t st);
-cudaError_t launch_stream_check(const GenParams& P, uint32_t grid, cudaStream_t st);  // 4 chunks per CTA
 cudaError_t launch_stream_fix(const GenParams& P, uint32_t grid, cudaStream_t st);
 cudaError_t launch_stream_commit(const GenParams& P, uint32_t grid, cudaStream_t st);
 // One warp, files in file_order, index inserts (GenParams::index_bits).

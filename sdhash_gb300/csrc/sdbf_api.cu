@@ -68,7 +68,7 @@ extern "C" void sdbfg_ctx_destroy(sdbfg_ctx* c) {
         b->release();
     for (auto& S : c->slot) {
         for (DevBuf* b : {&S.data, &S.chunks, &S.tiles, &S.files, &S.order, &S.tile_out, &S.features, &S.work,
-                          &S.redo, &S.rk_items, &S.fix_list})
+                          &S.rk_items, &S.fix_list})
             b->release();
         S.h_tables.release();
         if (S.stream) cudaStreamDestroy(S.stream);
@@ -456,7 +456,7 @@ static int commit_with_index(sdbfg_ctx* c, GenParams P, uint32_t cap_grid, cudaS
         uint32_t* pred[2] = {c->d_pred.as<uint32_t>(), c->d_seen[1].as<uint32_t>()};
         unsigned int* ndirty = c->d_diff.as<unsigned int>();
         uint8_t* dirty = c->d_diff.as<uint8_t>() + 8;
-        const uint32_t commit_grid = std::min<uint32_t>((P.nfiles + kCommitWarps - 1) / kCommitWarps, cap_grid);
+        const uint32_t commit_grid = std::min<uint32_t>(P.nfiles, cap_grid);
         const uint32_t fgrid = (uint32_t)std::min<uint64_t>((nfeat + 255) / 256, (uint64_t)c->sms * 32);
         const uint64_t pwords = (nfeat + 31) / 32;
         const uint32_t wgrid = (uint32_t)std::min<uint64_t>((pwords + 255) / 256, (uint64_t)c->sms * 8);
@@ -748,7 +748,6 @@ static int digest_stream_pipelined(sdbfg_ctx* c, const uint8_t* host_data, const
         CUDA_TRY(c, S.tile_out.ensure(std::max<uint64_t>(1, ntiles) * sizeof(TileOut)));
         CUDA_TRY(c, S.features.ensure(std::max<uint64_t>(1, ntiles) * 5ull * kTileCap * 4));
         CUDA_TRY(c, S.work.ensure(std::max<uint64_t>(1, work) * 256));
-        CUDA_TRY(c, S.redo.ensure(std::max<uint64_t>(1, nchunks) * 4));
         CUDA_TRY(c, S.fix_list.ensure((ntiles + 1) * 4));
         if (tb_chunks) CUDA_TRY(c, cudaMemcpyAsync(S.chunks.p, hc, tb_chunks, cudaMemcpyHostToDevice, st));
         if (tb_tiles) CUDA_TRY(c, cudaMemcpyAsync(S.tiles.p, ht, tb_tiles, cudaMemcpyHostToDevice, st));
@@ -773,7 +772,6 @@ static int digest_stream_pipelined(sdbfg_ctx* c, const uint8_t* host_data, const
         P.features = S.features.as<uint32_t>();
         P.out_filters = S.work.as<uint32_t>();
         P.out_info = c->d_binfo.as<FileInfoDev>() + g.first;
-        P.chunk_redo = S.redo.as<uint32_t>();
         P.fix_list = S.fix_list.as<uint32_t>();
         if (pre) {
             P.ranks = c->d_ranks.as<uint16_t>() + (gi & 1) * (rank_half / 2);
@@ -801,7 +799,6 @@ static int digest_stream_pipelined(sdbfg_ctx* c, const uint8_t* host_data, const
                 TIMED_LAUNCH_ON(c, "k_stream_fix_list", st,
                                 launch_stream_fix_list(P, std::min<uint32_t>(P.ntiles, (uint32_t)c->sms * 5), st));
             }
-            TIMED_LAUNCH_ON(c, "k_stream_check", st, launch_stream_check(P, (P.nchunks + 3) / 4, st));
             TIMED_LAUNCH_ON(c, "k_stream_fix", st,
                             launch_stream_fix(P, std::min<uint32_t>(P.nchunks, cap_grid), st));
         }
@@ -816,8 +813,7 @@ static int digest_stream_pipelined(sdbfg_ctx* c, const uint8_t* host_data, const
             if (rc) return rc;
         } else {
             TIMED_LAUNCH_ON(c, "k_stream_commit", st,
-                            launch_stream_commit(P, std::min<uint32_t>((g.count + kCommitWarps - 1) / kCommitWarps,
-                                                                       cap_grid), st));
+                            launch_stream_commit(P, std::min<uint32_t>(g.count, cap_grid), st));
         }
         // output slots follow input order: scan after the previous group's scan
         CUDA_TRY(c, cudaStreamWaitEvent(st, prev_scan, 0));
