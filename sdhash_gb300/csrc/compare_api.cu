@@ -33,7 +33,7 @@ extern "C" int sdbfg_set_upload(sdbfg_ctx* c, const sdbfg_digest_desc* ds, uint3
             delete s;
             return fail(c, SDBFG_ERR_ARG, "digest %u has no filters", i);
         }
-        dig[i] = {(uint32_t)total, ds[i].bf_count};
+        dig[i] = {(uint32_t)total, ds[i].bf_count, 0, 0, 0};
         total += ds[i].bf_count;
     }
     if (total >= (1ull << 32)) {
@@ -75,6 +75,7 @@ extern "C" int sdbfg_set_upload(sdbfg_ctx* c, const sdbfg_digest_desc* ds, uint3
             meta[dig[i].first + f] = (h << 16) | (e & 0xFFFFu);
             if (f + 1 == d.bf_count) s->last_elem[i] = e;
         }
+        digest_stats(dig[i], meta.data());
     }
     if (s->d_filters.ensure(std::max<uint64_t>(1, total) * 256) || s->d_meta.ensure(std::max<uint64_t>(1, total) * 4) ||
         s->d_digests.ensure(std::max<uint32_t>(1, n) * sizeof(CmpDigest))) {
@@ -204,6 +205,7 @@ static int upload_plan(sdbfg_ctx* c, MatPlan* p, UnitBuilder& ub, const std::vec
     const std::vector<MatUnit> units = ub.sorted_units();
     p->nunits = (uint32_t)units.size();
     p->nsplit = (uint32_t)ub.split.size();
+    p->nslots = ub.slots;
     p->filter_pairs = ub.filter_pairs;
     CUDA_TRY(c, p->d_units.ensure(std::max<size_t>(1, units.size()) * sizeof(MatUnit)));
     CUDA_TRY(c, p->d_targets.ensure(std::max<size_t>(1, targets.size()) * 4));
@@ -213,6 +215,7 @@ static int upload_plan(sdbfg_ctx* c, MatPlan* p, UnitBuilder& ub, const std::vec
         CUDA_TRY(c, cudaMemcpyAsync(p->d_refs.p, ub.refs.data(), ub.refs.size() * 4, cudaMemcpyHostToDevice,
                                     c->stream));
     CUDA_TRY(c, p->d_slots.ensure(std::max<uint64_t>(1, ub.slots) * 8));
+    CUDA_TRY(c, p->d_redo.ensure(kRedoBytes));
     CUDA_TRY(c, p->d_counter.ensure(64));
     cudaStream_t st = c->stream;
     if (!units.empty())
@@ -238,14 +241,21 @@ static int build_plan_all(sdbfg_ctx* c, const sdbfg_set* s, MatPlan* p) {
     std::stable_sort(sorted.begin(), sorted.end(),
                      [&](uint32_t x, uint32_t y) { return s->bf_count[x] < s->bf_count[y]; });
     std::vector<uint32_t> targets(sorted);
-    uint64_t sum = 0, sum2 = 0;
-    for (uint32_t i = 0; i < n; i++) {
-        sum += s->bf_count[i];
-        sum2 += (uint64_t)s->bf_count[i] * s->bf_count[i];
-    }
+    // the job's work: every class of equal counts (its rows packed) against
+    // the rest of the sorted order
     const uint64_t ctas = (uint64_t)c->sms * matrix_ctas_per_sm(c->mat_variant);
-    UnitBuilder ub(effective_unit_budget(c->mat_unit_work, (sum * sum - sum2) / 2, ctas),
-                   (uint32_t)kMatVariantTable[c->mat_variant].rows);
+    const uint64_t pad = c->mat_variant == kMatVariantTc ? (uint64_t)kMatVariantTable[c->mat_variant].rows : 1;
+    uint64_t rest = 0, total = 0;
+    for (uint32_t k = n; k > 0;) {
+        const uint32_t nf0 = s->bf_count[sorted[k - 1]];
+        uint32_t g = k;
+        while (g > 0 && s->bf_count[sorted[g - 1]] == nf0) g--;
+        const uint64_t rows = (uint64_t)(k - g) * nf0;
+        total += (rows + pad - 1) / pad * pad * (rest + rows / 2);
+        rest += rows;
+        k = g;
+    }
+    UnitBuilder ub(effective_unit_budget(c->mat_unit_work, total, ctas, c->mat_variant), c->mat_variant);
     const auto nf = [&](uint32_t e) { return s->bf_count[targets[e]]; };
     const auto id = [&](uint32_t e) { return targets[e]; };
     const auto nf_ref = [&](uint32_t d) { return s->bf_count[d]; };
@@ -280,8 +290,9 @@ static int build_plan_cross(sdbfg_ctx* c, const sdbfg_set* q, const sdbfg_set* t
     if ((uint64_t)q->n * t->n + q->n + t->n >= (1ull << 32))
         return fail(c, SDBFG_ERR_ARG, "compare_to: too many pairs for one plan");
     const uint64_t ctas = (uint64_t)c->sms * matrix_ctas_per_sm(c->mat_variant);
-    UnitBuilder ub(effective_unit_budget(c->mat_unit_work, (uint64_t)q->total_filters * t->total_filters, ctas),
-                   (uint32_t)kMatVariantTable[c->mat_variant].rows);
+    UnitBuilder ub(effective_unit_budget(c->mat_unit_work, cross_work(q->total_filters, t->total_filters, c->mat_variant), ctas,
+                                         c->mat_variant),
+                   c->mat_variant);
     std::vector<uint32_t> targets;
     build_cross_units(
         ub, targets, q->n, t->n, [&](uint32_t i, uint32_t j) { return swaps(q, i, t, j); },
@@ -337,11 +348,14 @@ static MatParams plan_params(sdbfg_ctx* c, const MatPlan* p, const sdbfg_set* a,
     P.split = p->d_split.as<MatSplit>();
     P.nsplit = p->nsplit;
     P.slots = p->d_slots.as<double>();
+    P.nslots = p->nslots;
     P.scores = scores;
+    P.nscores = p->nscores;
     P.mode = p->mode;
     P.n = p->mode == kMatModeAll ? a->n : b->n;
     P.cutoffs = c->d_cut.as<uint16_t>();
     P.cutoffs64 = c->d_cut64.as<uint16_t>();
+    P.redo = redo_list(p->d_redo.p);
     P.error = p->d_counter.as<uint32_t>() + 1;
     P.phase = c->profile ? c->d_mphase.as<unsigned long long>() : nullptr;
     return P;
@@ -350,8 +364,9 @@ static MatParams plan_params(sdbfg_ctx* c, const MatPlan* p, const sdbfg_set* a,
 static int enqueue_plan(sdbfg_ctx* c, const MatPlan* p, const MatParams& P, cudaStream_t st) {
     CUDA_TRY(c, cudaMemsetAsync(p->d_counter.p, 0, 8, st));  // work counter, error flag
     const uint32_t grid = (uint32_t)(c->sms * matrix_ctas_per_sm(p->variant));
-    TIMED_LAUNCH_ON(c, "k_matrix", st, launch_matrix(P, p->variant, std::max(1u, std::min(grid, P.nunits)), st));
-    if (P.nsplit) TIMED_LAUNCH_ON(c, "k_matrix_finalize", st, launch_matrix_finalize(P, st));
+    uint64_t launched = 0;
+    TIMED_LAUNCH_ON(c, "k_matrix", st, run_matrix(P, p->variant, grid, (uint32_t)c->sms, st, &launched));
+    c->launches += launched - 1;  // one is counted with the timer
     return SDBFG_OK;
 }
 
@@ -362,9 +377,10 @@ static int run_plan(sdbfg_ctx* c, MatPlan* p, const sdbfg_set* a, const sdbfg_se
     const MatParams P = plan_params(c, p, a, b, dev_scores);
     matrix_ctas_per_sm(p->variant);  // sets the kernel's attributes outside any capture
     if (!c->mat_graphs || c->profile) return enqueue_plan(c, p, P, st);
+    const uint64_t kernels = p->variant == kMatVariantTc ? 3 : 1 + (P.nsplit ? 1 : 0), before = c->launches;
     if (p->graph && p->graph_out == dev_scores) {
         CUDA_TRY(c, cudaGraphLaunch(p->graph, st));
-        c->launches += 1 + (P.nsplit ? 1 : 0);
+        c->launches += kernels;
         return SDBFG_OK;
     }
     if (p->graph) {
@@ -383,13 +399,13 @@ static int run_plan(sdbfg_ctx* c, MatPlan* p, const sdbfg_set* a, const sdbfg_se
     }
     cudaStreamDestroy(cs);
     if (rc) return rc;
-    c->launches -= 1 + (P.nsplit ? 1 : 0);  // counted when the graph runs
+    c->launches = before;  // counted when the graph runs
     if (e == cudaSuccess) e = cudaGraphInstantiate(&p->graph, g, 0);
     if (g) cudaGraphDestroy(g);
     if (e != cudaSuccess) return fail(c, SDBFG_ERR_CUDA, "comparison graph: %s", cudaGetErrorString(e));
     p->graph_out = dev_scores;
     CUDA_TRY(c, cudaGraphLaunch(p->graph, st));
-    c->launches += 1 + (P.nsplit ? 1 : 0);
+    c->launches += kernels;
     return SDBFG_OK;
 }
 

@@ -39,5 +39,34 @@ __device__ __forceinline__ int32_t final_score(double sum, uint32_t n1, uint32_t
     return (int32_t)floor(__dadd_rn(__ddiv_rn(__dmul_rn(100.0, sum), (double)denom), 0.5));
 }
 
+// Marks of scores that only the ordered sum in double precision decides: the
+// reference digest is the pair's first (-2) or second (-3) digest.
+constexpr int32_t kScoreRedoFirst = -2, kScoreRedoSecond = -3;
+
+// The score of (ref, tgt) from the sum of its row maxima in units of 2^-23
+// (each within two units; bit 63: left to exact arithmetic), or a mark.
+// score = floor(100 sum / denom + 0.5); the reference's sum in double
+// precision differs from the true one by far less than the rows' units do,
+// so the score is its score unless 100 sum / denom + 0.5 is closer to a whole
+// number than that.  A target without a filter of 16 elements gives every
+// active row -1 and every other row 0: the running sum is then -1 after an
+// active row and 0 after another one, so the last row decides.
+__device__ __forceinline__ int32_t fixed_score(const MatParams& P, uint32_t rs, uint32_t ref, uint32_t ts,
+                                               uint32_t tgt, unsigned long long sum) {
+    const CmpDigest A = P.digests[rs][ref], B = P.digests[ts][tgt];
+    const uint64_t denom = A.nfilters > 1 ? A.nfilters - A.sparse : A.nfilters;
+    if (denom == 0) return -1;
+    if (B.sparse == B.nfilters) return A.flags & kDigestLastActive ? -1 : 0;
+    const bool second = P.mode == kMatModeAll ? ref > tgt : rs != 0;
+    const int32_t redo = second ? kScoreRedoSecond : kScoreRedoFirst;
+    if (sum >> 63) return redo;
+    if (sum == 0) return 0;
+    const uint64_t one = denom << 24;  // a score of 1 in the units of t
+    const uint64_t t = 200ull * sum + (denom << 23);
+    const uint64_t score = t / one, rem = t - score * one;
+    const uint64_t tol = 400ull * denom;
+    return rem < tol || one - rem <= tol ? redo : (int32_t)score;
+}
+
 
 }  // namespace sdbfg

@@ -187,115 +187,143 @@ __device__ __forceinline__ void and_popc_16x2(const uint32_t (&a)[64], const uin
 
 }  // namespace
 
-__global__ void __launch_bounds__(kCmpThreads) k_compare_pairs(CmpParams P) {
-    __shared__ __align__(16) uint32_t tf[kTgtTile][64];
-    __shared__ uint32_t tmeta[kTgtTile];
-    __shared__ uint16_t cut_tab[SDBF_CUTOFF_BINS], cut64_tab[SDBF_CUTOFF_BINS];
-    __shared__ double msc[kCmpThreads];
-    __shared__ uint32_t sparse_flag[kCmpThreads];
+// Shared memory of one CTA scoring a pair.
+struct PairSmem {
+    alignas(16) uint32_t tf[kTgtTile][64];
+    uint32_t tmeta[kTgtTile];
+    uint16_t cut_tab[SDBF_CUTOFF_BINS], cut64_tab[SDBF_CUTOFF_BINS];
+    double msc[kCmpThreads];
+    uint32_t sparse_flag[kCmpThreads];
+};
+
+__device__ __forceinline__ void pair_tables(PairSmem& S, const uint16_t* cutoffs, const uint16_t* cutoffs64) {
     for (uint32_t i = threadIdx.x; i < SDBF_CUTOFF_BINS; i += blockDim.x) {
-        cut_tab[i] = P.cutoffs[i];
-        cut64_tab[i] = P.cutoffs64[i];
+        S.cut_tab[i] = cutoffs[i];
+        S.cut64_tab[i] = cutoffs64[i];
     }
     __syncthreads();
-    for (uint64_t pr = blockIdx.x; pr < P.npairs; pr += gridDim.x) {
-        const CmpPair pair = P.pairs[pr];
-        const uint32_t sa = pair.sides & 1u, sb = (pair.sides >> 1) & 1u;
-        const CmpDigest A = P.digests[sa][pair.ref];
-        const CmpDigest B = P.digests[sb][pair.tgt];
-        const uint32_t* __restrict__ fa = P.filters[sa];
-        const uint32_t* __restrict__ fb = P.filters[sb];
-        const uint32_t* __restrict__ ma = P.meta[sa];
-        const uint32_t* __restrict__ mb = P.meta[sb];
-        const uint32_t n1 = pair.n1;  // filters of A used (== A.nfilters, sampling not applied here)
-        const bool fastA = (A.flags & kDigestFast) != 0;  // the reference digest's fastmode decides
-        double sum = -1.0;
-        uint32_t sparse = 0;
-        for (uint32_t c0 = 0; c0 < n1; c0 += blockDim.x) {
-            const uint32_t i = c0 + threadIdx.x;
-            const bool have = i < n1;
-            uint32_t a[64];
-            uint32_t s1 = 0, e1 = 0;
-            if (have) {
-                const uint32_t meta = ma[A.first + i];
-                s1 = meta & 0xFFFFu;
-                e1 = meta >> 16;
-                const uint4* src = reinterpret_cast<const uint4*>(fa + (size_t)(A.first + i) * 64);
+}
+
+// The score of reference digest A (its first n1 filters) against target
+// digest B by all kCmpThreads threads of a CTA, the sum in filter order;
+// thread 0 returns it.
+__device__ __forceinline__ int32_t score_pair(PairSmem& S, const uint32_t* __restrict__ fa, const uint32_t* __restrict__ ma,
+                                              const CmpDigest A, const uint32_t* __restrict__ fb,
+                                              const uint32_t* __restrict__ mb, const CmpDigest B, uint32_t n1) {
+    const bool fastA = (A.flags & kDigestFast) != 0;  // the reference digest's fastmode decides
+    double sum = -1.0;
+    uint32_t sparse = 0;
+    for (uint32_t c0 = 0; c0 < n1; c0 += blockDim.x) {
+        const uint32_t i = c0 + threadIdx.x;
+        const bool have = i < n1;
+        uint32_t a[64];
+        uint32_t s1 = 0, e1 = 0;
+        if (have) {
+            const uint32_t meta = ma[A.first + i];
+            s1 = meta & 0xFFFFu;
+            e1 = meta >> 16;
+            const uint4* src = reinterpret_cast<const uint4*>(fa + (size_t)(A.first + i) * 64);
 #pragma unroll
-                for (int q = 0; q < 16; q++) {
-                    const uint4 v = __ldg(src + q);
-                    a[4 * q] = v.x; a[4 * q + 1] = v.y; a[4 * q + 2] = v.z; a[4 * q + 3] = v.w;
-                }
+            for (int q = 0; q < 16; q++) {
+                const uint4 v = __ldg(src + q);
+                a[4 * q] = v.x; a[4 * q + 1] = v.y; a[4 * q + 2] = v.z; a[4 * q + 3] = v.w;
             }
-            const bool active = have && s1 >= (uint32_t)kMinElem;
-            // best = num/den; counted: a target filter with >= 16 elements was seen
-            uint32_t bnum = 0, bden = 1;
-            bool counted = false;
-            for (uint32_t j0 = 0; j0 < B.nfilters; j0 += kTgtTile) {
-                const uint32_t nt = min((uint32_t)kTgtTile, B.nfilters - j0);
-                __syncthreads();
-                {
-                    const uint4* src = reinterpret_cast<const uint4*>(fb + (size_t)(B.first + j0) * 64);
-                    uint4* dst = reinterpret_cast<uint4*>(&tf[0][0]);
-                    for (uint32_t q = threadIdx.x; q < nt * 16; q += blockDim.x) dst[q] = __ldg(src + q);
-                    for (uint32_t q = threadIdx.x; q < nt; q += blockDim.x) tmeta[q] = mb[B.first + j0 + q];
-                }
-                __syncthreads();
-                if (active) {
-                    for (uint32_t j = 0; j < nt; j++) {
-                        const uint32_t meta = tmeta[j];
-                        const uint32_t s2 = meta & 0xFFFFu;
-                        if (s2 < (uint32_t)kMinElem) continue;
-                        const uint32_t e2 = meta >> 16;
-                        const uint32_t max_est = min(e1, e2);
-                        uint32_t cut, match;
-                        if (!fastA) {
-                            cut = cut_tab[4096u / (s1 + s2)];
-                            match = and_popc_hs(a, &tf[j][0]);
-                            if (match > cut && staged_exit(a, &tf[j][0], cut)) match = 0;
-                        } else {  // bf_bitcount_cut_64 (bf_utils.cc:78-110) on the folded 64 bytes
-                            cut = cut64_tab[1024u / (s1 + s2)];
-                            uint32_t h8, h16, u8, u16;
-                            and_popc_16x2(a, &tf[j][0], &tf[j][0], h8, h16, u8, u16);
-                            match = (2 * h8 + 48 < cut) ? 0u : h16;
-                        }
-                        uint32_t num = 0, den = 1;
-                        if (match > cut) {
-                            num = match - cut;
-                            den = max_est - cut;  // uint32 as in the reference
-                        }
-                        if (!counted || (uint64_t)num * bden > (uint64_t)bnum * den) {
-                            bnum = num;
-                            bden = den;
-                            counted = true;
-                        }
+        }
+        const bool active = have && s1 >= (uint32_t)kMinElem;
+        // best = num/den; counted: a target filter with >= 16 elements was seen
+        uint32_t bnum = 0, bden = 1;
+        bool counted = false;
+        for (uint32_t j0 = 0; j0 < B.nfilters; j0 += kTgtTile) {
+            const uint32_t nt = min((uint32_t)kTgtTile, B.nfilters - j0);
+            __syncthreads();
+            {
+                const uint4* src = reinterpret_cast<const uint4*>(fb + (size_t)(B.first + j0) * 64);
+                uint4* dst = reinterpret_cast<uint4*>(&S.tf[0][0]);
+                for (uint32_t q = threadIdx.x; q < nt * 16; q += blockDim.x) dst[q] = __ldg(src + q);
+                for (uint32_t q = threadIdx.x; q < nt; q += blockDim.x) S.tmeta[q] = mb[B.first + j0 + q];
+            }
+            __syncthreads();
+            if (active) {
+                for (uint32_t j = 0; j < nt; j++) {
+                    const uint32_t meta = S.tmeta[j];
+                    const uint32_t s2 = meta & 0xFFFFu;
+                    if (s2 < (uint32_t)kMinElem) continue;
+                    const uint32_t e2 = meta >> 16;
+                    const uint32_t max_est = min(e1, e2);
+                    uint32_t cut, match;
+                    if (!fastA) {
+                        cut = S.cut_tab[4096u / (s1 + s2)];
+                        match = and_popc_hs(a, &S.tf[j][0]);
+                        if (match > cut && staged_exit(a, &S.tf[j][0], cut)) match = 0;
+                    } else {  // bf_bitcount_cut_64 (bf_utils.cc:78-110) on the folded 64 bytes
+                        cut = S.cut64_tab[1024u / (s1 + s2)];
+                        uint32_t h8, h16, u8, u16;
+                        and_popc_16x2(a, &S.tf[j][0], &S.tf[j][0], h8, h16, u8, u16);
+                        match = (2 * h8 + 48 < cut) ? 0u : h16;
+                    }
+                    uint32_t num = 0, den = 1;
+                    if (match > cut) {
+                        num = match - cut;
+                        den = max_est - cut;  // uint32 as in the reference
+                    }
+                    if (!counted || (uint64_t)num * bden > (uint64_t)bnum * den) {
+                        bnum = num;
+                        bden = den;
+                        counted = true;
                     }
                 }
             }
-            if (have) {
-                msc[threadIdx.x] = max_value(active, bnum, bden, counted);
-                sparse_flag[threadIdx.x] = s1 < (uint32_t)kMinElem;
-            }
-            __syncthreads();
-            if (threadIdx.x == 0) {
-                const uint32_t lim = min((uint32_t)blockDim.x, n1 - c0);
-                for (uint32_t q = 0; q < lim; q++) {
-                    const double m = msc[q];
-                    sum = (sum < 0) ? m : __dadd_rn(sum, m);
-                    sparse += sparse_flag[q];
-                }
-            }
-            __syncthreads();
         }
+        if (have) {
+            S.msc[threadIdx.x] = max_value(active, bnum, bden, counted);
+            S.sparse_flag[threadIdx.x] = s1 < (uint32_t)kMinElem;
+        }
+        __syncthreads();
         if (threadIdx.x == 0) {
-            uint64_t denom = n1;
-            if (n1 > 1) denom -= sparse;
-            int32_t score;
-            if (denom == 0 || sum < 0) score = -1;
-            else score = (int32_t)floor(__dadd_rn(__ddiv_rn(__dmul_rn(100.0, sum), (double)denom), 0.5));
-            P.scores[pr] = score;
+            const uint32_t lim = min((uint32_t)blockDim.x, n1 - c0);
+            for (uint32_t q = 0; q < lim; q++) {
+                const double m = S.msc[q];
+                sum = (sum < 0) ? m : __dadd_rn(sum, m);
+                sparse += S.sparse_flag[q];
+            }
+        }
+        __syncthreads();
+    }
+    return final_score(sum, n1, sparse);
+}
+
+__global__ void __launch_bounds__(kCmpThreads) k_compare_pairs(CmpParams P) {
+    __shared__ PairSmem S;
+    pair_tables(S, P.cutoffs, P.cutoffs64);
+    for (uint64_t pr = blockIdx.x; pr < P.npairs; pr += gridDim.x) {
+        const CmpPair pair = P.pairs[pr];
+        const uint32_t sa = pair.sides & 1u, sb = (pair.sides >> 1) & 1u;
+        const int32_t score = score_pair(S, P.filters[sa], P.meta[sa], P.digests[sa][pair.ref], P.filters[sb], P.meta[sb],
+                                         P.digests[sb][pair.tgt], pair.n1);
+        if (threadIdx.x == 0) P.scores[pr] = score;
+    }
+}
+
+// One warp per digest: digest_stats from meta words on the device.
+__global__ void k_digest_stats(const uint32_t* __restrict__ meta, CmpDigest* __restrict__ digests, uint32_t n) {
+    const uint32_t lane = threadIdx.x & 31;
+    for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n; i += (gridDim.x * blockDim.x) >> 5) {
+        const CmpDigest D = digests[i];
+        uint32_t c = 0;
+        for (uint32_t f = lane; f < D.nfilters; f += 32) c += (meta[D.first + f] & 0xFFFFu) < (uint32_t)kMinElem;
+        c = __reduce_add_sync(0xffffffffu, c);
+        if (lane == 0) {
+            const uint32_t last = D.nfilters ? meta[D.first + D.nfilters - 1] & 0xFFFFu : 0u;
+            digests[i].sparse = c;
+            digests[i].last = last;
+            if (last >= (uint32_t)kMinElem) digests[i].flags = D.flags | kDigestLastActive;
         }
     }
+}
+
+cudaError_t launch_digest_stats(const uint32_t* meta, CmpDigest* digests, uint32_t n, cudaStream_t st) {
+    if (n) k_digest_stats<<<(n + 7) / 8 < 1024 ? (n + 7) / 8 : 1024, 256, 0, st>>>(meta, digests, n);
+    return cudaGetLastError();
 }
 
 // One warp per filter: 16 lanes fold words k, k+16, k+32, k+48 into word k
@@ -340,7 +368,7 @@ cudaError_t launch_compare_pairs(const CmpParams& P, uint32_t grid, cudaStream_t
 // ---------------------------------------------------------- matrix engine
 namespace sdbfg {
 
-const MatVariant kMatVariantTable[kMatVariants] = {{128, 32}, {128, 16}, {128, 64}, {64, 32}, {256, 32}, {128, 256}};
+const MatVariant kMatVariantTable[kMatVariants] = {{128, 32}, {128, 16}, {128, 64}, {64, 32}, {256, 32}, {128, 192}};
 
 template <int R, int TJ>
 struct MatSmem {
@@ -669,6 +697,220 @@ __global__ void k_matrix_finalize(MatParams P) {
     P.scores[out_index(P, rs != 0, sp.ref, sp.tgt)] = final_score(sum, A.nfilters, sparse);
 }
 
+__device__ __forceinline__ void pair_of(uint64_t k, uint32_t mode, uint64_t n, uint32_t& i, uint32_t& j) {
+    if (mode == kMatModeCross) {
+        i = (uint32_t)(k / n);
+        j = (uint32_t)(k % n);
+        return;
+    }
+    // row i of the upper triangle: start(i) = i*(2n-i-1)/2 <= k < start(i+1)
+    const double nn = (double)n;
+    double r = floor(((2.0 * nn - 1.0) - sqrt((2.0 * nn - 1.0) * (2.0 * nn - 1.0) - 8.0 * (double)k)) / 2.0);
+    uint64_t ii = r < 0 ? 0 : (uint64_t)r;
+    auto start = [&](uint64_t x) { return x * (2 * n - x - 1) / 2; };
+    while (ii > 0 && start(ii) > k) ii--;
+    while (ii + 1 < n && start(ii + 1) <= k) ii++;
+    i = (uint32_t)ii;
+    j = (uint32_t)(k - start(ii) + ii + 1);
+}
+
+// After the tensor-core kernel: the split pairs' scores from their row
+// maxima; every marked score goes to the redo list (k_matrix_redo), or, when
+// the list is full, is scored here.  A block takes a split pair, then 128
+// scores at a time.
+__global__ void __launch_bounds__(kCmpThreads) k_matrix_finish(MatParams P) {
+    __shared__ PairSmem S;
+    __shared__ unsigned long long total, place;
+    __shared__ uint32_t hits[kCmpThreads], nhits;
+    __shared__ int32_t mark;
+    pair_tables(S, P.cutoffs, P.cutoffs64);
+    const uint32_t* slots = reinterpret_cast<const uint32_t*>(P.slots);
+    // all threads: the marked pair's score, now or later
+    auto redo = [&](uint32_t rs, uint32_t ref, uint32_t ts, uint32_t tgt, uint64_t o) {
+        const CmpDigest A = P.digests[rs][ref];
+        if (threadIdx.x == 0) {  // (a full list takes no more places: the count stays small)
+            place = *reinterpret_cast<volatile unsigned long long*>(P.redo.place);
+            if ((uint32_t)(place >> 40) < kRedoPairs) place = atomicAdd(P.redo.place, (1ull << 40) | A.nfilters);
+        }
+        __syncthreads();
+        const uint32_t k = (uint32_t)(place >> 40);
+        const uint64_t first = place & ((1ull << 40) - 1);
+        if (k < kRedoPairs && first + A.nfilters <= kRedoRows) {
+            if (threadIdx.x == 0) P.redo.list[k] = RedoPair{o, first, ref, tgt, rs | ts << 1, 0};
+        } else {
+            const int32_t score = score_pair(S, P.filters[rs], P.meta[rs], A, P.filters[ts], P.meta[ts], P.digests[ts][tgt],
+                                             A.nfilters);
+            if (threadIdx.x == 0) {
+                P.scores[o] = score;
+                if (k < kRedoPairs) P.redo.list[k] = RedoPair{o, first, ref, tgt, rs | ts << 1, kRedoDone};
+            }
+        }
+        __syncthreads();
+    };
+    for (uint32_t i = blockIdx.x; i < P.nsplit; i += gridDim.x) {
+        const MatSplit sp = P.split[i];
+        const uint32_t rs = sp.flags & kUnitRefSide1 ? 1 : 0, ts = sp.flags & kUnitTgtSide1 ? 1 : 0;
+        const uint32_t n = P.digests[rs][sp.ref].nfilters;
+        if (threadIdx.x == 0) total = 0;
+        __syncthreads();
+        unsigned long long sum = 0;
+        for (uint32_t r = threadIdx.x; r < n; r += blockDim.x) {
+            const uint32_t v = slots[sp.slot_base + r];
+            sum = v == 0xFFFFFFFFu ? sum | (1ull << 63) : sum + v;
+        }
+        if (sum >> 63) atomicOr(&total, 1ull << 63);
+        atomicAdd(&total, sum & ~(1ull << 63));
+        __syncthreads();
+        const uint64_t o = out_index(P, rs != 0, sp.ref, sp.tgt);
+        if (threadIdx.x == 0) mark = fixed_score(P, rs, sp.ref, ts, sp.tgt, total);
+        __syncthreads();
+        if (mark <= kScoreRedoFirst) redo(rs, sp.ref, ts, sp.tgt, o);
+        else if (threadIdx.x == 0) P.scores[o] = mark;
+        __syncthreads();
+    }
+    for (uint64_t b = (uint64_t)blockIdx.x * kCmpThreads; b < P.nscores; b += (uint64_t)gridDim.x * kCmpThreads) {
+        const bool marked = b + threadIdx.x < P.nscores && P.scores[b + threadIdx.x] <= kScoreRedoFirst;
+        if (!__syncthreads_or(marked)) continue;
+        if (threadIdx.x == 0) nhits = 0;
+        __syncthreads();
+        if (marked) hits[atomicAdd(&nhits, 1u)] = threadIdx.x;
+        __syncthreads();
+        const uint32_t nh = nhits;
+        for (uint32_t k = 0; k < nh; k++) {
+            const uint64_t o = b + hits[k];
+            uint32_t x, y;
+            pair_of(o, P.mode, P.n, x, y);
+            const bool second = P.scores[o] == kScoreRedoSecond;
+            const uint32_t side_y = P.mode == kMatModeAll ? 0u : 1u;
+            __syncthreads();  // every thread has read the mark
+            if (second) redo(side_y, y, 0, x, o);
+            else redo(0, x, side_y, y, o);
+        }
+    }
+}
+
+// The listed pairs: one block per reference filter (its exact maximum over
+// the target's filters as the reference's double; eight lanes per target
+// filter), and the block that finishes a pair's last row adds them up in
+// filter order.  A pair of 64 x 8,192 filters by one block took 1.9 ms; a row
+// of it takes one of these about 16 us, and its rows run side by side.
+constexpr uint32_t kRedoThreads = 256;
+__global__ void __launch_bounds__(kRedoThreads) k_matrix_redo(MatParams P) {
+    const uint32_t npairs = min((uint32_t)(*P.redo.place >> 40), kRedoPairs);
+    if (npairs == 0) return;
+    __shared__ uint16_t cut_tab[SDBF_CUTOFF_BINS], cut64_tab[SDBF_CUTOFF_BINS];
+    __shared__ uint32_t best[3][kRedoThreads / 8], before;
+    for (uint32_t i = threadIdx.x; i < SDBF_CUTOFF_BINS; i += blockDim.x) {
+        cut_tab[i] = P.cutoffs[i];
+        cut64_tab[i] = P.cutoffs64[i];
+    }
+    __syncthreads();
+    const uint32_t lane = threadIdx.x & 31, sub = lane & 7, grp = threadIdx.x >> 3;
+    auto better = [](uint32_t n1, uint32_t d1, bool c1, uint32_t& num, uint32_t& den, bool& counted) {
+        if (c1 && (!counted || (uint64_t)n1 * den > (uint64_t)num * d1)) {
+            num = n1;
+            den = d1;
+            counted = true;
+        }
+    };
+    uint32_t turn = 0;  // rows of the pairs before, so that small pairs spread over the blocks
+    for (uint32_t k = 0; k < npairs; k++) {
+        const RedoPair rp = P.redo.list[k];
+        if (rp.done & kRedoDone) continue;
+        const uint32_t rs = rp.sides & 1u, ts = rp.sides >> 1;
+        const CmpDigest A = P.digests[rs][rp.ref], B = P.digests[ts][rp.tgt];
+        const bool fastA = (A.flags & kDigestFast) != 0;
+        const uint32_t row0 = (blockIdx.x + gridDim.x - turn % gridDim.x) % gridDim.x;
+        turn += A.nfilters;
+        for (uint32_t i = row0; i < A.nfilters; i += gridDim.x) {
+            const uint32_t m1 = P.meta[rs][A.first + i], s1 = m1 & 0xFFFFu, e1 = m1 >> 16;
+            const bool active = s1 >= (uint32_t)kMinElem;
+            uint32_t bnum = 0, bden = 1;
+            bool counted = false;
+            if (active) {
+                const uint4* src = reinterpret_cast<const uint4*>(P.filters[rs] + (size_t)(A.first + i) * 64) + sub;
+                const uint4 a0 = __ldg(src), a1 = __ldg(src + 8);
+                for (uint32_t j0 = 0; j0 < B.nfilters; j0 += kRedoThreads / 8) {
+                    const uint32_t j = j0 + grp, jc = min(j, B.nfilters - 1);
+                    const uint4* t = reinterpret_cast<const uint4*>(P.filters[ts] + (size_t)(B.first + jc) * 64) + sub;
+                    const uint4 t0 = __ldg(t), t1 = __ldg(t + 8);
+                    const uint32_t m2 = P.meta[ts][B.first + jc], s2 = m2 & 0xFFFFu;
+                    // the first of the eight lanes: counts of the first 8, 16
+                    // and 32 words, and above them those of the words 32 later
+                    uint32_t c = (__popc(a0.x & t0.x) + __popc(a0.y & t0.y) + __popc(a0.z & t0.z) + __popc(a0.w & t0.w)) |
+                                 (__popc(a1.x & t1.x) + __popc(a1.y & t1.y) + __popc(a1.z & t1.z) + __popc(a1.w & t1.w)) << 16;
+                    c += __shfl_xor_sync(0xffffffffu, c, 1);
+                    const uint32_t c8 = c & 0xFFFFu;
+                    c += __shfl_xor_sync(0xffffffffu, c, 2);
+                    const uint32_t c16 = c & 0xFFFFu;
+                    c += __shfl_xor_sync(0xffffffffu, c, 4);
+                    const uint32_t c32 = c & 0xFFFFu, c64 = c32 + (c >> 16);
+                    if (sub == 0 && j < B.nfilters && s2 >= (uint32_t)kMinElem) {
+                        const uint32_t cut = fastA ? cut64_tab[1024u / (s1 + s2)] : cut_tab[4096u / (s1 + s2)];
+                        uint32_t match = fastA ? c16 : c64;
+                        if (fastA ? 2 * c8 + 48 < cut : (8 * c8 + 48 < cut || 4 * c16 + 48 < cut || 2 * c32 + 48 < cut)) match = 0;
+                        uint32_t num = 0, den = 1;
+                        if (match > cut) {
+                            num = match - cut;
+                            den = min(e1, m2 >> 16) - cut;  // uint32 as in the reference
+                        }
+                        better(num, den, true, bnum, bden, counted);
+                    }
+                }
+            }
+            if (sub == 0) {
+                best[0][grp] = bnum;
+                best[1][grp] = bden;
+                best[2][grp] = counted;
+            }
+            __syncthreads();
+            if (threadIdx.x == 0) {
+                for (uint32_t q = 1; q < kRedoThreads / 8; q++) better(best[0][q], best[1][q], best[2][q], bnum, bden, counted);
+                P.redo.max[rp.first + i] = max_value(active, bnum, bden, counted);
+                __threadfence();
+                before = atomicAdd(&P.redo.list[k].done, 1u);
+            }
+            __syncthreads();
+            if (before + 1 == A.nfilters && threadIdx.x < 32) {  // the pair's last row: the ordered sum
+                __threadfence();
+                double sum = -1.0;
+                for (uint32_t c0 = 0; c0 < A.nfilters; c0 += 32) {
+                    const double m = c0 + lane < A.nfilters ? __ldcg(P.redo.max + rp.first + c0 + lane) : 0.0;
+                    const uint32_t lim = min(32u, A.nfilters - c0);
+                    for (uint32_t q = 0; q < lim; q++) {
+                        const double v = __shfl_sync(0xffffffffu, m, q);
+                        if (sum < 0) sum = v;
+                        else if (v != 0.0) sum = __dadd_rn(sum, v);
+                    }
+                }
+                if (lane == 0) P.scores[rp.score] = final_score(sum, A.nfilters, A.sparse);
+            }
+            __syncthreads();
+        }
+    }
+}
+
+cudaError_t run_matrix(const MatParams& P, int variant, uint32_t grid, uint32_t sms, cudaStream_t st, uint64_t* launches) {
+    if (P.nunits == 0) return cudaSuccess;
+    grid = grid < P.nunits ? grid : P.nunits;
+    cudaError_t e;
+    if (variant == kMatVariantTc) {
+        // sums of group units grow in the score array, split maxima in the slots
+        if ((e = cudaMemsetAsync(P.scores, 0, P.nscores * 4, st))) return e;
+        if (P.nslots && (e = cudaMemsetAsync(P.slots, 0, P.nslots * 4, st))) return e;
+        if ((e = cudaMemsetAsync(P.redo.place, 0, 8, st))) return e;
+        if ((e = launch_matrix_tc(P, grid, st))) return e;
+        const uint64_t work = P.nscores / kCmpThreads + 1 + P.nsplit;
+        k_matrix_finish<<<(uint32_t)(work < 8ull * sms ? work : 8ull * sms), kCmpThreads, 0, st>>>(P);
+        k_matrix_redo<<<4 * sms, kRedoThreads, 0, st>>>(P);
+        *launches += 3;
+        return cudaGetLastError();
+    }
+    if ((e = launch_matrix(P, variant, grid, st))) return e;
+    *launches += 1 + (P.nsplit ? 1 : 0);
+    return launch_matrix_finalize(P, st);
+}
+
 // The dynamic shared-memory attribute is set by matrix_ctas_per_sm, which
 // callers run before the first launch (and before any stream capture).
 template <int R, int TJ>
@@ -772,23 +1014,6 @@ __global__ void __launch_bounds__(1024) k_match_scan(const uint32_t* __restrict_
         run += counts[b];
     }
     if (threadIdx.x == 1023) offs[nb] = part[1023];
-}
-
-__device__ __forceinline__ void pair_of(uint64_t k, uint32_t mode, uint64_t n, uint32_t& i, uint32_t& j) {
-    if (mode == kMatModeCross) {
-        i = (uint32_t)(k / n);
-        j = (uint32_t)(k % n);
-        return;
-    }
-    // row i of the upper triangle: start(i) = i*(2n-i-1)/2 <= k < start(i+1)
-    const double nn = (double)n;
-    double r = floor(((2.0 * nn - 1.0) - sqrt((2.0 * nn - 1.0) * (2.0 * nn - 1.0) - 8.0 * (double)k)) / 2.0);
-    uint64_t ii = r < 0 ? 0 : (uint64_t)r;
-    auto start = [&](uint64_t x) { return x * (2 * n - x - 1) / 2; };
-    while (ii > 0 && start(ii) > k) ii--;
-    while (ii + 1 < n && start(ii + 1) <= k) ii++;
-    i = (uint32_t)ii;
-    j = (uint32_t)(k - start(ii) + ii + 1);
 }
 
 __global__ void __launch_bounds__(256) k_match_write(const int32_t* __restrict__ scores, uint64_t n, int32_t thr,

@@ -12,9 +12,21 @@ constexpr int kCmpThreads = 128;
 struct CmpDigest {
     uint32_t first;
     uint32_t nfilters;
-    uint32_t flags;  // kDigestFast: filters folded to 64 bytes (sdbf::fast)
+    uint32_t flags;  // kDigestFast: filters folded to 64 bytes (sdbf::fast); kDigestLastActive
+    uint32_t sparse; // filters with fewer than 16 elements
+    uint32_t last;   // element count of the last filter
 };
-constexpr uint32_t kDigestFast = 1u;
+constexpr uint32_t kDigestFast = 1u, kDigestLastActive = 2u;  // the last filter has 16 elements or more
+
+// The digest-level words of a set's meta words (element counts).
+inline void digest_stats(CmpDigest& d, const uint32_t* meta) {
+    d.sparse = 0;
+    for (uint32_t f = 0; f < d.nfilters; f++) d.sparse += (meta[d.first + f] & 0xFFFFu) < 16;
+    d.last = d.nfilters ? meta[d.first + d.nfilters - 1] & 0xFFFFu : 0u;
+    if (d.last >= 16) d.flags |= kDigestLastActive;
+}
+// The same from meta words on the device.
+cudaError_t launch_digest_stats(const uint32_t* meta, CmpDigest* digests, uint32_t n, cudaStream_t st);
 
 // One scored pair after the swap rule: `ref` is the side whose filters are
 // summed (sdbf_1 after the swap in sdbf_core.cc:351-359).
@@ -68,7 +80,10 @@ enum : uint32_t { kUnitRefSide1 = 1u, kUnitTgtSide1 = 2u, kUnitSplit = 4u, kUnit
 //    rows (ref = digest id, rows [r0, r1) = all its filters), running sums
 //    per target in shared memory;
 //  * split (kUnitSplit): rows [r0, r1) of one reference digest against one
-//    target; maxima to the slot array, summed by k_matrix_finalize.
+//    target; maxima to the slot array, summed by k_matrix_finalize.  The
+//    tensor-core kernel also splits the target's filters ([c0, c1), with a
+//    group's digests as rows too: their splits are consecutive), its maxima
+//    are unsigned integers of 2^-23 and k_matrix_finish sums them.
 struct MatUnit {
     uint32_t ref;     // digest id, or (group) position in MatParams::refs
     uint32_t r0, r1;  // rows [r0, r1) (group: 0 .. total filters of its digests)
@@ -76,6 +91,7 @@ struct MatUnit {
     uint32_t flags;
     uint32_t split;   // split units: index into MatParams::split
     uint32_t nref;    // group units: digests in the group
+    uint32_t c0, c1;  // tensor-core split units: filters [c0, c1) of the one target
 };
 
 struct MatSplit {
@@ -84,6 +100,29 @@ struct MatSplit {
     uint32_t pad;
     uint64_t slot_base;   // maxima of ref filter r at slots[slot_base + r]
 };
+
+// Pairs whose score only the ordered sum in double precision decides (listed
+// by k_matrix_finish, scored by k_matrix_redo).
+struct RedoPair {
+    uint64_t score;    // its place in the score array
+    uint64_t first;    // its row maxima at RedoList::max
+    uint32_t ref, tgt;
+    uint32_t sides;    // bit 0: ref is in set 1, bit 1: tgt is
+    uint32_t done;     // rows finished; kRedoDone: scored already (no room for its rows)
+};
+constexpr uint32_t kRedoPairs = 1024, kRedoDone = 0x80000000u;
+constexpr uint64_t kRedoRows = 1ull << 15;  // (296 KB in all: an allocation the driver serves quickly)
+struct RedoList {
+    unsigned long long* place;  // pairs << 40 | rows taken so far
+    RedoPair* list;             // kRedoPairs
+    double* max;                // kRedoRows
+};
+constexpr uint64_t kRedoBytes = 64 + kRedoPairs * sizeof(RedoPair) + kRedoRows * 8;
+inline RedoList redo_list(void* p) {  // in kRedoBytes of device memory
+    uint8_t* b = static_cast<uint8_t*>(p);
+    return RedoList{reinterpret_cast<unsigned long long*>(b), reinterpret_cast<RedoPair*>(b + 64),
+                    reinterpret_cast<double*>(b + 64 + kRedoPairs * sizeof(RedoPair))};
+}
 
 struct MatParams {
     const uint32_t* filters[2];
@@ -96,26 +135,29 @@ struct MatParams {
     const uint32_t* refs;      // reference digest ids of group units
     const MatSplit* split;
     uint32_t nsplit;
-    double* slots;
+    double* slots;             // row maxima of split pairs (tensor-core kernel: uint32_t)
+    uint64_t nslots;
     int32_t* scores;
+    uint64_t nscores;
     uint32_t mode;             // kMatModeAll: n*(n-1)/2 pair order; kMatModeCross: q*nt+t
     uint32_t n;                // set size (all) / number of targets (cross)
     const uint16_t* cutoffs;   // CUTOFFS256
     const uint16_t* cutoffs64; // CUTOFFS64 (fast mode)
+    RedoList redo;             // tensor-core kernel
     uint32_t* error;           // tensor-core kernel: set when a bounded wait gave up
     unsigned long long* phase; // tensor-core kernel: optional SM-cycle counters (kTcPh*), null = off
 };
-// phase counters of the tensor-core kernel (one producer and one consumer thread per CTA)
+// phase counters of the tensor-core kernel: per role the busy cycles of its
+// warps (first lane), then the cycles they waited, tiles, marked pairs
 enum : int {
-    kTcPhCompose = 0, kTcPhFill, kTcPhFetchWait, kTcPhStageWait, kTcPhWiden, kTcPhIssue, kTcPhProdStep,
-    kTcPhAccWait, kTcPhScore, kTcPhFold, kTcPhConsStep, kTcPhStepBarrier, kTcPhTiles, kTcPhLd, kTcPhMark,
-    kTcPhWalk, kTcPhCount
+    kTcPhCompose = 0, kTcPhWiden, kTcPhMma, kTcPhMark, kTcPhCheck, kTcPhWaits, kTcPhTiles = 2 * kTcPhWaits, kTcPhMarked,
+    kTcPhCount
 };
 
 // Kernel variants (rows per CTA x target filters per tile), chosen by the
 // autotuner.  Variants 0-4 count on the CUDA cores (carry-save AND-popcount);
-// variant 5 counts on the tensor cores (tcgen05, fp8 0/1 operands, fp32
-// accumulators in TMEM: the count is an exact dot product) and needs sm_100+.
+// variant 5 counts on the tensor cores (tcgen05, e2m1 operands, fp32
+// accumulators in TMEM: the count is an exact dot product) and needs sm_103a.
 struct MatVariant {
     int rows, tile;
 };
@@ -126,6 +168,9 @@ extern const MatVariant kMatVariantTable[kMatVariants];
 cudaError_t launch_matrix(const MatParams& P, int variant, uint32_t grid, cudaStream_t st);
 cudaError_t launch_matrix_tc(const MatParams& P, uint32_t grid, cudaStream_t st);
 int matrix_tc_ctas_per_sm();
+// A whole job on `grid` resident CTAs: what has to be zeroed, the kernel and
+// what finishes its scores; *launches grows by the kernels launched.
+cudaError_t run_matrix(const MatParams& P, int variant, uint32_t grid, uint32_t sms, cudaStream_t st, uint64_t* launches);
 cudaError_t launch_matrix_finalize(const MatParams& P, cudaStream_t st);
 int matrix_ctas_per_sm(int variant);
 

@@ -247,16 +247,16 @@ struct MatPlan {
     int variant = 0;
     uint64_t unit_work = 0;
     uint32_t nunits = 0, nsplit = 0;
-    uint64_t nscores = 0;
+    uint64_t nscores = 0, nslots = 0;
     uint64_t filter_pairs = 0;  // sum over scored pairs of n_ref * n_tgt
-    DevBuf d_units, d_targets, d_refs, d_split, d_slots, d_counter;
+    DevBuf d_units, d_targets, d_refs, d_split, d_slots, d_counter, d_redo;
     cudaGraphExec_t graph = nullptr;
     int32_t* graph_out = nullptr;
     cudaStream_t graph_stream = nullptr;
     uint64_t last_use = 0;
     ~MatPlan() {
         if (graph) cudaGraphExecDestroy(graph);
-        for (DevBuf* b : {&d_units, &d_targets, &d_refs, &d_split, &d_slots, &d_counter}) b->release();
+        for (DevBuf* b : {&d_units, &d_targets, &d_refs, &d_split, &d_slots, &d_counter, &d_redo}) b->release();
     }
 };
 

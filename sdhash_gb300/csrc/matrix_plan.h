@@ -24,15 +24,34 @@ struct UnitBuilder {
     uint64_t budget;
     uint32_t max_rows;
     uint64_t filter_pairs = 0;
-    UnitBuilder(uint64_t w, uint32_t rows) : budget(std::max<uint64_t>(w, 1)), max_rows(rows) {}
+    // Tensor-core units: a pass costs its 128 rows whatever it fills, so the
+    // budget counts padded rows, and a pair larger than the budget is split
+    // by reference rows and by target filters.
+    bool tc;
+    UnitBuilder(uint64_t w, int variant)
+        : budget(std::max<uint64_t>(w, 1)), max_rows((uint32_t)kMatVariantTable[variant].rows), tc(variant == kMatVariantTc) {}
+    uint64_t cost_rows(uint32_t rows) const { return tc ? ((uint64_t)rows + max_rows - 1) / max_rows * max_rows : rows; }
+    // target filters of a split unit of one pass: the budget's, in whole tiles
+    uint32_t split_cols() const {
+        const uint64_t tile = (uint64_t)kMatVariantTable[kMatVariantTc].tile;
+        return (uint32_t)std::min<uint64_t>(std::max<uint64_t>(tile, budget / max_rows / tile * tile), 1u << 30);
+    }
 
     // target run [t0, t1) of the target list for `rows` reference rows
-    template <class NF, class EMIT>
-    void cut_runs(uint32_t rows, uint32_t t0, uint32_t t1, NF nf, EMIT emit) {
+    // (huge(e): a target that is larger than the budget by itself)
+    template <class NF, class EMIT, class HUGE>
+    void cut_runs(uint32_t rows, uint32_t t0, uint32_t t1, NF nf, EMIT emit, HUGE huge) {
         uint32_t start = t0;
         uint64_t acc = 0;
         for (uint32_t e = t0; e < t1; e++) {
-            const uint64_t w = (uint64_t)rows * nf(e);
+            const uint64_t w = cost_rows(rows) * nf(e);
+            if (tc && w > budget && nf(e) > split_cols()) {
+                if (e > start) emit(start, e, acc);
+                huge(e);
+                start = e + 1;
+                acc = 0;
+                continue;
+            }
             if (e > start && (acc + w > budget || e - start >= kMatMaxTargets)) {
                 emit(start, e, acc);
                 start = e;
@@ -45,15 +64,30 @@ struct UnitBuilder {
 
     // digests ids[0..n) (side flags) all against targets [t0, t1); their
     // filters together must fit max_rows
-    template <class NF>
-    void add_group(const uint32_t* ids, uint32_t n, uint32_t rows, uint32_t flags, uint32_t t0, uint32_t t1, NF nf) {
+    template <class NFR, class NF, class ID>
+    void add_group(const uint32_t* ids, uint32_t n, uint32_t rows, NFR nf_ref, uint32_t flags, uint32_t t0, uint32_t t1,
+                   NF nf, ID id) {
         const uint32_t pos = (uint32_t)refs.size();
         refs.insert(refs.end(), ids, ids + n);
-        cut_runs(rows, t0, t1, nf, [&](uint32_t a, uint32_t b, uint64_t acc) {
-            units.push_back(MatUnit{pos, 0, rows, a, b, flags | kUnitGroup, 0, n});
-            work.push_back(acc + (uint64_t)(b - a) * rows * 4);
-            filter_pairs += acc;
-        });
+        for (uint32_t e = t0; e < t1; e++) filter_pairs += (uint64_t)rows * nf(e);
+        cut_runs(
+            rows, t0, t1, nf,
+            [&](uint32_t a, uint32_t b, uint64_t acc) {
+                units.push_back(MatUnit{pos, 0, rows, a, b, flags | kUnitGroup, 0, n, 0, 0});
+                work.push_back(acc + (uint64_t)(b - a) * rows * 4);
+            },
+            [&](uint32_t e) {  // every digest of the group against parts of one target
+                const uint32_t si = (uint32_t)split.size();
+                for (uint32_t k = 0; k < n; k++) {
+                    split.push_back(MatSplit{ids[k], id(e), flags & (kUnitRefSide1 | kUnitTgtSide1), 0, slots});
+                    slots += nf_ref(ids[k]);
+                }
+                for (uint32_t c = 0; c < nf(e); c += split_cols()) {
+                    const uint32_t c1 = std::min<uint32_t>(nf(e), c + split_cols());
+                    units.push_back(MatUnit{pos, 0, rows, e, e + 1, flags | kUnitGroup | kUnitSplit, si, n, c, c1});
+                    work.push_back(cost_rows(rows) * (c1 - c));
+                }
+            });
     }
 
     // one reference digest against targets [t0, t1)
@@ -61,33 +95,35 @@ struct UnitBuilder {
     void add(uint32_t ref, uint32_t nref, uint32_t flags, uint32_t t0, uint32_t t1, NF nf, ID id) {
         if (t1 <= t0) return;
         if (nref <= max_rows) {
-            add_group(&ref, 1, nref, flags, t0, t1, nf);
+            add_group(&ref, 1, nref, [&](uint32_t) { return nref; }, flags, t0, t1, nf, id);
             return;
         }
         uint32_t start = t0;
         uint64_t acc = 0;
         auto flush = [&](uint32_t end) {
             if (end > start) {
-                units.push_back(MatUnit{ref, 0, nref, start, end, flags, 0, 1});
+                units.push_back(MatUnit{ref, 0, nref, start, end, flags, 0, 1, 0, 0});
                 work.push_back(acc + (uint64_t)(end - start) * nref * 4);
             }
             start = end;
             acc = 0;
         };
         for (uint32_t e = t0; e < t1; e++) {
-            const uint64_t w = (uint64_t)nref * nf(e);
-            filter_pairs += w;
+            const uint64_t w = cost_rows(nref) * nf(e);
+            filter_pairs += (uint64_t)nref * nf(e);
             if (w > budget) {  // one pair larger than a unit: split the reference's rows
                 flush(e);
                 const uint32_t rows = (uint32_t)std::max<uint64_t>(128, budget / nf(e) / 128 * 128);
                 const uint32_t si = (uint32_t)split.size();
                 split.push_back(MatSplit{ref, id(e), flags & (kUnitRefSide1 | kUnitTgtSide1), 0, slots});
                 slots += nref;
-                for (uint32_t r = 0; r < nref; r += rows) {
-                    const uint32_t r1 = std::min(nref, r + rows);
-                    units.push_back(MatUnit{ref, r, r1, e, e + 1, flags | kUnitSplit, si, 1});
-                    work.push_back((uint64_t)(r1 - r) * nf(e));
-                }
+                const uint32_t cols = tc ? split_cols() : nf(e), rstep = tc && nf(e) > cols ? max_rows : rows;
+                for (uint32_t r = 0; r < nref; r += rstep)
+                    for (uint32_t c = 0; c < nf(e); c += cols) {
+                        const uint32_t r1 = std::min(nref, r + rstep), c1 = std::min<uint32_t>(nf(e), c + cols);
+                        units.push_back(MatUnit{ref, r, r1, e, e + 1, flags | kUnitSplit, si, 1, c, c1});
+                        work.push_back(cost_rows(r1 - r) * (c1 - c));
+                    }
                 start = e + 1;
                 continue;
             }
@@ -108,7 +144,7 @@ struct UnitBuilder {
         std::vector<uint32_t> cur;
         uint32_t rows = 0, cur_key = 0;
         auto flush = [&]() {
-            if (!cur.empty()) add_group(cur.data(), (uint32_t)cur.size(), rows, flags, t0, t1, nf);
+            if (!cur.empty()) add_group(cur.data(), (uint32_t)cur.size(), rows, nf_ref, flags, t0, t1, nf, id);
             cur.clear();
             rows = 0;
         };
@@ -185,13 +221,27 @@ void build_cross_units(UnitBuilder& ub, std::vector<uint32_t>& targets, uint32_t
     }
 }
 
-// Unit budget for a job of `total` filter pairs on `slots` resident CTAs:
-// the configured budget, lowered (to no less than 2^16) for small jobs so
-// that every CTA gets about four units.
-inline uint64_t effective_unit_budget(uint64_t configured, uint64_t total, uint64_t slots) {
-    const uint64_t fair = total / std::max<uint64_t>(1, 4 * slots);
-    return std::min(configured, std::max<uint64_t>(1ull << 16, fair));
+// Work of a query x target job: the side with fewer filters gives the rows.
+inline uint64_t cross_work(uint64_t q, uint64_t t, int variant) {
+    const uint64_t pad = variant == kMatVariantTc ? (uint64_t)kMatVariantTable[variant].rows : 1;
+    return (std::min(q, t) + pad - 1) / pad * pad * std::max(q, t);
 }
 
+// Unit budget for a job of `total` work (filter pairs; tensor-core units:
+// padded rows x target filters) on `slots` resident CTAs: the configured
+// budget, lowered for small jobs so that every CTA gets about four units
+// (no less than 2^16 filter pairs).  A tensor-core job of at most
+// 16 tiles per CTA is cut into one unit per CTA, of whole tiles: a unit's
+// start (rows fetched and widened, pipeline filled) costs about two tiles.
+inline uint64_t effective_unit_budget(uint64_t configured, uint64_t total, uint64_t slots, int variant) {
+    slots = std::max<uint64_t>(1, slots);
+    if (variant == kMatVariantTc) {
+        const uint64_t tile = (uint64_t)kMatVariantTable[variant].rows * kMatVariantTable[variant].tile;
+        const uint64_t tiles = (total + tile - 1) / tile;
+        const uint64_t per = tiles <= 16 * slots ? (tiles + slots - 1) / slots : tiles / (4 * slots);
+        return std::min(configured, std::max<uint64_t>(1, per) * tile);
+    }
+    return std::min(configured, std::max<uint64_t>(1ull << 16, total / (4 * slots)));
+}
 
 }  // namespace sdbfg

@@ -1,37 +1,64 @@
 // matrix_tc.cu -- the filter-matrix comparison counted on the tensor cores.
 //
 // popcount(a & b) of two 2048-bit filters is the dot product of their bit
-// vectors.  With each bit widened to an e4m3 byte (0x08 = 2^-6, or 0) and
-// fp32 accumulation, tcgen05.mma computes it exactly: every product is
-// 2^-12, every partial sum a multiple of 2^-12 no larger than 2048 * 2^-12,
-// well inside fp32's 24-bit significand; the count is the sum times 4096.  One CTA multiplies 128 reference filters (TMEM lanes)
-// by tiles of up to 256 target filters (TMEM columns) over K = 2048 in 16
-// chunks of 128.  The CTA is a two-stage software pipeline: warps 4-7
-// compose tile g, fetch its filter bits with cp.async, widen each chunk into
-// a 128-byte-swizzled shared-memory stage (two stages, so widening overlaps
-// the MMAs of the previous chunk) and issue the four K=32 MMAs per chunk into
-// accumulator g & 1 (512 TMEM columns hold two); meanwhile warps 0-3 read
-// tile g-1's counts from the other accumulator, one row per thread, and
-// score it exactly as the CUDA-core kernel does (compare_kernels.cu
-// k_matrix): a pair can score above 0 only if its full count exceeds the
-// cut, and for those rare pairs the reference's staged exits
-// (bf_utils.cc:114-206) are rechecked from the filters in memory.  Each
-// 32-column slice is scored in two passes: a branch-free pass marks the
-// row's counted columns and those above the cut, then the slice's segments
-// are walked in column order, re-checking only the marked columns.  Maxima
-// of completed targets collect in a ring of eight and are summed in filter
-// order as it fills.  Work units, group units, running sums and split pairs
-// are those of k_matrix.
+// vectors.  With every bit widened to an e2m1 value (4 bits) and fp32
+// accumulation, tcgen05.mma.kind::mxf4 computes it exactly: bit k of each
+// nibble keeps its place in the target filters (values 0.5, 1, 2, 2) and the
+// reference filters hold the reciprocal (2, 1, 0.5, 0.5), so every product of
+// two set bits is 1, all block scales are 1 and the sums are integers up to
+// 2,048.  Widening permutes K inside each 32-bit word identically for both.
 //
-// The widening permutes K inside each 32-bit word (output word k of a word
-// w holds bits k, k+8, k+16, k+24 of w), identically for both operands, so
-// the dot product is unchanged; bit k of each byte moves to bit 3 (the
-// single set bit of 0x08), one shift and one mask per output word.  --fast digests count only chunks 0-3 (their first
-// 64 bytes).
+// One persistent CTA per SM multiplies 128 reference filters (TMEM lanes, a
+// "pass": their 128 KB of e2m1 stay in shared memory) by tiles of up to 192
+// target filters (TMEM columns) over K = 2048 in eight chunks of 256.  Five
+// roles run as a pipeline over the tiles, joined by mbarriers only:
+//   compose (1 warp)  takes work units, writes the rows of a pass and the
+//                     columns of a tile (filter, hamming weight, element
+//                     count, target) into a ring of four tiles;
+//   widen (6 warps)   widen a pass's reference rows, then chunk by chunk the
+//                     tile's target filters (bits read from global memory four
+//                     chunks ahead) into two 24 KB stages;
+//   mma (1 warp)      four K=64 MMAs per chunk into one of two accumulators;
+//   mark (4 warps)    read the counts with tcgen05.ld, one row per lane, and
+//                     mark the columns above the pair's cut: one subtraction
+//                     and one funnel shift per column (the sign bit) when
+//                     the slice's element counts are equal, else a table
+//                     lookup per column;
+//   check (8 warps)   recompute the marked pairs (about 1 % on unrelated
+//                     content) from the filters in memory, eight lanes a
+//                     pair: full count and the reference's staged exits
+//                     (bf_utils.cc:114-206), and add the row's maximum.
+// A pair can score above 0 only if its full count exceeds the cut, so what
+// is not marked contributes 0.
 //
-// Every mbarrier wait is bounded; a wait that gives up sets P.error, all
-// threads leave together (the decision is made by __syncthreads_and), the
-// MMAs still in flight are waited for and the TMEM is released.
+// A digest pair's score is floor(100 * sum / denominator + 0.5) of the row
+// maxima's sum in double precision, in filter order.  The row maxima are
+// summed here as integers of 2^-23 (any order gives the same sum); each is
+// within two units of the true ratio, so the score is the reference's unless
+// 100 * sum / denominator + 0.5 lies within that error of a whole number.
+// Such a pair (about 1 in 20,000 of those above 0, or an exact half), and a
+// ratio that is not in [0, 1] (possible when --fast digests meet unfolded
+// ones), is marked and k_matrix_finish scores it with the ordered sum in
+// double precision.  Marks and sums live in the score array itself for units
+// of several reference digests.
+//
+// Every mbarrier wait is bounded; a role whose wait gives up sets P.error
+// and leaves, the others follow when their own waits run out, and the MMAs in
+// flight are waited for before the TMEM is released.
+//
+// What bounds it: shared-memory bandwidth and the hand-over between the
+// roles.  A tile takes about 10.4 K cycles, of which its 32 MMAs need 3 K on
+// the tensor pipe; they read 10 KB of shared memory each (2.5 K cycles of
+// its bandwidth a tile) beside 1.5 K cycles of widened stores.  Pairs of 128 x
+// 192 filters: 5.6e11 filter pairs/s (400 uneven digests, 4.7e9 pairs: 8.6
+// ms; 2,048 queries against 4 image segments, 8e8 pairs: 1.5 ms), against
+// 1.2e11 for e4m3 operands widened for both sides in every tile, one row per
+// scoring lane and ordered sums in the kernel (39 and 5.7 ms).  Measured on
+// the way: every check warp a share of the tile's marked pairs instead of
+// its own rows (three barriers a tile: 10.1 against 9.0 ms); unrolled role
+// loops (15 ms: the five roles share the instruction cache, and instruction
+// fetch was the first stall); a proxy fence in the widening warps (18.4 ms:
+// it waits for their loads in flight).
 #include <cstdint>
 #include <cuda_runtime.h>
 
@@ -43,64 +70,120 @@ namespace sdbfg {
 
 namespace {
 
-constexpr int kTcRows = 128;       // reference rows per pass = TMEM lanes
-constexpr int kTcCols = 256;       // target filters per tile = MMA N (max)
-constexpr int kTcThreads = 256;    // warps 0-3 score (one row each), warps 4-7 widen and issue
-constexpr int kTcChunk = 128;      // K elements (bits) per stage
-constexpr int kTcChunks = 2048 / kTcChunk;
-constexpr int kTcRing = 8;         // completed targets held before their maxima are summed
-constexpr uint32_t kTcAStage = kTcRows * kTcChunk;   // 16 KB of e4m3
-constexpr uint32_t kTcBStage = kTcCols * kTcChunk;   // 32 KB
-constexpr uint32_t kTcStage = kTcAStage + kTcBStage;
-constexpr uint32_t kTcWaitSpins = 1u << 20;
-constexpr int kTcBitSlots = 3;     // chunks of filter bits in flight (cp.async ring)
+constexpr uint32_t kTcRows = 128;       // reference rows per pass = TMEM lanes
+constexpr uint32_t kTcCols = 192;       // target filters per tile = MMA N (max)
+constexpr uint32_t kTcSlices = kTcCols / 32;
+constexpr uint32_t kTcMark = 4, kTcCheck = 8, kTcWiden = 6;  // warps of each role
+constexpr uint32_t kTcThreads = (kTcMark + kTcCheck + kTcWiden + 2) * 32;
+constexpr uint32_t kTcComposeWarp = kTcMark + kTcCheck + kTcWiden, kTcMmaWarp = kTcComposeWarp + 1;
+constexpr uint32_t kTcChunks = 8;                       // chunks of 256 bits: 128 bytes of e2m1 per row
+constexpr uint32_t kTcAChunk = kTcRows * 128, kTcA = kTcChunks * kTcAChunk;
+constexpr uint32_t kTcBStage = kTcCols * 128;
+constexpr uint32_t kTcRing = 4;         // composed tiles in flight
+constexpr uint32_t kTcScaleCol = 2 * kTcCols, kTcScaleCols = 32;  // TMEM columns of block scales (all 1.0)
+constexpr uint32_t kTcTmemCols = 512;
+constexpr uint32_t kTcMasks = 4;        // marked tiles in flight
+constexpr uint32_t kTcDense = 96;       // marked pairs a check warp takes at a time
+constexpr uint32_t kTcSpins = 1u << 20;
 
-// one tile's composition (double-buffered: warps 4-7 compose and count tile
-// k while warps 0-3 score tile k-1)
-struct TcTile {
-    uint4 tw[8][kTcCols];  // first 128 bytes of each target filter, chunk-major (staged re-check)
-    uint32_t gidx[kTcCols], tmeta[kTcCols], tinfo[kTcCols], comp[kTcCols];
-    uint32_t seg_first[kTcCols], seg_start[kTcCols + 1], seg_te[kTcCols];  // one segment per target
-    uint32_t lastmask[kTcCols / 32];
-    uint32_t ntile, ncomp, produced, nseg, last_open;
+enum : uint32_t { kTileFirst = 1u, kTilePassEnd = 2u, kTileUnitEnd = 4u, kTileExit = 8u, kTileFast = 16u };
+
+struct alignas(16) TcTile {
+    uint32_t gidx[kTcCols];                 // filter of each column
+    alignas(16) uint32_t meta[kTcCols];     // its hamming weight << 16 | element count (read four at a time)
+    uint16_t te[kTcCols];                   // its target's place in the unit's run
+    uint32_t e2min[kTcSlices];              // smallest hamming weight of the slice's columns that count
+    uint32_t kmask[kTcSlices];              // columns that count (elements >= 16)
+    uint32_t su[kTcSlices];                 // their element count where it is the same for all, else ~0
+    uint32_t ste[kTcSlices];                // their target's place where it is the same for all, else ~0
+    uint32_t nt, flags, pass, pseq, rc;     // columns, kTile*, pass slot and number, first row of the pass
+    MatUnit unit;
 };
+
+struct TcPass {
+    uint32_t rowf[kTcRows], rowmeta[kTcRows];  // filter of each row (~0: none), its meta word
+    uint32_t gref[kTcRows];                    // reference digests of the unit
+    uint8_t rowk[kTcRows];                     // the row's digest among them
+};
+
+// element-count sums of kTcSumMax and more share one cut: CUTOFFS256[0..3]
+// are equal (4096 / sum <= 3), and CUTOFFS64[0..3] (1024 / sum <= 3)
+constexpr uint32_t kTcSumMax = 1025;
 
 struct TcSmem {
-    uint4 bits[kTcBitSlots][kTcRows + kTcCols];  // 16 filter bytes per row per chunk
-    TcTile tile[2];
-    uint32_t rowf[kTcRows];           // filter index of each reference row (~0: none)
-    double mv[kTcRows][kTcRing + 1];  // row maxima of completed targets (ring)
-    uint16_t cstage[32][kTcRows];     // one 32-column slice of counts, column-major per row thread
-    double run[kMatMaxTargets];
-    uint32_t gref[kTcRows], gstart[kTcRows + 1], gsparse[kTcRows];
-    uint16_t cut_sum[1024], cut64_sum[1024], cut256[SDBF_CUTOFF_BINS], cut64[SDBF_CUTOFF_BINS];
-    MatUnit unit;
-    uint32_t unit_id, cur_t, cur_f, sparse, tmem;
-    alignas(8) uint64_t mbar[5];      // stage 0, stage 1 emptied; accumulator 0, 1 full; drain
+    TcTile tile[kTcRing];
+    TcPass pass[kTcRing];
+    uint32_t cm[kTcMasks][kTcSlices][kTcRows];     // marked columns of each row
+    float thr[kTcSumMax + 1], thr64[kTcSumMax + 1];  // cut by element-count sum
+    uint16_t dense[kTcCheck][kTcDense];     // check: marked pairs (row << 8 | column)
+    uint32_t res[kTcCheck][kTcDense];       // check: their ratios in units of 2^-23 (0: none)
+    uint2 rowbest[kTcRows];                 // a row's open target (pass number << 9 | place) and its maximum so far
+    uint32_t run[kMatMaxTargets];           // sums of the pass per target (one reference digest)
+    unsigned long long run64[kMatMaxTargets];  // and of the unit
+    uint32_t seg_first[kTcCols], seg_start[kTcCols + 1], seg_te[kTcCols];  // compose: one segment per target
+    uint32_t gfirst[kTcRows], gstart[kTcRows + 1];                          // compose: rows of a group
+    uint32_t tmem, fail;
+    alignas(8) uint64_t tile_full[kTcRing], tile_empty[kTcRing], stage_full[2], stage_empty[2], acc_full[2],
+        acc_empty[2], mask_full[kTcMasks], mask_empty[kTcMasks], check_bar, a_free, drain;
 };
 
-static_assert(kTcRows == 128 && kTcCols == 256 && kTcThreads == 256,
-              "producer threads widen one reference row and two target columns each");
-constexpr size_t kTcSmemBytes = 1024 /* alignment */ + 2 * kTcStage + sizeof(TcSmem);
+constexpr size_t kTcSmemBytes = 1024 /* alignment */ + kTcA + 2 * kTcBStage + sizeof(TcSmem);
 static_assert(kTcSmemBytes <= 227 * 1024, "tensor-core kernel exceeds the shared memory of one CTA");
+static_assert(sizeof(TcTile) % 16 == 0 && alignof(TcSmem) >= 16, "meta words are read as uint4");
+static_assert(kTcWiden * 32 == kTcCols, "eight lanes a row, whole rows to a warp");
 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
-__device__ __forceinline__ bool mbar_wait(uint32_t addr, uint32_t parity) {
-    for (uint32_t i = 0; i < kTcWaitSpins; i++) {
+__device__ __forceinline__ void mbar_init(uint64_t* b, uint32_t count) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(b)), "r"(count));
+}
+__device__ __forceinline__ void mbar_arrive(uint64_t* b) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(b)) : "memory");
+}
+// By a whole warp; false: the wait gave up (the limit is about a second).
+// The vote keeps the lanes together: without it they leave the loop one by
+// one and run what follows in parts.
+__device__ __forceinline__ bool mbar_wait(uint64_t* b, uint32_t parity) {
+    const uint32_t addr = smem_addr(b);
+#pragma unroll 1
+    for (uint32_t i = 0; i < kTcSpins; i++) {
         uint32_t done;
         asm volatile(
-            "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
+            "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n selp.u32 %0, 1, 0, p;\n}\n"
             : "=r"(done)
-            : "r"(addr), "r"(parity)
+            : "r"(addr), "r"(parity), "r"(1000u)
             : "memory");
-        if (done) return true;
+        if (__all_sync(0xffffffffu, done)) return true;
     }
     return false;
 }
-
-__device__ __forceinline__ void mma_commit(uint32_t mbar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(mbar)
+// mbar_wait that, when phases are counted (kPhases), adds the cycles waited
+// by the first lane of each of a role's warps (and the warp's other time)
+// when the role ends
+template <bool kPhases>
+struct TcWait {
+    unsigned long long* phase;
+    int what;
+    long long t0 = 0, waited = 0;
+    __device__ __forceinline__ TcWait(unsigned long long* p, int w) : phase(p), what(w) {
+        if constexpr (kPhases) t0 = clock64();
+    }
+    __device__ __forceinline__ bool operator()(uint64_t* b, uint32_t parity) {
+        if constexpr (!kPhases) return mbar_wait(b, parity);
+        const long long a = clock64();
+        const bool ok = mbar_wait(b, parity);
+        waited += clock64() - a;
+        return ok;
+    }
+    __device__ __forceinline__ ~TcWait() {
+        if (kPhases && (threadIdx.x & 31) == 0) {
+            atomicAdd(phase + what, (unsigned long long)(clock64() - t0 - waited));
+            atomicAdd(phase + kTcPhWaits + what, (unsigned long long)waited);
+        }
+    }
+};
+__device__ __forceinline__ void mma_commit(uint64_t* b) {
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_addr(b))
                  : "memory");
 }
 
@@ -115,36 +198,24 @@ __device__ __forceinline__ uint64_t sw128_desc(uint32_t saddr) {
     return d;
 }
 
-// bit k of every byte of w, as 0x08 or 0x00 in that byte
-__device__ __forceinline__ uint32_t bit_to_08(uint32_t w, int k) {
-    return (k <= 3 ? w << (3 - k) : w >> (k - 3)) & 0x08080808u;
-}
-
-// row r's 128 e4m3 bytes of one chunk from its 128 filter bits (4 words):
-// 8 granules of 16 bytes at their swizzled places
-__device__ __forceinline__ void widen_row(uint8_t* stage, uint32_t r, uint4 bits) {
-    const uint32_t w[4] = {bits.x, bits.y, bits.z, bits.w};
-    uint8_t* row = stage + (r >> 3) * 1024 + (r & 7) * 128;
-#pragma unroll
-    for (int m = 0; m < 4; m++) {
-#pragma unroll
-        for (int h = 0; h < 2; h++) {
-            uint4 g;
-            g.x = bit_to_08(w[m], 4 * h + 0);
-            g.y = bit_to_08(w[m], 4 * h + 1);
-            g.z = bit_to_08(w[m], 4 * h + 2);
-            g.w = bit_to_08(w[m], 4 * h + 3);
-            const uint32_t gi = 2 * m + h;
-            *reinterpret_cast<uint4*>(row + ((gi ^ (r & 7)) << 4)) = g;
-        }
+// One filter word as the 16-byte granule q of row r of a chunk, at its
+// swizzled place.
+template <bool kRef>
+__device__ __forceinline__ void widen_word(uint8_t* chunk, uint32_t r, uint32_t q, uint32_t x) {
+    uint4 g;
+    if (kRef) {
+        g.x = (x & 0x11111111u) << 2;
+        g.y = x & 0x22222222u;
+        g.z = (x & 0x44444444u) >> 2;
+        g.w = (x >> 3) & 0x11111111u;
+    } else {
+        g.x = x & 0x11111111u;
+        g.y = x & 0x22222222u;
+        g.z = x & 0x44444444u;
+        g.w = (x >> 1) & 0x44444444u;
     }
+    *reinterpret_cast<uint4*>(chunk + r * 128 + ((q ^ (r & 7)) << 4)) = g;
 }
-
-__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr(dst)), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait2() { asm volatile("cp.async.wait_group 2;" ::: "memory"); }
 
 // slot j of a composed tile: its segment k (seg_start[k] <= j < seg_start[k+1])
 __device__ __forceinline__ uint32_t find_segment(const uint32_t* seg_start, uint32_t nseg, uint32_t j) {
@@ -157,552 +228,775 @@ __device__ __forceinline__ uint32_t find_segment(const uint32_t* seg_start, uint
     return lo;
 }
 
-// the row's first 128 bytes (the staged re-check needs words 0..31)
-struct RowHead {
-    uint4 w[8];
-};
+// barrier of the check warps (bounded, unlike a hardware one); global
+// additions of a thread before it are seen by the others' L2 reads after it
+__device__ __forceinline__ bool check_sync(TcSmem& S, uint32_t lane, uint32_t& phase) {
+    __threadfence();
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&S.check_bar);
+    const bool ok = mbar_wait(&S.check_bar, phase);
+    phase ^= 1u;
+    return ok;
+}
 
-// A pair whose full count is above the cut (rare): the reference's staged
-// exits (normal mode: after 8, 16, 32 words) or its 32-byte stage (fast
-// mode), from the row's first 128 bytes and the target's (shared memory,
-// 16 bytes every kTcCols uint4s).
-// Returns (num << 32) | den of the pair's score (0 / 1 when it scores 0).
-__device__ __forceinline__ uint64_t candidate_fraction(const RowHead& aw, const uint4* tw, uint32_t cnt,
-                                                      uint32_t cut, bool fast, uint32_t max_est) {
-    // all eight loads first, then the three stage counts (an exit at any
-    // stage is an exit: the stages only end the count early)
-    uint32_t p[8];
+// ------------------------------------------------------------- compose
+template <bool kPhases>
+__device__ __forceinline__ void tc_compose(const MatParams& P, TcSmem& S, uint32_t lane) {
+    TcWait<kPhases> twait(P.phase, kTcPhCompose);
+    uint32_t t = 0, pass = 0;  // tiles composed, passes begun
+    uint32_t next = 0;
+    if (lane == 0) next = atomicAdd(P.next_unit, 1u);
+    for (;;) {
+        const uint32_t u = __shfl_sync(0xffffffffu, next, 0);
+        if (u >= P.nunits) {
+            TcTile& T = S.tile[t % kTcRing];
+            if (!twait(&S.tile_empty[t % kTcRing], ((t / kTcRing) & 1) ^ 1)) S.fail = 1;
+            if (lane == 0) {
+                T.flags = kTileExit;
+                T.nt = 0;
+                mbar_arrive(&S.tile_full[t % kTcRing]);
+            }
+            return;
+        }
+        if (lane == 0) next = atomicAdd(P.next_unit, 1u);  // the next unit, while this one is composed
+        const MatUnit U = P.units[u];
+        const uint32_t rs = U.flags & kUnitRefSide1 ? 1 : 0, ts = U.flags & kUnitTgtSide1 ? 1 : 0;
+        const bool split = (U.flags & kUnitSplit) != 0, group = (U.flags & kUnitGroup) != 0;
+        const uint32_t nref = group ? U.nref : 1, nT = U.t1 - U.t0;
+        if (group) {  // first rows of the group's digests
+            uint32_t base = 0;
+            for (uint32_t b = 0; b < nref; b += 32) {
+                const uint32_t k = b + lane;
+                uint32_t n = 0, first = 0;
+                if (k < nref) {
+                    const CmpDigest D = P.digests[rs][P.refs[U.ref + k]];
+                    n = D.nfilters;
+                    first = D.first;
+                }
+                uint32_t incl = n;
 #pragma unroll
-    for (int q = 0; q < 8; q++) {
-        const uint4 y = tw[q * kTcCols];
-        p[q] = __popc(aw.w[q].x & y.x) + __popc(aw.w[q].y & y.y) + __popc(aw.w[q].z & y.z) + __popc(aw.w[q].w & y.w);
+                for (int d = 1; d < 32; d <<= 1) {
+                    const uint32_t v = __shfl_up_sync(0xffffffffu, incl, d);
+                    if (lane >= (uint32_t)d) incl += v;
+                }
+                if (k < nref) {
+                    S.gfirst[k] = first;
+                    S.gstart[k] = base + incl - n;
+                }
+                base += __shfl_sync(0xffffffffu, incl, 31);
+            }
+            if (lane == 0) S.gstart[nref] = base;
+            __syncwarp();
+        }
+        const CmpDigest A = P.digests[rs][group ? P.refs[U.ref] : U.ref];
+        const uint32_t fast = A.flags & kDigestFast ? (uint32_t)kTileFast : 0u;
+        for (uint32_t rc = U.r0; rc < U.r1; rc += kTcRows) {
+            uint32_t ct = 0, cf = split ? U.c0 : 0u;  // target of the run, filter in it
+            uint32_t wb = 0, wn = 0, wfirst = 0;       // 32 targets from wb: filters, first filter
+            auto window = [&]() {
+                wb = ct;
+                wn = 0;
+                if (wb + lane < nT) {
+                    const CmpDigest B = P.digests[ts][P.targets[U.t0 + wb + lane]];
+                    wn = split ? U.c1 : B.nfilters;
+                    wfirst = B.first;
+                }
+            };
+            window();
+            bool first = true;
+            while (ct < nT) {
+                const uint32_t slot = t % kTcRing;
+                TcTile& T = S.tile[slot];
+                if (!twait(&S.tile_empty[slot], ((t / kTcRing) & 1) ^ 1)) {
+                    S.fail = 1;
+                    return;
+                }
+                if (first) {  // the rows of the pass (its slot was released with the tile's)
+                    TcPass& R = S.pass[pass % kTcRing];
+                    const uint32_t rows = U.r1 - rc;
+#pragma unroll
+                    for (uint32_t i = 0; i < kTcRows / 32; i++) {
+                        const uint32_t row = 32 * i + lane;
+                        uint32_t f = 0xFFFFFFFFu, m = 0, k = 0;
+                        if (row < rows) {
+                            if (group) {
+                                k = find_segment(S.gstart, nref, row);
+                                f = S.gfirst[k] + (row - S.gstart[k]);
+                            } else {
+                                f = A.first + rc + row;
+                            }
+                            m = P.meta[rs][f];
+                        }
+                        R.rowf[row] = f;
+                        R.rowmeta[row] = m;
+                        R.rowk[row] = (uint8_t)k;
+                        if (row < nref) R.gref[row] = group ? P.refs[U.ref + row] : U.ref;
+                    }
+                }
+                // targets from (ct, cf) on, up to kTcCols filters
+                uint32_t filled = 0, nseg = 0;
+                while (filled < kTcCols && ct < nT) {
+                    if (ct >= wb + 32) window();
+                    const uint32_t te = wb + lane;
+                    const uint32_t f0 = te == ct ? cf : 0u;
+                    const uint32_t rem = te >= ct && te < nT ? wn - f0 : 0u;
+                    uint32_t incl = rem;
+#pragma unroll
+                    for (int d = 1; d < 32; d <<= 1) {
+                        const uint32_t v = __shfl_up_sync(0xffffffffu, incl, d);
+                        if (lane >= (uint32_t)d) incl += v;
+                    }
+                    const uint32_t excl = incl - rem, room = kTcCols - filled;
+                    const bool has = rem > 0 && excl < room;
+                    const uint32_t has_mask = __ballot_sync(0xffffffffu, has);
+                    if (has) {
+                        const uint32_t k = nseg + __popc(has_mask & ((1u << lane) - 1u));
+                        S.seg_first[k] = wfirst + f0;
+                        S.seg_start[k] = filled + excl;
+                        S.seg_te[k] = te;
+                    }
+                    nseg += __popc(has_mask);
+                    const uint32_t over = __ballot_sync(0xffffffffu, rem > 0 && incl > room);
+                    if (over) {  // the first target that does not fit (any more)
+                        const uint32_t l = __ffs(over) - 1;
+                        const uint32_t ex_l = __shfl_sync(0xffffffffu, excl, l), f0_l = __shfl_sync(0xffffffffu, f0, l);
+                        ct = wb + l;
+                        cf = f0_l + (room - ex_l);
+                        filled = kTcCols;
+                    } else {
+                        filled += __shfl_sync(0xffffffffu, incl, 31);
+                        ct = min(wb + 32u, nT);
+                        cf = 0;
+                    }
+                }
+                if (lane == 0) S.seg_start[nseg] = filled;
+                __syncwarp();
+                uint32_t mj[kTcSlices];
+#pragma unroll 1
+                for (uint32_t j = lane; j < kTcCols; j += 32) {
+                    uint32_t f = 0, te = 0;
+                    if (j < filled) {
+                        const uint32_t k = find_segment(S.seg_start, nseg, j);
+                        f = S.seg_first[k] + (j - S.seg_start[k]);
+                        te = S.seg_te[k];
+                    }
+                    T.gidx[j] = f;
+                    T.te[j] = (uint16_t)te;
+                }
+#pragma unroll
+                for (uint32_t i = 0; i < kTcSlices; i++)  // (each lane reads what it wrote)
+                    mj[i] = 32 * i + lane < filled ? P.meta[ts][T.gidx[32 * i + lane]] : 0u;
+#pragma unroll
+                for (uint32_t i = 0; i < kTcSlices; i++) T.meta[32 * i + lane] = mj[i];
+#pragma unroll 1
+                for (uint32_t i = 0; i < kTcSlices; i++) {
+                    const uint32_t j = 32 * i + lane, m = T.meta[j], te = T.te[j];
+                    const uint32_t e = m & 0xFFFFu, s2 = min(e, kTcSumMax);
+                    const bool counts = j < filled && e >= (uint32_t)kMinElem;
+                    const uint32_t km = __ballot_sync(0xffffffffu, counts);
+                    const uint32_t lo = __reduce_min_sync(0xffffffffu, counts ? s2 : 0xFFFFu);
+                    const uint32_t hi = __reduce_max_sync(0xffffffffu, counts ? s2 : 0u);
+                    const uint32_t tlo = __reduce_min_sync(0xffffffffu, counts ? te : 0xFFFFu);
+                    const uint32_t thi = __reduce_max_sync(0xffffffffu, counts ? te : 0u);
+                    const uint32_t em = __reduce_min_sync(0xffffffffu, counts ? m >> 16 : 0xFFFFu);
+                    if (lane == 0) {
+                        T.kmask[i] = km;
+                        T.su[i] = lo == hi ? lo : 0xFFFFFFFFu;
+                        T.ste[i] = tlo == thi ? tlo : 0xFFFFFFFFu;
+                        T.e2min[i] = em;
+                    }
+                }
+                if (lane == 0) {
+                    const bool pass_end = ct >= nT;
+                    T.nt = filled;
+                    T.pass = pass % kTcRing;
+                    T.pseq = pass & 0x3FFFFFu;
+                    T.rc = rc;
+                    T.unit = U;
+                    T.flags = fast | (first ? (uint32_t)kTileFirst : 0u) | (pass_end ? (uint32_t)kTilePassEnd : 0u) |
+                              (pass_end && rc + kTcRows >= U.r1 ? (uint32_t)kTileUnitEnd : 0u);
+                }
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&S.tile_full[slot]);
+                first = false;
+                t++;
+            }
+            pass++;
+        }
     }
-    const uint32_t c1 = p[0] + p[1], c2 = c1 + p[2] + p[3], c3 = c2 + p[4] + p[5] + p[6] + p[7];
-    const bool exit = fast ? 2 * c1 + 48 < cut : (8 * c1 + 48 < cut || 4 * c2 + 48 < cut || 2 * c3 + 48 < cut);
-    if (exit || cnt <= cut) return 1;
-    return ((uint64_t)(cnt - cut) << 32) | (uint32_t)(max_est - cut);
 }
 
-// A row's maximum over a completed target (max_value), with the division
-// of the rare positive score out of line.
-__device__ __noinline__ double score_ratio(uint32_t bnum, uint32_t bden) { return __ddiv_rn((double)bnum, (double)bden); }
-
-__device__ __forceinline__ double row_maximum(bool active, uint32_t bnum, uint32_t bden, bool counted) {
-    if (!active) return 0.0;
-    if (!counted) return -1.0;
-    return bnum == 0 ? 0.0 : score_ratio(bnum, bden);
+// a read-only load that stays where it is written: the compiler moves a
+// plain one down to its use, behind the waits it is to overlap with
+__device__ __forceinline__ uint4 ldg_here(const uint4* p) {
+    uint4 v;
+    asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    return v;
 }
 
-// Sums the maxima of `done` completed targets (completion indices from
-// ring_base) in filter order: group units finish their (reference, target)
-// scores, multi-pass units extend the running sums.  All 128 consumer threads.
-__device__ __noinline__ void fold_ring(const MatParams& P, TcSmem& S, const TcTile& T, uint32_t ring_base,
-                                       uint32_t done, bool group, uint32_t nref, uint32_t nrows, uint32_t t0,
-                                       uint32_t rs, uint32_t tid) {
-    asm volatile("bar.sync 1, 128;" ::: "memory");
-    if (group) {
-        for (uint32_t t = tid; t < done * nref; t += 128) {
-            const uint32_t kk = t % nref, ci = ring_base + t / nref;
-            double sum = -1.0;
-            for (uint32_t r = S.gstart[kk]; r < S.gstart[kk + 1]; r++) {
-                const double m = S.mv[r][ci % kTcRing];
-                if (sum < 0) sum = m;
-                else if (m != 0.0) sum = __dadd_rn(sum, m);
+// --------------------------------------------------------------- widen
+// A warp load takes 128 bytes of four rows (eight lanes a row, four words a
+// lane: one "block" of four chunks), four cache lines instead of the sixteen
+// that 32-byte pieces of sixteen rows touch; chunk j of the block is word j of every
+// lane.  The order of the words in K is the same for both operands.
+template <bool kPhases>
+__device__ __forceinline__ void tc_widen(const MatParams& P, TcSmem& S, uint8_t* a_smem, uint8_t* b_smem, uint32_t wt,
+                                         uint32_t lane) {
+    TcWait<kPhases> twait(P.phase, kTcPhWiden);
+    const uint32_t g = wt & 7, r0 = wt >> 3;  // lane g of rows r0 + 24 k
+    constexpr uint32_t kRowStep = kTcWiden * 4, kRows = kTcCols / kRowStep;
+    const uint4 z = make_uint4(0, 0, 0, 0);
+    uint32_t pass = 0, q = 0;  // passes widened, chunks widened
+    uint4 x[kRows], y[kRows];  // this block's words, the next block's
+    uint32_t pt = 0, pb = 0;   // the next block: block pb of tile pt
+    bool more = true, ok = true;
+    auto fetch = [&]() {
+#pragma unroll
+        for (uint32_t k = 0; k < kRows; k++) y[k] = z;
+        if (!more) return;
+        const TcTile& T = S.tile[pt % kTcRing];
+        if (pb == 0) {
+            if (!twait(&S.tile_full[pt % kTcRing], (pt / kTcRing) & 1)) {
+                ok = more = false;
+                return;
             }
-            const uint32_t tgt = P.targets[t0 + T.comp[ci]];
-            P.scores[out_index(P, rs != 0, S.gref[kk], tgt)] =
-                final_score(sum, S.gstart[kk + 1] - S.gstart[kk], S.gsparse[kk]);
+            if (T.flags & kTileExit) {
+                more = false;
+                return;
+            }
         }
-    } else {
-        for (uint32_t t = tid; t < done; t += 128) {
-            const uint32_t ci = ring_base + t;
-            double sum = S.run[T.comp[ci]];
-            for (uint32_t r = 0; r < nrows; r++) {
-                const double m = S.mv[r][ci % kTcRing];
-                if (sum < 0) sum = m;
-                else if (m != 0.0) sum = __dadd_rn(sum, m);
+        const uint32_t* f = P.filters[T.unit.flags & kUnitTgtSide1 ? 1 : 0];
+#pragma unroll
+        for (uint32_t k = 0; k < kRows; k++)
+            if (r0 + kRowStep * k < T.nt)
+                y[k] = ldg_here(reinterpret_cast<const uint4*>(f + (size_t)T.gidx[r0 + kRowStep * k] * 64) + 8 * pb + g);
+        if (++pb == (T.flags & kTileFast ? 1u : 2u)) {
+            pb = 0;
+            pt++;
+        }
+    };
+    fetch();
+    uint32_t t = 0, blk = 0;
+    // one copy of the loop's code: five roles share the instruction cache
+#pragma unroll 1
+    while (ok) {
+        const uint32_t slot = t % kTcRing;
+        const TcTile& T = S.tile[slot];
+        // (its descriptor has arrived: the fetch position is past it or at the exit)
+        if (T.flags & kTileExit) return;
+        const uint32_t ncols = (T.nt + 15) & ~15u, nblk = T.flags & kTileFast ? 1u : 2u;
+        if (blk == 0 && (T.flags & kTileFirst)) {  // the pass's reference rows
+            if (pass > 0 && !twait(&S.a_free, (pass - 1) & 1)) break;
+            const TcPass& R = S.pass[T.pass];
+            const uint32_t* f = P.filters[T.unit.flags & kUnitRefSide1 ? 1 : 0];
+#pragma unroll 1
+            for (uint32_t i0 = wt; i0 < kTcRows * 8 * nblk; i0 += 4 * kTcWiden * 32) {
+                uint4 v[4];
+#pragma unroll
+                for (uint32_t k = 0; k < 4; k++) {  // lane g of row (i >> 3) & 127, block i >> 10
+                    const uint32_t i = i0 + k * kTcWiden * 32;
+                    v[k] = z;
+                    if (i < kTcRows * 8 * nblk) {
+                        const uint32_t fr = R.rowf[(i >> 3) & (kTcRows - 1)];
+                        // fast mode counts the first 16 words: four lanes
+                        if (fr != 0xFFFFFFFFu && (nblk == 2 || g < 4))
+                            v[k] = __ldg(reinterpret_cast<const uint4*>(f + (size_t)fr * 64) + 8 * (i >> 10) + g);
+                    }
+                }
+#pragma unroll
+                for (uint32_t k = 0; k < 4; k++) {
+                    const uint32_t i = i0 + k * kTcWiden * 32;
+                    if (i < kTcRows * 8 * nblk) {
+                        uint8_t* a = a_smem + 4 * (i >> 10) * kTcAChunk;
+                        const uint32_t r = (i >> 3) & (kTcRows - 1);
+                        widen_word<true>(a, r, g, v[k].x);
+                        widen_word<true>(a + kTcAChunk, r, g, v[k].y);
+                        widen_word<true>(a + 2 * kTcAChunk, r, g, v[k].z);
+                        widen_word<true>(a + 3 * kTcAChunk, r, g, v[k].w);
+                    }
+                }
             }
-            S.run[T.comp[ci]] = sum;
+            pass++;
+        }
+#pragma unroll
+        for (uint32_t k = 0; k < kRows; k++) x[k] = y[k];
+        fetch();
+#pragma unroll 1
+        for (uint32_t j = 0; j < 4 && ok; j++, q++) {
+            const uint32_t s = q & 1;
+            ok = twait(&S.stage_empty[s], ((q >> 1) & 1) ^ 1);
+            uint8_t* sb = b_smem + s * kTcBStage;
+#pragma unroll
+            for (uint32_t k = 0; k < kRows; k++) {
+                const uint32_t r = r0 + kRowStep * k;
+                if (r < ncols) widen_word<false>(sb, r, g, x[k].x);
+                x[k].x = x[k].y;
+                x[k].y = x[k].z;
+                x[k].z = x[k].w;
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&S.stage_full[s]);
+        }
+        if (++blk == nblk) {
+            blk = 0;
+            if (lane == 0) mbar_arrive(&S.tile_empty[slot]);
+            t++;
         }
     }
-    asm volatile("bar.sync 1, 128;" ::: "memory");
+    S.fail = 1;
+}
+
+// ----------------------------------------------------------------- mma
+template <bool kPhases>
+__device__ __forceinline__ void tc_mma(const MatParams& P, TcSmem& S, uint32_t a_addr, uint32_t b_addr, uint32_t tmem, uint32_t lane) {
+    TcWait<kPhases> twait(P.phase, kTcPhMma);
+    uint32_t q = 0;
+    for (uint32_t t = 0;; t++) {
+        const uint32_t slot = t % kTcRing, b = t & 1;
+        bool ok = twait(&S.tile_full[slot], (t / kTcRing) & 1);
+        const TcTile& T = S.tile[slot];
+        if (ok && (T.flags & kTileExit)) return;
+        ok = ok && twait(&S.acc_empty[b], ((t >> 1) & 1) ^ 1);
+        if (!ok) {
+            S.fail = 1;
+            return;
+        }
+        asm volatile("tcgen05.fence::after_thread_sync;");
+        const uint32_t nch = T.flags & kTileFast ? 4u : kTcChunks, ncols = (T.nt + 15) & ~15u;
+        const bool pass_end = (T.flags & kTilePassEnd) != 0;
+        if (kPhases && lane == 0) atomicAdd(P.phase + kTcPhTiles, 1ull);
+        // kind::mxf4: both operands e2m1 (1), N / 8, ue8m0 scales, M / 16, K = 64
+        const uint32_t idesc = (1u << 7) | (1u << 10) | ((ncols >> 3) << 17) | (1u << 23) | ((kTcRows >> 4) << 24);
+        const uint32_t dacc = tmem + b * kTcCols;
+        for (uint32_t c = 0; c < nch; c++, q++) {
+            const uint32_t s = q & 1;
+            if (!twait(&S.stage_full[s], (q >> 1) & 1)) {
+                S.fail = 1;
+                return;
+            }
+            if (lane == 0) {
+                // the widening warps' writes, seen through the barrier, become
+                // visible to the tensor core here: a fence in those warps
+                // would wait for their loads in flight
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                asm volatile("tcgen05.fence::after_thread_sync;");
+                const uint32_t a0 = a_addr + c * kTcAChunk, b0 = b_addr + s * kTcBStage;
+#pragma unroll
+                for (uint32_t kk = 0; kk < 4; kk++) {
+                    const uint64_t ad = sw128_desc(a0 + kk * 32), bd = sw128_desc(b0 + kk * 32);
+                    const uint32_t acc = (c > 0 || kk > 0) ? 1u : 0u;
+                    asm volatile(
+                        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+                        " tcgen05.mma.cta_group::1.kind::mxf4.block_scale.scale_vec::2X [%0], %1, %2, %3, [%5], [%6], p;\n}\n" ::"r"(
+                            dacc),
+                        "l"(ad), "l"(bd), "r"(idesc), "r"(acc), "r"(tmem + kTcScaleCol), "r"(tmem + kTcScaleCol + kTcScaleCols / 2));
+                }
+                mma_commit(&S.stage_empty[s]);
+                if (c + 1 == nch) {
+                    mma_commit(&S.acc_full[b]);
+                    if (pass_end) mma_commit(&S.a_free);
+                }
+            }
+            __syncwarp();
+        }
+        if (lane == 0) mbar_arrive(&S.tile_empty[slot]);
+    }
+}
+
+// ---------------------------------------------------------------- mark
+__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,"
+        "%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
+        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
+          "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]),
+          "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]),
+          "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
+        : "r"(taddr));
+}
+// the loads' registers pass through the wait, so that no use moves before it
+__device__ __forceinline__ void tmem_ld_wait(uint32_t (&v)[32]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]), "+r"(v[6]), "+r"(v[7]),
+                   "+r"(v[8]), "+r"(v[9]), "+r"(v[10]), "+r"(v[11]), "+r"(v[12]), "+r"(v[13]), "+r"(v[14]), "+r"(v[15])
+                 :
+                 : "memory");
+    asm volatile("" : "+r"(v[16]), "+r"(v[17]), "+r"(v[18]), "+r"(v[19]), "+r"(v[20]), "+r"(v[21]), "+r"(v[22]),
+                 "+r"(v[23]), "+r"(v[24]), "+r"(v[25]), "+r"(v[26]), "+r"(v[27]), "+r"(v[28]), "+r"(v[29]), "+r"(v[30]),
+                 "+r"(v[31]));
+}
+template <bool kPhases>
+__device__ __forceinline__ void tc_mark(const MatParams& P, TcSmem& S, uint32_t tmem, uint32_t warp, uint32_t lane) {
+    TcWait<kPhases> twait(P.phase, kTcPhMark);
+    const uint32_t row = warp * 32 + lane;
+    uint32_t s1 = 0, e1 = 0;
+    bool active = false;
+    for (uint32_t t = 0;; t++) {
+        const uint32_t slot = t % kTcRing, b = t & 1;
+        bool ok = twait(&S.tile_full[slot], (t / kTcRing) & 1);
+        const TcTile& T = S.tile[slot];
+        if (ok && (T.flags & kTileExit)) return;
+        const uint32_t mb = t % kTcMasks;
+        ok = ok && twait(&S.mask_empty[mb], ((t / kTcMasks) & 1) ^ 1) && twait(&S.acc_full[b], (t >> 1) & 1);
+        if (!ok) {
+            S.fail = 1;
+            return;
+        }
+        if (T.flags & kTileFirst) {
+            const uint32_t m = S.pass[T.pass].rowmeta[row] & 0xFFFFu;
+            active = m >= (uint32_t)kMinElem;
+            s1 = min(m, kTcSumMax);
+            e1 = S.pass[T.pass].rowmeta[row] >> 16;
+        }
+        asm volatile("tcgen05.fence::after_thread_sync;");
+        const float* thr = T.flags & kTileFast ? S.thr64 : S.thr;
+        const uint32_t nsl = (T.nt + 31) / 32;
+        const uint2 rb = S.rowbest[row];
+        const uint32_t tacc = tmem + ((warp * 32) << 16) + b * kTcCols;
+        // columns of slice i above the cut: the sign of cut - count, four
+        // chains of eight columns.  A row that has a maximum r of the
+        // slice's target already only improves on it where
+        // count - cut > r (weight - cut), weight the smaller hamming weight of the pair.
+        auto slice = [&](uint32_t i, const uint32_t (&v)[32]) {
+            const uint32_t km = T.kmask[i], su = T.su[i];
+            uint32_t m[4] = {0, 0, 0, 0};
+            if (km != 0) {
+                float r = 0.0f;
+                if (rb.x == (T.pseq << 9 | T.ste[i])) r = fmaxf((float)rb.y - 8.0f, 0.0f) * (1.0f / 8388608.0f);
+                const float keep = 1.0f - r, fe1 = (float)e1;
+                if (su != 0xFFFFFFFFu) {
+                    float cut = thr[min(s1 + su, kTcSumMax)];
+                    cut = fmaxf(cut, fmaf(cut, keep, r * fminf(fe1, (float)T.e2min[i]) - 0.0625f));
+#pragma unroll
+                    for (int q = 7; q >= 0; q--)
+#pragma unroll
+                        for (int z = 0; z < 4; z++)
+                            m[z] = __funnelshift_l(__float_as_uint(cut - __uint_as_float(v[8 * z + q])), m[z], 1);
+                } else {
+                    const uint4* m4 = reinterpret_cast<const uint4*>(&T.meta[32 * i]);
+#pragma unroll
+                    for (int z = 0; z < 4; z++) {
+                        const uint4 w = m4[2 * z], x = m4[2 * z + 1];
+                        const uint32_t mt[8] = {w.x, w.y, w.z, w.w, x.x, x.y, x.z, x.w};
+#pragma unroll
+                        for (int q = 7; q >= 0; q--) {
+                            float cut = thr[min(s1 + (mt[q] & 0xFFFFu), kTcSumMax)];
+                            const float we = fminf(fe1, (float)(mt[q] >> 16));
+                            cut = fmaxf(cut, fmaf(cut, keep, fmaf(r, we, -0.0625f)));
+                            m[z] = __funnelshift_l(__float_as_uint(cut - __uint_as_float(v[8 * z + q])), m[z], 1);
+                        }
+                    }
+                }
+            }
+            S.cm[mb][i][row] = active ? (m[0] | m[1] << 8 | m[2] << 16 | m[3] << 24) & km : 0u;
+        };
+#pragma unroll 1
+        for (uint32_t i = 0; i < nsl; i++) {
+            uint32_t v[32];
+            tmem_ld32(tacc + 32 * i, v);
+            tmem_ld_wait(v);
+            slice(i, v);
+        }
+        for (uint32_t i = nsl; i < kTcSlices; i++) S.cm[mb][i][row] = 0;
+        asm volatile("tcgen05.fence::before_thread_sync;");
+        __syncwarp();
+        if (lane == 0) {
+            mbar_arrive(&S.acc_empty[b]);
+            mbar_arrive(&S.mask_full[mb]);
+            mbar_arrive(&S.tile_empty[slot]);
+        }
+    }
+}
+
+// --------------------------------------------------------------- check
+template <bool kPhases>
+__device__ __forceinline__ void tc_check(const MatParams& P, TcSmem& S, uint32_t cw, uint32_t lane) {
+    TcWait<kPhases> twait(P.phase, kTcPhCheck);
+    const uint32_t half = lane >> 4, row = cw * 16 + (lane & 15);  // slices 3 half .. 3 half + 2 of the row
+    const uint32_t ct = cw * 32 + lane;                            // thread of the role
+    const uint32_t sub = lane & 7, grp = lane >> 3;
+    uint16_t* dense = S.dense[cw];
+    uint32_t* res = S.res[cw];
+    uint32_t phase = 0;
+    uint32_t cur_te = 0xFFFFFFFFu, best = 0;  // lanes 0..15: the row's open target and its maximum so far
+#pragma unroll 1
+    for (uint32_t t = 0;; t++) {
+        const uint32_t slot = t % kTcRing, b = t % kTcMasks;
+        bool ok = twait(&S.tile_full[slot], (t / kTcRing) & 1);
+        const TcTile& T = S.tile[slot];
+        if (ok && (T.flags & kTileExit)) return;
+        ok = ok && twait(&S.mask_full[b], (t / kTcMasks) & 1);
+        if (!ok) break;
+        uint32_t m[3];
+#pragma unroll
+        for (int k = 0; k < 3; k++) m[k] = S.cm[b][3 * half + k][row];
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&S.mask_empty[b]);
+        const uint32_t n = __popc(m[0]) + __popc(m[1]) + __popc(m[2]);
+        uint32_t incl = n;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, incl, d);
+            if (lane >= (uint32_t)d) incl += y;
+        }
+        const uint32_t off = incl - n, total = __shfl_sync(0xffffffffu, incl, 31);
+        const TcPass& R = S.pass[T.pass];
+        const uint32_t uflags = T.unit.flags;
+        const uint32_t rs = uflags & kUnitRefSide1 ? 1 : 0, ts = uflags & kUnitTgtSide1 ? 1 : 0;
+        const bool split = (uflags & kUnitSplit) != 0, fast = (T.flags & kTileFast) != 0;
+        const uint32_t nref = uflags & kUnitGroup ? T.unit.nref : 1u;
+        if (T.flags & kTileFirst) {
+            cur_te = 0xFFFFFFFFu;
+            best = 0;
+            if (half == 0) S.rowbest[row] = make_uint2(0xFFFFFFFFu, 0);
+        }
+        const uint32_t* __restrict__ fr = P.filters[rs];
+        const uint32_t* __restrict__ ft = P.filters[ts];
+        const float* thr = fast ? S.thr64 : S.thr;
+        if (kPhases && lane == 0) atomicAdd(P.phase + kTcPhMarked, (unsigned long long)total);
+        // the warp's marked pairs in one list: by lane (a row's first half
+        // before its second), then column; kTcDense of them at a time
+#pragma unroll 1
+        for (uint32_t base = 0; base < total; base += kTcDense) {
+            const uint32_t lim = min(total - base, kTcDense);
+#pragma unroll 1
+            for (uint32_t k = 0, i = off - base; k < n; k++, i++) {  // (i wraps below the round)
+                uint32_t col = 96 * half, mm[3] = {m[0], m[1], m[2]};
+                if (i >= lim) {
+                    if ((int32_t)i >= 0) break;  // past the round
+                    continue;                    // taken in an earlier one
+                }
+                if (mm[0]) {
+                    col += __ffs(mm[0]) - 1;
+                    m[0] &= m[0] - 1u;
+                } else if (mm[1]) {
+                    col += 32 + __ffs(mm[1]) - 1;
+                    m[1] &= m[1] - 1u;
+                } else {
+                    col += 64 + __ffs(mm[2]) - 1;
+                    m[2] &= m[2] - 1u;
+                }
+                dense[i] = (uint16_t)(row << 8 | col);
+            }
+            __syncwarp();
+            constexpr uint32_t kSteps = 3;  // pairs in flight per eight lanes
+#pragma unroll 1
+            for (uint32_t i0 = 0; i0 < lim; i0 += 4 * kSteps) {
+                uint4 x[kSteps][2], y[kSteps][2];
+                uint32_t e[kSteps];
+#pragma unroll
+                for (uint32_t s = 0; s < kSteps; s++) {  // (past the end: the last pair again)
+                    e[s] = dense[min(i0 + 4 * s + grp, lim - 1)];
+                    const uint4* a = reinterpret_cast<const uint4*>(fr + (size_t)R.rowf[e[s] >> 8] * 64) + sub;
+                    const uint4* c = reinterpret_cast<const uint4*>(ft + (size_t)T.gidx[e[s] & 0xFFu] * 64) + sub;
+                    x[s][0] = __ldg(a);
+                    x[s][1] = __ldg(a + 8);
+                    y[s][0] = __ldg(c);
+                    y[s][1] = __ldg(c + 8);
+                }
+                uint32_t pk0 = 0, pk1 = 0, ee = 0;  // lane sub < kSteps: step sub's counts (packed) and pair
+#pragma unroll
+                for (uint32_t s = 0; s < kSteps; s++) {
+                    uint32_t p[2];
+#pragma unroll
+                    for (int z = 0; z < 2; z++)
+                        p[z] = __popc(x[s][z].x & y[s][z].x) + __popc(x[s][z].y & y[s][z].y) +
+                               __popc(x[s][z].z & y[s][z].z) + __popc(x[s][z].w & y[s][z].w);
+                    // first of the eight lanes: counts of the first 8, 16 and
+                    // 32 words, and above them those of the words 32 later
+                    uint32_t c = p[0] | p[1] << 16;
+                    const uint32_t c1 = c + __shfl_xor_sync(0xffffffffu, c, 1);
+                    const uint32_t c2 = c1 + __shfl_xor_sync(0xffffffffu, c1, 2);
+                    const uint32_t c3 = c2 + __shfl_xor_sync(0xffffffffu, c2, 4);
+                    const uint32_t k0 = __shfl_sync(0xffffffffu, (c1 & 0xFFFFu) | c2 << 16, lane & 24);
+                    const uint32_t k1 = __shfl_sync(0xffffffffu, c3, lane & 24);
+                    if (sub == s) {
+                        pk0 = k0;
+                        pk1 = k1;
+                        ee = e[s];
+                    }
+                }
+                const uint32_t i = i0 + 4 * sub + grp;
+                if (sub < kSteps && i < lim) {
+                    const uint32_t p = pk0 & 0xFFFFu, p1 = pk0 >> 16, p2 = pk1 & 0xFFFFu, p3 = p2 + (pk1 >> 16);
+                    const uint32_t mr = R.rowmeta[ee >> 8], mc = T.meta[ee & 0xFFu];
+                    const uint32_t cut = (uint32_t)thr[min(min(mr & 0xFFFFu, kTcSumMax) + min(mc & 0xFFFFu, kTcSumMax), kTcSumMax)];
+                    const uint32_t cnt = fast ? p1 : p3;
+                    const bool out = fast ? 2 * p + 48 < cut : (8 * p + 48 < cut || 4 * p1 + 48 < cut || 2 * p2 + 48 < cut);
+                    uint32_t r = 0;
+                    if (!out && cnt > cut) {
+                        const uint32_t num = cnt - cut, den = min(mr >> 16, mc >> 16) - cut;
+                        // within two units of 2^-23 of num / den (two ulps of the quotient, rounding)
+                        r = num <= den ? (uint32_t)(__fdividef((float)num, (float)den) * 8388608.0f + 0.5f) : 0xFFFFFFFFu;
+                    }
+                    res[i] = r;
+                }
+            }
+            __syncwarp();
+            // the rows' maxima: lane < 16 takes its own entries of the round,
+            // then those of its row's second half
+            const uint32_t lo = min(max((int32_t)(off - base), 0), (int32_t)lim), hi = min(max((int32_t)(off + n - base), 0), (int32_t)lim);
+            const uint32_t lo2 = __shfl_down_sync(0xffffffffu, lo, 16), hi2 = __shfl_down_sync(0xffffffffu, hi, 16);
+            if (half == 0) {
+                const uint32_t n1 = hi - lo, nn = n1 + (hi2 - lo2);
+                const uint32_t was = best, was_te = cur_te;
+                for (uint32_t k = 0; k < nn; k++) {
+                    const uint32_t i = k < n1 ? lo + k : lo2 + (k - n1);
+                    const uint32_t r = res[i];
+                    if (r == 0) continue;
+                    const uint32_t te = T.te[dense[i] & 0xFFu];
+                    if (te != cur_te) {
+                        cur_te = te;
+                        best = 0;
+                    }
+                    if (r <= best) continue;
+                    // the sum grows by what the maximum grows
+                    if (split) {
+                        atomicMax(reinterpret_cast<uint32_t*>(P.slots) + P.split[T.unit.split].slot_base + T.rc + row, r);
+                    } else {
+                        uint32_t* sum;
+                        if (nref == 1) sum = &S.run[te];
+                        else
+                            sum = reinterpret_cast<uint32_t*>(P.scores) +
+                                  out_index(P, rs != 0, R.gref[R.rowk[row]], P.targets[T.unit.t0 + te]);
+                        if (r == 0xFFFFFFFFu) atomicOr(sum, 0x80000000u);  // left to k_matrix_finish
+                        else atomicAdd(sum, r - best);
+                    }
+                    best = r;
+                }
+                // what the mark warps may raise the row's cuts by
+                if (best != was || cur_te != was_te) S.rowbest[row] = make_uint2(T.pseq << 9 | cur_te, best);
+            }
+            __syncwarp();
+        }
+        if (!split && (T.flags & kTilePassEnd)) {
+            const uint32_t nT = T.unit.t1 - T.unit.t0;
+            if (!check_sync(S, lane, phase)) break;
+            if (nref == 1)
+                for (uint32_t k = ct; k < nT; k += kTcCheck * 32) {
+                    const uint32_t v = S.run[k];
+                    S.run[k] = 0;
+                    S.run64[k] = (S.run64[k] + (v & 0x7FFFFFFFu)) | ((unsigned long long)(v >> 31) << 63);
+                }
+            if (T.flags & kTileUnitEnd) {
+                for (uint32_t k = ct; k < nref * nT; k += kTcCheck * 32) {
+                    const uint32_t g = k % nref, te = k / nref;
+                    const uint32_t ref = R.gref[g], tgt = P.targets[T.unit.t0 + te];
+                    const uint64_t o = out_index(P, rs != 0, ref, tgt);
+                    unsigned long long sum;
+                    if (nref == 1) {
+                        sum = S.run64[te];
+                        S.run64[te] = 0;
+                    } else {
+                        const uint32_t v = (uint32_t)__ldcg(P.scores + o);
+                        sum = (v & 0x7FFFFFFFu) | ((unsigned long long)(v >> 31) << 63);
+                    }
+                    P.scores[o] = fixed_score(P, rs, ref, ts, tgt, sum);
+                }
+            }
+            if (!check_sync(S, lane, phase)) break;
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&S.tile_empty[slot]);
+    }
+    S.fail = 1;
 }
 
 }  // namespace
 
-// AND-reduction of a predicate over one 128-thread group (named barrier id)
-template <int ID>
-__device__ __forceinline__ bool group_and(bool v) {
-    uint32_t r;
-    asm volatile("{\n .reg .pred p, q;\n setp.ne.u32 p, %1, 0;\n bar.red.and.pred q, %2, 128, p;\n"
-                 " selp.u32 %0, 1, 0, q;\n}\n"
-                 : "=r"(r)
-                 : "r"((uint32_t)v), "n"(ID)
-                 : "memory");
-    return r != 0;
-}
-
-template <int ID>
-__device__ __forceinline__ void group_sync() {
-    asm volatile("bar.sync %0, 128;" ::"n"(ID) : "memory");
-}
-
-#define TC_STAMP(var) const long long var = P.phase ? clock64() : 0
-#define TC_ADD(ph, t0) \
-    do { if (P.phase) atomicAdd(P.phase + (ph), (unsigned long long)(clock64() - (t0))); } while (0)
-
+template <bool kPhases>
 __global__ void __launch_bounds__(kTcThreads, 1) k_matrix_tc(MatParams P) {
     extern __shared__ uint8_t tc_smem_raw[];
     const uint32_t raw = smem_addr(tc_smem_raw);
-    uint8_t* stages = tc_smem_raw + (((raw + 1023) & ~1023u) - raw);
-    TcSmem& S = *reinterpret_cast<TcSmem*>(stages + 2 * kTcStage);
+    uint8_t* a_smem = tc_smem_raw + (((raw + 1023) & ~1023u) - raw);
+    uint8_t* b_smem = a_smem + kTcA;
+    TcSmem& S = *reinterpret_cast<TcSmem*>(b_smem + 2 * kTcBStage);
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const bool producer = warp >= 4;
-    const uint32_t ptid = tid - 128;  // producers: 0..127
 
-    for (uint32_t i = tid; i < 1024; i += kTcThreads) {
-        S.cut_sum[i] = P.cutoffs[i >= 32 ? 4096u / i : (uint32_t)SDBF_CUTOFF_BINS - 1];
-        S.cut64_sum[i] = P.cutoffs64[i >= 8 ? 1024u / i : (uint32_t)SDBF_CUTOFF_BINS - 1];
+    for (uint32_t i = tid; i <= kTcSumMax; i += kTcThreads) {
+        // below 32 (8) the quotient is past the tables' end, as in the reference's last bin
+        S.thr[i] = (float)P.cutoffs[i >= 32 ? min(4096u / i, (uint32_t)SDBF_CUTOFF_BINS - 1) : (uint32_t)SDBF_CUTOFF_BINS - 1];
+        S.thr64[i] = (float)P.cutoffs64[i >= 8 ? min(1024u / i, (uint32_t)SDBF_CUTOFF_BINS - 1) : (uint32_t)SDBF_CUTOFF_BINS - 1];
     }
-    for (uint32_t i = tid; i < SDBF_CUTOFF_BINS; i += kTcThreads) {
-        S.cut256[i] = P.cutoffs[i];
-        S.cut64[i] = P.cutoffs64[i];
+    for (uint32_t i = tid; i < kTcRows; i += kTcThreads) S.rowbest[i] = make_uint2(0xFFFFFFFFu, 0);
+    for (uint32_t i = tid; i < kMatMaxTargets; i += kTcThreads) {
+        S.run[i] = 0;
+        S.run64[i] = 0;
     }
     if (tid == 0) {
-        for (int i = 0; i < 5; i++) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(&S.mbar[i])));
+        S.fail = 0;
+        for (uint32_t i = 0; i < kTcRing; i++) {
+            mbar_init(&S.tile_full[i], 1);
+            mbar_init(&S.tile_empty[i], kTcMark + kTcCheck + kTcWiden + 1);
+        }
+        for (uint32_t i = 0; i < 2; i++) {
+            mbar_init(&S.stage_full[i], kTcWiden);
+            mbar_init(&S.stage_empty[i], 1);
+            mbar_init(&S.acc_full[i], 1);
+            mbar_init(&S.acc_empty[i], kTcMark);
+        }
+        for (uint32_t i = 0; i < kTcMasks; i++) {
+            mbar_init(&S.mask_full[i], kTcMark);
+            mbar_init(&S.mask_empty[i], kTcCheck);
+        }
+        mbar_init(&S.check_bar, kTcCheck);
+        mbar_init(&S.a_free, 1);
+        mbar_init(&S.drain, 1);
         asm volatile("fence.mbarrier_init.release.cluster;");
     }
-    if (warp == 0) {  // two accumulators of 256 columns
+    if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(&S.tmem)),
-                     "r"(2 * kTcCols));
+                     "r"(kTcTmemCols));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     }
     asm volatile("tcgen05.fence::before_thread_sync;");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;");
     const uint32_t tmem = S.tmem;
-
-    uint32_t suses[2] = {0, 0};  // producers: commits to each stage barrier
-    uint32_t gtile = 0;          // tiles counted so far (all threads keep the same count)
-    bool ok = true;
-
-    for (;;) {
-        __syncthreads();
-        if (tid == 0) {
-            const uint32_t u = atomicAdd(P.next_unit, 1u);
-            S.unit_id = u;
-            if (u < P.nunits) S.unit = P.units[u];
-        }
-        __syncthreads();
-        if (S.unit_id >= P.nunits) break;
-        const MatUnit U = S.unit;
-        const uint32_t rs = U.flags & kUnitRefSide1 ? 1 : 0, ts = U.flags & kUnitTgtSide1 ? 1 : 0;
-        const bool split = (U.flags & kUnitSplit) != 0;
-        const bool group = (U.flags & kUnitGroup) != 0;
-        const uint32_t nref = group ? U.nref : 1;
-        const uint32_t nT = U.t1 - U.t0;
-        if (group) {
-            if (tid < 32) {
-                uint32_t base_row = 0;
-                for (uint32_t b = 0; b < nref; b += 32) {
-                    const uint32_t k = b + lane;
-                    uint32_t n = 0, id = 0;
-                    if (k < nref) {
-                        id = P.refs[U.ref + k];
-                        n = P.digests[rs][id].nfilters;
-                    }
-                    uint32_t incl = n;
+    if (warp < 4) {  // every block scale is 1.0 (ue8m0 127), whatever its place in these columns
+        const uint32_t one = 0x7F7F7F7Fu;
+        const uint32_t taddr = tmem + ((warp * 32) << 16) + kTcScaleCol;
 #pragma unroll
-                    for (int d = 1; d < 32; d <<= 1) {
-                        const uint32_t v = __shfl_up_sync(0xffffffffu, incl, d);
-                        if (lane >= (uint32_t)d) incl += v;
-                    }
-                    if (k < nref) {
-                        S.gref[k] = id;
-                        S.gstart[k] = base_row + incl - n;
-                        S.gsparse[k] = 0;
-                    }
-                    base_row += __shfl_sync(0xffffffffu, incl, 31);
-                }
-                if (lane == 0) S.gstart[nref] = base_row;
-            }
-        } else {
-            for (uint32_t k = tid; k < nT && !split; k += kTcThreads) S.run[k] = -1.0;
-        }
-        if (tid == 0) S.sparse = 0;
-        __syncthreads();
-        const CmpDigest A = P.digests[rs][group ? S.gref[0] : U.ref];
-        const bool fastA = (A.flags & kDigestFast) != 0;
-        const uint32_t nch = fastA ? 4 : kTcChunks;  // fast mode: the first 64 bytes
-
-        for (uint32_t rc = U.r0; rc < U.r1 && ok; rc += kTcRows) {
-            // ---- reference rows of this pass (threads 0..127)
-            const uint32_t row = rc + tid;
-            const bool have = tid < kTcRows && row < U.r1;
-            uint32_t s1 = 0, e1 = 0, gk = 0;
-            uint32_t fidx = A.first + row;
-            if (group && have) {
-                uint32_t lo = 0, hi = nref;
-                while (hi - lo > 1) {
-                    const uint32_t mid = (lo + hi) >> 1;
-                    if (S.gstart[mid] <= row) lo = mid;
-                    else hi = mid;
-                }
-                gk = lo;
-                fidx = P.digests[rs][S.gref[gk]].first + (row - S.gstart[gk]);
-            }
-            if (have) {
-                const uint32_t m = P.meta[rs][fidx];
-                s1 = m & 0xFFFFu;
-                e1 = m >> 16;
-            }
-            if (tid < kTcRows) S.rowf[tid] = have ? fidx : 0xFFFFFFFFu;
-            const bool active = have && s1 >= (uint32_t)kMinElem;
-            if (group && have && !active) atomicAdd(&S.gsparse[gk], 1u);
-            const uint32_t nsparse = __syncthreads_count(have && !active);
-            if (tid == 0) {
-                S.sparse += nsparse;
-                S.cur_t = 0;
-                S.cur_f = 0;
-                S.tile[0].produced = 0;
-                S.tile[1].produced = 0;
-            }
-            uint32_t bnum = 0, bden = 1;
-            bool counted = false;
-            const uint32_t nrows = min((uint32_t)kTcRows, U.r1 - rc);
-            RowHead aw;  // the row's first 128 bytes, for the staged re-check of candidates
-#pragma unroll
-            for (int q = 0; q < 8; q++)
-                aw.w[q] = have ? __ldg(reinterpret_cast<const uint4*>(P.filters[rs] + (size_t)fidx * 64) + q)
-                               : make_uint4(0, 0, 0, 0);
-            __syncthreads();
-            // ---- software pipeline: each step counts tile g (producers) and
-            // scores tile g-1 (consumers); one CTA barrier per step.  Tile g
-            // uses accumulator and tile slot g & 1, so accumulator b's n-th use
-            // is tile 2n + b and its barrier parity is (g >> 1) & 1.
-            bool pending = false;  // a counted tile waits to be scored
-            for (;;) {
-                const uint32_t b = gtile & 1;  // tile gtile is counted into accumulator / tile slot b
-                TC_STAMP(t_step);
-                if (producer) {
-                    TcTile& T = S.tile[b];
-                    TC_STAMP(t_comp);
-                    if (warp == 4) {  // compose tile g: up to 256 filters of up to 256 targets
-                        uint32_t filled = 0, ncomp = 0, nseg = 0, ct = S.cur_t, cf = S.cur_f;
-                        bool open = false;
-                        while (filled < (uint32_t)kTcCols && ct < nT) {
-                            const uint32_t te = ct + lane;
-                            const uint32_t f0 = lane == 0 ? cf : 0;
-                            uint32_t rem = 0, first = 0;
-                            if (te < nT) {
-                                const CmpDigest B = P.digests[ts][P.targets[U.t0 + te]];
-                                rem = B.nfilters - f0;
-                                first = B.first + f0;
-                            }
-                            uint32_t incl = rem;
-#pragma unroll
-                            for (int d = 1; d < 32; d <<= 1) {
-                                const uint32_t v = __shfl_up_sync(0xffffffffu, incl, d);
-                                if (lane >= (uint32_t)d) incl += v;
-                            }
-                            const uint32_t excl = incl - rem, room = (uint32_t)kTcCols - filled;
-                            const bool done_here = rem > 0 && incl <= room;
-                            const bool has = rem > 0 && excl < room;
-                            if (has) {  // every earlier segment of this tile completed, so index nseg + lane
-                                T.seg_first[nseg + lane] = first;
-                                T.seg_start[nseg + lane] = filled + excl;
-                                T.seg_te[nseg + lane] = te;
-                            }
-                            if (done_here) T.comp[ncomp + lane] = te;
-                            const uint32_t done_mask = __ballot_sync(0xffffffffu, done_here);
-                            const uint32_t has_mask = __ballot_sync(0xffffffffu, has);
-                            const uint32_t over_mask = __ballot_sync(0xffffffffu, rem > 0 && incl > room);
-                            const uint32_t open_mask = __ballot_sync(0xffffffffu, has && incl > room);
-                            const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
-                            ncomp += __popc(done_mask);
-                            nseg += __popc(has_mask);
-                            if (over_mask) {
-                                const uint32_t l = __ffs(over_mask) - 1;
-                                const uint32_t ex_l = __shfl_sync(0xffffffffu, excl, l);
-                                const uint32_t f0_l = __shfl_sync(0xffffffffu, f0, l);
-                                ct += l;
-                                cf = f0_l + (room - ex_l);
-                                filled = kTcCols;
-                                open = open_mask != 0;
-                            } else {
-                                ct = min(ct + 32u, nT);
-                                cf = 0;
-                                filled += total;
-                            }
-                        }
-                        if (lane < kTcCols / 32) T.lastmask[lane] = 0;
-                        if (lane == 0) {
-                            S.cur_t = ct;
-                            S.cur_f = cf;
-                            T.ntile = filled;
-                            T.ncomp = ncomp;
-                            T.nseg = nseg;
-                            T.seg_start[nseg] = filled;
-                            T.last_open = open;
-                            T.produced = filled > 0;
-                        }
-                    }
-                    group_sync<2>();
-                    if (ptid == 0) TC_ADD(kTcPhCompose, t_comp);
-                    TC_STAMP(t_fill);
-                    // slots of the tile, filled by all producers (loads in parallel)
-                    {
-                        const uint32_t nseg = T.nseg;
-                        for (uint32_t j = ptid; j < T.ntile; j += 128) {
-                            const uint32_t k = find_segment(T.seg_start, nseg, j);
-                            const uint32_t f = T.seg_first[k] + (j - T.seg_start[k]);
-                            const bool last = j + 1 == T.seg_start[k + 1] && !(k + 1 == nseg && T.last_open);
-                            T.gidx[j] = f;
-                            T.tmeta[j] = P.meta[ts][f];
-                            T.tinfo[j] = T.seg_te[k] | (k << 16) | (last ? 0x80000000u : 0u);
-                            if (last) atomicOr(&T.lastmask[j >> 5], 1u << (j & 31));
-                        }
-                    }
-                    group_sync<2>();
-                    if (ptid == 0) TC_ADD(kTcPhFill, t_fill);
-                    if (T.produced) {
-                        if (ptid == 0 && P.phase) atomicAdd(P.phase + kTcPhTiles, 1ull);
-                        const uint32_t nt = T.ntile;
-                        const uint32_t ncols = (nt + 15) & ~15u;  // MMA N: multiple of 16
-                        const uint32_t idesc = (1u << 4) | ((ncols >> 3) << 17) | ((uint32_t)(kTcRows >> 4) << 24);
-                        const uint32_t dacc = tmem + b * kTcCols;
-                        auto fetch = [&](uint32_t c) {
-                            uint4* slot = S.bits[c % kTcBitSlots];
-                            for (uint32_t i = ptid; i < kTcRows + ncols; i += 128) {
-                                if (i < kTcRows) {
-                                    const uint32_t f = S.rowf[i];
-                                    if (f != 0xFFFFFFFFu) cp_async16(slot + i, P.filters[rs] + (size_t)f * 64 + c * 4);
-                                } else if (i - kTcRows < nt) {
-                                    cp_async16(slot + i, P.filters[ts] + (size_t)T.gidx[i - kTcRows] * 64 + c * 4);
-                                }
-                            }
-                            cp_async_commit();
-                        };
-                        fetch(0);
-                        if (nch > 1) fetch(1);
-                        for (uint32_t c = 0; c < nch; c++) {
-                            TC_STAMP(t_fw);
-                            if (c + 2 < nch) fetch(c + 2);
-                            else cp_async_commit();
-                            cp_async_wait2();
-                            if (ptid == 0) TC_ADD(kTcPhFetchWait, t_fw);
-                            TC_STAMP(t_sw);
-                            const uint32_t s = (suses[0] + suses[1]) & 1;
-                            bool w = true;
-                            if (suses[s] > 0) w = mbar_wait(smem_addr(&S.mbar[s]), (suses[s] - 1) & 1);
-                            ok = group_and<2>(ok && w);
-                            if (ptid == 0) TC_ADD(kTcPhStageWait, t_sw);
-                            if (!ok) break;
-                            TC_STAMP(t_wd);
-                            uint8_t* sa = stages + s * kTcStage;
-                            uint8_t* sb = sa + kTcAStage;
-                            const uint4* slot = S.bits[c % kTcBitSlots];
-                            {
-                                // each producer thread: reference row ptid and target
-                                // columns ptid, ptid + 128 (zero bits past the tile);
-                                // the three loads first, then the three widenings
-                                const uint32_t c1 = ptid, c2 = ptid + 128;
-                                const uint4 z = make_uint4(0, 0, 0, 0);
-                                const uint4 ba = S.rowf[ptid] != 0xFFFFFFFFu ? slot[ptid] : z;
-                                const uint4 b1 = c1 < nt ? slot[kTcRows + c1] : z;
-                                const uint4 b2 = c2 < nt ? slot[kTcRows + c2] : z;
-                                if (c < 8) {
-                                    if (c1 < nt) T.tw[c][c1] = b1;
-                                    if (c2 < nt) T.tw[c][c2] = b2;
-                                }
-                                widen_row(sa, ptid, ba);
-                                if (c1 < ncols) widen_row(sb, c1, b1);
-                                if (c2 < ncols) widen_row(sb, c2, b2);
-                            }
-                            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                            group_sync<2>();
-                            if (ptid == 0) TC_ADD(kTcPhWiden, t_wd);
-                            TC_STAMP(t_is);
-                            if (ptid == 0) {
-                                asm volatile("tcgen05.fence::after_thread_sync;");
-                                const uint32_t a0 = smem_addr(sa), b0 = smem_addr(sb);
-#pragma unroll
-                                for (uint32_t kk = 0; kk < kTcChunk / 32; kk++) {
-                                    const uint64_t ad = sw128_desc(a0 + kk * 32), bd = sw128_desc(b0 + kk * 32);
-                                    const uint32_t acc = (c > 0 || kk > 0) ? 1u : 0u;
-                                    asm volatile(
-                                        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-                                        " tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n}\n" ::"r"(dacc),
-                                        "l"(ad), "l"(bd), "r"(idesc), "r"(acc));
-                                }
-                                mma_commit(smem_addr(&S.mbar[s]));
-                                TC_ADD(kTcPhIssue, t_is);
-                            }
-                            suses[s]++;
-                        }
-                        if (ok && ptid == 0) mma_commit(smem_addr(&S.mbar[2 + b]));
-                    }
-                    if (ptid == 0) TC_ADD(kTcPhProdStep, t_step);
-                } else if (pending) {
-                    // ---- consumers: score tile gtile-1 from accumulator 1-b
-                    const uint32_t pb = b ^ 1;
-                    const TcTile& T = S.tile[pb];
-                    const uint32_t g = gtile - 1;  // its tile number: the (g >> 1)-th use of accumulator pb
-                    TC_STAMP(t_aw);
-                    bool w = mbar_wait(smem_addr(&S.mbar[2 + pb]), (g >> 1) & 1);
-                    ok = group_and<1>(ok && w);
-                    if (tid == 0) TC_ADD(kTcPhAccWait, t_aw);
-                    TC_STAMP(t_sc);
-                    if (ok) {
-                        asm volatile("tcgen05.fence::after_thread_sync;");
-                        uint32_t ring_base = 0;                 // completion index of ring slot 0
-                        const uint32_t nt = T.ntile;
-                        uint32_t pend = 0;  // completed targets in the ring, not yet summed
-                        for (uint32_t c0 = 0; c0 < nt; c0 += 32) {
-                            TC_STAMP(t_ld);
-                            uint32_t v[32];
-                            const uint32_t taddr = tmem + ((warp * 32) << 16) + pb * kTcCols + c0;
-                            asm volatile(
-                                "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,"
-                                "%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
-                                : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]),
-                                  "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]),
-                                  "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]), "=r"(v[17]), "=r"(v[18]),
-                                  "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]),
-                                  "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]),
-                                  "=r"(v[31])
-                                : "r"(taddr));
-                            asm volatile("tcgen05.wait::ld.sync.aligned;");
-#pragma unroll
-                            for (int q = 0; q < 32; q++) S.cstage[q][tid] = (uint16_t)(__uint_as_float(v[q]) * 4096.0f);
-                            if (tid == 0) TC_ADD(kTcPhLd, t_ld);
-                            const uint32_t lim = min(32u, nt - c0);
-                            const uint32_t valid = lim == 32 ? 0xFFFFFFFFu : (1u << lim) - 1u;
-                            // pass 1, no branches: which columns count for this row
-                            // (kmask) and which are above the cut (cmask)
-                            uint32_t kmask = 0, cmask = 0;
-                            TC_STAMP(t_mk);
-                            // a table lookup only: element sums of 1024 and more (beyond
-                            // the reference's limits, never produced by its generator) are
-                            // marked and get their exact cut in pass 2
-                            const uint16_t* ctab = fastA ? S.cut64_sum : S.cut_sum;
-                            // (all 32 columns from the registers; c0 + 31 < 256, so the
-                            // columns past the tile read stale entries and are masked off)
-#pragma unroll
-                            for (uint32_t q = 0; q < 32; q++) {
-                                const uint32_t s2 = T.tmeta[c0 + q] & 0xFFFFu;
-                                const uint32_t sum = s1 + s2;
-                                const uint32_t cut = sum < 1024 ? ctab[sum] : 0u;
-                                const bool ct = s2 >= (uint32_t)kMinElem;
-                                kmask |= (uint32_t)ct << q;
-                                cmask |= (uint32_t)(ct && (uint32_t)(__uint_as_float(v[q]) * 4096.0f) > cut) << q;
-                            }
-                            kmask = active ? kmask & valid : 0u;
-                            cmask = active ? cmask & valid : 0u;
-                            // pass 2: the slice's segments in column order (the same for
-                            // every thread, so the ring fold's barrier stays uniform); in
-                            // each, this row's columns above the cut, then the segment end
-                            if (tid == 0) TC_ADD(kTcPhMark, t_mk);
-                            TC_STAMP(t_wk);
-                            uint32_t lmq = T.lastmask[c0 >> 5] & valid;
-                            uint32_t q0 = 0;
-                            for (;;) {
-                                const uint32_t qe = lmq ? (uint32_t)(__ffs(lmq) - 1) : lim;  // end column (incl.) or slice end
-                                const uint32_t upto = lmq ? qe + 1 : lim;
-                                const uint32_t range = (upto == 32 ? 0xFFFFFFFFu : (1u << upto) - 1u) & ~(q0 >= 32 ? 0xFFFFFFFFu : (1u << q0) - 1u);
-                                if (kmask & range) counted = true;  // a counted target filter scores at least 0
-                                for (uint32_t cm = cmask & range; cm; cm &= cm - 1u) {
-                                    const uint32_t q = __ffs(cm) - 1;
-                                    const uint32_t j = c0 + q;
-                                    const uint32_t tm = T.tmeta[j];
-                                    const uint32_t sum = s1 + (tm & 0xFFFFu);
-                                    const uint32_t cut = !fastA
-                                        ? (sum < 1024 ? S.cut_sum[sum] : S.cut256[4096u / sum])
-                                        : (sum < 1024 ? S.cut64_sum[sum] : S.cut64[1024u / sum]);
-                                    const uint64_t fr = candidate_fraction(aw, &T.tw[0][j], S.cstage[q][tid], cut, fastA,
-                                                                           min(e1, tm >> 16));
-                                    const uint32_t num = (uint32_t)(fr >> 32), den = (uint32_t)fr;
-                                    if ((uint64_t)num * bden > (uint64_t)bnum * den) {
-                                        bnum = num;
-                                        bden = den;
-                                    }
-                                }
-                                if (!lmq) break;  // the open segment goes on in the next slice
-                                lmq &= lmq - 1u;
-                                q0 = qe + 1;
-                                const uint32_t j = c0 + qe;
-                                {
-                                    const double m = row_maximum(active, bnum, bden, counted);
-                                    if (split) {
-                                        if (have) P.slots[P.split[U.split].slot_base + row] = m;
-                                    } else {
-                                        S.mv[tid][((T.tinfo[j] >> 16) & 0xFFu) % kTcRing] = m;
-                                    }
-                                    bnum = 0;
-                                    bden = 1;
-                                    counted = false;
-                                    if (!split && ++pend == (uint32_t)kTcRing) {  // ring full: sum it
-                                        TC_STAMP(t_fo);
-                                        fold_ring(P, S, T, ring_base, pend, group, nref, nrows, U.t0, rs, tid);
-                                        if (tid == 0) TC_ADD(kTcPhFold, t_fo);
-                                        ring_base += pend;
-                                        pend = 0;
-                                    }
-                                }
-                            }
-                            if (tid == 0) TC_ADD(kTcPhWalk, t_wk);
-                        }
-                        if (pend) {  // the tile's last completed targets
-                            TC_STAMP(t_fo);
-                            fold_ring(P, S, T, ring_base, pend, group, nref, nrows, U.t0, rs, tid);
-                            if (tid == 0) TC_ADD(kTcPhFold, t_fo);
-                        }
-                        asm volatile("tcgen05.fence::before_thread_sync;");
-                    }
-                    if (tid == 0) TC_ADD(kTcPhScore, t_sc);
-                    if (tid == 0) TC_ADD(kTcPhConsStep, t_step);
-                }
-                TC_STAMP(t_bar);
-                ok = __syncthreads_and(ok);
-                if (tid == 0) TC_ADD(kTcPhStepBarrier, t_bar);
-                if (!ok) break;
-                const bool produced = S.tile[b].produced != 0;
-                if (produced) gtile++;
-                pending = produced;
-                if (!produced) break;  // no tile counted in this step: the pass is done
-            }
-        }
-        if (!ok) break;
-        if (!split && !group) {
-            for (uint32_t k = tid; k < nT; k += kTcThreads) {
-                const uint32_t tgt = P.targets[U.t0 + k];
-                P.scores[out_index(P, rs != 0, U.ref, tgt)] = final_score(S.run[k], A.nfilters, S.sparse);
-            }
-        }
-    }
-    asm volatile("cp.async.wait_all;" ::: "memory");
-    if (!ok && tid == 0) {
-        atomicAdd(P.error, 1u);
-        // wait (bounded) for any MMA still reading shared memory or writing TMEM
-        mma_commit(smem_addr(&S.mbar[4]));
-        mbar_wait(smem_addr(&S.mbar[4]), 0);
+        for (uint32_t c = 0; c < kTcScaleCols; c += 8)
+            asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%1,%1,%1,%1,%1,%1,%1};" ::"r"(taddr + c), "r"(one)
+                         : "memory");
+        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
     }
     asm volatile("tcgen05.fence::before_thread_sync;");
     __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;");
+
+    if (warp < kTcMark) tc_mark<kPhases>(P, S, tmem, warp, lane);
+    else if (warp < kTcMark + kTcCheck) tc_check<kPhases>(P, S, warp - kTcMark, lane);
+    else if (warp < kTcComposeWarp) tc_widen<kPhases>(P, S, a_smem, b_smem, (warp - kTcMark - kTcCheck) * 32 + lane, lane);
+    else if (warp == kTcComposeWarp) tc_compose<kPhases>(P, S, lane);
+    else tc_mma<kPhases>(P, S, smem_addr(a_smem), smem_addr(b_smem), tmem, lane);
+    __syncwarp();
+    if (warp == kTcMmaWarp && S.fail) {
+        // wait (bounded) for any MMA still reading shared memory or writing TMEM
+        if (lane == 0) mma_commit(&S.drain);
+        __syncwarp();
+        mbar_wait(&S.drain, 0);
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;");
+    __syncthreads();
+    if (tid == 0 && S.fail) atomicAdd(P.error, 1u);
     if (warp == 0)
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2 * kTcCols));
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTcTmemCols));
 }
 
 cudaError_t launch_matrix_tc(const MatParams& P, uint32_t grid, cudaStream_t st) {
     if (P.nunits == 0) return cudaSuccess;
-    k_matrix_tc<<<grid, kTcThreads, kTcSmemBytes, st>>>(P);
+    if (P.phase) k_matrix_tc<true><<<grid, kTcThreads, kTcSmemBytes, st>>>(P);
+    else k_matrix_tc<false><<<grid, kTcThreads, kTcSmemBytes, st>>>(P);
     return cudaGetLastError();
 }
 
 int matrix_tc_ctas_per_sm() {
-    cudaFuncSetAttribute(k_matrix_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTcSmemBytes);
+    cudaFuncSetAttribute(k_matrix_tc<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTcSmemBytes);
+    cudaFuncSetAttribute(k_matrix_tc<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTcSmemBytes);
     int n = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_matrix_tc, kTcThreads, kTcSmemBytes);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_matrix_tc<false>, kTcThreads, kTcSmemBytes);
     return n > 0 ? n : 1;
 }
 

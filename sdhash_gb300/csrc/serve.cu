@@ -79,7 +79,7 @@ struct sdbfg_server {
         std::vector<Request> batch;
         uint32_t nunits = 0, nsplit = 0;
         HostBuf h_filters, h_meta, h_dig, h_units, h_targets, h_refs, h_split, h_scores;
-        DevBuf d_filters, d_meta, d_dig, d_units, d_targets, d_refs, d_split, d_slots, d_counter, d_scores;
+        DevBuf d_filters, d_meta, d_dig, d_units, d_targets, d_refs, d_split, d_slots, d_counter, d_scores, d_redo;
         uint64_t cap_units = 0, cap_targets = 0, cap_refs = 0, cap_split = 0, cap_slots = 0;
     };
     std::vector<Slot> slots;
@@ -111,13 +111,15 @@ static cudaError_t launch_batch(sdbfg_server* sv, sdbfg_server::Slot& S) {
         const Request& r = S.batch[i];
         memcpy(S.h_filters.as<uint8_t>() + tot * 256, r.filters.data(), (size_t)r.nf * 256);
         memcpy(S.h_meta.as<uint32_t>() + tot, r.meta.data(), (size_t)r.nf * 4);
-        dig[i] = CmpDigest{(uint32_t)tot, r.nf};
+        dig[i] = CmpDigest{(uint32_t)tot, r.nf, 0, 0, 0};
+        digest_stats(dig[i], S.h_meta.as<uint32_t>());
         tot += r.nf;
     }
     // work units: every query against every target, orientation by the swap rule
     const uint64_t ctas = (uint64_t)sv->ctx->sms * matrix_ctas_per_sm(sv->ctx->mat_variant);
-    UnitBuilder ub(effective_unit_budget(sv->ctx->mat_unit_work, tot * T->total_filters, ctas),
-                   (uint32_t)kMatVariantTable[sv->ctx->mat_variant].rows);
+    const int variant = sv->ctx->mat_variant;
+    UnitBuilder ub(effective_unit_budget(sv->ctx->mat_unit_work, cross_work(tot, T->total_filters, variant), ctas, variant),
+                   variant);
     std::vector<uint32_t> targets;
     build_cross_units(
         ub, targets, nq, nt, [&](uint32_t i, uint32_t j) { return server_swaps(S.batch[i], T, j); },
@@ -165,16 +167,18 @@ static cudaError_t launch_batch(sdbfg_server* sv, sdbfg_server::Slot& S) {
     P.split = S.d_split.as<MatSplit>();
     P.nsplit = S.nsplit;
     P.slots = S.d_slots.as<double>();
+    P.nslots = ub.slots;
     P.scores = S.d_scores.as<int32_t>();
+    P.nscores = (uint64_t)nq * nt;
     P.mode = kMatModeCross;
     P.n = nt;
     P.cutoffs = sv->ctx->d_cut.as<uint16_t>();
     P.cutoffs64 = sv->ctx->d_cut64.as<uint16_t>();
+    P.redo = redo_list(S.d_redo.p);
     P.error = S.d_counter.as<uint32_t>() + 1;
-    const uint32_t grid = (uint32_t)std::min<uint64_t>(ctas, std::max(1u, S.nunits));
-    if ((e = launch_matrix(P, sv->ctx->mat_variant, grid, st))) return e;
-    if ((e = launch_matrix_finalize(P, st))) return e;
-    sv->launches += 1 + (S.nsplit ? 1 : 0);
+    uint64_t launched = 0;
+    if ((e = run_matrix(P, variant, (uint32_t)ctas, (uint32_t)sv->ctx->sms, st, &launched))) return e;
+    sv->launches += launched;
     if ((e = cudaMemcpyAsync(S.h_scores.p, S.d_scores.p, (size_t)nq * nt * 4, cudaMemcpyDeviceToHost, st))) return e;
     return cudaEventRecord(S.ev, st);
 }
@@ -314,6 +318,7 @@ extern "C" int sdbfg_server_create(sdbfg_ctx* c, const sdbfg_set* refs, const sd
             if (e == cudaSuccess) e = hv->ensure(bytes);
         }
         if (e == cudaSuccess) e = S.d_counter.ensure(64);
+        if (e == cudaSuccess) e = S.d_redo.ensure(kRedoBytes);
         if (e == cudaSuccess) e = grow(S.d_units, &S.h_units, S.cap_units, 1 << 16, sizeof(MatUnit));
         if (e == cudaSuccess)
             e = grow(S.d_targets, &S.h_targets, S.cap_targets, (uint64_t)nq * refs->n + nq + refs->n + 1, 4);
@@ -409,7 +414,7 @@ extern "C" void sdbfg_server_destroy(sdbfg_server* sv) {
     cudaSetDevice(sv->ctx->device);
     for (auto& S : sv->slots) {
         for (DevBuf* b : {&S.d_filters, &S.d_meta, &S.d_dig, &S.d_units, &S.d_targets, &S.d_refs, &S.d_split,
-                          &S.d_slots, &S.d_counter, &S.d_scores})
+                          &S.d_slots, &S.d_counter, &S.d_scores, &S.d_redo})
             b->release();
         for (HostBuf* b : {&S.h_filters, &S.h_meta, &S.h_dig, &S.h_units, &S.h_targets, &S.h_refs, &S.h_split,
                            &S.h_scores})

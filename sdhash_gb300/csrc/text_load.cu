@@ -401,7 +401,7 @@ extern "C" int sdbfg_set_load_text(sdbfg_ctx* c, const char* text, uint64_t len,
         s->last_count[i] = p.last_count;
         s->dd_block[i] = p.dd_block;
         s->first[i] = p.line.first;
-        dig[i] = {p.line.first, p.line.nfilters};
+        dig[i] = {p.line.first, p.line.nfilters, 0, 0, 0};
     }
     auto cleanup = [&](int code) {
         s->d_filters.release();
@@ -508,15 +508,17 @@ extern "C" int sdbfg_set_load_text(sdbfg_ctx* c, const char* text, uint64_t len,
         return cleanup(fail(c, SDBFG_ERR_FORMAT, "line %lld: malformed SDBF (%d)",
                             (long long)(payload_first ? first_bad : hdr_bad), payload_first ? -2 : hdr_code));
     }
-    // element count of each digest's last filter (the swap rule's tie-break)
-    std::vector<uint32_t> lastmeta(nl);
-    for (uint32_t i = 0; i < nl; i++) {
-        const cudaError_t e = cudaMemcpyAsync(&lastmeta[i], s->d_meta.as<uint32_t>() + lines[i].first + lines[i].nfilters - 1,
-                                              4, cudaMemcpyDeviceToHost, st);
+    // the digests' element-count words; the last filter's count is the swap
+    // rule's tie-break (one copy back: a copy per digest cost 10 us each)
+    if (nl) {
+        cudaError_t e = launch_digest_stats(s->d_meta.as<uint32_t>(), s->d_digests.as<CmpDigest>(), nl, st);
+        c->launches += 1;
+        if (e == cudaSuccess)
+            e = cudaMemcpyAsync(dig.data(), s->d_digests.p, nl * sizeof(CmpDigest), cudaMemcpyDeviceToHost, st);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(st);
         if (e != cudaSuccess) return cleanup(fail(c, SDBFG_ERR_CUDA, "set load: %s", cudaGetErrorString(e)));
     }
-    if (cudaStreamSynchronize(st) != cudaSuccess) return cleanup(fail(c, SDBFG_ERR_CUDA, "set load: synchronize"));
-    for (uint32_t i = 0; i < nl; i++) s->last_elem[i] = lastmeta[i] & 0xFFFFu;
+    for (uint32_t i = 0; i < nl; i++) s->last_elem[i] = dig[i].last;
     *out = s;
     return SDBFG_OK;
 }
