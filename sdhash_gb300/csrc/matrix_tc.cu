@@ -50,12 +50,14 @@
 // roles.  A tile takes about 10.4 K cycles, of which its 32 MMAs need 3 K on
 // the tensor pipe; they read 10 KB of shared memory each (2.5 K cycles of
 // its bandwidth a tile) beside 1.5 K cycles of widened stores.  Pairs of 128 x
-// 192 filters: 5.6e11 filter pairs/s (400 uneven digests, 4.7e9 pairs: 8.6
+// 192 filters: 5.6e11 filter pairs/s (400 uneven digests, 4.7e9 pairs: 8.5
 // ms; 2,048 queries against 4 image segments, 8e8 pairs: 1.5 ms), against
 // 1.2e11 for e4m3 operands widened for both sides in every tile, one row per
 // scoring lane and ordered sums in the kernel (39 and 5.7 ms).  Measured on
 // the way: every check warp a share of the tile's marked pairs instead of
-// its own rows (three barriers a tile: 10.1 against 9.0 ms); unrolled role
+// its own rows (three barriers a tile: 10.1 against 9.0 ms); the marks of a
+// row listed and folded by its own lane (a last filter of few elements has
+// most of a tile's marks: 64 x 64 digests 240 against 145 us); unrolled role
 // loops (15 ms: the five roles share the instruction cache, and instruction
 // fetch was the first stall); a proxy fence in the widening warps (18.4 ms:
 // it waits for their loads in flight).
@@ -117,7 +119,9 @@ struct TcSmem {
     float thr[kTcSumMax + 1], thr64[kTcSumMax + 1];  // cut by element-count sum
     uint16_t dense[kTcCheck][kTcDense];     // check: marked pairs (row << 8 | column)
     uint32_t res[kTcCheck][kTcDense];       // check: their ratios in units of 2^-23 (0: none)
-    uint2 rowbest[kTcRows];                 // a row's open target (pass number << 9 | place) and its maximum so far
+    // check: a row's open target (pass number << 9 | place) in the high half, its
+    // maximum so far in the low one.  The mark warps read it while it changes: one 64-bit access.
+    unsigned long long rowbest[kTcRows];
     uint32_t run[kMatMaxTargets];           // sums of the pass per target (one reference digest)
     unsigned long long run64[kMatMaxTargets];  // and of the unit
     uint32_t seg_first[kTcCols], seg_start[kTcCols + 1], seg_te[kTcCols];  // compose: one segment per target
@@ -215,6 +219,14 @@ __device__ __forceinline__ void widen_word(uint8_t* chunk, uint32_t r, uint32_t 
         g.w = (x >> 1) & 0x44444444u;
     }
     *reinterpret_cast<uint4*>(chunk + r * 128 + ((q ^ (r & 7)) << 4)) = g;
+}
+
+__device__ __forceinline__ uint2 row_best(const TcSmem& S, uint32_t row) {
+    const unsigned long long v = *const_cast<const volatile unsigned long long*>(&S.rowbest[row]);
+    return make_uint2((uint32_t)(v >> 32), (uint32_t)v);
+}
+__device__ __forceinline__ void set_row_best(TcSmem& S, uint32_t row, uint32_t tag, uint32_t best) {
+    *const_cast<volatile unsigned long long*>(&S.rowbest[row]) = (unsigned long long)tag << 32 | best;
 }
 
 // slot j of a composed tile: its segment k (seg_start[k] <= j < seg_start[k+1])
@@ -651,7 +663,7 @@ __device__ __forceinline__ void tc_mark(const MatParams& P, TcSmem& S, uint32_t 
         asm volatile("tcgen05.fence::after_thread_sync;");
         const float* thr = T.flags & kTileFast ? S.thr64 : S.thr;
         const uint32_t nsl = (T.nt + 31) / 32;
-        const uint2 rb = S.rowbest[row];
+        const uint2 rb = row_best(S, row);
         const uint32_t tacc = tmem + ((warp * 32) << 16) + b * kTcCols;
         // columns of slice i above the cut: the sign of cut - count, four
         // chains of eight columns.  A row that has a maximum r of the
@@ -718,7 +730,6 @@ __device__ __forceinline__ void tc_check(const MatParams& P, TcSmem& S, uint32_t
     uint16_t* dense = S.dense[cw];
     uint32_t* res = S.res[cw];
     uint32_t phase = 0;
-    uint32_t cur_te = 0xFFFFFFFFu, best = 0;  // lanes 0..15: the row's open target and its maximum so far
 #pragma unroll 1
     for (uint32_t t = 0;; t++) {
         const uint32_t slot = t % kTcRing, b = t % kTcMasks;
@@ -746,37 +757,34 @@ __device__ __forceinline__ void tc_check(const MatParams& P, TcSmem& S, uint32_t
         const bool split = (uflags & kUnitSplit) != 0, fast = (T.flags & kTileFast) != 0;
         const uint32_t nref = uflags & kUnitGroup ? T.unit.nref : 1u;
         if (T.flags & kTileFirst) {
-            cur_te = 0xFFFFFFFFu;
-            best = 0;
-            if (half == 0) S.rowbest[row] = make_uint2(0xFFFFFFFFu, 0);
+            if (half == 0) set_row_best(S, row, 0xFFFFFFFFu, 0);
+            __syncwarp();
         }
         const uint32_t* __restrict__ fr = P.filters[rs];
         const uint32_t* __restrict__ ft = P.filters[ts];
         const float* thr = fast ? S.thr64 : S.thr;
         if (kPhases && lane == 0) atomicAdd(P.phase + kTcPhMarked, (unsigned long long)total);
-        // the warp's marked pairs in one list: by lane (a row's first half
-        // before its second), then column; kTcDense of them at a time
+        // the warp's marked pairs in one list, kTcDense of them at a time: by
+        // lane (a row's first half before its second), then column.  The
+        // warp writes one mask word at a time, so a row with many marks (a
+        // digest's last filter, of few elements and a low cut) costs it no more than others.
 #pragma unroll 1
         for (uint32_t base = 0; base < total; base += kTcDense) {
             const uint32_t lim = min(total - base, kTcDense);
+            uint32_t at = off - base;  // place of the lane's next word (wraps below the round)
+#pragma unroll
+            for (int k = 0; k < 3; k++) {
+                uint32_t lanes = __ballot_sync(0xffffffffu, m[k] != 0);
 #pragma unroll 1
-            for (uint32_t k = 0, i = off - base; k < n; k++, i++) {  // (i wraps below the round)
-                uint32_t col = 96 * half, mm[3] = {m[0], m[1], m[2]};
-                if (i >= lim) {
-                    if ((int32_t)i >= 0) break;  // past the round
-                    continue;                    // taken in an earlier one
+                while (lanes) {
+                    const uint32_t l = __ffs(lanes) - 1;
+                    lanes &= lanes - 1u;
+                    const uint32_t w = __shfl_sync(0xffffffffu, m[k], l), o = __shfl_sync(0xffffffffu, at, l);
+                    const uint32_t i = o + __popc(w & ((1u << lane) - 1u));
+                    if (((w >> lane) & 1u) && i < lim)
+                        dense[i] = (uint16_t)((cw * 16 + (l & 15)) << 8 | (96 * (l >> 4) + 32 * k + lane));
                 }
-                if (mm[0]) {
-                    col += __ffs(mm[0]) - 1;
-                    m[0] &= m[0] - 1u;
-                } else if (mm[1]) {
-                    col += 32 + __ffs(mm[1]) - 1;
-                    m[1] &= m[1] - 1u;
-                } else {
-                    col += 64 + __ffs(mm[2]) - 1;
-                    m[2] &= m[2] - 1u;
-                }
-                dense[i] = (uint16_t)(row << 8 | col);
+                at += __popc(m[k]);
             }
             __syncwarp();
             constexpr uint32_t kSteps = 3;  // pairs in flight per eight lanes
@@ -833,39 +841,48 @@ __device__ __forceinline__ void tc_check(const MatParams& P, TcSmem& S, uint32_t
                 }
             }
             __syncwarp();
-            // the rows' maxima: lane < 16 takes its own entries of the round,
-            // then those of its row's second half
-            const uint32_t lo = min(max((int32_t)(off - base), 0), (int32_t)lim), hi = min(max((int32_t)(off + n - base), 0), (int32_t)lim);
-            const uint32_t lo2 = __shfl_down_sync(0xffffffffu, lo, 16), hi2 = __shfl_down_sync(0xffffffffu, hi, 16);
-            if (half == 0) {
-                const uint32_t n1 = hi - lo, nn = n1 + (hi2 - lo2);
-                const uint32_t was = best, was_te = cur_te;
-                for (uint32_t k = 0; k < nn; k++) {
-                    const uint32_t i = k < n1 ? lo + k : lo2 + (k - n1);
-                    const uint32_t r = res[i];
-                    if (r == 0) continue;
-                    const uint32_t te = T.te[dense[i] & 0xFFu];
-                    if (te != cur_te) {
-                        cur_te = te;
-                        best = 0;
-                    }
-                    if (r <= best) continue;
-                    // the sum grows by what the maximum grows
-                    if (split) {
-                        atomicMax(reinterpret_cast<uint32_t*>(P.slots) + P.split[T.unit.split].slot_base + T.rc + row, r);
-                    } else {
-                        uint32_t* sum;
-                        if (nref == 1) sum = &S.run[te];
-                        else
-                            sum = reinterpret_cast<uint32_t*>(P.scores) +
-                                  out_index(P, rs != 0, R.gref[R.rowk[row]], P.targets[T.unit.t0 + te]);
-                        if (r == 0xFFFFFFFFu) atomicOr(sum, 0x80000000u);  // left to k_matrix_finish
-                        else atomicAdd(sum, r - best);
-                    }
-                    best = r;
+            // the rows' maxima, 32 entries at a time: the maximum of every run
+            // of one row and target, then the runs' last lanes update the
+            // rows (a row's runs one after another, in order)
+#pragma unroll 1
+            for (uint32_t i0 = 0; i0 < lim; i0 += 32) {
+                const uint32_t e = dense[min(i0 + lane, lim - 1)];
+                uint32_t r = i0 + lane < lim ? res[i0 + lane] : 0u;
+                const uint32_t te = T.te[e & 0xFFu], row = e >> 8, key = row << 9 | te;
+#pragma unroll
+                for (int d = 1; d < 32; d <<= 1) {
+                    const uint32_t kr = __shfl_up_sync(0xffffffffu, key, d), rr = __shfl_up_sync(0xffffffffu, r, d);
+                    if (lane >= (uint32_t)d && kr == key) r = max(r, rr);
                 }
-                // what the mark warps may raise the row's cuts by
-                if (best != was || cur_te != was_te) S.rowbest[row] = make_uint2(T.pseq << 9 | cur_te, best);
+                const uint32_t next = __shfl_down_sync(0xffffffffu, key, 1);
+                uint32_t todo = __ballot_sync(0xffffffffu, r != 0 && (lane == 31 || next != key));
+                const uint32_t same = __match_any_sync(0xffffffffu, row);
+#pragma unroll 1
+                while (todo) {
+                    const uint32_t mine = same & todo;
+                    if (((todo >> lane) & 1u) && (uint32_t)(__ffs(mine) - 1) == lane) {
+                        const uint32_t tag = T.pseq << 9 | te;
+                        const uint2 st = row_best(S, row);
+                        const uint32_t best = st.x == tag ? st.y : 0u;
+                        if (r > best) {
+                            set_row_best(S, row, tag, r);  // (the mark warps raise the row's cuts by it)
+                            // the sum grows by what the maximum grows
+                            if (split) {
+                                atomicMax(reinterpret_cast<uint32_t*>(P.slots) + P.split[T.unit.split].slot_base + T.rc + row, r);
+                            } else {
+                                uint32_t* sum;
+                                if (nref == 1) sum = &S.run[te];
+                                else
+                                    sum = reinterpret_cast<uint32_t*>(P.scores) +
+                                          out_index(P, rs != 0, R.gref[R.rowk[row]], P.targets[T.unit.t0 + te]);
+                                if (r == 0xFFFFFFFFu) atomicOr(sum, 0x80000000u);  // left to k_matrix_finish
+                                else atomicAdd(sum, r - best);
+                            }
+                        }
+                    }
+                    todo &= ~__ballot_sync(0xffffffffu, ((todo >> lane) & 1u) && (uint32_t)(__ffs(mine) - 1) == lane);
+                    __syncwarp();
+                }
             }
             __syncwarp();
         }
@@ -918,7 +935,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_matrix_tc(MatParams P) {
         S.thr[i] = (float)P.cutoffs[i >= 32 ? min(4096u / i, (uint32_t)SDBF_CUTOFF_BINS - 1) : (uint32_t)SDBF_CUTOFF_BINS - 1];
         S.thr64[i] = (float)P.cutoffs64[i >= 8 ? min(1024u / i, (uint32_t)SDBF_CUTOFF_BINS - 1) : (uint32_t)SDBF_CUTOFF_BINS - 1];
     }
-    for (uint32_t i = tid; i < kTcRows; i += kTcThreads) S.rowbest[i] = make_uint2(0xFFFFFFFFu, 0);
+    for (uint32_t i = tid; i < kTcRows; i += kTcThreads) S.rowbest[i] = ~0ull << 32;
     for (uint32_t i = tid; i < kMatMaxTargets; i += kTcThreads) {
         S.run[i] = 0;
         S.run64[i] = 0;

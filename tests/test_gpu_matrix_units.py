@@ -103,3 +103,21 @@ def test_folded_against_unfolded(ctx):
             f[i] = qs[i % 4].filters.reshape(-1, 256)[i % qs[i % 4].bf_count]
     q, t = ctx.upload(qs), ctx.upload(ts)
     assert np.array_equal(ctx.compare_to(q, t), pairwise(ctx, q, t, len(qs), len(ts)))
+
+
+def test_repeated_runs_agree(ctx):
+    """The roles of the tensor-core kernel hand each other a row's maximum while
+    it changes: forty runs of targets of many tiles give the CUDA-core kernel's scores."""
+    import sdhash_gb300 as g
+    rng = np.random.default_rng(11)
+    pool = np.stack([bits_to_bytes(rng.choice(2048, size=660, replace=False)) for _ in range(20)])
+    counts = np.rint(np.exp(rng.uniform(0, np.log(900), 70))).astype(int)
+    ds = [random_digest(g, rng, f"r{i:02d}", int(n), np.r_[np.full(int(n) - 1, 192), 40], pool) for i, n in enumerate(counts)]
+    dev = ctx.upload(ds)
+    ctx.set_compare_tuning(0, 1 << 22, False)
+    try:
+        want = ctx.compare_all(dev)
+    finally:
+        ctx.set_compare_tuning(5, 1 << 22, True)
+    for k in range(40):
+        assert np.array_equal(ctx.compare_all(dev), want), k
