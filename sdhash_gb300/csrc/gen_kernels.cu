@@ -955,6 +955,10 @@ __device__ __forceinline__ bool link_fails(const GenParams& P, const GenChunk& C
 // predecessors' exit states as they stand.  A tile whose predecessor is
 // recomputed in the same launch may start from the stale state; the
 // serial pass that follows finds and redoes it (normally nothing is left).
+// A group of at most one tile per resident CTA needs no list: fix_list is
+// null and each CTA checks its own tile's link (a stale or a fresh exit state
+// read there decides only what the serial pass is left with), which saves a
+// memset and a launch, 5 us of the 64 KiB file's digest.
 __global__ void __launch_bounds__(256) k_stream_fails(GenParams P) {
     for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < P.ntiles; t += gridDim.x * blockDim.x) {
         const GenChunk C = P.chunks[P.tiles[t].chunk];
@@ -966,9 +970,17 @@ template <bool kPre>
 __global__ void __launch_bounds__(kGenThreads) k_stream_fix_list(GenParams P) {
     extern __shared__ __align__(16) uint8_t smem[];
     __shared__ uint64_t entry;
-    const uint32_t n = P.fix_list[0];
+    const uint32_t n = P.fix_list ? P.fix_list[0] : P.ntiles;
     for (uint32_t k = blockIdx.x; k < n; k += gridDim.x) {
-        const uint32_t tile = P.fix_list[1 + k];
+        uint32_t tile = k;
+        if (P.fix_list) {
+            tile = P.fix_list[1 + k];
+        } else {
+            const GenChunk C = P.chunks[P.tiles[k].chunk];
+            bool fails = false;
+            if (threadIdx.x == 0) fails = k > C.first_tile && link_fails(P, C, k);
+            if (!__syncthreads_or(fails)) continue;
+        }
         if (threadIdx.x == 0) entry = P.tile_out[tile - 1].tau_out;
         __syncthreads();
         stream_tile_body<kPre>(P, tile, &entry, smem);
@@ -1033,14 +1045,20 @@ __device__ __forceinline__ void prefetch_l2(const void* gmem, uint32_t bytes) {
 
 // ------------------------------------------------ precomputed ranks
 // Entropy ranks of a stream launch group ahead of its tile kernel.  One CTA
-// item is a stretch of kRkSpan positions of a chunk, its bytes staged in
+// item is a stretch of kRkThreads x rk_per positions of a chunk, its bytes staged in
 // shared memory by 16-byte asynchronous copies (the CTA's next stretch
-// prefetched into L2 meanwhile); each thread ranks kRkPer consecutive
+// prefetched into L2 meanwhile); each thread ranks rk_per consecutive
 // positions with its own histogram (rank_run, the tile kernel's rank loop),
-// so a thread's 64-byte window set-up is spread over 312 positions instead
-// of a tile thread's 88.  Ranks of positions >= n-64 are 0; the chunk's
-// ranks run to a multiple of 8 (GenChunk::rank_off8).
-constexpr uint32_t kRkBytes = align_up(kRkSpan + 64 + 16, 16);  // staged bytes + zero padding
+// so a thread's 64-byte window set-up is spread over up to 312 positions
+// instead of a tile thread's 88.  Ranks of positions >= n-64 are 0; the
+// chunk's ranks run to a multiple of 8 (GenChunk::rank_off8).
+//
+// Positions per thread: the kernel's time is that of a thread's chain of
+// 64 + rk_per steps times the number of waves of stretches over the SMs
+// (three to an SM).  312 has the least set-up, but leaves most SMs idle
+// below 18 MB: rk_choose takes the smallest product.  One file of 64 KiB, 1, 4,
+// 8 and 16 MiB: 11, 13, 18, 24 and 37 us; always 312: 21, 21, 22, 27 and 36.
+constexpr uint32_t kRkBytes = align_up(rk_span(kRkPerMax) + 64 + 16, 16);  // staged bytes + zero padding
 constexpr uint32_t kRkSmem = 256 * kRkThreads + kRkBytes;
 
 __global__ void __launch_bounds__(kRkThreads, 3) k_stream_ranks(GenParams P) {
@@ -1051,13 +1069,13 @@ __global__ void __launch_bounds__(kRkThreads, 3) k_stream_ranks(GenParams P) {
     __shared__ uint16_t s_rank[(SDBF_RANK_BINS + 7) / 8 * 8];
     for (uint32_t i = threadIdx.x; i < 65; i += blockDim.x) dtab[i] = i < 64 ? (int32_t)P.ent_tab[i + 1] - (int32_t)P.ent_tab[i] : 0;
     for (uint32_t i = threadIdx.x; i < SDBF_RANK_BINS; i += blockDim.x) s_rank[i] = P.rank_tab[i];
-    const uint32_t tid = threadIdx.x;
+    const uint32_t tid = threadIdx.x, per = P.rk_per, span = rk_span(per);
     for (uint32_t item = blockIdx.x; item < P.nrk_items; item += gridDim.x) {
         const uint2 it = P.rk_items[item];
         const GenChunk C = P.chunks[it.x];
         const uint32_t s0 = it.y, n = C.n;
-        const uint32_t np = min(kRkSpan, align_up(n, 8) - s0);  // positions [s0, s0+np)
-        const uint32_t nb = min(kRkSpan + 64, n - s0);          // bytes [s0, s0+nb)
+        const uint32_t np = min(span, align_up(n, 8) - s0);  // positions [s0, s0+np)
+        const uint32_t nb = min(span + 64, n - s0);          // bytes [s0, s0+nb)
         __syncthreads();  // the previous stretch is done with the bytes and histograms
         // the stretch's bytes: 16-byte asynchronous copies, all in flight at once
         const uint8_t* src = P.data + C.data_off + s0;
@@ -1075,12 +1093,12 @@ __global__ void __launch_bounds__(kRkThreads, 3) k_stream_ranks(GenParams P) {
             const uint2 nx = P.rk_items[item + gridDim.x];
             const GenChunk Cn = P.chunks[nx.x];
             const uint8_t* ns = P.data + Cn.data_off + nx.y;
-            const uint32_t nnb = min(kRkSpan + 64, Cn.n - nx.y) & ~15u;
+            const uint32_t nnb = min(span + 64, Cn.n - nx.y) & ~15u;
             if ((reinterpret_cast<uintptr_t>(ns) & 15) == 0 && nnb) prefetch_l2(ns, nnb);
         }
         cp_async_wait_all();
         __syncthreads();
-        const uint32_t lo = min(np, tid * kRkPer), hi = min(np, lo + kRkPer);
+        const uint32_t lo = min(np, tid * per), hi = min(np, lo + per);
         const uint32_t last = n > kWin ? n - kWin : 0;  // ranks exist for o < n-64 only
         const uint32_t vend = last > s0 ? min(hi, last - s0) : lo;
         rank_run(b32, hist, hist_off(tid, 0), s_rank, dtab, lo, vend, hi,
@@ -1935,6 +1953,20 @@ static void set_stream_attrs() {
                           (const void*)k_stream_commit_index})
         cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared);
     done = true;
+}
+
+int rk_choose(const uint64_t* stretches, uint32_t sms) {
+    const uint64_t slots = (uint64_t)sms * 3;
+    int best = 0;
+    uint64_t cost = ~0ull;
+    for (int k = 0; k < kRkChoices; k++) {
+        const uint64_t c = (stretches[k] + slots - 1) / slots * (64 + kRkPers[k]);
+        if (c < cost) {
+            cost = c;
+            best = k;
+        }
+    }
+    return best;
 }
 
 cudaError_t launch_stream_ranks(const GenParams& P, uint32_t grid, cudaStream_t st) {

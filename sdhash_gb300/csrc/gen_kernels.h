@@ -40,13 +40,18 @@ struct GenChunk {
 };
 
 // Precomputed ranks of a stream launch group: k_stream_ranks gives each CTA
-// kRkThreads x kRkPer consecutive positions of one chunk (a "stretch"); one
-// work item (chunk, first position) per stretch.
+// kRkThreads x GenParams::rk_per consecutive positions of one chunk (a
+// "stretch"); one work item (chunk, first position) per stretch.  rk_per is
+// an odd multiple of 8, so its word count is 2 mod 4 and a warp's byte-word
+// reads are at most 2-way bank conflicts; at the largest, 73.3 KB per CTA
+// still fit three CTAs on an SM.
 constexpr int kRkThreads = 128;
-constexpr uint32_t kRkPer = 312;  // positions per thread: a multiple of 8 whose word count (78) is
-                                  // 2 mod 4, so a warp's byte-word reads are at most 2-way bank
-                                  // conflicts; 73.3 KB per CTA still fits three CTAs per SM
-constexpr uint32_t kRkSpan = kRkThreads * kRkPer;
+constexpr uint32_t kRkPers[] = {312, 152, 72, 40, 24};
+constexpr int kRkChoices = sizeof kRkPers / sizeof *kRkPers;
+constexpr uint32_t kRkPerMax = kRkPers[0];
+__host__ __device__ constexpr uint32_t rk_span(uint32_t per) { return kRkThreads * per; }
+// stretches of a chunk of n bytes
+inline uint32_t rk_stretches(uint32_t n, uint32_t per) { return ((n + 7) / 8 * 8 + rk_span(per) - 1) / rk_span(per); }
 
 struct GenTile {
     uint32_t chunk;
@@ -126,6 +131,7 @@ struct GenParams {
     uint16_t* ranks;
     const uint2* rk_items;
     uint32_t nrk_items;
+    uint32_t rk_per;  // positions per thread (one of kRkPers)
 };
 
 // Index search samples counted features 0, 4, 8, ... of a block
@@ -143,6 +149,9 @@ enum : int {
 
 size_t stream_tile_smem();
 size_t block_smem(uint32_t lmax);
+// Choice (index into kRkPers) for a group with stretches[k] work items at
+// kRkPers[k] on a GPU of sms SMs.
+int rk_choose(const uint64_t* stretches, uint32_t sms);
 // Ranks of every position of the group's chunks into P.ranks (P.rk_items stretches).
 cudaError_t launch_stream_ranks(const GenParams& P, uint32_t grid, cudaStream_t st);
 // Tile kernels: with P.ranks set they read the precomputed ranks (and the

@@ -643,6 +643,10 @@ static int digest_stream_pipelined(sdbfg_ctx* c, const uint8_t* host_data, const
             pre_ranks = false;
         }
     }
+    // A batch of one file has its filters at slot 0: the commit writes them
+    // straight into dev_out (where the file's bound fits) and neither the scan
+    // nor the packing runs.
+    const bool solo = n == 1 && !ib && lens[0] >= kMinFile && stream_cap(lens[0]) <= out_cap;
     cudaEvent_t prev_scan = c->ev_start, prev_tiles = c->ev_start, prev2_tiles = c->ev_start;
     const uint64_t rank_half = c->d_ranks.cap / 2 / 16 * 16;  // bytes per half, 16-byte aligned
     for (size_t gi = 0; gi < groups.size(); gi++) {
@@ -654,8 +658,8 @@ static int digest_stream_pipelined(sdbfg_ctx* c, const uint8_t* host_data, const
         S.used = true;
         CUDA_TRY(c, cudaStreamWaitEvent(st, c->ev_start, 0));
         // ---- work lists (pinned host staging, copied asynchronously)
-        // rank stretches: every chunk position (to a multiple of 8), kRkSpan at a time
-        uint64_t nchunks = 0, ntiles = 0, bytes = 0, nrk = 0;
+        // rank stretches: every chunk position (to a multiple of 8), rk_span(per) at a time
+        uint64_t nchunks = 0, ntiles = 0, bytes = 0, nrks[kRkChoices] = {};
         for (uint32_t k = 0; k < g.count; k++) {
             const uint64_t len = lens[g.first + k];
             bytes += (len + 15) & ~15ull;
@@ -664,9 +668,12 @@ static int digest_stream_pipelined(sdbfg_ctx* c, const uint8_t* host_data, const
                 const uint64_t m = std::min<uint64_t>(kChunkBytes, len - pos);
                 nchunks++;
                 if (m > 64) ntiles += (m - 64 + kTileL - 1) / kTileL;
-                nrk += ((m + 7) / 8 * 8 + kRkSpan - 1) / kRkSpan;
+                for (int q = 0; q < kRkChoices; q++) nrks[q] += rk_stretches((uint32_t)m, kRkPers[q]);
             }
         }
+        const int rk = rk_choose(nrks, (uint32_t)c->sms);
+        const uint64_t nrk = nrks[rk];
+        const uint32_t rspan = rk_span(kRkPers[rk]);
         bool pre = pre_ranks && ntiles;
         if (pre && S.rk_items.ensure(nrk * sizeof(uint2)) != cudaSuccess) {
             cudaGetLastError();
@@ -726,7 +733,7 @@ static int digest_stream_pipelined(sdbfg_ctx* c, const uint8_t* host_data, const
                         for (uint32_t t0 = 0; t0 < m - 64; t0 += kTileL) ht[ti++] = GenTile{ci, t0};
                     ch.ntiles = ti - ch.first_tile;
                     if (pre)
-                        for (uint32_t s0 = 0; s0 < (m + 7) / 8 * 8; s0 += kRkSpan) hr[ri++] = make_uint2(ci, s0);
+                        for (uint32_t s0 = 0; s0 < (m + 7) / 8 * 8; s0 += rspan) hr[ri++] = make_uint2(ci, s0);
                     r8 += (m + 7) / 8;
                     hc[ci++] = ch;
                     f.nchunks++;
@@ -746,7 +753,7 @@ static int digest_stream_pipelined(sdbfg_ctx* c, const uint8_t* host_data, const
         CUDA_TRY(c, S.order.ensure(std::max<size_t>(1, tb_order)));
         CUDA_TRY(c, S.tile_out.ensure(std::max<uint64_t>(1, ntiles) * sizeof(TileOut)));
         CUDA_TRY(c, S.features.ensure(std::max<uint64_t>(1, ntiles) * 5ull * kTileCap * 4));
-        CUDA_TRY(c, S.work.ensure(std::max<uint64_t>(1, work) * 256));
+        CUDA_TRY(c, S.work.ensure(solo ? 16 : std::max<uint64_t>(1, work) * 256));
         CUDA_TRY(c, S.fix_list.ensure((ntiles + 1) * 4));
         if (tb_chunks) CUDA_TRY(c, cudaMemcpyAsync(S.chunks.p, hc, tb_chunks, cudaMemcpyHostToDevice, st));
         if (tb_tiles) CUDA_TRY(c, cudaMemcpyAsync(S.tiles.p, ht, tb_tiles, cudaMemcpyHostToDevice, st));
@@ -769,13 +776,14 @@ static int digest_stream_pipelined(sdbfg_ctx* c, const uint8_t* host_data, const
         P.nfiles = g.count;
         P.tile_out = S.tile_out.as<TileOut>();
         P.features = S.features.as<uint32_t>();
-        P.out_filters = S.work.as<uint32_t>();
+        P.out_filters = solo ? dev_out : S.work.as<uint32_t>();
         P.out_info = c->d_binfo.as<FileInfoDev>() + g.first;
         P.fix_list = S.fix_list.as<uint32_t>();
         if (pre) {
             P.ranks = c->d_ranks.as<uint16_t>() + (gi & 1) * (rank_half / 2);
             P.rk_items = S.rk_items.as<uint2>();
             P.nrk_items = (uint32_t)nrk;
+            P.rk_per = kRkPers[rk];
         }
         const uint32_t cap_grid = (uint32_t)c->sms * 3 * 16;
         // the groups' tile kernels run one after another (each fills the GPU),
@@ -792,11 +800,16 @@ static int digest_stream_pipelined(sdbfg_ctx* c, const uint8_t* host_data, const
             TIMED_LAUNCH_ON(c, "k_stream_tiles", st, launch_stream_tiles(P, std::min<uint32_t>(P.ntiles, cap_grid), st));
         if (P.nchunks) {
             if (P.ntiles) {
-                CUDA_TRY(c, cudaMemsetAsync(P.fix_list, 0, 4, st));
-                TIMED_LAUNCH_ON(c, "k_stream_fails", st,
-                                launch_stream_fails(P, std::min<uint32_t>((P.ntiles + 255) / 256, cap_grid), st));
+                const uint32_t resident = (uint32_t)c->sms * 5;
+                if (P.ntiles <= resident) {  // one tile per CTA: no list
+                    P.fix_list = nullptr;
+                } else {
+                    CUDA_TRY(c, cudaMemsetAsync(P.fix_list, 0, 4, st));
+                    TIMED_LAUNCH_ON(c, "k_stream_fails", st,
+                                    launch_stream_fails(P, std::min<uint32_t>((P.ntiles + 255) / 256, cap_grid), st));
+                }
                 TIMED_LAUNCH_ON(c, "k_stream_fix_list", st,
-                                launch_stream_fix_list(P, std::min<uint32_t>(P.ntiles, (uint32_t)c->sms * 5), st));
+                                launch_stream_fix_list(P, std::min<uint32_t>(P.ntiles, resident), st));
             }
             TIMED_LAUNCH_ON(c, "k_stream_fix", st,
                             launch_stream_fix(P, std::min<uint32_t>(P.nchunks, cap_grid), st));
@@ -813,6 +826,10 @@ static int digest_stream_pipelined(sdbfg_ctx* c, const uint8_t* host_data, const
         } else {
             TIMED_LAUNCH_ON(c, "k_stream_commit", st,
                             launch_stream_commit(P, std::min<uint32_t>(g.count, cap_grid), st));
+        }
+        if (solo) {
+            CUDA_TRY(c, cudaEventRecord(S.done, st));
+            break;
         }
         // output slots follow input order: scan after the previous group's scan
         CUDA_TRY(c, cudaStreamWaitEvent(st, prev_scan, 0));
@@ -837,14 +854,15 @@ static int digest_stream_pipelined(sdbfg_ctx* c, const uint8_t* host_data, const
     std::vector<uint64_t> off(n);
     uint64_t flags_total[2] = {0, 0};
     uint32_t flags[2] = {0, 0};
-    if (n) {
-        CUDA_TRY(c, cudaMemcpyAsync(info.data(), c->d_binfo.p, n * sizeof(FileInfoDev), cudaMemcpyDeviceToHost, c->stream));
+    if (n) CUDA_TRY(c, cudaMemcpyAsync(info.data(), c->d_binfo.p, n * sizeof(FileInfoDev), cudaMemcpyDeviceToHost, c->stream));
+    if (n && !solo) {
         CUDA_TRY(c, cudaMemcpyAsync(off.data(), c->d_boff.p, n * sizeof(uint64_t), cudaMemcpyDeviceToHost, c->stream));
+        CUDA_TRY(c, cudaMemcpyAsync(flags_total, c->d_total.p, 8, cudaMemcpyDeviceToHost, c->stream));
     }
-    CUDA_TRY(c, cudaMemcpyAsync(flags_total, c->d_total.p, 8, cudaMemcpyDeviceToHost, c->stream));
     CUDA_TRY(c, cudaMemcpyAsync(flags, c->d_counters.p, sizeof flags, cudaMemcpyDeviceToHost, c->stream));
     CUDA_TRY(c, cudaStreamSynchronize(c->stream));
     if (flags[1]) return fail(c, SDBFG_ERR_CUDA, "internal error: stream digest exceeded its filter bound");
+    if (solo) flags_total[0] = info[0].bf_count;
     if (flags_total[0] > out_cap)
         return fail(c, SDBFG_ERR_CAPACITY, "output capacity %llu filters < %llu needed", (unsigned long long)out_cap,
                     (unsigned long long)flags_total[0]);
