@@ -159,13 +159,17 @@ static_assert(((kTileL + 64) / 15 + 8) * 4 <= (kTileL + 64 + kLead) * 2, "the li
 
 // Ranks [Q0, RE) of a tile from the chunk's precomputed ranks (src = the
 // chunk's first rank, 16-byte aligned; Q0 is a multiple of 64, and the
-// chunk's ranks extend to a multiple of 8), eight per 16-byte load.
+// chunk's ranks extend to a multiple of 8), eight per 16-byte load.  The
+// last 64 positions have rank 0 (a dd block inside a longer run of ranks has
+// a size that is a multiple of 8, so they are whole loads there).
+template <bool kBlock>
 __device__ inline void load_ranks(const uint16_t* __restrict__ src, const TileGeom& g, uint16_t* dst) {
     const uint32_t n8 = (g.RE - g.Q0 + 7) / 8;
     const uint4* s4 = reinterpret_cast<const uint4*>(src + g.Q0);
 #pragma unroll 4
     for (uint32_t i = threadIdx.x; i < n8; i += blockDim.x) {
-        const uint4 v = __ldg(s4 + i);
+        uint4 v = __ldg(s4 + i);
+        if (kBlock && g.Q0 + 8 * i >= g.n - kWin) v = make_uint4(0, 0, 0, 0);
         uint32_t* d = reinterpret_cast<uint32_t*>(dst + pidx(8 * i));
         d[0] = v.x;
         d[1] = v.y;
@@ -640,14 +644,14 @@ __device__ __forceinline__ ChainState walk_segment(const TileGeom& g, const Tile
 // starts speculatively `lead` steps early.  Writes sig_in / tau_out.
 // kPre: the ranks come from pre_ranks (the chunk's precomputed ranks)
 // instead of the chunk bytes.
-template <bool kPre = false>
+template <bool kPre = false, bool kBlock = kPre>
 __device__ void tile_pipeline(const uint8_t* __restrict__ chunk, const TileGeom& g, const TileSmem& s,
                               const uint16_t* rank_tab, const int32_t* dtab, const uint64_t* entry,
                               uint64_t* sig_in, uint64_t* tau_out, uint32_t lead, long long* tm,
                               const uint16_t* pre_ranks = nullptr) {
     stamp(tm, 0);
     if constexpr (kPre) {
-        load_ranks(pre_ranks, g, s.ranks);
+        load_ranks<kBlock>(pre_ranks, g, s.ranks);
         __syncthreads();
         stamp(tm, 1);
     } else {
@@ -689,12 +693,12 @@ __device__ void tile_pipeline(const uint8_t* __restrict__ chunk, const TileGeom&
             if (t == 0 && entry) {
                 st = unpack_state(*entry);
             } else {
-                // lead-in (never below Q0, since every lead <= kLead); a lead-in
+                // lead-in, not below the first simulated step; a lead-in
                 // from step 0 makes the walk exact.  The tile's first segment
                 // has the same lead as the others (a longer one would hold up
                 // its warp): its rare mis-speculation costs a tile recompute
                 // in k_stream_fix.
-                const uint32_t Ls = St > lead ? St - lead : 0;
+                const uint32_t Ls = St - min(St - g.Q0, lead);
                 st = walk(g, s, Ls, St, st, (Credit<1>*)nullptr);
             }
             s.sig[t] = pack_state(st);
@@ -878,7 +882,7 @@ __device__ void stream_tile_body(const GenParams& P, uint32_t tile, const uint64
     TileOut* out = P.tile_out + tile;
     long long tm[9];
     const uint8_t* chunk = P.data + C.data_off;
-    tile_pipeline<kPre>(chunk, g, s, rank_tab, dt, entry, &out->sig_in, &out->tau_out, P.lead,
+    tile_pipeline<kPre, false>(chunk, g, s, rank_tab, dt, entry, &out->sig_in, &out->tau_out, P.lead,
                         P.phase ? tm : nullptr, kPre ? P.ranks + (size_t)C.rank_off8 * 8 : nullptr);
     const uint32_t nown = g.SE > g.t0 ? g.SE - g.t0 : 0;
     __shared__ uint32_t counts[kGenThreads / 32];
@@ -1742,6 +1746,18 @@ __global__ void k_pred_dirty(const uint32_t* __restrict__ a, const uint32_t* __r
 }
 
 // ------------------------------------------------------------ block mode
+// kPre: the block's ranks come from k_stream_ranks (64-byte windows do not
+// know about blocks; only a block's last 64 positions have rank 0), and the
+// block is walked as one or two tiles of kBlkL steps, the second entered
+// with the first one's exit state.  55 KB of shared memory then hold four
+// blocks on an SM.  Without (block sizes that are no multiple of 8, or no
+// room for the ranks) the whole block is ranked and walked at once, two
+// blocks to an SM.  A 1 GiB image at 16 KiB blocks: ranks 1.6 ms and this
+// kernel 6.6 ms; with the ranks in the tile 10.9 ms, most of it the set-up of
+// 96 threads' windows for 170 positions each.
+constexpr uint32_t kBlkL = 8192;
+static_assert(kBlkL / kSegs == 64 && kBlkL % 64 == 0, "a segment is one block of the full-rescan table");
+
 __device__ inline TileGeom block_geom(uint32_t n) {
     TileGeom g;
     g.n = n;
@@ -1755,32 +1771,94 @@ __device__ inline TileGeom block_geom(uint32_t n) {
     return g;
 }
 
-__global__ void __launch_bounds__(kGenThreads) k_block_digest(GenParams P) {
+// tile h of a block with precomputed ranks: entered with a known state, so
+// no lead-in before its first credited step
+__device__ inline TileGeom block_tile_geom(uint32_t n, uint32_t h) {
+    TileGeom g;
+    g.n = n;
+    g.t0 = h * kBlkL;
+    g.S0 = g.t0 >= 64 ? g.t0 - 64 : 0;
+    g.Q0 = g.S0;
+    g.L = min(kBlkL, n - kWin - g.t0);
+    g.SE = g.t0 + g.L;
+    g.RE = min(g.SE + 64, n);
+    g.BE = n;
+    return g;
+}
+
+// ranks | fres (afterwards the candidate list and the insert's owner masks) |
+// scores of the whole block | sig | tau | misc
+constexpr uint32_t kBlkRanks = align_up(padded_len(kBlkL + 128 + 8) * 2, 16), kBlkFres = align_up(padded_len(kBlkL + 64) * 2, 16);
+constexpr uint32_t kBlkList = align_up(((kMaxBlockBytes - 64 + 64) / 15 + 8) * 4, 16);
+static_assert(kBlkList + kOwnBytes <= kBlkFres, "list and owner masks fit the full-rescan table");
+constexpr uint32_t kBlkSmem = kBlkRanks + kBlkFres + align_up(kMaxBlockBytes + 32, 16) + 2 * kSegs * 8 + 64 * 4;
+__device__ inline TileSmem carve_block_pre(uint8_t* p) {
+    TileSmem s;
+    s.bytes32 = nullptr;
+    s.hist = nullptr;
+    s.ranks = reinterpret_cast<uint16_t*>(p); p += kBlkRanks;
+    s.fres = reinterpret_cast<uint16_t*>(p);
+    s.list = reinterpret_cast<uint32_t*>(p);
+    s.own = reinterpret_cast<uint32_t*>(p + kBlkList); p += kBlkFres;
+    s.score32 = reinterpret_cast<uint32_t*>(p); p += align_up(kMaxBlockBytes + 32, 16);
+    s.sig = reinterpret_cast<uint64_t*>(p); p += kSegs * 8;
+    s.tau = reinterpret_cast<uint64_t*>(p); p += kSegs * 8;
+    s.misc = reinterpret_cast<uint32_t*>(p);
+    return s;
+}
+
+template <bool kPre>
+__global__ void __launch_bounds__(kGenThreads, kPre ? 4 : 1) k_block_digest(GenParams P) {
     extern __shared__ __align__(16) uint8_t smem[];
-    __shared__ int32_t dtab[65];
     __shared__ uint32_t histo[66];
     __shared__ uint32_t counts[kGenThreads / 32];
     __shared__ uint32_t filt[64];
     __shared__ uint32_t hsh[kGenThreads][5];
     __shared__ int state[4];  // k, allowed, hashed, done
-    for (uint32_t i = threadIdx.x; i < 65; i += blockDim.x) dtab[i] = i < 64 ? (int32_t)P.ent_tab[i + 1] - (int32_t)P.ent_tab[i] : 0;
-    __syncthreads();
-    __shared__ uint16_t s_rank[(SDBF_RANK_BINS + 7) / 8 * 8];
-    for (uint32_t i = threadIdx.x; i < SDBF_RANK_BINS; i += blockDim.x) s_rank[i] = P.rank_tab[i];
-    __syncthreads();
-    const uint16_t* rank_tab = s_rank;
-    TileSmem s = carve(smem, P.block_lmax);
+    const uint16_t* rank_tab = nullptr;
+    const int32_t* dt = nullptr;
+    if constexpr (!kPre) {
+        __shared__ int32_t dtab[65];
+        __shared__ uint16_t s_rank[(SDBF_RANK_BINS + 7) / 8 * 8];
+        for (uint32_t i = threadIdx.x; i < 65; i += blockDim.x) dtab[i] = i < 64 ? (int32_t)P.ent_tab[i + 1] - (int32_t)P.ent_tab[i] : 0;
+        for (uint32_t i = threadIdx.x; i < SDBF_RANK_BINS; i += blockDim.x) s_rank[i] = P.rank_tab[i];
+        __syncthreads();
+        rank_tab = s_rank;
+        dt = dtab;
+    }
+    TileSmem s = kPre ? carve_block_pre(smem) : carve(smem, P.block_lmax);
     for (uint32_t b = blockIdx.x; b < P.nchunks; b += gridDim.x) {
         const GenChunk C = P.chunks[b];
-        const TileGeom g = block_geom(C.n);
-        tile_pipeline(P.data + C.data_off, g, s, rank_tab, dtab, nullptr, nullptr, nullptr, P.lead, nullptr);
+        const uint8_t* chunk = P.data + C.data_off;
+        const uint32_t nown = C.n - kWin;
+        if constexpr (kPre) {
+            __shared__ uint64_t carry;
+            const uint32_t ntile = (nown + kBlkL - 1) / kBlkL;
+            for (uint32_t h = 0; h < ntile; h++) {
+                const TileGeom g = block_tile_geom(C.n, h);
+                TileSmem st = s;
+                st.score32 += g.t0 / 4;
+                tile_pipeline<true>(chunk, g, st, nullptr, nullptr, h ? &carry : nullptr, nullptr, nullptr, P.lead, nullptr,
+                                    P.ranks + (size_t)C.rank_off8 * 8);
+                if (threadIdx.x == 0) carry = *reinterpret_cast<uint64_t*>(&s.misc[10]);
+                __syncthreads();
+            }
+        } else {
+            tile_pipeline(chunk, block_geom(C.n), s, rank_tab, dt, nullptr, nullptr, nullptr, P.lead, nullptr);
+        }
         const uint8_t* sc = reinterpret_cast<const uint8_t*>(s.score32);
-        const uint32_t nown = g.SE;
         if (threadIdx.x < 66) histo[threadIdx.x] = 0;
         if (threadIdx.x < 64) filt[threadIdx.x] = 0;
         __syncthreads();
         if (C.kind == 0) {
-            for (uint32_t o = threadIdx.x; o < nown; o += blockDim.x) atomicAdd(&histo[sc[o]], 1u);
+            // only scores from the threshold on are looked at: most positions
+            // have score 0, and their additions to one bin would be serial
+            const uint32_t t4 = kThreshold * 0x01010101u;
+            for (uint32_t wd = threadIdx.x; wd < (nown + 3) / 4; wd += blockDim.x) {
+                uint32_t w = s.score32[wd];
+                if (4 * wd + 4 > nown) w &= (1u << (8 * (nown - 4 * wd))) - 1u;
+                for (uint32_t f = sel4(w, t4); f; f &= f - 1u) atomicAdd(&histo[(w >> (8 * (__ffs(f) - 1))) & 0xFFu], 1u);
+            }
             __syncthreads();
             if (threadIdx.x == 0) {
                 // thresholding of thread_gen_block_sdbf (sdbf_core.cc:271-276);
@@ -1816,7 +1894,10 @@ __global__ void __launch_bounds__(kGenThreads) k_block_digest(GenParams P) {
             if (ci < ncand) {
                 const uint32_t p = s.list[ci];
                 uint32_t w[16], h[5];
-                load_be16(s.bytes32, p, w);
+                if constexpr (kPre)
+                    load_be16_global(chunk + p, w);
+                else
+                    load_be16(s.bytes32, p, w);
                 sha1_feature(w, h);
 #pragma unroll
                 for (int q = 0; q < 5; q++) hsh[threadIdx.x][q] = h[q];
@@ -2049,10 +2130,18 @@ cudaError_t launch_stream_commit(const GenParams& P, uint32_t grid, cudaStream_t
     return cudaGetLastError();
 }
 
-cudaError_t launch_block(const GenParams& P, uint32_t grid, cudaStream_t st) {
-    const size_t sm = block_smem(P.block_lmax);
-    cudaFuncSetAttribute(k_block_digest, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    if (P.nchunks) k_block_digest<<<grid, kGenThreads, sm, st>>>(P);
+cudaError_t launch_block(const GenParams& P, uint32_t sms, cudaStream_t st) {
+    if (P.nchunks == 0) return cudaSuccess;
+    if (P.ranks) {
+        cudaFuncSetAttribute(k_block_digest<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBlkSmem);
+        cudaFuncSetAttribute(k_block_digest<true>, cudaFuncAttributePreferredSharedMemoryCarveout,
+                             (int)cudaSharedmemCarveoutMaxShared);
+        k_block_digest<true><<<min(P.nchunks, sms * 4 * 8), kGenThreads, kBlkSmem, st>>>(P);
+    } else {
+        const size_t sm = block_smem(P.block_lmax);
+        cudaFuncSetAttribute(k_block_digest<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+        k_block_digest<false><<<min(P.nchunks, sms * 2 * 8), kGenThreads, sm, st>>>(P);
+    }
     return cudaGetLastError();
 }
 

@@ -36,7 +36,7 @@ struct GenChunk {
     uint32_t ntiles;      // stream: tiles of this chunk
     uint32_t filter;      // block: output filter index
     uint32_t kind;        // block: 0 full block (histogram threshold), 1 tail (16 / 192)
-    uint32_t rank_off8;   // stream, ranks precomputed: the chunk's first rank in GenParams::ranks / 8
+    uint32_t rank_off8;   // ranks precomputed: the chunk's (block's) first rank in GenParams::ranks / 8
 };
 
 // Precomputed ranks of a stream launch group: k_stream_ranks gives each CTA
@@ -190,6 +190,8 @@ cudaError_t launch_pred_dirty(const GenParams& P, const uint32_t* a, const uint3
 // 256-byte filter, the big filter and bf_count / last_count / big-filter count.
 constexpr uint32_t kCkptTiles = 32;
 constexpr uint32_t kCkptWords = 64 + 4096 + 4;
-cudaError_t launch_block(const GenParams& P, uint32_t grid, cudaStream_t st);
+// Block mode; with P.ranks set (every block's GenChunk::rank_off8 into it) the
+// ranks are read, else computed.
+cudaError_t launch_block(const GenParams& P, uint32_t sms, cudaStream_t st);
 
 }  // namespace sdbfg

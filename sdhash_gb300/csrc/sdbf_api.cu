@@ -274,20 +274,39 @@ static int digest_group_device(sdbfg_ctx* c, const uint8_t* dev_base, const std:
     P.counters = c->d_counters.as<uint32_t>();
     P.lead = c->lead;
     if (dd) {
-        std::vector<GenChunk> chunks;
+        // Ranks ahead of the block kernel (2 bytes per input byte, in runs of
+        // whole blocks) where a block's ranks start 16-byte aligned; slabs
+        // bound their buffer.
+        struct Slab {
+            uint32_t first_chunk, nchunks, first_run, nruns;
+            uint64_t r8, stretches[kRkChoices];
+        };
+        std::vector<GenChunk> chunks, runs;
+        std::vector<Slab> slabs{Slab{}};
         uint32_t lmax = 0;
+        const uint64_t run_bytes = kChunkBytes / (2 * dd) * (2 * dd);  // a multiple of 16 with dd % 8 == 0
+        uint64_t most8 = 0;
         for (uint32_t k = 0; k < g.count; k++) {
             const uint32_t i = g.first + k;
             if (lens[i] < kMinFile) continue;
-            const uint64_t qt = lens[i] / dd, rem = lens[i] % dd;
-            uint64_t slot = res[i].filter_offset;
-            for (uint64_t b = 0; b < qt; b++) {
-                chunks.push_back({dev_off[k] + b * dd, dd, i, 0, 0, (uint32_t)(slot + b), 0});
-                lmax = std::max<uint32_t>(lmax, dd - 64);
-            }
-            if (rem >= kMinFile) {
-                chunks.push_back({dev_off[k] + qt * dd, (uint32_t)rem, i, 0, 0, (uint32_t)(slot + qt), 1});
-                lmax = std::max<uint32_t>(lmax, (uint32_t)rem - 64);
+            const uint64_t used = lens[i] % dd >= kMinFile ? lens[i] : lens[i] / dd * dd;  // full blocks and a counted tail
+            for (uint64_t pos = 0; pos < used; pos += run_bytes) {
+                const uint32_t m = (uint32_t)std::min<uint64_t>(run_bytes, used - pos);
+                if (slabs.back().r8 && (slabs.back().r8 * 8 + m) > kBlockSlabBytes)
+                    slabs.push_back(Slab{(uint32_t)chunks.size(), 0, (uint32_t)runs.size(), 0, 0, {}});
+                Slab& s = slabs.back();
+                for (uint32_t b = 0; b < m; b += dd) {
+                    const uint32_t len = std::min(dd, m - b);
+                    chunks.push_back({dev_off[k] + pos + b, len, i, 0, 0, (uint32_t)(res[i].filter_offset + (pos + b) / dd),
+                                      len < dd ? 1u : 0u, (uint32_t)(s.r8 + b / 8)});
+                    lmax = std::max<uint32_t>(lmax, len - 64);
+                    s.nchunks++;
+                }
+                runs.push_back({dev_off[k] + pos, m, i, 0, 0, 0, 0, (uint32_t)s.r8});
+                s.nruns++;
+                for (int q = 0; q < kRkChoices; q++) s.stretches[q] += rk_stretches(m, kRkPers[q]);
+                s.r8 += (m + 7) / 8;
+                most8 = std::max(most8, s.r8);
             }
         }
         if (chunks.empty()) return SDBFG_OK;
@@ -302,8 +321,45 @@ static int digest_group_device(sdbfg_ctx* c, const uint8_t* dev_base, const std:
         P.nprobes = c->probe_counts;
         P.feats = c->feat_words;
         P.block_lmax = (lmax + 63) / 64 * 64;
-        const uint32_t grid = (uint32_t)std::min<size_t>(chunks.size(), (size_t)c->sms * 2 * 8);
-        TIMED_LAUNCH(c, "k_block_digest", launch_block(P, grid, st));
+        std::vector<uint2> items;
+        std::vector<uint32_t> first_item, per;
+        for (const Slab& s : slabs) {
+            const int q = rk_choose(s.stretches, (uint32_t)c->sms);
+            first_item.push_back((uint32_t)items.size());
+            per.push_back(kRkPers[q]);
+            for (uint32_t r = 0; r < s.nruns; r++)
+                for (uint32_t s0 = 0; s0 < (runs[s.first_run + r].n + 7) / 8 * 8; s0 += rk_span(per.back()))
+                    items.push_back(make_uint2(s.first_run + r, s0));
+        }
+        first_item.push_back((uint32_t)items.size());
+        bool pre = c->pre_ranks && dd % 8 == 0;
+        if (pre && (c->d_ranks.ensure(most8 * 16 + 256) != cudaSuccess ||
+                    c->d_files.ensure(runs.size() * sizeof(GenChunk)) != cudaSuccess ||
+                    c->d_tiles.ensure(items.size() * sizeof(uint2)) != cudaSuccess)) {
+            cudaGetLastError();
+            c->d_ranks.release();
+            pre = false;
+        }
+        if (!pre) {
+            TIMED_LAUNCH(c, "k_block_digest", launch_block(P, (uint32_t)c->sms, st));
+        } else {
+            CUDA_TRY(c, cudaMemcpyAsync(c->d_files.p, runs.data(), runs.size() * sizeof(GenChunk), cudaMemcpyHostToDevice, st));
+            CUDA_TRY(c, cudaMemcpyAsync(c->d_tiles.p, items.data(), items.size() * sizeof(uint2), cudaMemcpyHostToDevice, st));
+            P.ranks = c->d_ranks.as<uint16_t>();
+            for (size_t k = 0; k < slabs.size(); k++) {
+                GenParams R = P;
+                R.chunks = c->d_files.as<GenChunk>();
+                R.rk_items = c->d_tiles.as<uint2>() + first_item[k];
+                R.nrk_items = first_item[k + 1] - first_item[k];
+                R.rk_per = per[k];
+                TIMED_LAUNCH(c, "k_stream_ranks",
+                             launch_stream_ranks(R, std::min<uint32_t>(R.nrk_items, (uint32_t)c->sms * 3 * 16), st));
+                GenParams B = P;
+                B.chunks = P.chunks + slabs[k].first_chunk;
+                B.nchunks = slabs[k].nchunks;
+                TIMED_LAUNCH(c, "k_block_digest", launch_block(B, (uint32_t)c->sms, st));
+            }
+        }
         // the chunk table must outlive the async copy
         CUDA_TRY(c, cudaStreamSynchronize(st));
         return SDBFG_OK;
