@@ -63,7 +63,7 @@ struct TileSmem {
     uint32_t* list;        // selected positions (relative to t0)
     uint64_t* sig;         // per-segment entry state
     uint64_t* tau;         // per-segment exit state
-    uint32_t* own;         // block mode, insert phase: 2,048 owner masks over dead space
+    uint32_t* own;         // block mode, insert phase: 2,048 owners over dead space
     uint32_t* misc;        // scalars
 };
 
@@ -739,79 +739,28 @@ __device__ void tile_pipeline(const uint8_t* __restrict__ chunk, const TileGeom&
 }
 
 // ------------------------------------------- phase 6: ordered compaction
-// Writes the positions (relative to t0) with score > thr (or >= thr when
-// ge) among [t0, t0+nown) into s.list in ascending order; returns count.
-// Each warp owns a contiguous run of score words; lanes read consecutive
-// 32-bit words (4 positions each), so the reads are conflict-free.  A
-// position's place in the list comes from four ballots (one per byte of
-// the word): the selected positions of earlier lanes, plus those earlier in
-// the lane's own word.
-__device__ __forceinline__ uint32_t word_flags(const uint32_t* sc32, uint32_t wd, uint32_t nown, uint32_t thr,
-                                               bool ge) {
-    const uint32_t w = sc32[wd];
-    // per byte: bit 7 set when selected (bytes are scores <= 65 and the
-    // threshold byte is <= 66, so no byte borrows from its neighbour)
-    const uint32_t t4 = (ge ? thr : thr + 1) * 0x01010101u;
-    const uint32_t hb = ((w | 0x80808080u) - t4) & 0x80808080u;
-    uint32_t f = (hb >> 7 | hb >> 14 | hb >> 21 | hb >> 28) & 0xFu;
-    const uint32_t p0 = 4 * wd;
-    if (p0 + 4 > nown) f &= (p0 >= nown) ? 0u : ((1u << (nown - p0)) - 1u);
-    return f;
-}
-
-__device__ uint32_t compact(const TileSmem& s, uint32_t nown, uint32_t thr, bool ge, uint32_t* tmp_counts) {
-    const uint32_t nwords = (nown + 3) / 4;
-    const uint32_t nwarps = blockDim.x / 32, lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const uint32_t per = ((nwords + nwarps - 1) / nwarps + 31) / 32 * 32;
-    const uint32_t w0 = min(nwords, wid * per), w1 = min(nwords, w0 + per);
-    uint32_t c = 0;
-    for (uint32_t wd = w0 + lane; wd < w1; wd += 32) c += __popc(word_flags(s.score32, wd, nown, thr, ge));
-    c = __reduce_add_sync(0xffffffffu, c);
-    if (lane == 0) tmp_counts[wid] = c;
-    __syncthreads();
-    uint32_t base = 0, total = 0;
-    for (uint32_t w = 0; w < nwarps; w++) {
-        if (w < wid) base += tmp_counts[w];
-        total += tmp_counts[w];
-    }
-    const uint32_t lt = (1u << lane) - 1u;
-    for (uint32_t wd0 = w0; wd0 < w1; wd0 += 32) {
-        const uint32_t wd = wd0 + lane;
-        const uint32_t f = wd < w1 ? word_flags(s.score32, wd, nown, thr, ge) : 0u;
-        const uint32_t m0 = __ballot_sync(0xffffffffu, f & 1u), m1 = __ballot_sync(0xffffffffu, f & 2u);
-        const uint32_t m2 = __ballot_sync(0xffffffffu, f & 4u), m3 = __ballot_sync(0xffffffffu, f & 8u);
-        uint32_t pos = base + __popc(m0 & lt) + __popc(m1 & lt) + __popc(m2 & lt) + __popc(m3 & lt);
-#pragma unroll
-        for (int b = 0; b < 4; b++)
-            if ((f >> b) & 1u) s.list[pos++] = 4 * wd + b;
-        base += __popc(m0) + __popc(m1) + __popc(m2) + __popc(m3);
-    }
-    __syncthreads();
-    return total;
-}
-
-// Stream tiles (threshold 16): one pass.  Warp w writes its selected
-// positions to its own list s.list[w * kWarpList ..] and their number to
-// counts[w]; feature f of the tile is entry f - (the counts of earlier
-// warps) of the first warp list that reaches it.  A lane reads 16 scores
-// (one 16-byte load; a warp's 32 loads are one contiguous 512-byte run) and
-// gets their selection bits from four byte-parallel compares; a shuffle scan
-// of the lanes' counts places them.  A warp's range holds at most 2,048
-// positions, so at most (2048 + 64) / 17 = 124 of them reach a score of 17
-// (each step credits one position in [i, i+64]).
-constexpr uint32_t kWarpList = 128;
+// The positions (relative to t0) whose score is at least kGe, in one pass.
+// Warp w writes its own to lists + w * stride and their number to counts[w];
+// entry f of all is entry f - (the counts of earlier warps) of the first warp
+// list that reaches it.  A lane reads 16 scores (one 16-byte load; a warp's
+// 32 loads are one contiguous 512-byte run) and gets their selection bits
+// from four byte-parallel compares; a shuffle scan of the lanes' counts
+// places them.  (Bytes are scores <= 65, so no byte borrows from its
+// neighbour.)  Each step credits one position in [i, i+64], so at most
+// (R + 64) / kGe positions of a warp's range of R reach kGe.
 __device__ __forceinline__ uint32_t sel4(uint32_t w, uint32_t t4) {
     const uint32_t hb = ((w | 0x80808080u) - t4) & 0x80808080u;
     return (hb >> 7 | hb >> 14 | hb >> 21 | hb >> 28) & 0xFu;
 }
-__device__ void compact_stream(const TileSmem& s, uint32_t nown, uint32_t* counts) {
+template <uint32_t kGe, class T>
+__device__ __forceinline__ uint32_t compact_warp(const uint32_t* score32, uint32_t nown, T* lists, uint32_t stride) {
     const uint32_t nq = (nown + 15) / 16;  // 16-position quads
     const uint32_t nwarps = blockDim.x / 32, lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const uint32_t per = ((nq + nwarps - 1) / nwarps + 31) / 32 * 32;
     const uint32_t q0 = min(nq, wid * per), q1 = min(nq, q0 + per);
-    uint32_t* list = s.list + wid * kWarpList;
-    const uint4* sc4 = reinterpret_cast<const uint4*>(s.score32);
-    const uint32_t t4 = (kThreshold + 1) * 0x01010101u;
+    T* list = lists + wid * stride;
+    const uint4* sc4 = reinterpret_cast<const uint4*>(score32);
+    const uint32_t t4 = kGe * 0x01010101u;
     uint32_t n = 0;
     for (uint32_t qb = q0; qb < q1; qb += 32) {
         const uint32_t q = qb + lane;
@@ -830,14 +779,14 @@ __device__ void compact_stream(const TileSmem& s, uint32_t nown, uint32_t* count
         }
         uint32_t pos = n + incl - c;
         while (m) {
-            list[pos++] = 16 * q + (uint32_t)(__ffs(m) - 1);
+            list[pos++] = (T)(16 * q + (uint32_t)(__ffs(m) - 1));
             m &= m - 1u;
         }
         n += __shfl_sync(0xffffffffu, incl, 31);
     }
-    if (lane == 0) counts[wid] = n;
-    __syncthreads();
+    return n;
 }
+constexpr uint32_t kWarpList = 128;  // stream tiles: at most (2,048 + 64) / 17 = 124 per warp
 
 // ---------------------------------------------------------- stream tiles
 __device__ inline TileGeom stream_geom(uint32_t n, uint32_t t0) {
@@ -887,7 +836,9 @@ __device__ void stream_tile_body(const GenParams& P, uint32_t tile, const uint64
     const uint32_t nown = g.SE > g.t0 ? g.SE - g.t0 : 0;
     __shared__ uint32_t counts[kGenThreads / 32];
     static_assert(kGenThreads / 32 == 4 && 4 * kWarpList <= (kTileL + 64) / 15 + 8, "stream list layout");
-    compact_stream(s, nown, counts);
+    const uint32_t nsel = compact_warp<kThreshold + 1>(s.score32, nown, s.list, kWarpList);
+    if ((threadIdx.x & 31) == 0) counts[threadIdx.x >> 5] = nsel;
+    __syncthreads();
     const uint32_t c1 = counts[0], c2 = c1 + counts[1], c3 = c2 + counts[2], nf = c3 + counts[3];
     stamp(P.phase ? tm : nullptr, 6);
     // SHA-1 of each selected feature (sdbf_core.cc:103-105)
@@ -1198,11 +1149,6 @@ struct CommitSmem {
 // barrier of the window's threads (the loading warp does not take part)
 __device__ __forceinline__ void commit_sync() { asm volatile("bar.sync 1, %0;" ::"n"(kCmWin) : "memory"); }
 
-__device__ inline uint32_t lanemask_le() {
-    uint32_t m;
-    asm("mov.u32 %0, %%lanemask_le;" : "=r"(m));
-    return m;
-}
 __device__ inline uint32_t lanemask_lt() {
     uint32_t m;
     asm("mov.u32 %0, %%lanemask_lt;" : "=r"(m));
@@ -1753,8 +1699,8 @@ __global__ void k_pred_dirty(const uint32_t* __restrict__ a, const uint32_t* __r
 // blocks on an SM.  Without (block sizes that are no multiple of 8, or no
 // room for the ranks) the whole block is ranked and walked at once, two
 // blocks to an SM.  A 1 GiB image at 16 KiB blocks: ranks 1.6 ms and this
-// kernel 6.6 ms; with the ranks in the tile 10.9 ms, most of it the set-up of
-// 96 threads' windows for 170 positions each.
+// kernel 5.1 ms; with the ranks in the tile it took 4.3 ms more than both,
+// most of it the set-up of 96 threads' windows for 170 positions each.
 constexpr uint32_t kBlkL = 8192;
 static_assert(kBlkL / kSegs == 64 && kBlkL % 64 == 0, "a segment is one block of the full-rescan table");
 
@@ -1786,20 +1732,19 @@ __device__ inline TileGeom block_tile_geom(uint32_t n, uint32_t h) {
     return g;
 }
 
-// ranks | fres (afterwards the candidate list and the insert's owner masks) |
-// scores of the whole block | sig | tau | misc
+// ranks | fres (afterwards the insert's owner table) | scores of the whole
+// block | sig | tau | misc
 constexpr uint32_t kBlkRanks = align_up(padded_len(kBlkL + 128 + 8) * 2, 16), kBlkFres = align_up(padded_len(kBlkL + 64) * 2, 16);
-constexpr uint32_t kBlkList = align_up(((kMaxBlockBytes - 64 + 64) / 15 + 8) * 4, 16);
-static_assert(kBlkList + kOwnBytes <= kBlkFres, "list and owner masks fit the full-rescan table");
+static_assert(kOwnBytes <= kBlkFres, "the owner table fits the full-rescan table");
 constexpr uint32_t kBlkSmem = kBlkRanks + kBlkFres + align_up(kMaxBlockBytes + 32, 16) + 2 * kSegs * 8 + 64 * 4;
 __device__ inline TileSmem carve_block_pre(uint8_t* p) {
     TileSmem s;
     s.bytes32 = nullptr;
     s.hist = nullptr;
     s.ranks = reinterpret_cast<uint16_t*>(p); p += kBlkRanks;
+    s.list = nullptr;
     s.fres = reinterpret_cast<uint16_t*>(p);
-    s.list = reinterpret_cast<uint32_t*>(p);
-    s.own = reinterpret_cast<uint32_t*>(p + kBlkList); p += kBlkFres;
+    s.own = reinterpret_cast<uint32_t*>(p); p += kBlkFres;
     s.score32 = reinterpret_cast<uint32_t*>(p); p += align_up(kMaxBlockBytes + 32, 16);
     s.sig = reinterpret_cast<uint64_t*>(p); p += kSegs * 8;
     s.tau = reinterpret_cast<uint64_t*>(p); p += kSegs * 8;
@@ -1807,14 +1752,44 @@ __device__ inline TileSmem carve_block_pre(uint8_t* p) {
     return s;
 }
 
+// Selection and ordered insert (kind 0: thread_gen_block_sdbf's histogram
+// threshold, sdbf_core.cc:271-276; kind 1, a tail: 16, sdbf_core.cc:315).
+// The block's positions of score >= 15 are listed once (a threshold is never
+// lower), the histogram counts the list, every warp finds the threshold from
+// its suffix sums, and each warp drops the entries below it from its list.
+// The insert (gen_block_hash, sdbf_core.cc:157-183) takes kGenThreads
+// candidates at once, one per thread: a candidate is eligible if its score is
+// above the threshold k, or equal to it while `allowed` lasts; an eligible one
+// sets its 5 filter bits and is counted if one was new -- unset before, with
+// this candidate as its smallest holder (a table of the smallest candidate
+// per filter bit; the key's high part counts passes down, so a pass overrides
+// its predecessors).  A pass takes every candidate as eligible, then keeps
+// those before the first one counted past the allowance (it is skipped and
+// the rest re-run with the allowance spent) and stops after the one that
+// reaches 192.
+// (One warp that inserted 32 candidates at a time after the whole CTA had
+// counted all 16 K scores one by one and compacted them in two passes: 54 K
+// of a block's 119 K cycles, 6.6 ms for a 1 GiB image; now 5.1 ms.)
+constexpr uint32_t kBlkWarpList = ((kMaxBlockBytes / (kGenThreads / 32)) + 64) / 15 + 3;  // scores >= 15 in a warp's range
+
+// Index of the n-th (from 1) set bit of a mask of kGenThreads bits that has as many.
+__device__ __forceinline__ uint32_t nth_bit(const uint32_t* m, uint32_t n) {
+    uint32_t w = 0;
+    while (n > (uint32_t)__popc(m[w])) n -= __popc(m[w++]);
+    return 32 * w + __fns(m[w], 0, (int)n);
+}
+
 template <bool kPre>
 __global__ void __launch_bounds__(kGenThreads, kPre ? 4 : 1) k_block_digest(GenParams P) {
     extern __shared__ __align__(16) uint8_t smem[];
     __shared__ uint32_t histo[66];
-    __shared__ uint32_t counts[kGenThreads / 32];
+    constexpr uint32_t kWarps = kGenThreads / 32;
+    static_assert(kWarps == 4, "candidate lists are walked as four");
+    __shared__ uint32_t counts[kWarps];
     __shared__ uint32_t filt[64];
-    __shared__ uint32_t hsh[kGenThreads][5];
-    __shared__ int state[4];  // k, allowed, hashed, done
+    __shared__ uint16_t lists[kWarps][kBlkWarpList];
+    __shared__ uint32_t madd[kWarps], maddk[kWarps];  // candidates counted in a pass; those of score k
+    const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const uint16_t* rank_tab = nullptr;
     const int32_t* dt = nullptr;
     if constexpr (!kPre) {
@@ -1831,6 +1806,8 @@ __global__ void __launch_bounds__(kGenThreads, kPre ? 4 : 1) k_block_digest(GenP
         const GenChunk C = P.chunks[b];
         const uint8_t* chunk = P.data + C.data_off;
         const uint32_t nown = C.n - kWin;
+        if (threadIdx.x < 66) histo[threadIdx.x] = 0;
+        if (threadIdx.x < 64) filt[threadIdx.x] = 0;
         if constexpr (kPre) {
             __shared__ uint64_t carry;
             const uint32_t ntile = (nown + kBlkL - 1) / kBlkL;
@@ -1847,159 +1824,155 @@ __global__ void __launch_bounds__(kGenThreads, kPre ? 4 : 1) k_block_digest(GenP
             tile_pipeline(chunk, block_geom(C.n), s, rank_tab, dt, nullptr, nullptr, nullptr, P.lead, nullptr);
         }
         const uint8_t* sc = reinterpret_cast<const uint8_t*>(s.score32);
-        if (threadIdx.x < 66) histo[threadIdx.x] = 0;
-        if (threadIdx.x < 64) filt[threadIdx.x] = 0;
+        uint16_t* list = lists[wid];
+        uint32_t nw = compact_warp<kThreshold - 1>(s.score32, nown, &lists[0][0], kBlkWarpList);
+        __syncwarp();
+        if (C.kind == 0)
+            for (uint32_t i = lane; i < nw; i += 32) atomicAdd(&histo[sc[list[i]]], 1u);
+        uint4* own4 = reinterpret_cast<uint4*>(s.own);
+        for (uint32_t i = threadIdx.x; i < kOwnBytes / 16; i += kGenThreads) own4[i] = make_uint4(~0u, ~0u, ~0u, ~0u);
         __syncthreads();
+        // threshold k: the largest score >= 16 that more than 192 positions
+        // reach (15 if none does); the allowance is what those above it leave
+        uint32_t k = kThreshold, allowed = kMaxElemDD;
         if (C.kind == 0) {
-            // only scores from the threshold on are looked at: most positions
-            // have score 0, and their additions to one bin would be serial
-            const uint32_t t4 = kThreshold * 0x01010101u;
-            for (uint32_t wd = threadIdx.x; wd < (nown + 3) / 4; wd += blockDim.x) {
-                uint32_t w = s.score32[wd];
-                if (4 * wd + 4 > nown) w &= (1u << (8 * (nown - 4 * wd))) - 1u;
-                for (uint32_t f = sel4(w, t4); f; f &= f - 1u) atomicAdd(&histo[(w >> (8 * (__ffs(f) - 1))) & 0xFFu], 1u);
+            static_assert(66 - kThreshold == 2 * 25, "two scores per lane");
+            const uint32_t c0 = lane < 25 ? histo[kThreshold + 2 * lane] : 0u;
+            const uint32_t c1 = lane < 25 ? histo[kThreshold + 1 + 2 * lane] : 0u;
+            uint32_t s0 = c0 + c1;  // positions of score >= 16 + 2 lane
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+                const uint32_t y = __shfl_down_sync(0xffffffffu, s0, d);
+                if (lane + d < 32) s0 += y;
             }
-            __syncthreads();
-            if (threadIdx.x == 0) {
-                // thresholding of thread_gen_block_sdbf (sdbf_core.cc:271-276);
-                // k may end at 15 when the loop does not break
-                int k = 65;
-                uint32_t sum = 0;
-                for (; k >= kThreshold; k--) {
-                    if (sum <= (uint32_t)kMaxElemDD && sum + histo[k] > (uint32_t)kMaxElemDD) break;
-                    sum += histo[k];
-                }
-                state[0] = k;
-                state[1] = kMaxElemDD - (int)sum;
+            const uint32_t s1 = s0 - c0;  // of score >= 17 + 2 lane
+            const uint32_t over = __ballot_sync(0xffffffffu, s0 > (uint32_t)kMaxElemDD);
+            const uint32_t odd = __ballot_sync(0xffffffffu, s1 > (uint32_t)kMaxElemDD);
+            const uint32_t L = over ? 31 - __clz(over) : 0;
+            const bool hi = (odd >> L) & 1u;
+            const uint32_t above = __shfl_sync(0xffffffffu, hi ? s1 - c1 : s1, L);
+            const uint32_t all = __shfl_sync(0xffffffffu, s0, 0);
+            k = over ? kThreshold + 2 * L + hi : kThreshold - 1;
+            allowed = kMaxElemDD - (over ? above : all);
+        }
+        if (k >= kThreshold) {
+            uint32_t m = 0;
+            for (uint32_t i0 = 0; i0 < nw; i0 += 32) {
+                const bool have = i0 + lane < nw;
+                const uint16_t p = have ? list[i0 + lane] : (uint16_t)0;
+                const bool sel = have && sc[p] >= k;
+                const uint32_t bm = __ballot_sync(0xffffffffu, sel);
+                if (sel) list[m + __popc(bm & lanemask_lt())] = p;
+                m += __popc(bm);
+                __syncwarp();
             }
-        } else if (threadIdx.x == 0) {
-            state[0] = kThreshold;  // tail block (sdbf_core.cc:315)
-            state[1] = kMaxElemDD;
+            nw = m;
         }
-        if (threadIdx.x == 0) {
-            state[2] = 0;
-            state[3] = 0;
-        }
+        if (lane == 0) counts[wid] = nw;
         __syncthreads();
-        const uint32_t k = (uint32_t)state[0];
-        const uint32_t ncand = compact(s, nown, k, true, counts);
-        // owner masks of the insert passes, over space dead once the scores
-        // are known
-        uint32_t* own = s.own;
-        for (uint32_t i = threadIdx.x; i < 2048; i += blockDim.x) own[i] = 0;
-        __syncthreads();
-        for (uint32_t base = 0; base < ncand; base += blockDim.x) {
-            if (state[3]) break;
-            const uint32_t ci = base + threadIdx.x;
-            if (ci < ncand) {
-                const uint32_t p = s.list[ci];
-                uint32_t w[16], h[5];
+        const uint32_t n1 = counts[0], n2 = n1 + counts[1], n3 = n2 + counts[2], ncand = n3 + counts[3];
+        uint32_t hashed = 0, pass = 0xFFFFu;
+        for (uint32_t base = 0; base < ncand && hashed < (uint32_t)kMaxElemDD; base += kGenThreads) {
+            const uint32_t f = base + threadIdx.x;
+            const bool have = f < ncand;
+            uint32_t h[5] = {0, 0, 0, 0, 0};
+            bool isk = false;
+            if (have) {
+                const uint32_t wl = (f >= n1) + (f >= n2) + (f >= n3);
+                const uint32_t before = wl == 0 ? 0u : wl == 1 ? n1 : wl == 2 ? n2 : n3;
+                const uint32_t p = lists[wl][f - before];
+                isk = sc[p] == k;
+                uint32_t w[16];
                 if constexpr (kPre)
                     load_be16_global(chunk + p, w);
                 else
                     load_be16(s.bytes32, p, w);
                 sha1_feature(w, h);
-#pragma unroll
-                for (int q = 0; q < 5; q++) hsh[threadIdx.x][q] = h[q];
             }
-            __syncthreads();
-            if (threadIdx.x < 32) {
-                // gen_block_hash ordered insert (sdbf_core.cc:157-183) by warp 0,
-                // 32 candidates per pass: a candidate is eligible if its score
-                // is above k, or equal to k while `allowed` lasts; an eligible
-                // one sets its 5 filter bits and is counted if one was new.
-                // A pass takes every lane as eligible, then keeps the lanes
-                // before the first one that was counted past the allowance
-                // (that lane is skipped and the rest re-run with the allowance
-                // spent) and stops after the lane that reaches 192.
-                const uint32_t lane = threadIdx.x;
-                int allowed = state[1];
-                int hashed = state[2];
-                const uint32_t lim = min(ncand - base, (uint32_t)blockDim.x);
-                for (uint32_t g0 = 0; g0 < lim && hashed < kMaxElemDD; g0 += 32) {
-                    const uint32_t q = g0 + lane;
-                    const bool have = q < lim;
-                    const bool isK = have && sc[s.list[base + (have ? q : 0)]] == k;
-                    uint32_t a[5];
+            uint32_t start = 0;
+            while (true) {
+                const bool act = have && threadIdx.x >= start && (!isk || allowed > 0);
+                const uint32_t key = (--pass << 16) | threadIdx.x;
+                uint32_t fresh = 0;
+                if (act) {
 #pragma unroll
-                    for (int z = 0; z < 5; z++) a[z] = have ? (hsh[q][z] & kBfMask) : 0u;
-                    uint32_t start = 0;
-                    bool stop = false;
-                    while (true) {
-                        const bool act = have && lane >= start && (!isK || allowed > 0);
-                        if (!__any_sync(0xffffffffu, act)) break;
-                        uint32_t fpre = 0;
-                        if (act) {
-#pragma unroll
-                            for (int z = 0; z < 5; z++) {
-                                fpre |= ((filt[a[z] >> 5] >> (a[z] & 31)) & 1u) << z;
-                                atomicOr(&own[a[z]], 1u << lane);
-                            }
-                        }
-                        __syncwarp();
-                        uint32_t m[5];
-#pragma unroll
-                        for (int z = 0; z < 5; z++) m[z] = act ? own[a[z]] : 0u;
-                        __syncwarp();
-                        if (act) {
-#pragma unroll
-                            for (int z = 0; z < 5; z++) own[a[z]] = 0;
-                        }
-                        bool added = false;
-#pragma unroll
-                        for (int z = 0; z < 5; z++)
-                            if (act && !((fpre >> z) & 1u) && (uint32_t)(__ffs(m[z]) - 1) == lane) added = true;
-                        const uint32_t cm = __ballot_sync(0xffffffffu, added);
-                        const uint32_t ckm = __ballot_sync(0xffffffffu, added && isK);
-                        const uint32_t le = lanemask_le();
-                        const uint32_t om =
-                            __ballot_sync(0xffffffffu, added && isK && __popc(ckm & le) > allowed);
-                        const uint32_t L = om ? (uint32_t)(__ffs(om) - 1) : 32u;
-                        const uint32_t fm =
-                            __ballot_sync(0xffffffffu, added && hashed + __popc(cm & le) == kMaxElemDD);
-                        const uint32_t H = fm ? (uint32_t)(__ffs(fm) - 1) : 32u;
-                        const uint32_t rx = min(L, H + 1);  // lanes [0, rx) stand
-                        const uint32_t keep = rx >= 32 ? 0xffffffffu : ((1u << rx) - 1u);
-                        if (act && lane < rx) {
-#pragma unroll
-                            for (int z = 0; z < 5; z++) atomicOr(&filt[a[z] >> 5], 1u << (a[z] & 31));
-                            if (added) {
-                                const uint32_t idx = (uint32_t)hashed + __popc(cm & lanemask_lt());
-                                if (P.feats) {  // index build: every counted feature (sdbf_core.cc:164-167)
-                                    uint32_t* fw = P.feats + (size_t)C.filter * kFeatWords + idx * 5;
-#pragma unroll
-                                    for (int z = 0; z < 5; z++) fw[z] = hsh[q][z];
-                                }
-                                if (P.probes && (idx & 3) == 0) {  // index search sample (sdbf_core.cc:168-175)
-                                    uint32_t* pr = P.probes + (size_t)C.filter * kProbeWords + (idx >> 2) * 5;
-#pragma unroll
-                                    for (int z = 0; z < 5; z++) pr[z] = hsh[q][z];
-                                }
-                            }
-                        }
-                        hashed += __popc(cm & keep);
-                        allowed -= __popc(ckm & keep);
-                        __syncwarp();
-                        if (H < L) {  // the 192nd element: the block is full
-                            stop = true;
-                            break;
-                        }
-                        if (L >= 32) break;
-                        start = L + 1;  // lane L is skipped (allowance spent)
+                    for (int z = 0; z < 5; z++) {
+                        const uint32_t a = h[z] & kBfMask;
+                        fresh |= (~(filt[a >> 5] >> (a & 31)) & 1u) << z;
+                        atomicMin(&s.own[a], key);
                     }
-                    if (stop) break;
                 }
+                __syncthreads();
+                bool added = false;
+                if (act) {
+#pragma unroll
+                    for (int z = 0; z < 5; z++) added |= ((fresh >> z) & 1u) && s.own[h[z] & kBfMask] == key;
+                }
+                const uint32_t bm = __ballot_sync(0xffffffffu, added), bk = __ballot_sync(0xffffffffu, added && isk);
                 if (lane == 0) {
-                    state[1] = allowed;
-                    state[2] = hashed;
-                    if (hashed >= kMaxElemDD) state[3] = 1;
+                    madd[wid] = bm;
+                    maddk[wid] = bk;
                 }
+                __syncthreads();
+                uint32_t total = 0, totalk = 0, before = __popc(bm & lanemask_lt());
+#pragma unroll
+                for (uint32_t q = 0; q < kWarps; q++) {
+                    total += __popc(madd[q]);
+                    totalk += __popc(maddk[q]);
+                    if (q < wid) before += __popc(madd[q]);
+                }
+                uint32_t end = kGenThreads;  // candidates [start, end) stand
+                bool skip = false, full = false;
+                if (totalk > allowed) {
+                    end = nth_bit(maddk, allowed + 1);
+                    skip = true;
+                }
+                if (hashed + total >= (uint32_t)kMaxElemDD) {
+                    const uint32_t last = nth_bit(madd, kMaxElemDD - hashed);  // the block's 192nd
+                    if (last < end) {
+                        end = last + 1;
+                        full = true;
+                    }
+                }
+                if (act && threadIdx.x < end) {
+#pragma unroll
+                    for (int z = 0; z < 5; z++) {
+                        const uint32_t a = h[z] & kBfMask;
+                        atomicOr(&filt[a >> 5], 1u << (a & 31));
+                    }
+                    if (added) {
+                        const uint32_t idx = hashed + before;
+                        if (P.feats) {  // index build: every counted feature (sdbf_core.cc:164-167)
+                            uint32_t* fw = P.feats + (size_t)C.filter * kFeatWords + idx * 5;
+#pragma unroll
+                            for (int z = 0; z < 5; z++) fw[z] = h[z];
+                        }
+                        if (P.probes && (idx & 3) == 0) {  // index search sample (sdbf_core.cc:168-175)
+                            uint32_t* pr = P.probes + (size_t)C.filter * kProbeWords + (idx >> 2) * 5;
+#pragma unroll
+                            for (int z = 0; z < 5; z++) pr[z] = h[z];
+                        }
+                    }
+                }
+                if (end < (uint32_t)kGenThreads) {  // count those that stand only
+                    total = totalk = 0;
+#pragma unroll
+                    for (uint32_t q = 0; q < kWarps; q++) {
+                        const uint32_t keep = end >= 32 * q + 32 ? 0xffffffffu : end <= 32 * q ? 0u : (1u << (end - 32 * q)) - 1u;
+                        total += __popc(madd[q] & keep);
+                        totalk += __popc(maddk[q] & keep);
+                    }
+                }
+                hashed += total;
+                allowed -= totalk;
+                __syncthreads();  // the filter's bits are set, the masks read
+                if (full || !skip) break;
+                start = end + 1;  // candidate `end` is skipped (allowance spent)
             }
-            __syncthreads();
         }
         if (threadIdx.x < 64) P.out_filters[(size_t)C.filter * 64 + threadIdx.x] = filt[threadIdx.x];
-        if (threadIdx.x == 0) P.out_counts[C.filter] = (uint16_t)state[2];
-        if (threadIdx.x == 0 && P.nprobes) P.nprobes[C.filter] = (uint8_t)((state[2] + 3) >> 2);
+        if (threadIdx.x == 0) P.out_counts[C.filter] = (uint16_t)hashed;
+        if (threadIdx.x == 0 && P.nprobes) P.nprobes[C.filter] = (uint8_t)((hashed + 3) >> 2);
         __syncthreads();
     }
 }

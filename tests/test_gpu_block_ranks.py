@@ -34,6 +34,33 @@ def test_block_sizes(ctx, oracle, dd):
         assert got[k].to_string() == oracle.digest(names[k], f, dd).to_string(), (dd, len(f))
 
 
+def crowded(n):
+    """Content whose blocks select more than 192 positions, many of equal score."""
+    d = synth.random_bytes(44, 0, n)
+    for k, o in enumerate(range(0, n, 40_000)):
+        m = min(30_000, n - o)
+        d[o:o + m] = np.resize(synth.random_bytes(45, k, 65 + 37 * k), m)
+    return d
+
+
+CONTENT = {
+    "random": lambda: synth.random_bytes(46, 0, 600_007),
+    "random_low": lambda: synth.random_bytes(46, 1, 600_007) & 0x3F,
+    "periods": lambda: crowded(1_000_003),
+    "ramps": lambda: (np.arange(500_001) // 3 % 251).astype(np.uint8),
+    "zeros": lambda: np.zeros(100_000, dtype=np.uint8),
+}
+
+
+@pytest.mark.parametrize("dd", [16_384, 16_379, 4096, 2048, 512])
+@pytest.mark.parametrize("name", list(CONTENT))
+def test_selection(ctx, oracle, name, dd):
+    """The threshold, its allowance and the 192nd element of a block."""
+    data = CONTENT[name]().tobytes()
+    got = ctx.digest_buffers([data], [name], dd)[0]
+    assert got.to_string() == oracle.digest(name, data, dd).to_string()
+
+
 @pytest.mark.parametrize("lead", [0, 128])
 @pytest.mark.parametrize("dd", [8264, 16_384])
 def test_leads(ctx, oracle, dd, lead):
