@@ -23,6 +23,7 @@ namespace sdbfg_host {
 constexpr uint32_t kMaxTilesPerLaunch = 1u << 18;  // 2 GiB of stream input per launch group
 constexpr uint64_t kMaxBytesPerLaunch = 2ull << 30;
 constexpr uint64_t kBlockSlabBytes = 256ull << 20;  // block-mode input whose ranks are held at once (512 MiB of them)
+constexpr uint64_t kFirstHostSlabBytes = 16ull << 20;  // first slab of a host-input block batch (each later one at most twice it)
 constexpr uint64_t kFirstHostGroupBytes = 256ull << 20;  // first group of a host-input stream batch
 constexpr uint32_t kMinFile = 512;                 // MIN_FILE_SIZE (sdbf_defines.h:56)
 constexpr uint64_t kPairsPerLaunch = 1ull << 22;
@@ -147,6 +148,7 @@ struct sdbfg_ctx {
     uint32_t lead = kDefaultLead;
     bool pre_ranks = true;  // stream mode: ranks by k_stream_ranks ahead of the tile kernel
     DevBuf d_ranks;         // their ranks (two halves, by launch-group parity)
+    bool reads_pageable = false;  // the device reads pageable memory through the host's page tables
     // constant tables
     DevBuf d_rank, d_ent, d_cut, d_cut64;
     // generation buffers

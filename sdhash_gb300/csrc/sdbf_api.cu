@@ -30,6 +30,9 @@ extern "C" int sdbfg_ctx_create(int device, sdbfg_ctx** out) {
         return SDBFG_ERR_CUDA;
     }
     cudaDeviceGetAttribute(&c->sms, cudaDevAttrMultiProcessorCount, device);
+    int pageable = 0;
+    cudaDeviceGetAttribute(&pageable, cudaDevAttrPageableMemoryAccessUsesHostPageTables, device);
+    c->reads_pageable = pageable != 0;
     if (cudaStreamCreateWithFlags(&c->own, cudaStreamNonBlocking) != cudaSuccess) {
         delete c;
         return SDBFG_ERR_CUDA;
@@ -258,115 +261,6 @@ std::vector<Group> make_groups(const uint64_t* lens, uint32_t n, uint32_t dd,
 
 }  // namespace
 
-// Core: inputs for files [g.first, g.first+g.count) are in device memory at
-// dev_base + dev_off[i].  Writes packed filters to dev_out (+ counts) at the
-// offsets in results[] (already assigned for block mode, assigned here for
-// stream mode starting at *next_slot).
-static int digest_group_device(sdbfg_ctx* c, const uint8_t* dev_base, const std::vector<uint64_t>& dev_off,
-                               const uint64_t* lens, const Group& g, uint32_t dd, uint32_t* dev_out,
-                               uint16_t* dev_counts, sdbfg_digest_result* res, uint64_t* next_slot,
-                               uint64_t out_cap) {
-    cudaStream_t st = c->stream;
-    GenParams P{};
-    P.data = dev_base;
-    P.rank_tab = c->d_rank.as<uint16_t>();
-    P.ent_tab = c->d_ent.as<uint32_t>();
-    P.counters = c->d_counters.as<uint32_t>();
-    P.lead = c->lead;
-    if (dd) {
-        // Ranks ahead of the block kernel (2 bytes per input byte, in runs of
-        // whole blocks) where a block's ranks start 16-byte aligned; slabs
-        // bound their buffer.
-        struct Slab {
-            uint32_t first_chunk, nchunks, first_run, nruns;
-            uint64_t r8, stretches[kRkChoices];
-        };
-        std::vector<GenChunk> chunks, runs;
-        std::vector<Slab> slabs{Slab{}};
-        uint32_t lmax = 0;
-        const uint64_t run_bytes = kChunkBytes / (2 * dd) * (2 * dd);  // a multiple of 16 with dd % 8 == 0
-        uint64_t most8 = 0;
-        for (uint32_t k = 0; k < g.count; k++) {
-            const uint32_t i = g.first + k;
-            if (lens[i] < kMinFile) continue;
-            const uint64_t used = lens[i] % dd >= kMinFile ? lens[i] : lens[i] / dd * dd;  // full blocks and a counted tail
-            for (uint64_t pos = 0; pos < used; pos += run_bytes) {
-                const uint32_t m = (uint32_t)std::min<uint64_t>(run_bytes, used - pos);
-                if (slabs.back().r8 && (slabs.back().r8 * 8 + m) > kBlockSlabBytes)
-                    slabs.push_back(Slab{(uint32_t)chunks.size(), 0, (uint32_t)runs.size(), 0, 0, {}});
-                Slab& s = slabs.back();
-                for (uint32_t b = 0; b < m; b += dd) {
-                    const uint32_t len = std::min(dd, m - b);
-                    chunks.push_back({dev_off[k] + pos + b, len, i, 0, 0, (uint32_t)(res[i].filter_offset + (pos + b) / dd),
-                                      len < dd ? 1u : 0u, (uint32_t)(s.r8 + b / 8)});
-                    lmax = std::max<uint32_t>(lmax, len - 64);
-                    s.nchunks++;
-                }
-                runs.push_back({dev_off[k] + pos, m, i, 0, 0, 0, 0, (uint32_t)s.r8});
-                s.nruns++;
-                for (int q = 0; q < kRkChoices; q++) s.stretches[q] += rk_stretches(m, kRkPers[q]);
-                s.r8 += (m + 7) / 8;
-                most8 = std::max(most8, s.r8);
-            }
-        }
-        if (chunks.empty()) return SDBFG_OK;
-        CUDA_TRY(c, c->d_chunks.ensure(chunks.size() * sizeof(GenChunk)));
-        CUDA_TRY(c, cudaMemcpyAsync(c->d_chunks.p, chunks.data(), chunks.size() * sizeof(GenChunk),
-                                    cudaMemcpyHostToDevice, st));
-        P.chunks = c->d_chunks.as<GenChunk>();
-        P.nchunks = (uint32_t)chunks.size();
-        P.out_filters = dev_out;
-        P.out_counts = dev_counts;
-        P.probes = c->probe_words;
-        P.nprobes = c->probe_counts;
-        P.feats = c->feat_words;
-        P.block_lmax = (lmax + 63) / 64 * 64;
-        std::vector<uint2> items;
-        std::vector<uint32_t> first_item, per;
-        for (const Slab& s : slabs) {
-            const int q = rk_choose(s.stretches, (uint32_t)c->sms);
-            first_item.push_back((uint32_t)items.size());
-            per.push_back(kRkPers[q]);
-            for (uint32_t r = 0; r < s.nruns; r++)
-                for (uint32_t s0 = 0; s0 < (runs[s.first_run + r].n + 7) / 8 * 8; s0 += rk_span(per.back()))
-                    items.push_back(make_uint2(s.first_run + r, s0));
-        }
-        first_item.push_back((uint32_t)items.size());
-        bool pre = c->pre_ranks && dd % 8 == 0;
-        if (pre && (c->d_ranks.ensure(most8 * 16 + 256) != cudaSuccess ||
-                    c->d_files.ensure(runs.size() * sizeof(GenChunk)) != cudaSuccess ||
-                    c->d_tiles.ensure(items.size() * sizeof(uint2)) != cudaSuccess)) {
-            cudaGetLastError();
-            c->d_ranks.release();
-            pre = false;
-        }
-        if (!pre) {
-            TIMED_LAUNCH(c, "k_block_digest", launch_block(P, (uint32_t)c->sms, st));
-        } else {
-            CUDA_TRY(c, cudaMemcpyAsync(c->d_files.p, runs.data(), runs.size() * sizeof(GenChunk), cudaMemcpyHostToDevice, st));
-            CUDA_TRY(c, cudaMemcpyAsync(c->d_tiles.p, items.data(), items.size() * sizeof(uint2), cudaMemcpyHostToDevice, st));
-            P.ranks = c->d_ranks.as<uint16_t>();
-            for (size_t k = 0; k < slabs.size(); k++) {
-                GenParams R = P;
-                R.chunks = c->d_files.as<GenChunk>();
-                R.rk_items = c->d_tiles.as<uint2>() + first_item[k];
-                R.nrk_items = first_item[k + 1] - first_item[k];
-                R.rk_per = per[k];
-                TIMED_LAUNCH(c, "k_stream_ranks",
-                             launch_stream_ranks(R, std::min<uint32_t>(R.nrk_items, (uint32_t)c->sms * 3 * 16), st));
-                GenParams B = P;
-                B.chunks = P.chunks + slabs[k].first_chunk;
-                B.nchunks = slabs[k].nchunks;
-                TIMED_LAUNCH(c, "k_block_digest", launch_block(B, (uint32_t)c->sms, st));
-            }
-        }
-        // the chunk table must outlive the async copy
-        CUDA_TRY(c, cudaStreamSynchronize(st));
-        return SDBFG_OK;
-    }
-    return fail(c, SDBFG_ERR_ARG, "internal: stream mode goes through the pipeline");
-}
-
 // ---------------------------------------------------- stream pipeline
 // Output slots of one launch group: exclusive scan of the files' filter
 // counts, continuing from the running total of the earlier groups
@@ -414,23 +308,45 @@ __global__ void k_pack_group(const uint32_t* __restrict__ work, const GenFile* _
     }
 }
 
-// Staging of pinned host inputs: each piece (at most kStagePiece bytes of
-// one input) is read straight from host memory through the device's mapping
-// of the pinned buffer and written to its 16-byte aligned staging offset;
-// 16-byte loads where the source allows them, else 4-byte or single bytes.
+// Staging of host inputs: each piece (at most kStagePiece bytes of one input)
+// is read straight from host memory (host_view) and written to its 16-byte
+// aligned staging offset, 16 bytes per load.  A source off that alignment is
+// read as the aligned 16-byte words inside the piece, lane by lane, and each
+// output is put together from a lane's word and its neighbour's; only the
+// first 16 bytes and the end of such a piece go byte by byte.
 // kGatherThreads threads and few registers, so a CTA fits on an SM beside
-// the tile kernel's four.
+// the tile kernel's four.  Bound by the link to the host: 200 GB/s from pinned
+// and from pageable memory.
 constexpr int kGatherThreads = 128;
+
+// Bytes [off, off + 16) of the 32 bytes a | b (off: 1..15, the same in every lane).
+__device__ __forceinline__ uint4 shift_pair(uint4 a, uint4 b, uint32_t off) {
+    uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+    if (off & 8) {
+#pragma unroll
+        for (int k = 0; k < 6; k++) w[k] = w[k + 2];
+    }
+    if (off & 4) {
+#pragma unroll
+        for (int k = 0; k < 5; k++) w[k] = w[k + 1];
+    }
+    const uint32_t sh = 8 * (off & 3);
+    return make_uint4(__funnelshift_r(w[0], w[1], sh), __funnelshift_r(w[1], w[2], sh),
+                      __funnelshift_r(w[2], w[3], sh), __funnelshift_r(w[3], w[4], sh));
+}
+
 __global__ void __launch_bounds__(kGatherThreads) k_stage_gather(const StagePiece* __restrict__ items, uint32_t n,
                                                                   uint8_t* __restrict__ dst) {
+    const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     for (uint32_t f = blockIdx.x; f < n; f += gridDim.x) {
         const StagePiece it = items[f];
         const uint8_t* s = reinterpret_cast<const uint8_t*>(it.src);
         uint8_t* d = dst + it.dst;
+        uint4* d4 = reinterpret_cast<uint4*>(d);
+        const uint32_t off = (uint32_t)(it.src & 15);
         uint64_t done = 0;
-        if ((it.src & 15) == 0) {
+        if (off == 0) {
             const uint4* s4 = reinterpret_cast<const uint4*>(s);
-            uint4* d4 = reinterpret_cast<uint4*>(d);
             const uint64_t n4 = it.len / 16;
             uint64_t q = threadIdx.x;
             for (; q + 3 * kGatherThreads < n4; q += 4 * kGatherThreads) {
@@ -443,15 +359,63 @@ __global__ void __launch_bounds__(kGatherThreads) k_stage_gather(const StagePiec
             }
             for (; q < n4; q += kGatherThreads) d4[q] = s4[q];
             done = n4 * 16;
-        } else if ((it.src & 3) == 0) {
-            const uint32_t* s1 = reinterpret_cast<const uint32_t*>(s);
-            uint32_t* d1 = reinterpret_cast<uint32_t*>(d);
-            const uint64_t n1 = it.len / 4;
-            for (uint64_t q = threadIdx.x; q < n1; q += kGatherThreads) d1[q] = s1[q];
-            done = n1 * 4;
+        } else {
+            // output j is made of the aligned words j and j + 1, both inside
+            // the piece for 1 <= j < end; a warp takes 31 outputs per step
+            const uint4* s4 = reinterpret_cast<const uint4*>(s - off);
+            const uint64_t words = (off + it.len) / 16;  // whole words up to the piece's end
+            const uint64_t end = words > 2 ? words - 1 : 1;
+            constexpr uint32_t kStep = 31 * (kGatherThreads / 32);
+            for (uint64_t j0 = 1 + 31 * wid; j0 < end; j0 += 4 * kStep) {
+                uint4 v[4];
+#pragma unroll
+                for (int u = 0; u < 4; u++) {
+                    const uint64_t j = j0 + u * kStep + lane;
+                    v[u] = j <= end && end > 1 ? s4[j] : make_uint4(0, 0, 0, 0);
+                }
+#pragma unroll
+                for (int u = 0; u < 4; u++) {
+                    const uint64_t j = j0 + u * kStep + lane;
+                    const uint4 nx = make_uint4(__shfl_down_sync(0xffffffffu, v[u].x, 1), __shfl_down_sync(0xffffffffu, v[u].y, 1),
+                                                __shfl_down_sync(0xffffffffu, v[u].z, 1), __shfl_down_sync(0xffffffffu, v[u].w, 1));
+                    if (lane < 31 && j < end) d4[j] = shift_pair(v[u], nx, off);
+                }
+            }
+            for (uint64_t q = threadIdx.x; q < 16 && q < it.len; q += kGatherThreads) d[q] = s[q];
+            done = 16 * end;
         }
         for (uint64_t q = done + threadIdx.x; q < it.len; q += kGatherThreads) d[q] = s[q];
     }
+}
+
+// The device's view of host memory that starts at p: the mapping of a pinned
+// buffer, or p itself where the device reads pageable memory through the
+// host's page tables; null where neither holds.
+static const uint8_t* host_view(sdbfg_ctx* c, const uint8_t* p) {
+    cudaPointerAttributes attr{};
+    const bool pinned = cudaPointerGetAttributes(&attr, p) == cudaSuccess && attr.type == cudaMemoryTypeHost &&
+                        attr.devicePointer != nullptr;
+    cudaGetLastError();
+    if (pinned) return static_cast<const uint8_t*>(attr.devicePointer) + (p - static_cast<const uint8_t*>(attr.hostPointer));
+    return c->reads_pageable ? p : nullptr;
+}
+
+static int ensure_copy_stream(sdbfg_ctx* c, size_t events) {
+    if (!c->copy_stream) {
+        int lo = 0, hi = 0;
+        CUDA_TRY(c, cudaDeviceGetStreamPriorityRange(&lo, &hi));
+        CUDA_TRY(c, cudaStreamCreateWithPriority(&c->copy_stream, cudaStreamNonBlocking, hi));
+    }
+    while (c->ev_copy.size() < events) {
+        cudaEvent_t e;
+        CUDA_TRY(c, cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+        c->ev_copy.push_back(e);
+    }
+    if (!c->ev_start) CUDA_TRY(c, cudaEventCreateWithFlags(&c->ev_start, cudaEventDisableTiming));
+    // beside the tile kernels' shared-memory / L1 split
+    cudaFuncSetAttribute(k_stage_gather, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared);
+    cudaGetLastError();
+    return SDBFG_OK;
 }
 
 static int ensure_pipeline(sdbfg_ctx* c) {
@@ -466,7 +430,7 @@ static int ensure_pipeline(sdbfg_ctx* c) {
     if (!c->ev_start) CUDA_TRY(c, cudaEventCreateWithFlags(&c->ev_start, cudaEventDisableTiming));
     // the pipeline's small kernels take the tile kernels' shared-memory / L1
     // split, so their CTAs can share an SM with them
-    for (const void* f : {(const void*)k_stage_gather, (const void*)k_scan_offsets, (const void*)k_pack_group})
+    for (const void* f : {(const void*)k_scan_offsets, (const void*)k_pack_group})
         cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared);
     cudaGetLastError();
     return SDBFG_OK;
@@ -572,34 +536,24 @@ static int digest_stream_pipelined(sdbfg_ctx* c, const uint8_t* host_data, const
     // results[] records where each input's filters are.
     // (an index build keeps input order: every file's digest depends on the
     // index inserts of the files before it)
-    // Pinned host inputs are staged whole on the device when they fit.  A
-    // gather kernel per launch group reads the group's inputs straight from
-    // host memory (the device's mapping of the pinned buffer) on a
-    // high-priority stream of its own, one event per group: the copies cost
+    // Host inputs that the device can read are staged whole on the device when
+    // they fit.  A gather kernel per launch group reads the group's inputs
+    // straight from host memory (host_view) on a high-priority stream of its own, one event per group: the copies cost
     // one launch per group instead of one API call per input (tens of
     // microseconds each), and no copy waits behind an earlier group's commit
     // or a slot's reuse.  Its small CTAs fit beside the tile kernel's.
     bool staged = false;
-    const uint8_t* host_dev = nullptr;  // the device's view of the pinned input
+    const uint8_t* host_dev = nullptr;  // the device's view of the input
     if (host_data && !ib && n) {
-        cudaPointerAttributes attr{};
-        const bool pinned = cudaPointerGetAttributes(&attr, host_data) == cudaSuccess &&
-                            attr.type == cudaMemoryTypeHost && attr.devicePointer != nullptr;
-        cudaGetLastError();
-        if (pinned)
-            host_dev = static_cast<const uint8_t*>(attr.devicePointer) +
-                       (host_data - static_cast<const uint8_t*>(attr.hostPointer));
+        host_dev = host_view(c, host_data);
         uint64_t tot = 0;
         for (uint32_t i = 0; i < n; i++) tot += (lens_in[i] + 15) & ~15ull;
         size_t freeb = 0, totb = 0;
-        if (pinned && tot <= kStageMaxBytes && cudaMemGetInfo(&freeb, &totb) == cudaSuccess &&
+        // (one pageable input: a plain copy of it)
+        const bool gather = host_dev && (n > 1 || host_dev != host_data);
+        if (gather && tot <= kStageMaxBytes && cudaMemGetInfo(&freeb, &totb) == cudaSuccess &&
             (c->d_stage_in.cap >= tot || tot <= freeb / 2)) {
             CUDA_TRY(c, c->d_stage_in.ensure(std::max<uint64_t>(16, tot)));
-            if (!c->copy_stream) {
-                int lo = 0, hi = 0;
-                CUDA_TRY(c, cudaDeviceGetStreamPriorityRange(&lo, &hi));
-                CUDA_TRY(c, cudaStreamCreateWithPriority(&c->copy_stream, cudaStreamNonBlocking, hi));
-            }
             staged = true;
         }
         cudaGetLastError();
@@ -630,11 +584,8 @@ static int digest_stream_pipelined(sdbfg_ctx* c, const uint8_t* host_data, const
             stage_off[i] = tot;
             tot += (lens[i] + 15) & ~15ull;
         }
-        while (c->ev_copy.size() < groups.size()) {
-            cudaEvent_t e;
-            CUDA_TRY(c, cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-            c->ev_copy.push_back(e);
-        }
+        rc = ensure_copy_stream(c, groups.size());
+        if (rc) return rc;
         // after the previous batch's work on the caller's stream
         CUDA_TRY(c, cudaStreamWaitEvent(c->copy_stream, c->ev_start, 0));
     }
@@ -933,6 +884,146 @@ static int digest_stream_pipelined(sdbfg_ctx* c, const uint8_t* host_data, const
     return SDBFG_OK;
 }
 
+// Block-mode digests of a launch group: inputs for files [g.first,
+// g.first+g.count) are in device memory at dev_base + dev_off[i], or are
+// brought there from host_dev + host_off[i] (the device's view of host
+// memory), slab by slab beside the kernels of the slabs before.  Writes
+// filters to dev_out (+ counts) at the offsets in results[].
+static int digest_block_group(sdbfg_ctx* c, const uint8_t* dev_base, const std::vector<uint64_t>& dev_off,
+                               const uint64_t* lens, const Group& g, uint32_t dd, uint32_t* dev_out,
+                               uint16_t* dev_counts, sdbfg_digest_result* res, const uint8_t* host_dev,
+                               const uint64_t* host_off) {
+    cudaStream_t st = c->stream;
+    GenParams P{};
+    P.data = dev_base;
+    P.rank_tab = c->d_rank.as<uint16_t>();
+    P.ent_tab = c->d_ent.as<uint32_t>();
+    P.counters = c->d_counters.as<uint32_t>();
+    P.lead = c->lead;
+    // Ranks ahead of the block kernel (2 bytes per input byte, in runs of
+    // whole blocks) where a block's ranks start 16-byte aligned; slabs
+    // bound their buffer.
+    struct Slab {
+        uint32_t first_chunk, nchunks, first_run, nruns;
+        uint64_t r8, stretches[kRkChoices];
+    };
+    std::vector<GenChunk> chunks, runs;
+    std::vector<Slab> slabs{Slab{}};
+    uint32_t lmax = 0;
+    const uint64_t run_bytes = kChunkBytes / (16 * dd) * (16 * dd);  // so every run starts 16-byte aligned
+    uint64_t most8 = 0, cap = host_dev ? kFirstHostSlabBytes : kBlockSlabBytes;
+    for (uint32_t k = 0; k < g.count; k++) {
+        const uint32_t i = g.first + k;
+        if (lens[i] < kMinFile) continue;
+        const uint64_t used = lens[i] % dd >= kMinFile ? lens[i] : lens[i] / dd * dd;  // full blocks and a counted tail
+        for (uint64_t pos = 0; pos < used; pos += run_bytes) {
+            const uint32_t m = (uint32_t)std::min<uint64_t>(run_bytes, used - pos);
+            if (slabs.back().r8 && (slabs.back().r8 * 8 + m) > cap) {
+                cap = std::min(2 * cap, kBlockSlabBytes);
+                slabs.push_back(Slab{(uint32_t)chunks.size(), 0, (uint32_t)runs.size(), 0, 0, {}});
+            }
+            Slab& s = slabs.back();
+            for (uint32_t b = 0; b < m; b += dd) {
+                const uint32_t len = std::min(dd, m - b);
+                chunks.push_back({dev_off[k] + pos + b, len, i, 0, 0, (uint32_t)(res[i].filter_offset + (pos + b) / dd),
+                                  len < dd ? 1u : 0u, (uint32_t)(s.r8 + b / 8)});
+                lmax = std::max<uint32_t>(lmax, len - 64);
+                s.nchunks++;
+            }
+            runs.push_back({dev_off[k] + pos, m, i, 0, 0, 0, 0, (uint32_t)s.r8});
+            s.nruns++;
+            for (int q = 0; q < kRkChoices; q++) s.stretches[q] += rk_stretches(m, kRkPers[q]);
+            s.r8 += (m + 7) / 8;
+            most8 = std::max(most8, s.r8);
+        }
+    }
+    if (chunks.empty()) return SDBFG_OK;
+    CUDA_TRY(c, c->d_chunks.ensure(chunks.size() * sizeof(GenChunk)));
+    CUDA_TRY(c, cudaMemcpyAsync(c->d_chunks.p, chunks.data(), chunks.size() * sizeof(GenChunk),
+                                cudaMemcpyHostToDevice, st));
+    P.chunks = c->d_chunks.as<GenChunk>();
+    P.nchunks = (uint32_t)chunks.size();
+    P.out_filters = dev_out;
+    P.out_counts = dev_counts;
+    P.probes = c->probe_words;
+    P.nprobes = c->probe_counts;
+    P.feats = c->feat_words;
+    P.block_lmax = (lmax + 63) / 64 * 64;
+    std::vector<uint2> items;
+    std::vector<uint32_t> first_item, per;
+    for (const Slab& s : slabs) {
+        const int q = rk_choose(s.stretches, (uint32_t)c->sms);
+        first_item.push_back((uint32_t)items.size());
+        per.push_back(kRkPers[q]);
+        for (uint32_t r = 0; r < s.nruns; r++)
+            for (uint32_t s0 = 0; s0 < (runs[s.first_run + r].n + 7) / 8 * 8; s0 += rk_span(per.back()))
+                items.push_back(make_uint2(s.first_run + r, s0));
+    }
+    first_item.push_back((uint32_t)items.size());
+    bool pre = c->pre_ranks && dd % 8 == 0;
+    if (pre && (c->d_ranks.ensure(most8 * 16 + 256) != cudaSuccess ||
+                c->d_files.ensure(runs.size() * sizeof(GenChunk)) != cudaSuccess ||
+                c->d_tiles.ensure(items.size() * sizeof(uint2)) != cudaSuccess)) {
+        cudaGetLastError();
+        c->d_ranks.release();
+        pre = false;
+    }
+    std::vector<StagePiece> pieces;
+    if (host_dev) {
+        std::vector<uint32_t> first_piece;
+        for (const Slab& s : slabs) {
+            first_piece.push_back((uint32_t)pieces.size());
+            for (uint32_t r = s.first_run; r < s.first_run + s.nruns; r++) {
+                const GenChunk& R = runs[r];
+                const uint64_t src = reinterpret_cast<uint64_t>(host_dev) + host_off[R.file] + (R.data_off - dev_off[R.file - g.first]);
+                for (uint64_t pos = 0; pos < R.n; pos += kStagePiece)
+                    pieces.push_back({R.data_off + pos, src + pos, std::min<uint64_t>(kStagePiece, R.n - pos)});
+            }
+        }
+        first_piece.push_back((uint32_t)pieces.size());
+        const int rc = ensure_copy_stream(c, slabs.size());
+        if (rc) return rc;
+        CUDA_TRY(c, c->d_stage_items.ensure(pieces.size() * sizeof(StagePiece)));
+        CUDA_TRY(c, cudaMemcpyAsync(c->d_stage_items.p, pieces.data(), pieces.size() * sizeof(StagePiece),
+                                    cudaMemcpyHostToDevice, st));
+        CUDA_TRY(c, cudaEventRecord(c->ev_start, st));
+        CUDA_TRY(c, cudaStreamWaitEvent(c->copy_stream, c->ev_start, 0));
+        for (size_t k = 0; k < slabs.size(); k++) {
+            const uint32_t np = first_piece[k + 1] - first_piece[k];
+            TIMED_LAUNCH_ON(c, "k_stage_gather", c->copy_stream,
+                            (k_stage_gather<<<std::min<uint32_t>(np, (uint32_t)c->sms), kGatherThreads, 0,
+                                              c->copy_stream>>>(c->d_stage_items.as<StagePiece>() + first_piece[k], np,
+                                                                const_cast<uint8_t*>(dev_base)),
+                             cudaGetLastError()));
+            CUDA_TRY(c, cudaEventRecord(c->ev_copy[k], c->copy_stream));
+        }
+    }
+    if (pre) {
+        CUDA_TRY(c, cudaMemcpyAsync(c->d_files.p, runs.data(), runs.size() * sizeof(GenChunk), cudaMemcpyHostToDevice, st));
+        CUDA_TRY(c, cudaMemcpyAsync(c->d_tiles.p, items.data(), items.size() * sizeof(uint2), cudaMemcpyHostToDevice, st));
+        P.ranks = c->d_ranks.as<uint16_t>();
+    }
+    for (size_t k = 0; k < slabs.size(); k++) {
+        if (host_dev) CUDA_TRY(c, cudaStreamWaitEvent(st, c->ev_copy[k], 0));
+        if (pre) {
+            GenParams R = P;
+            R.chunks = c->d_files.as<GenChunk>();
+            R.rk_items = c->d_tiles.as<uint2>() + first_item[k];
+            R.nrk_items = first_item[k + 1] - first_item[k];
+            R.rk_per = per[k];
+            TIMED_LAUNCH(c, "k_stream_ranks",
+                         launch_stream_ranks(R, std::min<uint32_t>(R.nrk_items, (uint32_t)c->sms * 3 * 16), st));
+        }
+        GenParams B = P;
+        B.chunks = P.chunks + slabs[k].first_chunk;
+        B.nchunks = slabs[k].nchunks;
+        TIMED_LAUNCH(c, "k_block_digest", launch_block(B, (uint32_t)c->sms, st));
+    }
+    // the tables must outlive their copies
+    CUDA_TRY(c, cudaStreamSynchronize(st));
+    return SDBFG_OK;
+}
+
 static int validate_batch(sdbfg_ctx* c, const uint64_t* offsets, const uint64_t* lens, uint32_t n, uint32_t dd,
                           sdbfg_digest_result* res) {
     if (!c || (!offsets && n) || (!lens && n) || (!res && n)) return SDBFG_ERR_ARG;
@@ -966,7 +1057,6 @@ extern "C" int sdbfg_digest_batch_device(sdbfg_ctx* c, const uint8_t* dev_data, 
     for (uint32_t i = 0; i < n; i++)
         if (offsets[i] % 16) return fail(c, SDBFG_ERR_ARG, "device input %u not 16-byte aligned", i);
     CUDA_TRY(c, cudaSetDevice(c->device));
-    uint64_t next = 0;
     if (dd) {
         const uint64_t need = assign_block_slots(lens, n, dd, res);
         if (need > out_cap) return fail(c, SDBFG_ERR_CAPACITY, "need %llu filter slots", (unsigned long long)need);
@@ -976,8 +1066,8 @@ extern "C" int sdbfg_digest_batch_device(sdbfg_ctx* c, const uint8_t* dev_data, 
                                             out_cap, res, nullptr);
     for (const Group& g : make_groups(lens, n, dd)) {
         std::vector<uint64_t> off(offsets + g.first, offsets + g.first + g.count);
-        rc = digest_group_device(c, dev_data, off, lens, g, dd, reinterpret_cast<uint32_t*>(dev_out), dev_counts, res,
-                                 &next, out_cap);
+        rc = digest_block_group(c, dev_data, off, lens, g, dd, reinterpret_cast<uint32_t*>(dev_out), dev_counts, res,
+                                nullptr, nullptr);
         if (rc) return rc;
     }
     return SDBFG_OK;
@@ -990,11 +1080,6 @@ static int digest_block_host(sdbfg_ctx* c, const uint8_t* host_data, const uint6
                              sdbfg_digest_result* res, const sdbfg_index* const* indexes, uint32_t nidx,
                              uint8_t* out_hits, const IndexBuild* ib = nullptr, uint32_t* d_first = nullptr) {
     cudaStream_t st = c->stream;
-    cudaPointerAttributes attr{};
-    const bool pinned = cudaPointerGetAttributes(&attr, host_data) == cudaSuccess &&
-                        (attr.type == cudaMemoryTypeHost || attr.type == cudaMemoryTypeManaged);
-    cudaGetLastError();
-    uint64_t next = 0;
     for (const Group& g : make_groups(lens, n, dd)) {
         // lay the group's inputs out 16-byte aligned on the device
         std::vector<uint64_t> off(g.count);
@@ -1005,13 +1090,19 @@ static int digest_block_host(sdbfg_ctx* c, const uint8_t* host_data, const uint6
         }
         CUDA_TRY(c, c->d_data.ensure(std::max<uint64_t>(bytes, 16)));
         uint8_t* d = c->d_data.as<uint8_t>();
-        // contiguous source range with the same layout -> one copy
+        // Small contiguous inputs: one copy (exactly to the last input's end).
+        // Else the gather kernel brings them over slab by slab, where the
+        // device can read them (768 fragments of 140 MB in 4 KiB to 1 MiB: one
+        // copy call per input took 8.3 ms, the gather 0.8).
         bool contiguous = true;
         for (uint32_t k = 0; k < g.count && contiguous; k++)
             contiguous = offsets[g.first + k] - offsets[g.first] == off[k];
-        if (contiguous && pinned) {
-            CUDA_TRY(c, cudaMemcpyAsync(d, host_data + offsets[g.first], bytes, cudaMemcpyHostToDevice, st));
-        } else {
+        const uint8_t* view = nullptr;
+        if (contiguous && bytes <= kFirstHostSlabBytes) {
+            const uint32_t last = g.count - 1;
+            CUDA_TRY(c, cudaMemcpyAsync(d, host_data + offsets[g.first], off[last] + lens[g.first + last],
+                                        cudaMemcpyHostToDevice, st));
+        } else if (!(view = host_view(c, host_data))) {
             for (uint32_t k = 0; k < g.count; k++) {
                 const uint32_t i = g.first + k;
                 if (lens[i] < kMinFile) continue;
@@ -1049,8 +1140,8 @@ static int digest_block_host(sdbfg_ctx* c, const uint8_t* host_data, const uint6
             saved[k] = res[g.first + k].filter_offset;
             res[g.first + k].filter_offset -= group_first_slot;
         }
-        int rc = digest_group_device(c, d, off, lens, g, dd, c->d_out_filters.as<uint32_t>(),
-                                     c->d_out_counts.as<uint16_t>(), res, &next, UINT64_MAX);
+        int rc = digest_block_group(c, d, off, lens, g, dd, c->d_out_filters.as<uint32_t>(),
+                                    c->d_out_counts.as<uint16_t>(), res, view, offsets);
         c->probe_words = nullptr;
         c->probe_counts = nullptr;
         c->feat_words = nullptr;
