@@ -41,8 +41,9 @@ extern "C" int sdbfg_set_upload(sdbfg_ctx* c, const sdbfg_digest_desc* ds, uint3
         return fail(c, SDBFG_ERR_ARG, "set too large");
     }
     s->total_filters = total;
-    std::vector<uint32_t> meta(total);
-    std::vector<uint8_t> filt(total * 256);
+    std::vector<uint8_t> image(sdbfg_set::bytes(total, n));  // the set's device memory, copied at once
+    uint8_t* filt = image.data();
+    uint32_t* meta = reinterpret_cast<uint32_t*>(filt + sdbfg_set::meta_at(total));
     s->names.resize(n);
     s->fast.assign(n, 0);
     s->bf_count.resize(n);
@@ -61,7 +62,7 @@ extern "C" int sdbfg_set_upload(sdbfg_ctx* c, const sdbfg_digest_desc* ds, uint3
         s->last_count[i] = d.elem_counts ? 0 : d.last_count;
         s->dd_block[i] = d.elem_counts ? d.dd_block_size : 0;
         s->first[i] = dig[i].first;
-        memcpy(&filt[(uint64_t)dig[i].first * 256], d.filters, (uint64_t)d.bf_count * 256);
+        memcpy(filt + (uint64_t)dig[i].first * 256, d.filters, (uint64_t)d.bf_count * 256);
         for (uint32_t f = 0; f < d.bf_count; f++) {
             // get_elem_count (sdbf_class.cc:406-415)
             uint32_t e = d.elem_counts ? d.elem_counts[f] : (f + 1 < d.bf_count ? d.max_elem : d.last_count);
@@ -75,19 +76,15 @@ extern "C" int sdbfg_set_upload(sdbfg_ctx* c, const sdbfg_digest_desc* ds, uint3
             meta[dig[i].first + f] = (h << 16) | (e & 0xFFFFu);
             if (f + 1 == d.bf_count) s->last_elem[i] = e;
         }
-        digest_stats(dig[i], meta.data());
+        digest_stats(dig[i], meta);
     }
-    if (s->d_filters.ensure(std::max<uint64_t>(1, total) * 256) || s->d_meta.ensure(std::max<uint64_t>(1, total) * 4) ||
-        s->d_digests.ensure(std::max<uint32_t>(1, n) * sizeof(CmpDigest))) {
-        s->d_filters.release();
-        s->d_meta.release();
-        s->d_digests.release();
+    if (n) memcpy(filt + sdbfg_set::digests_at(total), dig.data(), n * sizeof(CmpDigest));
+    if (s->allocate(total, n) != cudaSuccess) {
+        cudaGetLastError();
         delete s;
         return fail(c, SDBFG_ERR_NOMEM, "set upload: out of device memory");
     }
-    cudaMemcpy(s->d_filters.p, filt.data(), total * 256, cudaMemcpyHostToDevice);
-    cudaMemcpy(s->d_meta.p, meta.data(), total * 4, cudaMemcpyHostToDevice);
-    cudaMemcpy(s->d_digests.p, dig.data(), n * sizeof(CmpDigest), cudaMemcpyHostToDevice);
+    cudaMemcpy(s->d_all.p, image.data(), image.size(), cudaMemcpyHostToDevice);
     *out = s;
     return SDBFG_OK;
 }
@@ -120,9 +117,7 @@ extern "C" void sdbfg_set_free(sdbfg_set* s) {
     if (!s) return;
     cudaSetDevice(s->ctx->device);
     drop_plans(s->ctx, s->serial);
-    s->d_filters.release();
-    s->d_meta.release();
-    s->d_digests.release();
+    s->d_all.release();
     delete s;
 }
 
@@ -207,26 +202,31 @@ static int upload_plan(sdbfg_ctx* c, MatPlan* p, UnitBuilder& ub, const std::vec
     p->nsplit = (uint32_t)ub.split.size();
     p->nslots = ub.slots;
     p->filter_pairs = ub.filter_pairs;
-    CUDA_TRY(c, p->d_units.ensure(std::max<size_t>(1, units.size()) * sizeof(MatUnit)));
-    CUDA_TRY(c, p->d_targets.ensure(std::max<size_t>(1, targets.size()) * 4));
-    CUDA_TRY(c, p->d_split.ensure(std::max<size_t>(1, ub.split.size()) * sizeof(MatSplit)));
-    CUDA_TRY(c, p->d_refs.ensure(std::max<size_t>(1, ub.refs.size()) * 4));
-    if (!ub.refs.empty())
-        CUDA_TRY(c, cudaMemcpyAsync(p->d_refs.p, ub.refs.data(), ub.refs.size() * 4, cudaMemcpyHostToDevice,
-                                    c->stream));
-    CUDA_TRY(c, p->d_slots.ensure(std::max<uint64_t>(1, ub.slots) * 8));
-    CUDA_TRY(c, p->d_redo.ensure(kRedoBytes));
-    CUDA_TRY(c, p->d_counter.ensure(64));
-    cudaStream_t st = c->stream;
-    if (!units.empty())
-        CUDA_TRY(c, cudaMemcpyAsync(p->d_units.p, units.data(), units.size() * sizeof(MatUnit),
-                                    cudaMemcpyHostToDevice, st));
-    if (!targets.empty())
-        CUDA_TRY(c, cudaMemcpyAsync(p->d_targets.p, targets.data(), targets.size() * 4, cudaMemcpyHostToDevice, st));
-    if (!ub.split.empty())
-        CUDA_TRY(c, cudaMemcpyAsync(p->d_split.p, ub.split.data(), ub.split.size() * sizeof(MatSplit),
-                                    cudaMemcpyHostToDevice, st));
-    CUDA_TRY(c, cudaStreamSynchronize(st));  // host vectors go out of scope
+    const auto up = [](uint64_t v) { return (v + 255) / 256 * 256; };
+    const uint64_t at_targets = up(units.size() * sizeof(MatUnit)), at_refs = at_targets + up(targets.size() * 4),
+                   at_split = at_refs + up(ub.refs.size() * 4), at_redo = at_split + up(ub.split.size() * sizeof(MatSplit)),
+                   at_counter = at_redo + up(kRedoBytes);
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    CUDA_TRY(c, cudaStreamIsCapturing(c->stream, &cap));
+    if (cap != cudaStreamCaptureStatusNone)
+        return fail(c, SDBFG_ERR_CUDA, "a comparison's first run cannot be captured");
+    CUDA_TRY(c, p->d_all.ensure(at_counter + kMatCounterBytes + std::max<uint64_t>(1, ub.slots) * 8));
+    uint8_t* d = p->d_all.as<uint8_t>();
+    p->d_units.p = d;
+    p->d_targets.p = d + at_targets;
+    p->d_refs.p = d + at_refs;
+    p->d_split.p = d + at_split;
+    p->d_redo.p = d + at_redo;
+    p->d_counter.p = d + at_counter;
+    p->tables.resize(at_redo);
+    const auto put = [&](uint64_t at, const void* src, uint64_t bytes) {
+        if (bytes) memcpy(p->tables.data() + at, src, bytes);
+    };
+    put(0, units.data(), units.size() * sizeof(MatUnit));
+    put(at_targets, targets.data(), targets.size() * 4);
+    put(at_refs, ub.refs.data(), ub.refs.size() * 4);
+    put(at_split, ub.split.data(), ub.split.size() * sizeof(MatSplit));
+    if (at_redo) CUDA_TRY(c, cudaMemcpyAsync(d, p->tables.data(), at_redo, cudaMemcpyHostToDevice, c->stream));
     return SDBFG_OK;
 }
 
@@ -347,7 +347,7 @@ static MatParams plan_params(sdbfg_ctx* c, const MatPlan* p, const sdbfg_set* a,
     P.refs = p->d_refs.as<uint32_t>();
     P.split = p->d_split.as<MatSplit>();
     P.nsplit = p->nsplit;
-    P.slots = p->d_slots.as<double>();
+    P.slots = p->d_counter.as<double>() + kMatCounterBytes / 8;
     P.nslots = p->nslots;
     P.scores = scores;
     P.nscores = p->nscores;
@@ -355,14 +355,13 @@ static MatParams plan_params(sdbfg_ctx* c, const MatPlan* p, const sdbfg_set* a,
     P.n = p->mode == kMatModeAll ? a->n : b->n;
     P.cutoffs = c->d_cut.as<uint16_t>();
     P.cutoffs64 = c->d_cut64.as<uint16_t>();
-    P.redo = redo_list(p->d_redo.p);
+    P.redo = redo_list(p->d_redo.p, P.next_unit);
     P.error = p->d_counter.as<uint32_t>() + 1;
     P.phase = c->profile ? c->d_mphase.as<unsigned long long>() : nullptr;
     return P;
 }
 
 static int enqueue_plan(sdbfg_ctx* c, const MatPlan* p, const MatParams& P, cudaStream_t st) {
-    CUDA_TRY(c, cudaMemsetAsync(p->d_counter.p, 0, 8, st));  // work counter, error flag
     const uint32_t grid = (uint32_t)(c->sms * matrix_ctas_per_sm(p->variant));
     uint64_t launched = 0;
     TIMED_LAUNCH_ON(c, "k_matrix", st, run_matrix(P, p->variant, grid, (uint32_t)c->sms, st, &launched));
@@ -370,13 +369,24 @@ static int enqueue_plan(sdbfg_ctx* c, const MatPlan* p, const MatParams& P, cuda
     return SDBFG_OK;
 }
 
-// Runs a plan on the context stream, replaying its CUDA graph when the
-// output array is the one it was captured with.
+// Runs a plan on the context stream: launch by launch the first time (a
+// capture costs more than it saves there), and through a CUDA graph once the
+// output array is that of the run before.
 static int run_plan(sdbfg_ctx* c, MatPlan* p, const sdbfg_set* a, const sdbfg_set* b, int32_t* dev_scores) {
     cudaStream_t st = c->stream;
     const MatParams P = plan_params(c, p, a, b, dev_scores);
     matrix_ctas_per_sm(p->variant);  // sets the kernel's attributes outside any capture
     if (!c->mat_graphs || c->profile) return enqueue_plan(c, p, P, st);
+    if (p->graph_out != dev_scores) {
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        CUDA_TRY(c, cudaStreamIsCapturing(st, &cap));
+        if (cap == cudaStreamCaptureStatusNone) {
+            if (p->graph) cudaGraphExecDestroy(p->graph);
+            p->graph = nullptr;
+            p->graph_out = dev_scores;
+            return enqueue_plan(c, p, P, st);
+        }
+    }
     const uint64_t kernels = p->variant == kMatVariantTc ? 3 : 1 + (P.nsplit ? 1 : 0), before = c->launches;
     if (p->graph && p->graph_out == dev_scores) {
         CUDA_TRY(c, cudaGraphLaunch(p->graph, st));
@@ -409,12 +419,14 @@ static int run_plan(sdbfg_ctx* c, MatPlan* p, const sdbfg_set* a, const sdbfg_se
     return SDBFG_OK;
 }
 
-// waits for the plan's launches and reports a bounded wait that gave up
-static int check_plan_error(sdbfg_ctx* c, const MatPlan* p) {
-    uint32_t err = 0;
-    CUDA_TRY(c, cudaMemcpyAsync(&err, p->d_counter.as<uint32_t>() + 1, 4, cudaMemcpyDeviceToHost, c->stream));
+// Copies a run's scores to out, waits, and reports a bounded wait that gave up.
+static int fetch_scores(sdbfg_ctx* c, const MatPlan* p, int32_t* out) {
+    CUDA_TRY(c, c->h_flags.ensure(64));  // pinned: this copy does not block
+    uint32_t* err = static_cast<uint32_t*>(c->h_flags.p);
+    CUDA_TRY(c, cudaMemcpyAsync(err, p->d_counter.as<uint32_t>() + 1, 4, cudaMemcpyDeviceToHost, c->stream));
+    if (out) CUDA_TRY(c, cudaMemcpyAsync(out, c->d_scores.p, p->nscores * 4, cudaMemcpyDeviceToHost, c->stream));
     CUDA_TRY(c, cudaStreamSynchronize(c->stream));
-    if (err) return fail(c, SDBFG_ERR_CUDA, "comparison kernel: %u CTAs gave up waiting for the tensor cores", err);
+    if (*err) return fail(c, SDBFG_ERR_CUDA, "comparison kernel: %u CTAs gave up waiting for the tensor cores", *err);
     return SDBFG_OK;
 }
 
@@ -448,8 +460,7 @@ extern "C" int sdbfg_compare_all(sdbfg_ctx* c, const sdbfg_set* s, int32_t* out)
     CUDA_TRY(c, c->d_scores.ensure(p->nscores * 4));
     rc = run_plan(c, p, s, nullptr, c->d_scores.as<int32_t>());
     if (rc) return rc;
-    CUDA_TRY(c, cudaMemcpyAsync(out, c->d_scores.p, p->nscores * 4, cudaMemcpyDeviceToHost, c->stream));
-    return check_plan_error(c, p);
+    return fetch_scores(c, p, out);
 }
 
 extern "C" int sdbfg_compare_to(sdbfg_ctx* c, const sdbfg_set* q, const sdbfg_set* t, int32_t* out) {
@@ -462,8 +473,7 @@ extern "C" int sdbfg_compare_to(sdbfg_ctx* c, const sdbfg_set* q, const sdbfg_se
     CUDA_TRY(c, c->d_scores.ensure(p->nscores * 4));
     rc = run_plan(c, p, q, t, c->d_scores.as<int32_t>());
     if (rc) return rc;
-    CUDA_TRY(c, cudaMemcpyAsync(out, c->d_scores.p, p->nscores * 4, cudaMemcpyDeviceToHost, c->stream));
-    return check_plan_error(c, p);
+    return fetch_scores(c, p, out);
 }
 
 // scores (already queued into c->d_scores) -> matches on the host
@@ -504,7 +514,7 @@ extern "C" int sdbfg_compare_all_matches(sdbfg_ctx* c, const sdbfg_set* s, int32
     CUDA_TRY(c, c->d_scores.ensure(p->nscores * 4));
     rc = run_plan(c, p, s, nullptr, c->d_scores.as<int32_t>());
     if (rc) return rc;
-    if ((rc = check_plan_error(c, p))) return rc;
+    if ((rc = fetch_scores(c, p, nullptr))) return rc;
     return collect_matches(c, p->nscores, kMatModeAll, s->n, threshold, out, cap, count);
 }
 
@@ -520,7 +530,7 @@ extern "C" int sdbfg_compare_to_matches(sdbfg_ctx* c, const sdbfg_set* q, const 
     CUDA_TRY(c, c->d_scores.ensure(p->nscores * 4));
     rc = run_plan(c, p, q, t, c->d_scores.as<int32_t>());
     if (rc) return rc;
-    if ((rc = check_plan_error(c, p))) return rc;
+    if ((rc = fetch_scores(c, p, nullptr))) return rc;
     return collect_matches(c, p->nscores, kMatModeCross, t->n, threshold, out, cap, count);
 }
 
@@ -607,7 +617,7 @@ extern "C" int sdbfg_compare_autotune(sdbfg_ctx* c, const sdbfg_set* a, const sd
             cudaStream_t st = c->stream;
             float best_ms = 1e30f;
             for (int rep = 0; rep < 2; rep++) {
-                CUDA_TRY(c, cudaMemsetAsync(p->d_counter.p, 0, 8, st));
+                CUDA_TRY(c, cudaMemsetAsync(p->d_counter.p, 0, kMatCounterBytes, st));
                 CUDA_TRY(c, cudaEventRecord(e0, st));
                 const uint32_t grid = (uint32_t)(c->sms * matrix_ctas_per_sm(v));
                 CUDA_TRY(c, launch_matrix(P, v, std::max(1u, std::min(grid, P.nunits)), st));

@@ -897,8 +897,7 @@ cudaError_t run_matrix(const MatParams& P, int variant, uint32_t grid, uint32_t 
     if (variant == kMatVariantTc) {
         // sums of group units grow in the score array, split maxima in the slots
         if ((e = cudaMemsetAsync(P.scores, 0, P.nscores * 4, st))) return e;
-        if (P.nslots && (e = cudaMemsetAsync(P.slots, 0, P.nslots * 4, st))) return e;
-        if ((e = cudaMemsetAsync(P.redo.place, 0, 8, st))) return e;
+        if ((e = cudaMemsetAsync(P.next_unit, 0, kMatCounterBytes + P.nslots * 4, st))) return e;
         if ((e = launch_matrix_tc(P, grid, st))) return e;
         const uint64_t work = P.nscores / kCmpThreads + 1 + P.nsplit;
         k_matrix_finish<<<(uint32_t)(work < 8ull * sms ? work : 8ull * sms), kCmpThreads, 0, st>>>(P);
@@ -906,6 +905,7 @@ cudaError_t run_matrix(const MatParams& P, int variant, uint32_t grid, uint32_t 
         *launches += 3;
         return cudaGetLastError();
     }
+    if ((e = cudaMemsetAsync(P.next_unit, 0, kMatCounterBytes, st))) return e;
     if ((e = launch_matrix(P, variant, grid, st))) return e;
     *launches += 1 + (P.nsplit ? 1 : 0);
     return launch_matrix_finalize(P, st);

@@ -117,12 +117,15 @@ struct RedoList {
     RedoPair* list;             // kRedoPairs
     double* max;                // kRedoRows
 };
-constexpr uint64_t kRedoBytes = 64 + kRedoPairs * sizeof(RedoPair) + kRedoRows * 8;
-inline RedoList redo_list(void* p) {  // in kRedoBytes of device memory
+constexpr uint64_t kRedoBytes = kRedoPairs * sizeof(RedoPair) + kRedoRows * 8;
+inline RedoList redo_list(void* p, uint32_t* counters) {  // in kRedoBytes of device memory; its place in the counters
     uint8_t* b = static_cast<uint8_t*>(p);
-    return RedoList{reinterpret_cast<unsigned long long*>(b), reinterpret_cast<RedoPair*>(b + 64),
-                    reinterpret_cast<double*>(b + 64 + kRedoPairs * sizeof(RedoPair))};
+    return RedoList{reinterpret_cast<unsigned long long*>(counters + 2), reinterpret_cast<RedoPair*>(b),
+                    reinterpret_cast<double*>(b + kRedoPairs * sizeof(RedoPair))};
 }
+// A run's counters -- next unit, error, the redo list's place -- with the
+// slots behind them, so that one memset clears both.
+constexpr uint64_t kMatCounterBytes = 64;
 
 struct MatParams {
     const uint32_t* filters[2];

@@ -81,6 +81,13 @@ struct DevBuf {
     T* as() const { return static_cast<T*>(p); }
 };
 
+// A part of a DevBuf.
+struct DevView {
+    void* p = nullptr;
+    template <class T>
+    T* as() const { return static_cast<T*>(p); }
+};
+
 struct HostBuf {
     void* p = nullptr;
     size_t cap = 0;
@@ -155,6 +162,7 @@ struct sdbfg_ctx {
     DevBuf d_data, d_chunks, d_tiles, d_files, d_order, d_tile_out, d_features, d_work_filters, d_info, d_counters,
         d_pack_src, d_pack_dst_off, d_out_filters, d_out_counts;
     HostBuf h_stage;
+    HostBuf h_flags;  // small read-backs (pinned)
     // comparison buffers
     DevBuf d_pairs, d_scores;
     // stream-mode pipeline: two launch-group slots on their own streams
@@ -162,12 +170,16 @@ struct sdbfg_ctx {
         cudaStream_t stream = nullptr;
         cudaEvent_t done = nullptr;
         bool used = false;
-        DevBuf data, chunks, tiles, files, order, tile_out, features, work, fix_list;
-        DevBuf rk_items;  // stretches of the group's chunks for k_stream_ranks
+        DevBuf data, tile_out, features, work;
+        // chunks, tiles, files, order, rank stretches and the (zero) head of
+        // the list of failing links, uploaded in one copy; the list follows
+        DevBuf tables;
         HostBuf h_tables;
     } slot[kSlots];
     int depth = 4;  // launch groups in flight
-    DevBuf d_binfo, d_boff, d_total, d_phase;
+    DevBuf d_result, d_phase;  // of a stream batch: total filters, per-file info and output slots
+    HostBuf h_result;
+    HostBuf h_block;  // a block-mode launch group's tables
     // host-input stream batches staged whole on the device: per-file copies
     // in launch-group order on their own stream, one event per group
     DevBuf d_stage_in, d_stage_items;
@@ -235,7 +247,19 @@ struct sdbfg_set {
     uint64_t serial = 0;               // identifies the set in cached comparison plans
     uint64_t total_filters = 0;
     std::vector<uint32_t> first;       // first filter of each digest in d_filters
-    DevBuf d_filters, d_meta, d_digests;
+    DevBuf d_all;  // one allocation: filters, meta, digests
+    DevView d_filters, d_meta, d_digests;
+    static uint64_t meta_at(uint64_t filters) { return std::max<uint64_t>(1, filters) * 256; }
+    static uint64_t digests_at(uint64_t filters) { return meta_at(filters) + (filters * 4 + 255) / 256 * 256; }
+    static uint64_t bytes(uint64_t filters, uint64_t digests) { return digests_at(filters) + (digests + 1) * sizeof(CmpDigest); }
+    cudaError_t allocate(uint64_t filters, uint64_t digests) {
+        const cudaError_t e = d_all.ensure(bytes(filters, digests));
+        if (e != cudaSuccess) return e;
+        d_filters.p = d_all.p;
+        d_meta.p = d_all.as<uint8_t>() + meta_at(filters);
+        d_digests.p = d_all.as<uint8_t>() + digests_at(filters);
+        return e;
+    }
 };
 
 // Serial number of a new set (cached comparison plans are keyed by it).
@@ -252,14 +276,15 @@ struct MatPlan {
     uint32_t nunits = 0, nsplit = 0;
     uint64_t nscores = 0, nslots = 0;
     uint64_t filter_pairs = 0;  // sum over scored pairs of n_ref * n_tgt
-    DevBuf d_units, d_targets, d_refs, d_split, d_slots, d_counter, d_redo;
+    DevBuf d_all;  // one allocation: units, targets, refs, split | redo list | counters, slots
+    DevView d_units, d_targets, d_refs, d_split, d_redo, d_counter;
+    std::vector<uint8_t> tables;  // the uploaded tables: alive for the copy, which nothing waits for
     cudaGraphExec_t graph = nullptr;
-    int32_t* graph_out = nullptr;
-    cudaStream_t graph_stream = nullptr;
+    int32_t* graph_out = nullptr;  // output of the captured (or, before that, of the last) run
     uint64_t last_use = 0;
     ~MatPlan() {
         if (graph) cudaGraphExecDestroy(graph);
-        for (DevBuf* b : {&d_units, &d_targets, &d_refs, &d_split, &d_slots, &d_counter, &d_redo}) b->release();
+        d_all.release();  // waits for the device: the tables' copy is done
     }
 };
 

@@ -63,16 +63,14 @@ extern "C" void sdbfg_ctx_destroy(sdbfg_ctx* c) {
     for (DevBuf* b : {&c->d_rank, &c->d_ent, &c->d_cut, &c->d_cut64, &c->d_data, &c->d_chunks, &c->d_tiles, &c->d_files,
                       &c->d_order, &c->d_tile_out, &c->d_features, &c->d_work_filters, &c->d_info,
                       &c->d_counters, &c->d_pack_src, &c->d_pack_dst_off, &c->d_out_filters, &c->d_out_counts,
-                      &c->d_pairs, &c->d_scores, &c->d_binfo, &c->d_boff, &c->d_total, &c->d_phase,
+                      &c->d_pairs, &c->d_scores, &c->d_result, &c->d_phase,
                       &c->d_match_counts, &c->d_match_offs, &c->d_matches, &c->d_mphase, &c->d_probes,
                       &c->d_nprobes, &c->d_hits, &c->d_index_tab, &c->d_feats, &c->d_idx_bits, &c->d_idx_first,
                       &c->d_idx_count, &c->d_seen[0], &c->d_seen[1], &c->d_pred, &c->d_diff, &c->d_ckpt,
                       &c->d_from, &c->d_ranks})
         b->release();
     for (auto& S : c->slot) {
-        for (DevBuf* b : {&S.data, &S.chunks, &S.tiles, &S.files, &S.order, &S.tile_out, &S.features, &S.work,
-                          &S.rk_items, &S.fix_list})
-            b->release();
+        for (DevBuf* b : {&S.data, &S.tables, &S.tile_out, &S.features, &S.work}) b->release();
         S.h_tables.release();
         if (S.stream) cudaStreamDestroy(S.stream);
         if (S.done) cudaEventDestroy(S.done);
@@ -89,6 +87,9 @@ extern "C" void sdbfg_ctx_destroy(sdbfg_ctx* c) {
     if (c->copy_stream) cudaStreamDestroy(c->copy_stream);
     if (c->ev_start) cudaEventDestroy(c->ev_start);
     c->h_stage.release();
+    c->h_flags.release();
+    c->h_result.release();
+    c->h_block.release();
     timer_collect(c);
     if (c->own) cudaStreamDestroy(c->own);
     delete c;
@@ -569,11 +570,14 @@ static int digest_stream_pipelined(sdbfg_ctx* c, const uint8_t* host_data, const
     }
     const uint64_t* lens = lens_v.data();
     const uint64_t* offsets = offs_v.data();
-    CUDA_TRY(c, c->d_binfo.ensure(std::max<size_t>(1, n) * sizeof(FileInfoDev)));
-    CUDA_TRY(c, c->d_boff.ensure(std::max<size_t>(1, n) * sizeof(uint64_t)));
-    CUDA_TRY(c, c->d_total.ensure(64));
-    CUDA_TRY(c, cudaMemsetAsync(c->d_binfo.p, 0, std::max<size_t>(1, n) * sizeof(FileInfoDev), c->stream));
-    CUDA_TRY(c, cudaMemsetAsync(c->d_total.p, 0, 64, c->stream));
+    // results: total | output slot per file | info per file, read back in one copy
+    const size_t at_info = 64 + (size_t)n * sizeof(uint64_t), result_bytes = at_info + n * sizeof(FileInfoDev);
+    CUDA_TRY(c, c->d_result.ensure(result_bytes));
+    CUDA_TRY(c, c->h_result.ensure(result_bytes + 64));
+    CUDA_TRY(c, cudaMemsetAsync(c->d_result.p, 0, result_bytes, c->stream));
+    uint64_t* d_total = c->d_result.as<uint64_t>();
+    uint64_t* d_off = d_total + 8;
+    FileInfoDev* d_info = reinterpret_cast<FileInfoDev*>(d_off + n);
     CUDA_TRY(c, cudaEventRecord(c->ev_start, c->stream));
     const std::vector<Group> groups = make_groups(lens, n, 0, host_data ? kFirstHostGroupBytes : kMaxBytesPerLaunch);
     std::vector<uint64_t> stage_off;
@@ -681,21 +685,21 @@ static int digest_stream_pipelined(sdbfg_ctx* c, const uint8_t* host_data, const
         const int rk = rk_choose(nrks, (uint32_t)c->sms);
         const uint64_t nrk = nrks[rk];
         const uint32_t rspan = rk_span(kRkPers[rk]);
-        bool pre = pre_ranks && ntiles;
-        if (pre && S.rk_items.ensure(nrk * sizeof(uint2)) != cudaSuccess) {
-            cudaGetLastError();
-            S.rk_items.release();
-            pre = false;
-        }
-        const size_t tb_chunks = nchunks * sizeof(GenChunk), tb_tiles = ntiles * sizeof(GenTile);
-        const size_t tb_files = g.count * sizeof(GenFile), tb_order = g.count * sizeof(uint32_t);
-        const size_t tb_rk = pre ? nrk * sizeof(uint2) : 0;
-        CUDA_TRY(c, S.h_tables.ensure(tb_chunks + tb_tiles + tb_files + tb_order + tb_rk + 64));
-        GenChunk* hc = reinterpret_cast<GenChunk*>(S.h_tables.p);
-        GenTile* ht = reinterpret_cast<GenTile*>(reinterpret_cast<uint8_t*>(S.h_tables.p) + tb_chunks);
-        GenFile* hf = reinterpret_cast<GenFile*>(reinterpret_cast<uint8_t*>(ht) + tb_tiles);
-        uint32_t* ho = reinterpret_cast<uint32_t*>(reinterpret_cast<uint8_t*>(hf) + tb_files);
-        uint2* hr = reinterpret_cast<uint2*>(reinterpret_cast<uint8_t*>(ho) + tb_order);
+        const bool pre = pre_ranks && ntiles;
+        const auto up = [](size_t v) { return (v + 15) / 16 * 16; };
+        const size_t at_tiles = up(nchunks * sizeof(GenChunk)), at_files = at_tiles + up(ntiles * sizeof(GenTile));
+        const size_t at_order = at_files + up(g.count * sizeof(GenFile)), at_rk = at_order + up(g.count * sizeof(uint32_t));
+        const size_t at_fix = at_rk + up(pre ? nrk * sizeof(uint2) : 0), table_bytes = at_fix + 4;
+        CUDA_TRY(c, S.h_tables.ensure(table_bytes));
+        CUDA_TRY(c, S.tables.ensure(table_bytes + ntiles * 4));
+        uint8_t* hb = static_cast<uint8_t*>(S.h_tables.p);
+        uint8_t* db = S.tables.as<uint8_t>();
+        GenChunk* hc = reinterpret_cast<GenChunk*>(hb);
+        GenTile* ht = reinterpret_cast<GenTile*>(hb + at_tiles);
+        GenFile* hf = reinterpret_cast<GenFile*>(hb + at_files);
+        uint32_t* ho = reinterpret_cast<uint32_t*>(hb + at_order);
+        uint2* hr = reinterpret_cast<uint2*>(hb + at_rk);
+        *reinterpret_cast<uint32_t*>(hb + at_fix) = 0;
         const uint8_t* gdata;
         std::vector<uint64_t> doff(g.count);
         if (dev_data) {
@@ -754,19 +758,10 @@ static int digest_stream_pipelined(sdbfg_ctx* c, const uint8_t* host_data, const
         if (!ib)
             std::stable_sort(ho, ho + g.count,
                              [&](uint32_t a, uint32_t b) { return lens[g.first + a] > lens[g.first + b]; });
-        CUDA_TRY(c, S.chunks.ensure(std::max<size_t>(1, tb_chunks)));
-        CUDA_TRY(c, S.tiles.ensure(std::max<size_t>(1, tb_tiles)));
-        CUDA_TRY(c, S.files.ensure(std::max<size_t>(1, tb_files)));
-        CUDA_TRY(c, S.order.ensure(std::max<size_t>(1, tb_order)));
         CUDA_TRY(c, S.tile_out.ensure(std::max<uint64_t>(1, ntiles) * sizeof(TileOut)));
         CUDA_TRY(c, S.features.ensure(std::max<uint64_t>(1, ntiles) * 5ull * kTileCap * 4));
         CUDA_TRY(c, S.work.ensure(solo ? 16 : std::max<uint64_t>(1, work) * 256));
-        CUDA_TRY(c, S.fix_list.ensure((ntiles + 1) * 4));
-        if (tb_chunks) CUDA_TRY(c, cudaMemcpyAsync(S.chunks.p, hc, tb_chunks, cudaMemcpyHostToDevice, st));
-        if (tb_tiles) CUDA_TRY(c, cudaMemcpyAsync(S.tiles.p, ht, tb_tiles, cudaMemcpyHostToDevice, st));
-        CUDA_TRY(c, cudaMemcpyAsync(S.files.p, hf, tb_files, cudaMemcpyHostToDevice, st));
-        CUDA_TRY(c, cudaMemcpyAsync(S.order.p, ho, tb_order, cudaMemcpyHostToDevice, st));
-        if (tb_rk) CUDA_TRY(c, cudaMemcpyAsync(S.rk_items.p, hr, tb_rk, cudaMemcpyHostToDevice, st));
+        CUDA_TRY(c, cudaMemcpyAsync(db, hb, table_bytes, cudaMemcpyHostToDevice, st));
         GenParams P{};
         P.data = gdata;
         P.rank_tab = c->d_rank.as<uint16_t>();
@@ -774,21 +769,21 @@ static int digest_stream_pipelined(sdbfg_ctx* c, const uint8_t* host_data, const
         P.counters = c->d_counters.as<uint32_t>();
         P.lead = c->lead;
         P.phase = c->profile ? c->d_phase.as<unsigned long long>() : nullptr;
-        P.chunks = S.chunks.as<GenChunk>();
+        P.chunks = reinterpret_cast<GenChunk*>(db);
         P.nchunks = (uint32_t)nchunks;
-        P.tiles = S.tiles.as<GenTile>();
+        P.tiles = reinterpret_cast<GenTile*>(db + at_tiles);
         P.ntiles = (uint32_t)ntiles;
-        P.files = S.files.as<GenFile>();
-        P.file_order = S.order.as<uint32_t>();
+        P.files = reinterpret_cast<GenFile*>(db + at_files);
+        P.file_order = reinterpret_cast<uint32_t*>(db + at_order);
         P.nfiles = g.count;
         P.tile_out = S.tile_out.as<TileOut>();
         P.features = S.features.as<uint32_t>();
         P.out_filters = solo ? dev_out : S.work.as<uint32_t>();
-        P.out_info = c->d_binfo.as<FileInfoDev>() + g.first;
-        P.fix_list = S.fix_list.as<uint32_t>();
+        P.out_info = d_info + g.first;
+        P.fix_list = reinterpret_cast<uint32_t*>(db + at_fix);
         if (pre) {
             P.ranks = c->d_ranks.as<uint16_t>() + (gi & 1) * (rank_half / 2);
-            P.rk_items = S.rk_items.as<uint2>();
+            P.rk_items = reinterpret_cast<uint2*>(db + at_rk);
             P.nrk_items = (uint32_t)nrk;
             P.rk_per = kRkPers[rk];
         }
@@ -811,7 +806,6 @@ static int digest_stream_pipelined(sdbfg_ctx* c, const uint8_t* host_data, const
                 if (P.ntiles <= resident) {  // one tile per CTA: no list
                     P.fix_list = nullptr;
                 } else {
-                    CUDA_TRY(c, cudaMemsetAsync(P.fix_list, 0, 4, st));
                     TIMED_LAUNCH_ON(c, "k_stream_fails", st,
                                     launch_stream_fails(P, std::min<uint32_t>((P.ntiles + 255) / 256, cap_grid), st));
                 }
@@ -841,38 +835,32 @@ static int digest_stream_pipelined(sdbfg_ctx* c, const uint8_t* host_data, const
         // output slots follow input order: scan after the previous group's scan
         CUDA_TRY(c, cudaStreamWaitEvent(st, prev_scan, 0));
         TIMED_LAUNCH_ON(c, "k_scan_offsets", st,
-                        (k_scan_offsets<<<1, 1024, 0, st>>>(c->d_binfo.as<FileInfoDev>() + g.first,
-                                                             c->d_boff.as<uint64_t>() + g.first, g.count,
-                                                             c->d_total.as<uint64_t>()),
+                        (k_scan_offsets<<<1, 1024, 0, st>>>(d_info + g.first, d_off + g.first, g.count, d_total),
                          cudaGetLastError()));
         CUDA_TRY(c, cudaEventRecord(c->ev_scan[gi % depth], st));
         prev_scan = c->ev_scan[gi % depth];
         TIMED_LAUNCH_ON(c, "k_pack_filters", st,
                         (k_pack_group<<<std::min<uint32_t>(g.count, (uint32_t)c->sms * 8), 256, 0, st>>>(
-                             S.work.as<uint32_t>(), S.files.as<GenFile>(), c->d_binfo.as<FileInfoDev>() + g.first,
-                             c->d_boff.as<uint64_t>() + g.first, dev_out, g.count),
+                             S.work.as<uint32_t>(), P.files, d_info + g.first, d_off + g.first, dev_out, g.count),
                          cudaGetLastError()));
         CUDA_TRY(c, cudaEventRecord(S.done, st));
     }
     // join: the caller's stream waits for both slots, then results come back
     for (int k = 0; k < kSlots; k++)
         if (c->slot[k].used) CUDA_TRY(c, cudaStreamWaitEvent(c->stream, c->slot[k].done, 0));
-    std::vector<FileInfoDev> info(n);
-    std::vector<uint64_t> off(n);
-    uint64_t flags_total[2] = {0, 0};
-    uint32_t flags[2] = {0, 0};
-    if (n) CUDA_TRY(c, cudaMemcpyAsync(info.data(), c->d_binfo.p, n * sizeof(FileInfoDev), cudaMemcpyDeviceToHost, c->stream));
-    if (n && !solo) {
-        CUDA_TRY(c, cudaMemcpyAsync(off.data(), c->d_boff.p, n * sizeof(uint64_t), cudaMemcpyDeviceToHost, c->stream));
-        CUDA_TRY(c, cudaMemcpyAsync(flags_total, c->d_total.p, 8, cudaMemcpyDeviceToHost, c->stream));
-    }
-    CUDA_TRY(c, cudaMemcpyAsync(flags, c->d_counters.p, sizeof flags, cudaMemcpyDeviceToHost, c->stream));
+    uint8_t* hr = static_cast<uint8_t*>(c->h_result.p);
+    uint64_t* total = reinterpret_cast<uint64_t*>(hr);
+    const uint64_t* off = total + 8;
+    const FileInfoDev* info = reinterpret_cast<const FileInfoDev*>(hr + at_info);
+    const uint32_t* flags = reinterpret_cast<const uint32_t*>(hr + result_bytes);
+    CUDA_TRY(c, cudaMemcpyAsync(hr, c->d_result.p, result_bytes, cudaMemcpyDeviceToHost, c->stream));
+    CUDA_TRY(c, cudaMemcpyAsync(hr + result_bytes, c->d_counters.p, 8, cudaMemcpyDeviceToHost, c->stream));
     CUDA_TRY(c, cudaStreamSynchronize(c->stream));
     if (flags[1]) return fail(c, SDBFG_ERR_CUDA, "internal error: stream digest exceeded its filter bound");
-    if (solo) flags_total[0] = info[0].bf_count;
-    if (flags_total[0] > out_cap)
+    if (solo) *total = info[0].bf_count;
+    if (*total > out_cap)
         return fail(c, SDBFG_ERR_CAPACITY, "output capacity %llu filters < %llu needed", (unsigned long long)out_cap,
-                    (unsigned long long)flags_total[0]);
+                    (unsigned long long)*total);
     for (uint32_t i = 0; i < n; i++) {
         if (lens[i] < kMinFile) continue;
         sdbfg_digest_result& r = res[perm[i]];
@@ -880,7 +868,7 @@ static int digest_stream_pipelined(sdbfg_ctx* c, const uint8_t* host_data, const
         r.last_count = info[i].last_count;
         r.filter_offset = off[i];
     }
-    if (total_out) *total_out = flags_total[0];
+    if (total_out) *total_out = *total;
     return SDBFG_OK;
 }
 
@@ -904,122 +892,140 @@ static int digest_block_group(sdbfg_ctx* c, const uint8_t* dev_base, const std::
     // whole blocks) where a block's ranks start 16-byte aligned; slabs
     // bound their buffer.
     struct Slab {
-        uint32_t first_chunk, nchunks, first_run, nruns;
+        uint32_t first_run, nruns, nchunks;
         uint64_t r8, stretches[kRkChoices];
     };
-    std::vector<GenChunk> chunks, runs;
+    std::vector<GenChunk> runs;
     std::vector<Slab> slabs{Slab{}};
     uint32_t lmax = 0;
     const uint64_t run_bytes = kChunkBytes / (16 * dd) * (16 * dd);  // so every run starts 16-byte aligned
-    uint64_t most8 = 0, cap = host_dev ? kFirstHostSlabBytes : kBlockSlabBytes;
+    uint64_t most8 = 0, nchunks = 0, cap = host_dev ? kFirstHostSlabBytes : kBlockSlabBytes;
     for (uint32_t k = 0; k < g.count; k++) {
         const uint32_t i = g.first + k;
         if (lens[i] < kMinFile) continue;
         const uint64_t used = lens[i] % dd >= kMinFile ? lens[i] : lens[i] / dd * dd;  // full blocks and a counted tail
         for (uint64_t pos = 0; pos < used; pos += run_bytes) {
-            const uint32_t m = (uint32_t)std::min<uint64_t>(run_bytes, used - pos);
+            const uint32_t m = (uint32_t)std::min<uint64_t>(run_bytes, used - pos), nb = (m + dd - 1) / dd;
             if (slabs.back().r8 && (slabs.back().r8 * 8 + m) > cap) {
                 cap = std::min(2 * cap, kBlockSlabBytes);
-                slabs.push_back(Slab{(uint32_t)chunks.size(), 0, (uint32_t)runs.size(), 0, 0, {}});
+                slabs.push_back(Slab{(uint32_t)runs.size(), 0, 0, 0, {}});
             }
             Slab& s = slabs.back();
-            for (uint32_t b = 0; b < m; b += dd) {
-                const uint32_t len = std::min(dd, m - b);
-                chunks.push_back({dev_off[k] + pos + b, len, i, 0, 0, (uint32_t)(res[i].filter_offset + (pos + b) / dd),
-                                  len < dd ? 1u : 0u, (uint32_t)(s.r8 + b / 8)});
-                lmax = std::max<uint32_t>(lmax, len - 64);
-                s.nchunks++;
-            }
-            runs.push_back({dev_off[k] + pos, m, i, 0, 0, 0, 0, (uint32_t)s.r8});
+            // (a run's first output slot; its blocks' are consecutive)
+            runs.push_back({dev_off[k] + pos, m, i, 0, nb, (uint32_t)(res[i].filter_offset + pos / dd), 0, (uint32_t)s.r8});
             s.nruns++;
+            s.nchunks += nb;
+            nchunks += nb;
+            lmax = std::max(lmax, std::min(m, dd) - 64);
             for (int q = 0; q < kRkChoices; q++) s.stretches[q] += rk_stretches(m, kRkPers[q]);
             s.r8 += (m + 7) / 8;
             most8 = std::max(most8, s.r8);
         }
     }
-    if (chunks.empty()) return SDBFG_OK;
-    CUDA_TRY(c, c->d_chunks.ensure(chunks.size() * sizeof(GenChunk)));
-    CUDA_TRY(c, cudaMemcpyAsync(c->d_chunks.p, chunks.data(), chunks.size() * sizeof(GenChunk),
-                                cudaMemcpyHostToDevice, st));
-    P.chunks = c->d_chunks.as<GenChunk>();
-    P.nchunks = (uint32_t)chunks.size();
+    if (runs.empty()) return SDBFG_OK;
+    std::vector<uint32_t> first_item, per;
+    uint64_t nitems = 0;
+    for (const Slab& s : slabs) {
+        const int q = rk_choose(s.stretches, (uint32_t)c->sms);
+        first_item.push_back((uint32_t)nitems);
+        per.push_back(kRkPers[q]);
+        nitems += s.stretches[q];
+    }
+    first_item.push_back((uint32_t)nitems);
+    CUDA_TRY(c, c->d_chunks.ensure(nchunks * sizeof(GenChunk)));
+    bool pre = c->pre_ranks && dd % 8 == 0;
+    if (pre && (c->d_ranks.ensure(most8 * 16 + 256) != cudaSuccess ||
+                c->d_files.ensure(runs.size() * sizeof(GenChunk)) != cudaSuccess ||
+                c->d_tiles.ensure(nitems * sizeof(uint2)) != cudaSuccess)) {
+        cudaGetLastError();
+        c->d_ranks.release();
+        pre = false;
+    }
     P.out_filters = dev_out;
     P.out_counts = dev_counts;
     P.probes = c->probe_words;
     P.nprobes = c->probe_counts;
     P.feats = c->feat_words;
     P.block_lmax = (lmax + 63) / 64 * 64;
-    std::vector<uint2> items;
-    std::vector<uint32_t> first_item, per;
-    for (const Slab& s : slabs) {
-        const int q = rk_choose(s.stretches, (uint32_t)c->sms);
-        first_item.push_back((uint32_t)items.size());
-        per.push_back(kRkPers[q]);
-        for (uint32_t r = 0; r < s.nruns; r++)
-            for (uint32_t s0 = 0; s0 < (runs[s.first_run + r].n + 7) / 8 * 8; s0 += rk_span(per.back()))
-                items.push_back(make_uint2(s.first_run + r, s0));
-    }
-    first_item.push_back((uint32_t)items.size());
-    bool pre = c->pre_ranks && dd % 8 == 0;
-    if (pre && (c->d_ranks.ensure(most8 * 16 + 256) != cudaSuccess ||
-                c->d_files.ensure(runs.size() * sizeof(GenChunk)) != cudaSuccess ||
-                c->d_tiles.ensure(items.size() * sizeof(uint2)) != cudaSuccess)) {
-        cudaGetLastError();
-        c->d_ranks.release();
-        pre = false;
-    }
-    std::vector<StagePiece> pieces;
+    // the tables' pinned copy: blocks | rank stretches | runs | pieces
+    uint64_t npieces = 0;
+    for (const GenChunk& R : runs) npieces += (R.n + kStagePiece - 1) / kStagePiece;
+    CUDA_TRY(c, c->h_block.ensure(nchunks * sizeof(GenChunk) + nitems * sizeof(uint2) + runs.size() * sizeof(GenChunk) +
+                                  npieces * sizeof(StagePiece)));
+    GenChunk* chunks = static_cast<GenChunk*>(c->h_block.p);
+    uint2* items = reinterpret_cast<uint2*>(chunks + nchunks);
+    GenChunk* hruns = reinterpret_cast<GenChunk*>(items + nitems);
+    StagePiece* pieces = reinterpret_cast<StagePiece*>(hruns + runs.size());
     if (host_dev) {
         std::vector<uint32_t> first_piece;
+        uint32_t np = 0;
         for (const Slab& s : slabs) {
-            first_piece.push_back((uint32_t)pieces.size());
+            first_piece.push_back(np);
             for (uint32_t r = s.first_run; r < s.first_run + s.nruns; r++) {
                 const GenChunk& R = runs[r];
                 const uint64_t src = reinterpret_cast<uint64_t>(host_dev) + host_off[R.file] + (R.data_off - dev_off[R.file - g.first]);
                 for (uint64_t pos = 0; pos < R.n; pos += kStagePiece)
-                    pieces.push_back({R.data_off + pos, src + pos, std::min<uint64_t>(kStagePiece, R.n - pos)});
+                    pieces[np++] = {R.data_off + pos, src + pos, std::min<uint64_t>(kStagePiece, R.n - pos)};
             }
         }
-        first_piece.push_back((uint32_t)pieces.size());
+        first_piece.push_back(np);
         const int rc = ensure_copy_stream(c, slabs.size());
         if (rc) return rc;
-        CUDA_TRY(c, c->d_stage_items.ensure(pieces.size() * sizeof(StagePiece)));
-        CUDA_TRY(c, cudaMemcpyAsync(c->d_stage_items.p, pieces.data(), pieces.size() * sizeof(StagePiece),
-                                    cudaMemcpyHostToDevice, st));
+        CUDA_TRY(c, c->d_stage_items.ensure(np * sizeof(StagePiece)));
+        CUDA_TRY(c, cudaMemcpyAsync(c->d_stage_items.p, pieces, np * sizeof(StagePiece), cudaMemcpyHostToDevice, st));
         CUDA_TRY(c, cudaEventRecord(c->ev_start, st));
         CUDA_TRY(c, cudaStreamWaitEvent(c->copy_stream, c->ev_start, 0));
         for (size_t k = 0; k < slabs.size(); k++) {
-            const uint32_t np = first_piece[k + 1] - first_piece[k];
+            const uint32_t m = first_piece[k + 1] - first_piece[k];
             TIMED_LAUNCH_ON(c, "k_stage_gather", c->copy_stream,
-                            (k_stage_gather<<<std::min<uint32_t>(np, (uint32_t)c->sms), kGatherThreads, 0,
-                                              c->copy_stream>>>(c->d_stage_items.as<StagePiece>() + first_piece[k], np,
+                            (k_stage_gather<<<std::min<uint32_t>(m, (uint32_t)c->sms), kGatherThreads, 0,
+                                              c->copy_stream>>>(c->d_stage_items.as<StagePiece>() + first_piece[k], m,
                                                                 const_cast<uint8_t*>(dev_base)),
                              cudaGetLastError()));
             CUDA_TRY(c, cudaEventRecord(c->ev_copy[k], c->copy_stream));
         }
     }
     if (pre) {
-        CUDA_TRY(c, cudaMemcpyAsync(c->d_files.p, runs.data(), runs.size() * sizeof(GenChunk), cudaMemcpyHostToDevice, st));
-        CUDA_TRY(c, cudaMemcpyAsync(c->d_tiles.p, items.data(), items.size() * sizeof(uint2), cudaMemcpyHostToDevice, st));
+        memcpy(hruns, runs.data(), runs.size() * sizeof(GenChunk));
+        CUDA_TRY(c, cudaMemcpyAsync(c->d_files.p, hruns, runs.size() * sizeof(GenChunk), cudaMemcpyHostToDevice, st));
         P.ranks = c->d_ranks.as<uint16_t>();
     }
+    // a slab's block table is made while the slab before it runs
+    uint64_t first = 0;
     for (size_t k = 0; k < slabs.size(); k++) {
+        const Slab& s = slabs[k];
         if (host_dev) CUDA_TRY(c, cudaStreamWaitEvent(st, c->ev_copy[k], 0));
         if (pre) {
+            uint2* it = items + first_item[k];
+            for (uint32_t r = s.first_run; r < s.first_run + s.nruns; r++)
+                for (uint32_t s0 = 0; s0 < (runs[r].n + 7) / 8 * 8; s0 += rk_span(per[k])) *it++ = make_uint2(r, s0);
             GenParams R = P;
             R.chunks = c->d_files.as<GenChunk>();
             R.rk_items = c->d_tiles.as<uint2>() + first_item[k];
             R.nrk_items = first_item[k + 1] - first_item[k];
             R.rk_per = per[k];
+            CUDA_TRY(c, cudaMemcpyAsync(c->d_tiles.as<uint2>() + first_item[k], items + first_item[k],
+                                        R.nrk_items * sizeof(uint2), cudaMemcpyHostToDevice, st));
             TIMED_LAUNCH(c, "k_stream_ranks",
                          launch_stream_ranks(R, std::min<uint32_t>(R.nrk_items, (uint32_t)c->sms * 3 * 16), st));
         }
+        GenChunk* ch = chunks + first;
+        for (uint32_t r = s.first_run; r < s.first_run + s.nruns; r++) {
+            const GenChunk& R = runs[r];
+            for (uint32_t b = 0, q = 0; b < R.n; b += dd, q++) {
+                const uint32_t len = std::min(dd, R.n - b);
+                *ch++ = {R.data_off + b, len, R.file, 0, 0, R.filter + q, len < dd ? 1u : 0u, R.rank_off8 + b / 8};
+            }
+        }
         GenParams B = P;
-        B.chunks = P.chunks + slabs[k].first_chunk;
-        B.nchunks = slabs[k].nchunks;
+        B.chunks = c->d_chunks.as<GenChunk>() + first;
+        B.nchunks = s.nchunks;
+        CUDA_TRY(c, cudaMemcpyAsync(c->d_chunks.as<GenChunk>() + first, chunks + first, s.nchunks * sizeof(GenChunk),
+                                    cudaMemcpyHostToDevice, st));
         TIMED_LAUNCH(c, "k_block_digest", launch_block(B, (uint32_t)c->sms, st));
+        first += s.nchunks;
     }
-    // the tables must outlive their copies
+    // the tables are rewritten by the next call
     CUDA_TRY(c, cudaStreamSynchronize(st));
     return SDBFG_OK;
 }

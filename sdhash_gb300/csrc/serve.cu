@@ -79,7 +79,7 @@ struct sdbfg_server {
         std::vector<Request> batch;
         uint32_t nunits = 0, nsplit = 0;
         HostBuf h_filters, h_meta, h_dig, h_units, h_targets, h_refs, h_split, h_scores;
-        DevBuf d_filters, d_meta, d_dig, d_units, d_targets, d_refs, d_split, d_slots, d_counter, d_scores, d_redo;
+        DevBuf d_filters, d_meta, d_dig, d_units, d_targets, d_refs, d_split, d_slots, d_scores, d_redo;  // slots behind the counters
         uint64_t cap_units = 0, cap_targets = 0, cap_refs = 0, cap_split = 0, cap_slots = 0;
     };
     std::vector<Slot> slots;
@@ -132,7 +132,7 @@ static cudaError_t launch_batch(sdbfg_server* sv, sdbfg_server::Slot& S) {
     if ((e = grow(S.d_split, &S.h_split, S.cap_split, ub.split.size() + 1, sizeof(MatSplit)))) return e;
     if ((e = grow(S.d_refs, &S.h_refs, S.cap_refs, ub.refs.size() + 1, 4))) return e;
     memcpy(S.h_refs.p, ub.refs.data(), ub.refs.size() * 4);
-    if ((e = grow(S.d_slots, nullptr, S.cap_slots, ub.slots + 1, 8))) return e;
+    if ((e = grow(S.d_slots, nullptr, S.cap_slots, ub.slots + 1 + kMatCounterBytes / 8, 8))) return e;
     memcpy(S.h_units.p, units.data(), units.size() * sizeof(MatUnit));
     memcpy(S.h_targets.p, targets.data(), targets.size() * 4);
     memcpy(S.h_split.p, ub.split.data(), ub.split.size() * sizeof(MatSplit));
@@ -151,7 +151,6 @@ static cudaError_t launch_batch(sdbfg_server* sv, sdbfg_server::Slot& S) {
     if (S.nsplit &&
         (e = cudaMemcpyAsync(S.d_split.p, S.h_split.p, S.nsplit * sizeof(MatSplit), cudaMemcpyHostToDevice, st)))
         return e;
-    if ((e = cudaMemsetAsync(S.d_counter.p, 0, 8, st))) return e;  // work counter, error flag
     MatParams P{};
     P.filters[0] = S.d_filters.as<uint32_t>();
     P.meta[0] = S.d_meta.as<uint32_t>();
@@ -161,12 +160,12 @@ static cudaError_t launch_batch(sdbfg_server* sv, sdbfg_server::Slot& S) {
     P.digests[1] = T->d_digests.as<CmpDigest>();
     P.units = S.d_units.as<MatUnit>();
     P.nunits = S.nunits;
-    P.next_unit = S.d_counter.as<uint32_t>();
+    P.next_unit = S.d_slots.as<uint32_t>();
     P.targets = S.d_targets.as<uint32_t>();
     P.refs = S.d_refs.as<uint32_t>();
     P.split = S.d_split.as<MatSplit>();
     P.nsplit = S.nsplit;
-    P.slots = S.d_slots.as<double>();
+    P.slots = S.d_slots.as<double>() + kMatCounterBytes / 8;
     P.nslots = ub.slots;
     P.scores = S.d_scores.as<int32_t>();
     P.nscores = (uint64_t)nq * nt;
@@ -174,8 +173,8 @@ static cudaError_t launch_batch(sdbfg_server* sv, sdbfg_server::Slot& S) {
     P.n = nt;
     P.cutoffs = sv->ctx->d_cut.as<uint16_t>();
     P.cutoffs64 = sv->ctx->d_cut64.as<uint16_t>();
-    P.redo = redo_list(S.d_redo.p);
-    P.error = S.d_counter.as<uint32_t>() + 1;
+    P.redo = redo_list(S.d_redo.p, P.next_unit);
+    P.error = P.next_unit + 1;
     uint64_t launched = 0;
     if ((e = run_matrix(P, variant, (uint32_t)ctas, (uint32_t)sv->ctx->sms, st, &launched))) return e;
     sv->launches += launched;
@@ -317,14 +316,13 @@ extern "C" int sdbfg_server_create(sdbfg_ctx* c, const sdbfg_set* refs, const sd
             if (e == cudaSuccess) e = dv->ensure(bytes);
             if (e == cudaSuccess) e = hv->ensure(bytes);
         }
-        if (e == cudaSuccess) e = S.d_counter.ensure(64);
         if (e == cudaSuccess) e = S.d_redo.ensure(kRedoBytes);
         if (e == cudaSuccess) e = grow(S.d_units, &S.h_units, S.cap_units, 1 << 16, sizeof(MatUnit));
         if (e == cudaSuccess)
             e = grow(S.d_targets, &S.h_targets, S.cap_targets, (uint64_t)nq * refs->n + nq + refs->n + 1, 4);
         if (e == cudaSuccess) e = grow(S.d_refs, &S.h_refs, S.cap_refs, (uint64_t)nq + refs->n + 1, 4);
         if (e == cudaSuccess) e = grow(S.d_split, &S.h_split, S.cap_split, (uint64_t)nq * refs->n + 1, sizeof(MatSplit));
-        if (e == cudaSuccess) e = grow(S.d_slots, nullptr, S.cap_slots, (uint64_t)nf * refs->n + 1, 8);
+        if (e == cudaSuccess) e = grow(S.d_slots, nullptr, S.cap_slots, (uint64_t)nf * refs->n + 1 + kMatCounterBytes / 8, 8);
         if (e != cudaSuccess) {
             sdbfg_server_destroy(sv);
             return fail(c, e == cudaErrorMemoryAllocation ? SDBFG_ERR_NOMEM : SDBFG_ERR_CUDA, "server slots: %s",
@@ -414,7 +412,7 @@ extern "C" void sdbfg_server_destroy(sdbfg_server* sv) {
     cudaSetDevice(sv->ctx->device);
     for (auto& S : sv->slots) {
         for (DevBuf* b : {&S.d_filters, &S.d_meta, &S.d_dig, &S.d_units, &S.d_targets, &S.d_refs, &S.d_split,
-                          &S.d_slots, &S.d_counter, &S.d_scores, &S.d_redo})
+                          &S.d_slots, &S.d_scores, &S.d_redo})
             b->release();
         for (HostBuf* b : {&S.h_filters, &S.h_meta, &S.h_dig, &S.h_units, &S.h_targets, &S.h_refs, &S.h_split,
                            &S.h_scores})

@@ -404,9 +404,7 @@ extern "C" int sdbfg_set_load_text(sdbfg_ctx* c, const char* text, uint64_t len,
         dig[i] = {p.line.first, p.line.nfilters, 0, 0, 0};
     }
     auto cleanup = [&](int code) {
-        s->d_filters.release();
-        s->d_meta.release();
-        s->d_digests.release();
+        s->d_all.release();
         delete s;
         return code;
     };
@@ -418,9 +416,7 @@ extern "C" int sdbfg_set_load_text(sdbfg_ctx* c, const char* text, uint64_t len,
         d_flags.release();
         d_recs.release();
     };
-    if (s->d_filters.ensure(std::max<uint64_t>(1, total) * 256) || s->d_meta.ensure(std::max<uint64_t>(1, total) * 4) ||
-        s->d_digests.ensure(std::max<uint32_t>(1, nl) * sizeof(CmpDigest)) ||
-        d_text.ensure(std::max<uint64_t>(16, text_used + 16)) ||
+    if (s->allocate(total, nl) || d_text.ensure(std::max<uint64_t>(16, text_used + 16)) ||
         d_lines.ensure(std::max<uint32_t>(1, nl) * sizeof(TextLine)) || d_flags.ensure(std::max<uint32_t>(1, nl) * 4)) {
         release_scratch();
         cudaGetLastError();
