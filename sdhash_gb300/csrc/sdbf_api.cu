@@ -227,16 +227,16 @@ struct Group {  // consecutive inputs processed by one launch sequence
 
 // Splits inputs into launch groups bounded by tiles (stream) or bytes.
 // Launch groups of consecutive inputs, each at most kMaxTilesPerLaunch tiles
-// and kMaxBytesPerLaunch bytes; the first group at most first_cap bytes and
+// and max_bytes bytes; the first group at most first_cap bytes and
 // each later one at most twice its predecessor's cap (host inputs: a short
 // first copy lets the kernels start early, and the ramp keeps each later
 // group's copy shorter than the kernels of the groups before it).
 std::vector<Group> make_groups(const uint64_t* lens, uint32_t n, uint32_t dd,
-                               uint64_t first_cap = kMaxBytesPerLaunch) {
+                               uint64_t first_cap = kMaxBytesPerLaunch, uint64_t max_bytes = kMaxBytesPerLaunch) {
     std::vector<Group> gs;
     uint32_t start = 0;
     uint64_t tiles = 0, bytes = 0;
-    uint64_t cap_bytes = std::min(first_cap, kMaxBytesPerLaunch);
+    uint64_t cap_bytes = std::min(first_cap, max_bytes);
     for (uint32_t i = 0; i < n; i++) {
         uint64_t t = 0;
         if (!dd && lens[i] >= kMinFile) {
@@ -251,7 +251,7 @@ std::vector<Group> make_groups(const uint64_t* lens, uint32_t n, uint32_t dd,
             start = i;
             tiles = 0;
             bytes = 0;
-            cap_bytes = std::min(2 * cap_bytes, kMaxBytesPerLaunch);
+            cap_bytes = std::min(2 * cap_bytes, max_bytes);
         }
         tiles += t;
         bytes += b;
@@ -579,7 +579,9 @@ static int digest_stream_pipelined(sdbfg_ctx* c, const uint8_t* host_data, const
     uint64_t* d_off = d_total + 8;
     FileInfoDev* d_info = reinterpret_cast<FileInfoDev*>(d_off + n);
     CUDA_TRY(c, cudaEventRecord(c->ev_start, c->stream));
-    const std::vector<Group> groups = make_groups(lens, n, 0, host_data ? kFirstHostGroupBytes : kMaxBytesPerLaunch);
+    const std::vector<Group> groups =
+        ib ? make_groups(lens, n, 0, host_data ? kFirstIndexGroupBytes : kMaxBytesPerLaunch)
+           : make_groups(lens, n, 0, host_data ? kFirstHostGroupBytes : kStreamGroupBytes, kStreamGroupBytes);
     std::vector<uint64_t> stage_off;
     if (staged) {
         stage_off.resize(n);
