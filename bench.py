@@ -48,7 +48,7 @@ CONFIG_BASE = {"workload": "bulk stream-mode digest generation", "files": 4096, 
 
 
 KERNELS = ("k_stream_ranks", "k_stream_tiles", "k_stream_fails", "k_stream_fix_list", "k_stream_fix",
-           "k_stream_commit", "k_pack_filters", "k_scan_offsets")
+           "k_stream_commit", "k_feat_links", "k_stream_chain", "k_stream_emit", "k_pack_filters", "k_scan_offsets")
 
 
 def parse():

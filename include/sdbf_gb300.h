@@ -55,15 +55,15 @@ uint64_t sdbfg_ctx_launch_count(const sdbfg_ctx *ctx);
  * every launch (off by default; enabling clears previous totals).
  * sdbfg_ctx_kernel_time reports the accumulated milliseconds and launch
  * count of one kernel ("k_stream_tiles", "k_stream_fix",
- * "k_stream_commit", "k_pack_filters", "k_block_digest", "k_compare_pairs",
- * "k_scan_offsets").  While profiling, the stream kernels also count SM
+ * "k_stream_commit", "k_feat_links" (the five kernels before
+ * "k_stream_chain"), "k_stream_emit", "k_pack_filters", "k_block_digest",
+ * "k_compare_pairs", "k_scan_offsets").  While profiling, the stream kernels also count SM
  * cycles per phase; the names "k_stream_tiles.{load,ranks,fres,walk,link,
  * compact,sha1}" and "k_stream_commit.{wait,busy,max_file}" report those
  * cycles in *total_ms (and the tile count in *launches); ".count",
  * ".groups", ".loops" report counts.  The tensor-core comparison kernel
- * reports "k_matrix_tc.{compose,fill,fetch_wait,stage_wait,widen,issue,
- * producer_step,acc_wait,score,mark,walk,fold,consumer_step,step_barrier,
- * tmem_ld}" in SM cycles and ".tiles" as a count.
+ * reports "k_matrix_tc.{compose,widen,mma,mark,check}" and their waits
+ * ("..._wait") in SM cycles, ".tiles" and ".marked" as counts.
  * Instrumentation without a counterpart in the reference. */
 int sdbfg_ctx_profile(sdbfg_ctx *ctx, int enable);
 int sdbfg_ctx_kernel_time(sdbfg_ctx *ctx, const char *kernel, double *total_ms, uint64_t *launches);

@@ -34,6 +34,13 @@ constexpr uint64_t kStreamGroupBytes = 256ull << 20;
 // its copy is the one nothing hides.  64 files of 1 MiB: 1.06 ms, with 16 MiB
 // 1.11, with 64 MiB (one group) 1.17.
 constexpr uint64_t kFirstHostGroupBytes = 32ull << 20;
+// A group with a file of this many tiles, and at least half of all, commits
+// through links (k_stream_chain): there the group waits for that one file's
+// chain.  One file of 2, 3, 8 and 32 MiB on the device: 209, 267, 537 and 1,698
+// us, through k_stream_commit 191, 289, 717 and 2,646.  Where many files'
+// commits run beside tiles anyway, the links are only more work: 3.1 GB of
+// uneven files 22.9 ms against 21.2.
+constexpr uint32_t kChainTiles = 384;
 constexpr uint64_t kFirstIndexGroupBytes = 256ull << 20;  // with an index being built (groups one after another)
 constexpr uint32_t kMinFile = 512;                 // MIN_FILE_SIZE (sdbf_defines.h:56)
 constexpr uint64_t kPairsPerLaunch = 1ull << 22;
@@ -181,6 +188,7 @@ struct sdbfg_ctx {
         cudaEvent_t done = nullptr;
         bool used = false;
         DevBuf data, tile_out, features, work;
+        DevBuf links, last_tab, chain;  // linked commit; chain: tile places, file totals, filter ends
         // chunks, tiles, files, order, rank stretches and the (zero) head of
         // the list of failing links, uploaded in one copy; the list follows
         DevBuf tables;

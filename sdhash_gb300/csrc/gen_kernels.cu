@@ -17,7 +17,8 @@
 //                   zero-new-bit suppression, the 16 KiB "big filter"
 //                   dedupe (bloom_filter.cc:333-359), roll-over at 160
 //                   elements, big-filter roll-over at 8738 per chunk, and the
-//                   final chop (:235-238).
+//                   final chop (:235-238).  A file that a batch waits for
+//                   commits through links instead (k_stream_chain).
 //  k_block_digest   one CTA per dd block (gen_block_sdbf_mt :251-324,
 //                   gen_block_hash :141-191): histogram threshold, <=192
 //                   ordered inserts.
@@ -1691,6 +1692,468 @@ __global__ void k_pred_dirty(const uint32_t* __restrict__ a, const uint32_t* __r
     }
 }
 
+// ------------------------------------------------------ linked commit
+// The ordered filter fill again, for files long enough that its chain of
+// passes is what a batch waits for.  Whether a feature sets a new bit in the
+// filter F does not need F: F holds exactly the bits of the features since
+// the filter's start fs (a feature that fails either test sets no bit that is
+// new), so feature i passes iff one of its five bits was last held before fs,
+// that is iff min over its words of (place of the last earlier holder of the
+// same 11-bit index) is before fs.  That minimum depends on the features
+// alone and is computed for all of them at once:
+//  k_feat_scan   the place of every tile's features in its file;
+//  k_feat_pack   the features packed per file: five 17-bit big-filter indices
+//                (the filter's are their low 11 bits);
+//  k_feat_last   per block of kLkBlock features, the last holder of each
+//                filter bit in the block;
+//  k_feat_carry  per block, the last holder before it;
+//  k_feat_links  the minimum (0: a bit that no earlier feature holds, else
+//                place + 1), and for each word whether a feature of the last
+//                kLkNear may hold the same big-filter index.
+// k_stream_chain then walks a file's features in windows as k_stream_commit
+// does, with one compare for F; the big filter G is kept, and its bits that
+// are unset before a window and near no other holder are new.  It leaves the
+// ends of the filters; k_stream_emit fills them.
+//
+// What bounds it: the chain, ~200 instructions a pass that wait for one
+// another, three barriers, the random reads and stores of G (a byte per bit,
+// so that its bits are set without atomics).  One 200 MiB file: 16,693 passes
+// of 1,034 cycles, 8.35 ms, and 0.43 ms for links and filters; k_stream_commit
+// takes 15.2 ms.  On the way: G as bits set by atomics, one table of 13 bits
+// for the near flags (0.44 ambiguous features a pass, 1,100 cycles each; with
+// two tables 0.02): 1,745 cycles; the next window's features read only after
+// barrier (1): 1,135.
+constexpr uint32_t kLkNear = 192 + 32;  // a window, and what a stale place in the table may be off
+static_assert(kLkNear % 32 == 0 && kLkBlock % 32 == 0 && kLkNear <= kLkBlock && kLkBlock + kLkNear < 65535, "places in whole groups, in 16 bits");
+
+__global__ void __launch_bounds__(1024) k_feat_scan(GenParams P) {
+    __shared__ uint32_t warp_sums[32];
+    const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    for (uint32_t f = blockIdx.x; f < P.nfiles; f += gridDim.x) {
+        const GenFile Fd = P.files[f];
+        if (Fd.nchunks == 0) {
+            if (threadIdx.x == 0) P.file_total[f] = 0;
+            continue;
+        }
+        const GenChunk cl = P.chunks[Fd.first_chunk + Fd.nchunks - 1];
+        const uint32_t t0 = P.chunks[Fd.first_chunk].first_tile, t1 = cl.first_tile + cl.ntiles;
+        uint32_t run = t0 * kTileCap;
+        for (uint32_t b = t0; b < t1; b += 4096) {
+            uint32_t c[4], sum = 0;
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                const uint32_t t = b + 4 * threadIdx.x + k;
+                c[k] = t < t1 ? min(P.tile_out[t].count, kTileCap) : 0u;
+            }
+#pragma unroll
+            for (int k = 0; k < 4; k++) sum += c[k];
+            uint32_t incl = sum;
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xffffffffu, incl, d);
+                if (lane >= (uint32_t)d) incl += y;
+            }
+            __syncthreads();  // the last stretch's sums are read
+            if (lane == 31) warp_sums[wid] = incl;
+            __syncthreads();
+            uint32_t ws = warp_sums[lane];
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xffffffffu, ws, d);
+                if (lane >= (uint32_t)d) ws += y;
+            }
+            uint32_t at = run + incl - sum + (wid ? __shfl_sync(0xffffffffu, ws, wid - 1) : 0u);
+            run += __shfl_sync(0xffffffffu, ws, 31);
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                const uint32_t t = b + 4 * threadIdx.x + k;
+                if (t < t1) P.tile_base[t] = at;
+                at += c[k];
+            }
+        }
+        if (threadIdx.x == 0) P.file_total[f] = run - t0 * kTileCap;
+    }
+}
+
+// links entry: x = index 0 | low 15 bits of index 3 << 17, y = index 1 | low
+// 15 bits of index 4 << 17, z = index 2 | high bits of 3 << 17 | of 4 << 19 |
+// near flags << 21, w = the minimum
+__device__ __forceinline__ void link_unpack(const uint4& v, uint32_t (&b)[5]) {
+    b[0] = v.x & kBigMask;
+    b[1] = v.y & kBigMask;
+    b[2] = v.z & kBigMask;
+    b[3] = (v.x >> 17) | ((v.z >> 2) & 0x18000u);
+    b[4] = (v.y >> 17) | ((v.z >> 4) & 0x18000u);
+}
+
+__global__ void __launch_bounds__(256) k_feat_pack(GenParams P) {
+    const uint32_t lane = threadIdx.x & 31, w0 = blockIdx.x * 8 + (threadIdx.x >> 5), nw = gridDim.x * 8;
+    for (uint32_t t = w0; t < P.ntiles; t += nw) {
+        const uint32_t c = min(P.tile_out[t].count, kTileCap);
+        const uint32_t* src = P.features + (size_t)t * 5 * kTileCap;
+        uint4* dst = P.links + P.tile_base[t];
+        for (uint32_t q = lane; q < c; q += 32) {
+            const uint4 h = __ldg(reinterpret_cast<const uint4*>(src) + q);
+            const uint32_t b3 = h.w & kBigMask, b4 = __ldg(src + 4 * kTileCap + q) & kBigMask;
+            dst[q] = make_uint4((h.x & kBigMask) | (b3 << 17), (h.y & kBigMask) | (b4 << 17),
+                                (h.z & kBigMask) | ((b3 >> 15) << 17) | ((b4 >> 15) << 19), 0u);
+        }
+    }
+}
+
+// first place of a file's features in links
+__device__ __forceinline__ uint32_t link_base(const GenParams& P, const GenFile& Fd) {
+    return P.chunks[Fd.first_chunk].first_tile * kTileCap;
+}
+
+__global__ void __launch_bounds__(32) k_feat_last(GenParams P) {
+    __shared__ uint32_t last[kLkTab];
+    const uint32_t lane = threadIdx.x;
+    for (uint32_t f = blockIdx.y; f < P.nfiles; f += gridDim.y) {
+        const uint32_t total = P.file_total[f];
+        if (total <= kLkBlock) continue;
+        const uint4* v = P.links + link_base(P, P.files[f]);
+        const uint32_t nblk = (total + kLkBlock - 1) / kLkBlock;
+        for (uint32_t b = blockIdx.x; b + 1 < nblk; b += gridDim.x) {  // (nothing follows the last block)
+            for (uint32_t i = lane; i < kLkTab; i += 32) last[i] = 0;
+            __syncwarp();
+#pragma unroll 4
+            for (uint32_t q = lane; q < kLkBlock; q += 32) {
+                const uint32_t o = b * kLkBlock + q;
+                uint32_t x[5];
+                link_unpack(v[o], x);
+#pragma unroll
+                for (int k = 0; k < 5; k++) atomicMax(&last[x[k] & kBfMask], o + 1);
+            }
+            __syncwarp();
+            uint32_t* row = P.last_tab + ((size_t)P.link_first[f] + b) * kLkTab;
+            for (uint32_t i = lane; i < kLkTab; i += 32) row[i] = last[i];
+            __syncwarp();
+        }
+    }
+}
+
+// Rows of a file: last holder in the block -> last holder before the block.
+__global__ void __launch_bounds__(128) k_feat_carry(GenParams P) {
+    const uint32_t col = blockIdx.x * 128 + threadIdx.x;
+    for (uint32_t f = blockIdx.y; f < P.nfiles; f += gridDim.y) {
+        const uint32_t total = P.file_total[f];
+        if (total <= kLkBlock) continue;
+        const uint32_t nblk = (total + kLkBlock - 1) / kLkBlock;
+        uint32_t* c = P.last_tab + (size_t)P.link_first[f] * kLkTab + col;
+        uint32_t run = 0;
+        for (uint32_t b = 0; b < nblk; b += 16) {
+            uint32_t x[16];
+#pragma unroll
+            for (uint32_t k = 0; k < 16; k++) x[k] = b + k + 1 < nblk ? c[(size_t)(b + k) * kLkTab] : 0u;
+#pragma unroll
+            for (uint32_t k = 0; k < 16; k++) {
+                if (b + k < nblk) c[(size_t)(b + k) * kLkTab] = run;
+                run = max(run, x[k]);
+            }
+        }
+    }
+}
+
+struct LinkSmem {
+    uint32_t last[kLkTab];   // place + 1 of the last holder of each filter bit
+    uint32_t own[kLkTab];    // lanes of the current 32 features that hold it
+    uint32_t idx[32][5];     // their big-filter indices
+    // place (from the first one looked at) + 1 of a late holder of an index's
+    // low and of its high 13 bits: an index held late is late in both (chance
+    // matches in both are one in 50, in one table one in 7)
+    uint16_t near_[2][8192];
+};
+__global__ void __launch_bounds__(32) k_feat_links(GenParams P) {
+    extern __shared__ __align__(16) uint8_t smem[];
+    LinkSmem& S = *reinterpret_cast<LinkSmem*>(smem);
+    const uint32_t lane = threadIdx.x;
+    for (uint32_t i = lane; i < kLkTab; i += 32) S.own[i] = 0;
+    for (uint32_t f = blockIdx.y; f < P.nfiles; f += gridDim.y) {
+        const uint32_t total = P.file_total[f];
+        if (total == 0) continue;
+        uint4* v = P.links + link_base(P, P.files[f]);
+        const uint32_t nblk = (total + kLkBlock - 1) / kLkBlock;
+        for (uint32_t b = blockIdx.x; b < nblk; b += gridDim.x) {
+            __syncwarp();
+            const uint32_t* row = P.last_tab + ((size_t)P.link_first[f] + b) * kLkTab;
+            for (uint32_t i = lane; i < kLkTab; i += 32) S.last[i] = b ? __ldg(row + i) : 0u;
+            uint4* n4 = reinterpret_cast<uint4*>(S.near_);
+            for (uint32_t i = lane; i < sizeof S.near_ / 16; i += 32) n4[i] = make_uint4(0, 0, 0, 0);
+            const uint32_t o0 = b * kLkBlock, o1 = min(total, o0 + kLkBlock), h0 = b ? o0 - kLkNear : 0u;
+            __syncwarp();
+            // the features before the block that a window may still hold
+            // (other blocks' warps write these entries' flags meanwhile; the
+            // indices stay)
+            for (uint32_t o = h0 + lane; o < o0; o += 32) {  // whole groups of 32
+                uint32_t x[5];
+                link_unpack(v[o], x);
+#pragma unroll
+                for (int k = 0; k < 5; k++) S.near_[0][x[k] & 8191u] = S.near_[1][x[k] >> 4] = (uint16_t)(o - h0 + 1);
+                __syncwarp();
+            }
+            __syncwarp();
+            uint4 cur = o0 + lane < o1 ? v[o0 + lane] : make_uint4(0, 0, 0, 0);
+            for (uint32_t g = o0; g < o1; g += 32) {
+                const uint32_t o = g + lane;
+                const bool have = o < o1;
+                const uint4 nxt = o + 32 < o1 ? v[o + 32] : make_uint4(0, 0, 0, 0);
+                uint32_t x[5], held[5], own[5], nr[5], nh[5];
+                link_unpack(cur, x);
+                const uint32_t here = o - h0 + 1;
+#pragma unroll
+                for (int k = 0; k < 5; k++) {
+                    held[k] = S.last[x[k] & kBfMask];
+                    nr[k] = S.near_[0][x[k] & 8191u];
+                    nh[k] = S.near_[1][x[k] >> 4];
+                    if (have) atomicOr(&S.own[x[k] & kBfMask], 1u << lane);
+                    S.idx[lane][k] = x[k];
+                }
+                __syncwarp();
+#pragma unroll
+                for (int k = 0; k < 5; k++) own[k] = S.own[x[k] & kBfMask];
+                __syncwarp();
+                if (have) {
+                    uint32_t least = 0xFFFFFFFFu, flags = 0;
+#pragma unroll
+                    for (int k = 0; k < 5; k++) {
+                        const uint32_t lower = own[k] & lanemask_lt();
+                        least = min(least, lower ? g + 32 - __clz(lower) : held[k]);
+                        const bool late = nr[k] != 0 && nh[k] != 0 && here - min(nr[k], nh[k]) < kLkNear;
+                        bool same = late;
+                        for (uint32_t l = lower; l && !same; l &= l - 1u) {  // earlier ones of these 32, word by word
+                            const uint32_t* e = S.idx[31 - __clz(l & (0u - l))];
+                            same = e[0] == x[k] || e[1] == x[k] || e[2] == x[k] || e[3] == x[k] || e[4] == x[k];
+                        }
+                        flags |= (uint32_t)same << k;
+                        if ((own[k] >> lane) == 1u) S.last[x[k] & kBfMask] = o + 1;
+                        S.own[x[k] & kBfMask] = 0;
+                        S.near_[0][x[k] & 8191u] = S.near_[1][x[k] >> 4] = (uint16_t)here;
+                    }
+                    reinterpret_cast<uint2*>(v + o)[1] = make_uint2((cur.z & 0x1FFFFFu) | (flags << 21), least);
+                }
+                __syncwarp();
+                cur = nxt;
+            }
+        }
+    }
+}
+
+constexpr uint32_t kChRing = 1024;
+struct ChainSmem {
+    uint4 ring[kChRing];                  // links staged ahead
+    alignas(16) uint8_t G[kBigMask + 1];  // big filter, a byte per bit: set by plain stores
+    uint32_t match[kCmWin];               // slow path: big-filter values held by an earlier feature
+    alignas(8) uint8_t counted[8];        // features counted per warp
+    uint32_t ambig[8];                    // slow path, per warp
+    uint32_t end;                         // features the pass consumes, when F or G rolls over
+};
+static_assert(offsetof(ChainSmem, G) % 16 == 0 && offsetof(ChainSmem, counted) % 8 == 0, "read as 16- and 8-byte words");
+
+__global__ void __launch_bounds__(kCmWin) k_stream_chain(GenParams P) {
+    extern __shared__ __align__(16) uint8_t smem[];
+    ChainSmem& S = *reinterpret_cast<ChainSmem*>(smem);
+    const uint32_t tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    S.match[tid] = 0;
+    // ones in the bytes of the warps before this one
+    const uint32_t below_x = wid >= 4 ? 0x01010101u : 0x01010101u & ((1u << (8 * wid)) - 1u);
+    const uint32_t below_y = wid == 5 ? 1u : 0u;
+    for (uint32_t fi = blockIdx.x; fi < P.nfiles; fi += gridDim.x) {
+        const uint32_t file = P.file_order[fi];
+        const GenFile Fd = P.files[file];
+        if (Fd.nchunks == 0) continue;
+        const GenChunk cl = P.chunks[Fd.first_chunk + Fd.nchunks - 1];
+        const uint32_t t_end = cl.first_tile + cl.ntiles, base = link_base(P, Fd), total = P.file_total[file];
+        const uint4* v = P.links + base;
+        uint32_t* ends = P.ends + Fd.filter_base;
+        // a chunk's first feature; the big filter's counter restarts there
+        uint32_t chunk = 0;
+        const auto chunk_start = [&](uint32_t k) {
+            if (k >= Fd.nchunks) return total;
+            const uint32_t t = P.chunks[Fd.first_chunk + k].first_tile;
+            return t < t_end ? P.tile_base[t] - base : total;
+        };
+        uint32_t seg_end = chunk_start(1);
+        uint32_t bf_count = 1, last_count = 0, bigfi = 0, fs = 0, pos = 0;
+        uint32_t e0 = 0, e1 = 0, e2 = 0, e3 = 0;  // ends of the copies started up to this pass, the ones before
+        uint32_t n_pass = 0, n_ambig = 0;
+        const long long t_file = P.phase ? clock64() : 0;
+        // this thread's feature of the window: five indices, near flags, last holder
+        uint32_t h[5] = {0, 0, 0, 0, 0}, near_ = 0, held = 0;
+        bool loaded = false;
+        __syncthreads();  // the previous file is done with the shared state
+        for (uint32_t i = tid; i < sizeof S.G / 16; i += kCmWin) reinterpret_cast<uint4*>(S.G)[i] = make_uint4(0, 0, 0, 0);
+        for (; e0 < min(total, 4u * kCmWin); e0 += kCmWin)
+            if (e0 + tid < total) cp_async16(&S.ring[e0 + tid], v + e0 + tid);
+        e0 = min(e0, total);
+        while (pos < total) {
+            while (pos == seg_end) {
+                bigfi = 0;
+                seg_end = chunk_start(++chunk + 1);
+            }
+            n_pass++;
+            // stage on: places below this window's start are free (reads that
+            // may still be under way are of this window's features)
+            e3 = e2;
+            e2 = e1;
+            e1 = e0;
+            const uint32_t room = min(min((uint32_t)kCmWin, total - e0), pos + kChRing - e0);
+            if (tid < room) cp_async16(&S.ring[(e0 + tid) & (kChRing - 1)], v + e0 + tid);
+            e0 += room;
+            cp_async_commit();
+            uint32_t avail = e3;
+            if (e3 - pos < min((uint32_t)kCmWin, total - pos)) {
+                cp_async_wait_all();
+                avail = e3 = e2 = e1 = e0;
+            } else {
+                asm volatile("cp.async.wait_group 3;\n" ::);
+            }
+            __syncthreads();  // (1) copies and the last pass's big-filter bits are there
+            const uint32_t W = min(min((uint32_t)kCmWin, avail - pos), seg_end - pos);
+            const bool have = tid < W;
+            if (have && !loaded) {
+                const uint4 x = S.ring[(pos + tid) & (kChRing - 1)];
+                link_unpack(x, h);
+                near_ = x.z >> 21;
+                held = x.w;
+            }
+            const bool gate = have && held <= fs;
+            // a big-filter bit that is unset (0) before the window, and one
+            // that is unset and near no other holder
+            uint32_t g[5], un = 1, sure = 1;
+#pragma unroll
+            for (int k = 0; k < 5; k++) g[k] = S.G[h[k]];
+#pragma unroll
+            for (int k = 0; k < 5; k++) {
+                un = min(un, g[k]);
+                sure = min(sure, g[k] | (near_ & (1u << k)));
+            }
+            bool cnt_def = gate && sure == 0;
+            const bool amb = gate && un == 0 && sure != 0;
+            uint32_t mc = __ballot_sync(0xffffffffu, cnt_def);
+            if (lane == 0) S.counted[wid] = (uint8_t)__popc(mc);
+            if (__syncthreads_or(amb)) {  // (2)
+                // an ambiguous feature's value k is held by an earlier
+                // F-passing feature of the window?
+                const uint32_t ma = __ballot_sync(0xffffffffu, amb);
+                if (lane == 0) S.ambig[wid] = ma;
+                __syncthreads();
+                for (uint32_t w = 0; w < (uint32_t)kCmWarps; w++) {
+                    for (uint32_t am = S.ambig[w]; am; am &= am - 1u) {
+                        const uint32_t j = 32 * w + (uint32_t)(__ffs(am) - 1);
+                        n_ambig++;
+                        if (wid > w) continue;  // later features only
+                        uint32_t mm = 0;
+                        if (gate && tid < j) {
+                            uint32_t x[5];
+                            link_unpack(S.ring[(pos + j) & (kChRing - 1)], x);
+#pragma unroll
+                            for (int k = 0; k < 5; k++)
+#pragma unroll
+                                for (int q = 0; q < 5; q++) mm |= (uint32_t)(h[q] == x[k]) << k;
+                        }
+                        mm = __reduce_or_sync(0xffffffffu, mm);
+                        if (lane == 0 && mm) atomicOr(&S.match[j], mm);
+                    }
+                }
+                __syncthreads();
+                if (amb) {
+                    const uint32_t mm = S.match[tid];
+#pragma unroll
+                    for (int k = 0; k < 5; k++) cnt_def |= g[k] == 0 && !((mm >> k) & 1u);
+                    S.match[tid] = 0;
+                }
+                mc = __ballot_sync(0xffffffffu, cnt_def);
+                if (lane == 0) S.counted[wid] = (uint8_t)__popc(mc);
+                __syncthreads();
+            }
+            // counted features before this one and in all: byte sums
+            const uint2 cw = *reinterpret_cast<const uint2*>(S.counted);
+            const uint32_t all = __dp4a(cw.x, 0x01010101u, __dp4a(cw.y, 0x00000101u, 0u));
+            const uint32_t before = __dp4a(cw.x, below_x, __dp4a(cw.y, below_y, (uint32_t)__popc(mc & lanemask_lt())));
+            const uint32_t need_s = (uint32_t)kMaxElem - last_count, need_b = (uint32_t)kBigElem - bigfi;
+            const uint32_t need = min(need_s, need_b);
+            const bool roll = all >= need;  // the need-th counted feature ends the pass
+            if (roll && cnt_def && before + 1 == need) S.end = tid + 1;
+            __syncthreads();  // (3)
+            const uint32_t n = roll ? S.end : W;
+            const bool roll_small = roll && need == need_s, roll_big = roll && need == need_b;
+            // the next window's feature is read while this one's bits are set
+            const uint32_t next = pos + n + tid;
+            loaded = next < avail;
+            uint4 x = make_uint4(0, 0, 0, 0);
+            if (loaded) x = S.ring[next & (kChRing - 1)];
+            if (gate && tid < n && !roll_big) {
+#pragma unroll
+                for (int k = 0; k < 5; k++) S.G[h[k]] = 1;
+            }
+            if (roll_big)
+                for (uint32_t i = tid; i < sizeof S.G / 16; i += kCmWin)
+                    reinterpret_cast<uint4*>(S.G)[i] = make_uint4(0, 0, 0, 0);
+            link_unpack(x, h);
+            near_ = x.z >> 21;
+            held = x.w;
+            last_count += min(all, need);
+            bigfi += min(all, need);
+            pos += n;
+            if (roll_small) {
+                if (tid == 0) {
+                    if (bf_count <= Fd.filter_cap) ends[bf_count - 1] = pos;
+                    else atomicAdd(P.counters + 1, 1u);
+                }
+                bf_count++;
+                last_count = 0;
+                fs = pos;
+            }
+            if (roll_big) bigfi = 0;
+        }
+        cp_async_wait_all();
+        if (tid == 0) {
+            if (bf_count <= Fd.filter_cap) ends[bf_count - 1] = total;
+            else atomicAdd(P.counters + 1, 1u);
+            commit_result(P, file, bf_count, last_count);
+            if (P.phase) {
+                const long long busy = clock64() - t_file;
+                atomicAdd(P.phase + kPhCommitBusy, (unsigned long long)busy);
+                atomicAdd(P.phase + kPhCommitGroups, (unsigned long long)n_pass);
+                atomicAdd(P.phase + kPhCommitLoops, (unsigned long long)n_ambig);
+                atomicMax(P.phase + kPhCommitMaxFile, (unsigned long long)busy);
+            }
+        }
+    }
+}
+
+// A warp per filter: the bits of its features, written to the file's output
+// slots (dst_off; null: a batch of one file, from slot 0).
+__global__ void __launch_bounds__(256) k_stream_emit(GenParams P, const uint64_t* __restrict__ dst_off,
+                                                     uint32_t* __restrict__ dst, uint64_t dst_cap) {
+    __shared__ uint32_t F[8][64];
+    const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    for (uint32_t f = blockIdx.y; f < P.nfiles; f += gridDim.y) {
+        const GenFile Fd = P.files[f];
+        if (Fd.nchunks == 0) continue;
+        const uint32_t nf = P.out_info[f].bf_count;
+        const uint4* v = P.links + link_base(P, Fd);
+        const uint32_t* ends = P.ends + Fd.filter_base;
+        const uint64_t slot = dst_off ? dst_off[f] : 0;
+        for (uint32_t k = blockIdx.x * 8 + wid; k < nf && k < Fd.filter_cap && slot + k < dst_cap; k += gridDim.x * 8) {
+            F[wid][lane] = 0;
+            F[wid][lane + 32] = 0;
+            __syncwarp();
+            const uint32_t b = k ? ends[k - 1] : 0u, e = ends[k];
+            for (uint32_t o = b + lane; o < e; o += 32) {
+                uint32_t x[5];
+                link_unpack(__ldg(v + o), x);
+#pragma unroll
+                for (int q = 0; q < 5; q++) atomicOr(&F[wid][(x[q] & kBfMask) >> 5], 1u << (x[q] & 31));
+            }
+            __syncwarp();
+            reinterpret_cast<uint2*>(dst + (slot + k) * 64)[lane] = reinterpret_cast<const uint2*>(F[wid])[lane];
+            __syncwarp();
+        }
+    }
+}
+
 // ------------------------------------------------------------ block mode
 // kPre: the block's ranks come from k_stream_ranks (64-byte windows do not
 // know about blocks; only a block's last 64 positions have rank 0), and the
@@ -1996,6 +2459,8 @@ static void set_stream_attrs() {
     cudaFuncSetAttribute(k_stream_commit, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(CommitSmem<false>));
     cudaFuncSetAttribute(k_stream_commit_round, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)sizeof(CommitSmem<true>));
+    cudaFuncSetAttribute(k_stream_chain, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(ChainSmem));
+    cudaFuncSetAttribute(k_feat_links, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(LinkSmem));
     // one shared-memory / L1 split for every kernel of the stream pipeline
     // (the largest shared memory): CTAs of different kernels can then share
     // an SM
@@ -2004,7 +2469,9 @@ static void set_stream_attrs() {
                           (const void*)k_stream_fix_list<true>,
                           (const void*)k_stream_fix<false>, (const void*)k_stream_fix<true>,
                           (const void*)k_stream_commit, (const void*)k_stream_commit_round,
-                          (const void*)k_stream_commit_index})
+                          (const void*)k_stream_commit_index, (const void*)k_feat_scan, (const void*)k_feat_pack,
+                          (const void*)k_feat_last, (const void*)k_feat_carry, (const void*)k_feat_links,
+                          (const void*)k_stream_chain, (const void*)k_stream_emit})
         cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared);
     done = true;
 }
@@ -2094,6 +2561,32 @@ cudaError_t launch_stream_index_mark(const GenParams& P, const uint32_t* seen, c
 cudaError_t launch_pred_dirty(const GenParams& P, const uint32_t* a, const uint32_t* b, uint64_t nwords,
                               uint8_t* dirty, uint32_t* from, unsigned int* ndirty, uint32_t grid, cudaStream_t st) {
     k_pred_dirty<<<grid, 256, 0, st>>>(a, b, nwords, P.tiles, P.chunks, P.ntiles, dirty, from, ndirty);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_stream_links(const GenParams& P, uint32_t sms, cudaStream_t st) {
+    set_stream_attrs();
+    const uint32_t files = min(P.nfiles, 4096u);
+    // CTAs per file: enough to fill the SMs with one-warp CTAs
+    const uint32_t x = max(4u, 24 * sms / files);
+    k_feat_scan<<<min(P.nfiles, 2 * sms), 1024, 0, st>>>(P);
+    k_feat_pack<<<min((P.ntiles + 7) / 8, 8 * sms), 256, 0, st>>>(P);
+    k_feat_last<<<dim3(x, files), 32, 0, st>>>(P);
+    k_feat_carry<<<dim3(kLkTab / 128, files), 128, 0, st>>>(P);
+    k_feat_links<<<dim3(x, files), 32, sizeof(LinkSmem), st>>>(P);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_stream_chain(const GenParams& P, uint32_t grid, cudaStream_t st) {
+    set_stream_attrs();
+    k_stream_chain<<<grid, kCmWin, sizeof(ChainSmem), st>>>(P);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_stream_emit(const GenParams& P, const uint64_t* dst_off, uint32_t* dst, uint64_t dst_cap, uint32_t sms,
+                               cudaStream_t st) {
+    const uint32_t files = min(P.nfiles, 4096u);
+    k_stream_emit<<<dim3(max(1u, 8 * sms / files), files), 256, 0, st>>>(P, dst_off, dst, dst_cap);
     return cudaGetLastError();
 }
 

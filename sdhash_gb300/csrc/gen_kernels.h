@@ -132,6 +132,14 @@ struct GenParams {
     const uint2* rk_items;
     uint32_t nrk_items;
     uint32_t rk_per;  // positions per thread (one of kRkPers)
+    // linked commit (null links: k_stream_commit): a file's features packed
+    // behind one another from links[first tile of the file * kTileCap] on
+    uint4* links;
+    uint32_t* tile_base;         // per tile: its first feature's place in links
+    uint32_t* file_total;        // per file: its features
+    const uint32_t* link_first;  // per file: its first row of last_tab
+    uint32_t* last_tab;          // per block of kLkBlock features: 2,048 last holders
+    uint32_t* ends;              // [GenFile::filter_base + k]: end of a file's filter k, in features
 };
 
 // Index search samples counted features 0, 4, 8, ... of a block
@@ -162,6 +170,18 @@ cudaError_t launch_stream_tiles(const GenParams& P, uint32_t grid, cudaStream_t 
 cudaError_t launch_stream_fails(const GenParams& P, uint32_t grid, cudaStream_t st);
 cudaError_t launch_stream_fix_list(const GenParams& P, uint32_t grid, cudaStream_t st);
 cudaError_t launch_stream_fix(const GenParams& P, uint32_t grid, cudaStream_t st);
+// Commit with links (P.links): what the ordered pass needs to know of a
+// feature's predecessors is worked out by all SMs first, and its filters are
+// filled afterwards (launch_stream_emit, once their output slots are known).
+constexpr uint32_t kLkBlock = 1024;
+constexpr uint32_t kLkTab = 2048;  // filter bits
+// Most blocks of a file of this many tiles.
+inline uint64_t link_blocks(uint64_t tiles) { return (tiles * kTileCap + kLkBlock - 1) / kLkBlock; }
+constexpr uint32_t kLkMaxTiles = 1u << 22;  // of a group: places in links fit 32 bits
+cudaError_t launch_stream_links(const GenParams& P, uint32_t sms, cudaStream_t st);
+cudaError_t launch_stream_chain(const GenParams& P, uint32_t grid, cudaStream_t st);
+cudaError_t launch_stream_emit(const GenParams& P, const uint64_t* dst_off, uint32_t* dst, uint64_t dst_cap, uint32_t sms,
+                               cudaStream_t st);
 cudaError_t launch_stream_commit(const GenParams& P, uint32_t grid, cudaStream_t st);
 // One warp, files in file_order, index inserts (GenParams::index_bits).
 cudaError_t launch_stream_commit_index(const GenParams& P, cudaStream_t st);

@@ -70,7 +70,7 @@ extern "C" void sdbfg_ctx_destroy(sdbfg_ctx* c) {
                       &c->d_from, &c->d_ranks})
         b->release();
     for (auto& S : c->slot) {
-        for (DevBuf* b : {&S.data, &S.tables, &S.tile_out, &S.features, &S.work}) b->release();
+        for (DevBuf* b : {&S.data, &S.tables, &S.tile_out, &S.features, &S.work, &S.links, &S.last_tab, &S.chain}) b->release();
         S.h_tables.release();
         if (S.stream) cudaStreamDestroy(S.stream);
         if (S.done) cudaEventDestroy(S.done);
@@ -673,25 +673,40 @@ static int digest_stream_pipelined(sdbfg_ctx* c, const uint8_t* host_data, const
         // ---- work lists (pinned host staging, copied asynchronously)
         // rank stretches: every chunk position (to a multiple of 8), rk_span(per) at a time
         uint64_t nchunks = 0, ntiles = 0, bytes = 0, nrks[kRkChoices] = {};
+        uint64_t most_tiles = 0, nlinks = 0, nfilters = 0;  // of a file; link blocks and filter slots of all
         for (uint32_t k = 0; k < g.count; k++) {
             const uint64_t len = lens[g.first + k];
             bytes += (len + 15) & ~15ull;
             if (len < kMinFile) continue;
+            const uint64_t tiles0 = ntiles;
             for (uint64_t pos = 0; pos < len; pos += kChunkBytes) {
                 const uint64_t m = std::min<uint64_t>(kChunkBytes, len - pos);
                 nchunks++;
                 if (m > 64) ntiles += (m - 64 + kTileL - 1) / kTileL;
                 for (int q = 0; q < kRkChoices; q++) nrks[q] += rk_stretches((uint32_t)m, kRkPers[q]);
             }
+            most_tiles = std::max(most_tiles, ntiles - tiles0);
+            nlinks += link_blocks(ntiles - tiles0);
+            nfilters += stream_cap(len);
+        }
+        const auto up = [](size_t v) { return (v + 15) / 16 * 16; };
+        bool chain = !ib && most_tiles >= kChainTiles && 2 * most_tiles >= ntiles && ntiles < kLkMaxTiles;
+        const size_t at_total = up(ntiles * 4), at_ends = at_total + up(g.count * 4);
+        if (chain && (S.links.ensure(ntiles * kTileCap * sizeof(uint4)) != cudaSuccess ||
+                      S.last_tab.ensure(nlinks * kLkTab * 4) != cudaSuccess || S.chain.ensure(at_ends + nfilters * 4) != cudaSuccess)) {
+            cudaGetLastError();
+            S.links.release();
+            S.last_tab.release();
+            chain = false;
         }
         const int rk = rk_choose(nrks, (uint32_t)c->sms);
         const uint64_t nrk = nrks[rk];
         const uint32_t rspan = rk_span(kRkPers[rk]);
         const bool pre = pre_ranks && ntiles;
-        const auto up = [](size_t v) { return (v + 15) / 16 * 16; };
         const size_t at_tiles = up(nchunks * sizeof(GenChunk)), at_files = at_tiles + up(ntiles * sizeof(GenTile));
         const size_t at_order = at_files + up(g.count * sizeof(GenFile)), at_rk = at_order + up(g.count * sizeof(uint32_t));
-        const size_t at_fix = at_rk + up(pre ? nrk * sizeof(uint2) : 0), table_bytes = at_fix + 4;
+        const size_t at_first = at_rk + up(pre ? nrk * sizeof(uint2) : 0);
+        const size_t at_fix = at_first + up(g.count * 4), table_bytes = at_fix + 4;
         CUDA_TRY(c, S.h_tables.ensure(table_bytes));
         CUDA_TRY(c, S.tables.ensure(table_bytes + ntiles * 4));
         uint8_t* hb = static_cast<uint8_t*>(S.h_tables.p);
@@ -701,6 +716,7 @@ static int digest_stream_pipelined(sdbfg_ctx* c, const uint8_t* host_data, const
         GenFile* hf = reinterpret_cast<GenFile*>(hb + at_files);
         uint32_t* ho = reinterpret_cast<uint32_t*>(hb + at_order);
         uint2* hr = reinterpret_cast<uint2*>(hb + at_rk);
+        uint32_t* hl = reinterpret_cast<uint32_t*>(hb + at_first);
         *reinterpret_cast<uint32_t*>(hb + at_fix) = 0;
         const uint8_t* gdata;
         std::vector<uint64_t> doff(g.count);
@@ -733,11 +749,13 @@ static int digest_stream_pipelined(sdbfg_ctx* c, const uint8_t* host_data, const
                 }
             }
         }
-        uint32_t ci = 0, ti = 0, ri = 0, r8 = 0;
+        uint32_t ci = 0, ti = 0, ri = 0, r8 = 0, li = 0;
         uint64_t work = 0;
         for (uint32_t k = 0; k < g.count; k++) {
             const uint32_t i = g.first + k;
             GenFile f{ci, 0, work, 0};
+            hl[k] = li;
+            const uint32_t file_tile = ti;
             if (lens[i] >= kMinFile) {
                 for (uint64_t pos = 0; pos < lens[i]; pos += kChunkBytes) {
                     const uint32_t m = (uint32_t)std::min<uint64_t>(kChunkBytes, lens[i] - pos);
@@ -753,6 +771,7 @@ static int digest_stream_pipelined(sdbfg_ctx* c, const uint8_t* host_data, const
                 }
                 f.filter_cap = stream_cap(lens[i]);
                 work += f.filter_cap;
+                li += (uint32_t)link_blocks(ti - file_tile);
             }
             hf[k] = f;
             ho[k] = k;
@@ -762,7 +781,7 @@ static int digest_stream_pipelined(sdbfg_ctx* c, const uint8_t* host_data, const
                              [&](uint32_t a, uint32_t b) { return lens[g.first + a] > lens[g.first + b]; });
         CUDA_TRY(c, S.tile_out.ensure(std::max<uint64_t>(1, ntiles) * sizeof(TileOut)));
         CUDA_TRY(c, S.features.ensure(std::max<uint64_t>(1, ntiles) * 5ull * kTileCap * 4));
-        CUDA_TRY(c, S.work.ensure(solo ? 16 : std::max<uint64_t>(1, work) * 256));
+        CUDA_TRY(c, S.work.ensure(solo || chain ? 16 : std::max<uint64_t>(1, work) * 256));
         CUDA_TRY(c, cudaMemcpyAsync(db, hb, table_bytes, cudaMemcpyHostToDevice, st));
         GenParams P{};
         P.data = gdata;
@@ -788,6 +807,14 @@ static int digest_stream_pipelined(sdbfg_ctx* c, const uint8_t* host_data, const
             P.rk_items = reinterpret_cast<uint2*>(db + at_rk);
             P.nrk_items = (uint32_t)nrk;
             P.rk_per = kRkPers[rk];
+        }
+        if (chain) {
+            P.links = S.links.as<uint4>();
+            P.last_tab = S.last_tab.as<uint32_t>();
+            P.link_first = reinterpret_cast<uint32_t*>(db + at_first);
+            P.tile_base = S.chain.as<uint32_t>();
+            P.file_total = reinterpret_cast<uint32_t*>(S.chain.as<uint8_t>() + at_total);
+            P.ends = reinterpret_cast<uint32_t*>(S.chain.as<uint8_t>() + at_ends);
         }
         const uint32_t cap_grid = (uint32_t)c->sms * 3 * 16;
         // the groups' tile kernels run one after another (each fills the GPU),
@@ -826,11 +853,17 @@ static int digest_stream_pipelined(sdbfg_ctx* c, const uint8_t* host_data, const
             P.index_new = ib->count;
             rc = commit_with_index(c, P, cap_grid, st);
             if (rc) return rc;
+        } else if (chain) {
+            TIMED_LAUNCH_ON(c, "k_feat_links", st, launch_stream_links(P, (uint32_t)c->sms, st));
+            c->launches += 4;  // five kernels, one is counted with the timer
+            TIMED_LAUNCH_ON(c, "k_stream_chain", st, launch_stream_chain(P, std::min<uint32_t>(g.count, cap_grid), st));
         } else {
             TIMED_LAUNCH_ON(c, "k_stream_commit", st,
                             launch_stream_commit(P, std::min<uint32_t>(g.count, cap_grid), st));
         }
         if (solo) {
+            if (chain)
+                TIMED_LAUNCH_ON(c, "k_stream_emit", st, launch_stream_emit(P, nullptr, dev_out, out_cap, (uint32_t)c->sms, st));
             CUDA_TRY(c, cudaEventRecord(S.done, st));
             break;
         }
@@ -841,10 +874,14 @@ static int digest_stream_pipelined(sdbfg_ctx* c, const uint8_t* host_data, const
                          cudaGetLastError()));
         CUDA_TRY(c, cudaEventRecord(c->ev_scan[gi % depth], st));
         prev_scan = c->ev_scan[gi % depth];
-        TIMED_LAUNCH_ON(c, "k_pack_filters", st,
-                        (k_pack_group<<<std::min<uint32_t>(g.count, (uint32_t)c->sms * 8), 256, 0, st>>>(
-                             S.work.as<uint32_t>(), P.files, d_info + g.first, d_off + g.first, dev_out, g.count),
-                         cudaGetLastError()));
+        if (chain)
+            TIMED_LAUNCH_ON(c, "k_stream_emit", st,
+                            launch_stream_emit(P, d_off + g.first, dev_out, out_cap, (uint32_t)c->sms, st));
+        else
+            TIMED_LAUNCH_ON(c, "k_pack_filters", st,
+                            (k_pack_group<<<std::min<uint32_t>(g.count, (uint32_t)c->sms * 8), 256, 0, st>>>(
+                                 S.work.as<uint32_t>(), P.files, d_info + g.first, d_off + g.first, dev_out, g.count),
+                             cudaGetLastError()));
         CUDA_TRY(c, cudaEventRecord(S.done, st));
     }
     // join: the caller's stream waits for both slots, then results come back
