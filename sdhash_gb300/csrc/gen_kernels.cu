@@ -375,27 +375,38 @@ __device__ inline void compute_ranks(const TileGeom& g, const TileSmem& s, const
 // For step k with rank[k] > 0 the full rescan of gen_chunk_scores picks the
 // smallest non-zero rank m of window [k, k+63], at its leftmost position f,
 // extended right over the run of equal ranks (capped at k+63).  Stored as
-// (m << 6) | (p - k); 0 when rank[k] == 0 (no credit, next step rescans).
+// (m << 6) | (p - k); kNoRes when rank[k] == 0 (no credit, next step rescans).
 //
-// One thread per aligned 64-step block A (steps base..base+63); the window
-// of step base+u is A[u..63] followed by B[0..u-1], B the next block.
-//  pass 1, u = 63..0: the leftmost minimum of A[u..63] and the end of its
-//    run inside A, as a running state -- a rank equal to the minimum
-//    becomes the new leftmost one, keeping the run end only when its right
-//    neighbour continues the run.  Written to fres[base+u] (0 when
-//    rank[base+u] == 0).
-//  pass 2, v = 0..62: the same state for the prefix B[0..v] (a run end
-//    advances only while the run is contiguous) and the end of B's leading
-//    run; step u = v+1 takes A's minimum on ties (leftmost), continuing its
-//    run into B when it reaches A's last position and B starts with the
-//    same rank.  Both run ends stay within the window, so no cap is needed.
+// A position's key is (its rank, the end of its run of equal ranks): the
+// smallest key of a window is the leftmost run of its smallest rank, and it
+// holds that run's end.  Keys are (r - 1) * 64 + e, so that a rank of 0 wraps
+// around to above every key.  One thread per aligned 64-step block A (steps
+// base..base+63); the window of step base+u is A[u..63] followed by
+// B[0..u-1], B the next block.
+//  pass 1, u = 63..0: suffix minimum of A's keys (run ends inside A), written
+//    to fres[base+u] (kNoRes when rank[base+u] == 0);
+//  pass 2, v = 0..62: the smallest rank of the prefix B[0..v] and the end of
+//    its leftmost run so far.  T is what a rank's (r - 1) * 64 + 63 may be at
+//    most to change them: that of the minimum while its run is open (an equal
+//    rank extends the run), less than it once the run has ended.  Step
+//    u = v+1 takes A's minimum on ties (leftmost); when A's is the run that
+//    ends at A's last position and B starts with the same rank, the run goes
+//    on into B.  Run ends stay within the window, so no cap is needed.
 // Positions past the tile's last step are read but only feed steps that no
 // walk uses (every array extends past them).
+//
+// What bounds the tile kernels is the integer pipe (79 % busy, issue 72 %):
+// both passes are a handful of compares, selects and minima per step, the
+// multiplications and additions left to the other pipe: 8,300 cycles of a
+// tile's 47,600 (running minimum, run end and previous rank as separate states:
+// 12,100), the tile kernel 14.8 to 13.7 ms on 3.1 GB, k_block_digest 5.1 to
+// 4.6 ms on 1 GiB.
 //
 // Both passes move eight steps at a time: the next group's ranks (two per
 // 32-bit word; pidx keeps a block contiguous and 4-byte aligned) are loaded
 // before the current group's results are stored, so no load waits behind a
 // store.
+constexpr uint32_t kNoRes = kNoRank << 6;  // full-rescan result: no rank
 __device__ inline void compute_fres(const TileGeom& g, const TileSmem& s) {
     const uint32_t nsteps = g.SE - g.Q0;
     const uint32_t nblk = (nsteps + 63) / 64;
@@ -404,15 +415,16 @@ __device__ inline void compute_fres(const TileGeom& g, const TileSmem& s) {
         const uint32_t* __restrict__ Ra = reinterpret_cast<const uint32_t*>(s.ranks + pidx(base));
         const uint32_t* __restrict__ Rb = reinterpret_cast<const uint32_t*>(s.ranks + pidx(base + 64));
         uint32_t* __restrict__ Fa = reinterpret_cast<uint32_t*>(s.fres + pidx(base));
-        // pass 1: suffix states of A, steps 63..0
-        uint32_t m = 1023, e = 63, rn = 0;
+        // pass 1: suffix minima of A's keys, steps 63..0
+        uint32_t key = 0xFFFFFFFFu, e = 0, rn = 0xFFFFu;  // e: the run's end - 64
         uint32_t cur[4], nxt[4] = {0, 0, 0, 0};
 #pragma unroll
         for (int q = 0; q < 4; q++) cur[q] = Ra[28 + q];
-        uint32_t first = 0;  // result of step 0 (final after pass 1)
+        uint32_t first = 0;  // key of step 0
         uint32_t any = 0;    // OR of block A's ranks
+        uint32_t u0 = 0u - 8u;  // position of the group's first step - 64
 #pragma unroll 1
-        for (int gi = 7; gi >= 0; gi--) {
+        for (int gi = 7; gi >= 0; gi--, u0 -= 8) {
             any |= cur[0] | cur[1] | cur[2] | cur[3];
             if (gi > 0) {
 #pragma unroll
@@ -421,20 +433,16 @@ __device__ inline void compute_fres(const TileGeom& g, const TileSmem& s) {
             uint32_t out[4];
 #pragma unroll
             for (int q = 3; q >= 0; q--) {
-                uint32_t o2 = 0;
+                uint32_t o2[2];
 #pragma unroll
                 for (int h = 1; h >= 0; h--) {
-                    const uint32_t u = 8u * gi + 2 * q + h;
                     const uint32_t r = h ? (cur[q] >> 16) : (cur[q] & 0xFFFFu);
-                    // r != 0 and (r < m, or r == m after a run break), as one
-                    // unsigned compare (m >= 1): r - 1 < m - (rn == m)
-                    const bool take = (r - 1u) < (m - (uint32_t)(rn == m));
-                    m = take ? r : m;
-                    e = take ? u : e;
+                    e = r == rn ? e : u0 + 2 * q + h;
+                    key = min(key, r * 64 + e);
+                    o2[h] = r == 0 ? kNoRes : key;
                     rn = r;
-                    o2 |= (r == 0 ? 0u : ((m << 6) | e)) << (16 * h);
                 }
-                out[q] = o2;
+                out[q] = __byte_perm(o2[0], o2[1], 0x5410);
             }
             first = out[0] & 0xFFFFu;
 #pragma unroll
@@ -442,8 +450,8 @@ __device__ inline void compute_fres(const TileGeom& g, const TileSmem& s) {
 #pragma unroll
             for (int q = 0; q < 4; q++) cur[q] = nxt[q];
         }
-        // a block whose ranks are all 0 (low-entropy content) is done: every
-        // step's result is 0, as pass 1 wrote
+        // a block whose ranks are all 0 (low-entropy content) is done: no
+        // step has a result, as pass 1 wrote
         if (any == 0) continue;
         // pass 2: prefix states of B, steps u = v + 1 = 1..63; results are
         // packed into aligned words with the previous group's last one
@@ -452,18 +460,17 @@ __device__ inline void compute_fres(const TileGeom& g, const TileSmem& s) {
         for (int q = 0; q < 4; q++) rb[q] = Rb[q];
 #pragma unroll
         for (int q = 0; q < 5; q++) fa[q] = Fa[q];
-        const uint32_t rb0 = rb[0] & 0xFFFFu;
-        // A's leftmost minimum whose run reaches A's last position has A's
-        // last rank, so it continues into B iff B starts with that rank
-        const uint32_t r63 = Ra[31] >> 16;
-        const bool contB = r63 != 0 && r63 == rb0;
-        // pm / pe64: minimum of B[0..v] and 64 + the end of its leftmost run;
-        // open: that run ends at v; lead64: 64 + the end of B's leading run
-        uint32_t pm = 1023, pe64 = 64, lead64 = 64;
-        bool open = false, lead_open = true;
-        uint32_t carry = first;
+        // A's run up to its last position goes on into B's leading run
+        const uint32_t rb0 = rb[0] & 0xFFFFu, r63 = Ra[31] >> 16;
+        const bool cont = r63 != 0 && r63 == rb0;
+        const uint32_t tail = cont ? r63 * 64 - 1 : 0xFFFFFFFFu;  // that run's key in A
+        bool lead_open = true;
+        uint32_t lead = tail;  // with its end so far in B
+        uint32_t pm = kNoRes - 1, T = pm, pval = 0;  // smallest rank of B's prefix as (r - 1) * 64 + 63; its key
+        uint32_t carry = first == kNoRes ? kNoRes : first + 64;
+        uint32_t v0 = 0;
 #pragma unroll 1
-        for (uint32_t gi = 0; gi < 8; gi++) {
+        for (uint32_t gi = 0; gi < 8; gi++, v0 += 8) {
             if (gi < 7) {
 #pragma unroll
                 for (int q = 0; q < 4; q++) nrb[q] = Rb[4 * (gi + 1) + q];
@@ -474,28 +481,25 @@ __device__ inline void compute_fres(const TileGeom& g, const TileSmem& s) {
             uint32_t res[8];
 #pragma unroll
             for (int t = 0; t < 8; t++) {
-                const uint32_t v = 8 * gi + t;
                 const uint32_t r = (t & 1) ? (rb[t >> 1] >> 16) : (rb[t >> 1] & 0xFFFFu);
                 lead_open = lead_open && r == rb0;
-                lead64 = lead_open ? 64 + v : lead64;
-                const bool lower = (r - 1u) < (pm - 1u);  // r != 0 && r < pm (pm >= 1)
-                const bool cont = open && r == pm;  // pm > 0, so r != 0
-                pm = lower ? r : pm;
-                open = lower || cont;
-                pe64 = open ? 64 + v : pe64;
-                const uint32_t u = v + 1;  // its suffix state is halfword t + 1 of fa
+                lead += lead_open;
+                const uint32_t q = r * 64 - 1;
+                const bool upd = q <= T;
+                pm = upd ? q : pm;
+                pval = upd ? q + v0 + (t + 1) : pval;
+                T = upd ? q : pm - 1;
+                // step u = v + 1: its suffix minimum is halfword t + 1 of fa
                 const uint32_t sv = ((t + 1) & 1) ? (fa[(t + 1) >> 1] >> 16) : (fa[(t + 1) >> 1] & 0xFFFFu);
-                const uint32_t sm = sv >> 6, se = sv & 63;
-                const bool a_wins = sm <= pm;
-                const uint32_t mm = a_wins ? sm : pm;
-                const uint32_t p = a_wins ? ((se == 63 && contB) ? lead64 : se) : pe64;
-                res[t] = sv == 0 ? 0u : ((mm << 6) | (p - u));
+                const uint32_t a = sv == tail ? lead : sv;
+                const uint32_t w = sv <= pm ? a : pval;
+                res[t] = sv == kNoRes ? kNoRes : w + (63 - t) - v0;  // + 64 - u
             }
             // steps 8gi .. 8gi+7 as words 4gi .. 4gi+3 (step 8gi from the carry)
-            Fa[4 * gi] = carry | (res[0] << 16);
-            Fa[4 * gi + 1] = res[1] | (res[2] << 16);
-            Fa[4 * gi + 2] = res[3] | (res[4] << 16);
-            Fa[4 * gi + 3] = res[5] | (res[6] << 16);
+            Fa[4 * gi] = __byte_perm(carry, res[0], 0x5410);
+            Fa[4 * gi + 1] = __byte_perm(res[1], res[2], 0x5410);
+            Fa[4 * gi + 2] = __byte_perm(res[3], res[4], 0x5410);
+            Fa[4 * gi + 3] = __byte_perm(res[5], res[6], 0x5410);
             carry = res[7];  // step 8gi + 8 (the next block's step 0 when gi == 7: dropped)
 #pragma unroll
             for (int q = 0; q < 4; q++) rb[q] = nrb[q];
@@ -523,7 +527,7 @@ struct Credit {
             else atomicSub(&score32[o >> 2], inc);
         }
     }
-    // step i credits p when act (its min rank is not 0); a step that
+    // step i credits p when act (its window has a rank); a step that
     // credits nothing opens a run of ~0u, which is never added
     // (the open run is closed inline: one predicate for "changed and in range")
     __device__ __forceinline__ void add(uint32_t i, uint32_t p, bool act) {
@@ -535,7 +539,7 @@ struct Credit {
             if (kSign > 0) atomicAdd(&score32[o >> 2], inc);
             else atomicSub(&score32[o >> 2], inc);
         }
-        cur = chg ? key : cur;
+        cur = key;
         start = chg ? i : start;
     }
 };
@@ -544,11 +548,11 @@ struct Credit {
 // rank[i+64] and the full-rescan result of step i.
 template <typename CR>
 __device__ __forceinline__ void walk_step(ChainState& st, uint32_t i, uint32_t r64, uint32_t f, CR* cr) {
-    const bool cheap = (st.M != 0) & (r64 >= st.M) & (i < st.P);
+    const bool cheap = (r64 >= st.M) & (i < st.P);  // never with M == kNoRank
     const uint32_t cheapP = (r64 == st.M) ? i + 64 : st.P;
     st.P = cheap ? cheapP : i + (f & 63);
     st.M = cheap ? st.M : (f >> 6);
-    if (cr) cr->add(i, st.P, st.M != 0);
+    if (cr) cr->add(i, st.P, st.M != kNoRank);
 }
 
 // Eight consecutive 16-bit entries starting at an 8-aligned index (inside
@@ -562,7 +566,7 @@ __device__ __forceinline__ uint32_t half16(const uint32_t* w, int k) {
     return (k & 1) ? (w[k >> 1] >> 16) : (w[k >> 1] & 0xFFFFu);
 }
 
-// Walk steps [a, b) of gen_chunk_scores from state `st` (st.M == 0 makes step
+// Walk steps [a, b) of gen_chunk_scores from state `st` (st.M == kNoRank makes step
 // a a full rescan: the speculative start, or step 0).  Single steps up to an
 // 8-aligned step (Q0 is a multiple of 64, so tile offsets are aligned too),
 // then groups of eight whose operands (rank[i+64..], fres[i..]) are loaded
@@ -690,7 +694,7 @@ __device__ void tile_pipeline(const uint8_t* __restrict__ chunk, const TileGeom&
     const bool has_seg = t < kSegs && SL > 0 && St < g.SE;
     if (t < kSegs) {
         if (has_seg) {
-            ChainState st{0, 0};
+            ChainState st{0, kNoRank};
             if (t == 0 && entry) {
                 st = unpack_state(*entry);
             } else {

@@ -97,19 +97,21 @@ __device__ __forceinline__ void load_be16_global(const uint8_t* src, uint32_t (&
 
 // ------------------------------------------------- popularity-chain state
 // State entering a window step i of gen_chunk_scores (sdbf_core.cc:58-82):
-// (P, M) = current (min_pos, min_rank).  M == 0 means the next step is a
-// full rescan regardless of P, so P is normalised to 0 in that case.
+// (P, M) = current (min_pos, min_rank).  M == kNoRank (above every rank, so
+// no rank is at least M) means the next step is a full rescan regardless of
+// P; a packed state is 0 in that case.
+constexpr uint32_t kNoRank = 1023;
 struct ChainState {
     uint32_t P;
     uint32_t M;
 };
 __device__ __forceinline__ uint64_t pack_state(ChainState s) {
-    return s.M == 0 ? 0ull : ((uint64_t)s.M << 32) | s.P;
+    return s.M == kNoRank ? 0ull : ((uint64_t)s.M << 32) | s.P;
 }
 __device__ __forceinline__ ChainState unpack_state(uint64_t v) {
     ChainState s;
     s.P = (uint32_t)v;
-    s.M = (uint32_t)(v >> 32);
+    s.M = v ? (uint32_t)(v >> 32) : kNoRank;
     return s;
 }
 
