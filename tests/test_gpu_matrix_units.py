@@ -121,3 +121,23 @@ def test_repeated_runs_agree(ctx):
         ctx.set_compare_tuning(5, 1 << 22, True)
     for k in range(40):
         assert np.array_equal(ctx.compare_all(dev), want), k
+
+
+@pytest.mark.parametrize("counts", [list(range(1, 60)), [1] * 100 + [2] * 30 + [3] * 3 + [900], [5, 5, 6, 6, 6, 7, 127, 128, 129, 400],
+                                    [60, 64, 64, 65, 2000], [1, 2, 3], [40] * 5 + [41] * 5 + [1500] * 2])
+@pytest.mark.parametrize("folded", [False, True])
+def test_bundles_of_small_digests(ctx, counts, folded):
+    """All pairs of digests whose small ones share passes: every pair scored
+    once, in the swap rule's order, classes of equal counts and folded digests among them."""
+    import sdhash_gb300 as g
+    rng = np.random.default_rng(len(counts) + sum(counts))
+    pool = np.stack([bits_to_bytes(rng.choice(2048, size=660, replace=False)) for _ in range(12)])
+    order = rng.permutation(len(counts))
+    ds = [random_digest(g, rng, f"d{i:03d}", counts[k], pool=pool) for i, k in enumerate(order)]
+    if folded:
+        ds = [d.fast() if i % 3 == 1 else d for i, d in enumerate(ds)]
+    s = ctx.upload(ds)
+    i, j = np.triu_indices(len(ds), 1)
+    want = ctx.score_pairs(s, s, i, j)
+    assert (want > 0).any()
+    assert np.array_equal(ctx.compare_all(s), want)
