@@ -42,6 +42,7 @@ constexpr uint64_t kFirstHostGroupBytes = 32ull << 20;
 // uneven files 22.9 ms against 21.2.
 constexpr uint32_t kChainTiles = 384;
 constexpr uint64_t kFirstIndexGroupBytes = 256ull << 20;  // with an index being built (groups one after another)
+constexpr uint64_t kFetchFilters = 512;  // output filters (128 KiB) that a host batch reads back with its results
 constexpr uint32_t kMinFile = 512;                 // MIN_FILE_SIZE (sdbf_defines.h:56)
 constexpr uint64_t kPairsPerLaunch = 1ull << 22;
 constexpr int kSlots = 8;  // stream-mode launch groups in flight (at most)

@@ -528,7 +528,7 @@ static int commit_with_index(sdbfg_ctx* c, GenParams P, uint32_t cap_grid, cudaS
 static int digest_stream_pipelined(sdbfg_ctx* c, const uint8_t* host_data, const uint8_t* dev_data,
                                    const uint64_t* offsets_in, const uint64_t* lens_in, uint32_t n, uint32_t* dev_out,
                                    uint64_t out_cap, sdbfg_digest_result* res, uint64_t* total_out,
-                                   const IndexBuild* ib = nullptr) {
+                                   const IndexBuild* ib = nullptr, uint64_t fetch = 0) {
     int rc = ensure_pipeline(c);
     if (rc) return rc;
     // Launch groups are formed over the inputs sorted by size (largest first),
@@ -573,7 +573,8 @@ static int digest_stream_pipelined(sdbfg_ctx* c, const uint8_t* host_data, const
     // results: total | output slot per file | info per file, read back in one copy
     const size_t at_info = 64 + (size_t)n * sizeof(uint64_t), result_bytes = at_info + n * sizeof(FileInfoDev);
     CUDA_TRY(c, c->d_result.ensure(result_bytes));
-    CUDA_TRY(c, c->h_result.ensure(result_bytes + 64));
+    const size_t at_fetch = (result_bytes + 64 + 255) / 256 * 256;  // the first `fetch` filters, with the results
+    CUDA_TRY(c, c->h_result.ensure(at_fetch + fetch * 256));
     CUDA_TRY(c, cudaMemsetAsync(c->d_result.p, 0, result_bytes, c->stream));
     uint64_t* d_total = c->d_result.as<uint64_t>();
     uint64_t* d_off = d_total + 8;
@@ -894,6 +895,7 @@ static int digest_stream_pipelined(sdbfg_ctx* c, const uint8_t* host_data, const
     const uint32_t* flags = reinterpret_cast<const uint32_t*>(hr + result_bytes);
     CUDA_TRY(c, cudaMemcpyAsync(hr, c->d_result.p, result_bytes, cudaMemcpyDeviceToHost, c->stream));
     CUDA_TRY(c, cudaMemcpyAsync(hr + result_bytes, c->d_counters.p, 8, cudaMemcpyDeviceToHost, c->stream));
+    if (fetch) CUDA_TRY(c, cudaMemcpyAsync(hr + at_fetch, dev_out, fetch * 256, cudaMemcpyDeviceToHost, c->stream));
     CUDA_TRY(c, cudaStreamSynchronize(c->stream));
     if (flags[1]) return fail(c, SDBFG_ERR_CUDA, "internal error: stream digest exceeded its filter bound");
     if (solo) *total = info[0].bf_count;
@@ -1228,10 +1230,19 @@ extern "C" int sdbfg_digest_batch(sdbfg_ctx* c, const uint8_t* host_data, const 
         for (uint32_t i = 0; i < n; i++)
             if (lens[i] >= kMinFile) cap_needed += stream_cap(lens[i]);
         CUDA_TRY(c, c->d_out_filters.ensure(std::max<uint64_t>(1, cap_needed) * 256));
+        // a few filters come back with the results, as many as there can be,
+        // instead of in a copy of their own behind a second wait (one 64 KiB
+        // file: 104 us, 112 with them)
+        const uint64_t cap = std::min(cap_needed, out_cap), fetch = cap <= kFetchFilters ? cap : 0;
         uint64_t total = 0;
-        rc = digest_stream_pipelined(c, host_data, nullptr, offsets, lens, n, c->d_out_filters.as<uint32_t>(),
-                                     std::min(cap_needed, out_cap), res, &total);
+        rc = digest_stream_pipelined(c, host_data, nullptr, offsets, lens, n, c->d_out_filters.as<uint32_t>(), cap, res,
+                                     &total, nullptr, fetch);
         if (rc) return rc;
+        if (fetch) {
+            const size_t at = (64 + (size_t)n * (sizeof(uint64_t) + sizeof(FileInfoDev)) + 64 + 255) / 256 * 256;
+            memcpy(out_filters, static_cast<uint8_t*>(c->h_result.p) + at, total * 256);
+            return SDBFG_OK;
+        }
         if (total) CUDA_TRY(c, cudaMemcpyAsync(out_filters, c->d_out_filters.p, total * 256, cudaMemcpyDeviceToHost, st));
         CUDA_TRY(c, cudaStreamSynchronize(st));
         return SDBFG_OK;
