@@ -215,11 +215,12 @@ def peaks():
 
 def compare_roofline(pairs_per_s: float, variant: int, sm_mhz=None):
     """Roofline of the comparison kernel.  The tensor-core variant counts
-    popcount(a & b) of two 2,048-bit filters as an e4m3 dot product of length
-    2,048 (4,096 fp8 FLOPs per filter pair) against the fp8 dense rate, taken
-    as twice the measured bf16 rate (MEASURED_PEAKS.json has no fp8 figure;
-    nominal dense fp8 is 4.5 PFLOP/s).  The CUDA-core variants are integer
-    issue bound: 64 AND + 64 POPC + 63 adds per filter pair against 128
+    popcount(a & b) of two 2,048-bit filters as an e2m1 dot product of length
+    2,048 (4,096 FLOPs per filter pair), stated against the fp8 dense rate,
+    taken as twice the measured bf16 rate (MEASURED_PEAKS.json has no figure
+    below bf16; nominal dense fp8 is 4.5 PFLOP/s, fp4 13.5): the bound earlier
+    builds, which counted in e4m3, are stated against.  The CUDA-core variants
+    are integer issue bound: 64 AND + 64 POPC + 63 adds per filter pair against 128
     integer lanes per SM per clock."""
     try:
         with open(os.path.join(REPO, "MEASURED_PEAKS.json")) as f:
@@ -232,7 +233,7 @@ def compare_roofline(pairs_per_s: float, variant: int, sm_mhz=None):
         ach = pairs_per_s * 4096 / 1e12
         return {"bound": "tensor", "kernel": "k_matrix_tc", "achieved": ach, "peak": peak, "unit": "TFLOP/s",
                 "frac": ach / peak, "traffic": None,
-                "work_per_filter_pair": "4096 fp8 FLOPs (2048-bit AND-popcount as an e4m3 0/1 dot product)",
+                "work_per_filter_pair": "4096 FLOPs (2048-bit AND-popcount as an e2m1 dot product, counted at the fp8 rate)",
                 "peak_source": f"2 x {src} bf16 burst (MEASURED_PEAKS.json bf16_tflops; fp8 dense = 2 x bf16)",
                 "mma_bound_filter_pairs_per_s": peak * 1e12 / 4096}
     mhz = sm_mhz or 2070.0
@@ -411,20 +412,21 @@ def allpairs_digests(args, ctx):
     return digs, counts, int(sizes.sum())
 
 
-TC_PHASES = ("compose", "fill", "fetch_wait", "stage_wait", "widen", "issue", "producer_step", "acc_wait", "score",
-             "mark", "walk", "fold", "consumer_step", "step_barrier", "tmem_ld")
+TC_WARPS = {"compose": 1, "widen": 6, "mma": 1, "mark": 4, "check": 8}  # roles of the kernel
 
 
 def tc_phases(ctx, run):
-    """SM cycles per tile of each phase of the tensor-core kernel (one CTA's
-    clock, summed over CTAs, divided by the tiles counted) for one more run."""
+    """SM cycles per tile of each role of the tensor-core kernel, busy and
+    waiting (a warp's, of the tiles counted), for one more run."""
     import torch
     ctx.profile(True)
     run()
     torch.cuda.synchronize()
     tiles = ctx.kernel_time("k_matrix_tc.tiles")[0] or 1.0
-    out = {k: round(ctx.kernel_time("k_matrix_tc." + k)[0] / tiles) for k in TC_PHASES}
+    out = {k + w: round(ctx.kernel_time("k_matrix_tc." + k + w)[0] / tiles / n)
+           for k, n in TC_WARPS.items() for w in ("", "_wait")}
     out["tiles"] = int(tiles)
+    out["marked_per_tile"] = round(ctx.kernel_time("k_matrix_tc.marked")[0] / tiles, 1)
     ctx.profile(False)
     return out
 

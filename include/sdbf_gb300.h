@@ -72,8 +72,9 @@ int sdbfg_ctx_kernel_time(sdbfg_ctx *ctx, const char *kernel, double *total_ms, 
  * lead-ins only make the re-walk path run more often; tests use this to
  * exercise it.  No counterpart in the reference (its walk is sequential). */
 int sdbfg_ctx_set_lead(sdbfg_ctx *ctx, uint32_t steps);
-/* Stream-mode launch groups (<= 2 GiB of input each) kept in flight on
- * separate streams, 1..8 (default 4): the ordered commit of one group
+/* Stream-mode launch groups (<= 256 MiB of input each, or one larger input)
+ * kept in flight on separate streams, 1..8 (default 8: up to eight, four of
+ * 1 GiB in batches of more than 4 GiB): the ordered commit of one group
  * overlaps the next groups' tile kernels.  Depth 1 runs groups one after
  * another (used to time kernels without overlap).  Tuning knob without a
  * counterpart in the reference. */
@@ -113,8 +114,8 @@ uint64_t sdbfg_digest_capacity(const uint64_t *lens, uint32_t n, uint32_t dd_blo
  * The file / istream constructors (sdbf_class.cc:34,71) read the bytes and
  * then do exactly this.
  * host_data + offsets[i] holds input i (lens[i] bytes) in HOST memory
- * (pinned memory is copied directly, pageable memory through a staging
- * buffer).  Filters land in out_filters (host, 256 bytes per slot,
+ * (read by the device itself where it can: pinned memory, and pageable
+ * memory on systems whose devices use the host's page tables).  Filters land in out_filters (host, 256 bytes per slot,
  * capacity out_cap filter slots, see sdbfg_digest_capacity); block-mode
  * element counts in out_elem_counts (one uint16 per slot; may be NULL for
  * stream mode). */

@@ -64,7 +64,7 @@ cudaError_t launch_fold(uint32_t* filters, uint32_t* meta, CmpDigest* digests, u
 // whose filters are summed after the swap rule) against a run of target
 // digests from a target list, or -- for a single pair too large for one unit --
 // a row range of the reference digest against one target ("split" unit, its
-// per-filter maxima go to a slot array and k_matrix_finalize sums them).
+// per-filter maxima go to a slot array and are summed at the end).
 namespace sdbfg {
 
 constexpr uint32_t kMatMaxTargets = 512;  // targets per unit (running sums in shared memory)
@@ -80,7 +80,7 @@ enum : uint32_t { kUnitRefSide1 = 1u, kUnitTgtSide1 = 2u, kUnitSplit = 4u, kUnit
 //    rows (ref = digest id, rows [r0, r1) = all its filters), running sums
 //    per target in shared memory;
 //  * split (kUnitSplit): rows [r0, r1) of one reference digest against one
-//    target; maxima to the slot array, summed by k_matrix_finalize.  The
+//    target; maxima to the slot array, summed at the end.  The
 //    tensor-core kernel also splits the target's filters ([c0, c1), with a
 //    group's digests as rows too: their splits are consecutive), its maxima
 //    are unsigned integers of 2^-23 and k_matrix_finish sums them.

@@ -30,6 +30,12 @@ constexpr uint64_t kFirstHostSlabBytes = 16ull << 20;  // first slab of a host-i
 // 3.1 GB on the device: 21.2 ms, in groups of 2 GiB 22.2, of 128 MiB 25.4;
 // 0.9 GB from the host: 10.9 ms against 11.9 in groups of 512 MiB and more.
 constexpr uint64_t kStreamGroupBytes = 256ull << 20;
+// A long batch keeps the GPU busy whatever the groups' size, and many commits in
+// flight take the registers that the staging gather's CTAs need on an SM: groups
+// of 1 GiB, four in flight.  28.4 GB: 160 ms on the device and 201 from the
+// host; 256 MiB, eight in flight: 164 and 303; 2 GiB, four: 160 and 200.
+constexpr uint64_t kLongBatchBytes = 4ull << 30;
+constexpr uint64_t kLongGroupBytes = 1ull << 30;
 // First group of a host-input stream batch (each later one at most twice it):
 // its copy is the one nothing hides.  64 files of 1 MiB: 1.06 ms, with 16 MiB
 // 1.11, with 64 MiB (one group) 1.17.
@@ -195,7 +201,7 @@ struct sdbfg_ctx {
         DevBuf tables;
         HostBuf h_tables;
     } slot[kSlots];
-    int depth = 8;  // launch groups in flight
+    int depth = kSlots;  // launch groups in flight (at kSlots: fewer in long batches)
     DevBuf d_result, d_phase;  // of a stream batch: total filters, per-file info and output slots
     HostBuf h_result;
     HostBuf h_block;  // a block-mode launch group's tables

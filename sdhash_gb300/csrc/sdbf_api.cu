@@ -580,9 +580,13 @@ static int digest_stream_pipelined(sdbfg_ctx* c, const uint8_t* host_data, const
     uint64_t* d_off = d_total + 8;
     FileInfoDev* d_info = reinterpret_cast<FileInfoDev*>(d_off + n);
     CUDA_TRY(c, cudaEventRecord(c->ev_start, c->stream));
+    uint64_t batch_bytes = 0;
+    for (uint32_t i = 0; i < n; i++) batch_bytes += lens[i];
+    const bool long_batch = batch_bytes > kLongBatchBytes;
+    const uint64_t group_bytes = long_batch ? kLongGroupBytes : kStreamGroupBytes;
     const std::vector<Group> groups =
         ib ? make_groups(lens, n, 0, host_data ? kFirstIndexGroupBytes : kMaxBytesPerLaunch)
-           : make_groups(lens, n, 0, host_data ? kFirstHostGroupBytes : kStreamGroupBytes, kStreamGroupBytes);
+           : make_groups(lens, n, 0, host_data ? kFirstHostGroupBytes : group_bytes, group_bytes);
     std::vector<uint64_t> stage_off;
     if (staged) {
         stage_off.resize(n);
@@ -663,9 +667,24 @@ static int digest_stream_pipelined(sdbfg_ctx* c, const uint8_t* host_data, const
     const bool solo = n == 1 && !ib && lens[0] >= kMinFile && stream_cap(lens[0]) <= out_cap;
     cudaEvent_t prev_scan = c->ev_start, prev_tiles = c->ev_start, prev2_tiles = c->ev_start;
     const uint64_t rank_half = c->d_ranks.cap / 2 / 16 * 16;  // bytes per half, 16-byte aligned
+    // A buffer that must be had: without room the linked commit's, which need
+    // not, are given back first (cudaFree waits for their users).
+    const auto need = [&](DevBuf& b, size_t bytes) {
+        cudaError_t e = b.ensure(bytes);
+        if (e == cudaErrorMemoryAllocation) {
+            cudaGetLastError();
+            for (sdbfg_ctx::Slot& s : c->slot) {
+                s.links.release();
+                s.last_tab.release();
+            }
+            e = b.ensure(bytes);
+        }
+        return e;
+    };
+    const int max_depth = c->depth == kSlots && long_batch ? 4 : kSlots;  // (a lower depth is taken as it is)
     for (size_t gi = 0; gi < groups.size(); gi++) {
         const Group& g = groups[gi];
-        const int depth = ib ? 1 : std::max(1, std::min(c->depth, kSlots));
+        const int depth = ib ? 1 : std::max(1, std::min(c->depth, max_depth));
         sdbfg_ctx::Slot& S = c->slot[gi % depth];
         cudaStream_t st = S.stream;
         if (S.used) CUDA_TRY(c, cudaEventSynchronize(S.done));  // its pinned tables may be reused now
@@ -691,15 +710,6 @@ static int digest_stream_pipelined(sdbfg_ctx* c, const uint8_t* host_data, const
             nfilters += stream_cap(len);
         }
         const auto up = [](size_t v) { return (v + 15) / 16 * 16; };
-        bool chain = !ib && most_tiles >= kChainTiles && 2 * most_tiles >= ntiles && ntiles < kLkMaxTiles;
-        const size_t at_total = up(ntiles * 4), at_ends = at_total + up(g.count * 4);
-        if (chain && (S.links.ensure(ntiles * kTileCap * sizeof(uint4)) != cudaSuccess ||
-                      S.last_tab.ensure(nlinks * kLkTab * 4) != cudaSuccess || S.chain.ensure(at_ends + nfilters * 4) != cudaSuccess)) {
-            cudaGetLastError();
-            S.links.release();
-            S.last_tab.release();
-            chain = false;
-        }
         const int rk = rk_choose(nrks, (uint32_t)c->sms);
         const uint64_t nrk = nrks[rk];
         const uint32_t rspan = rk_span(kRkPers[rk]);
@@ -709,7 +719,7 @@ static int digest_stream_pipelined(sdbfg_ctx* c, const uint8_t* host_data, const
         const size_t at_first = at_rk + up(pre ? nrk * sizeof(uint2) : 0);
         const size_t at_fix = at_first + up(g.count * 4), table_bytes = at_fix + 4;
         CUDA_TRY(c, S.h_tables.ensure(table_bytes));
-        CUDA_TRY(c, S.tables.ensure(table_bytes + ntiles * 4));
+        CUDA_TRY(c, need(S.tables, table_bytes + ntiles * 4));
         uint8_t* hb = static_cast<uint8_t*>(S.h_tables.p);
         uint8_t* db = S.tables.as<uint8_t>();
         GenChunk* hc = reinterpret_cast<GenChunk*>(hb);
@@ -729,7 +739,7 @@ static int digest_stream_pipelined(sdbfg_ctx* c, const uint8_t* host_data, const
             for (uint32_t k = 0; k < g.count; k++) doff[k] = stage_off[g.first + k];
             CUDA_TRY(c, cudaStreamWaitEvent(st, c->ev_copy[gi], 0));
         } else {
-            CUDA_TRY(c, S.data.ensure(std::max<uint64_t>(16, bytes)));
+            CUDA_TRY(c, need(S.data, std::max<uint64_t>(16, bytes)));
             gdata = S.data.as<uint8_t>();
             uint64_t b = 0;
             for (uint32_t k = 0; k < g.count; k++) {
@@ -780,9 +790,22 @@ static int digest_stream_pipelined(sdbfg_ctx* c, const uint8_t* host_data, const
         if (!ib)
             std::stable_sort(ho, ho + g.count,
                              [&](uint32_t a, uint32_t b) { return lens[g.first + a] > lens[g.first + b]; });
-        CUDA_TRY(c, S.tile_out.ensure(std::max<uint64_t>(1, ntiles) * sizeof(TileOut)));
-        CUDA_TRY(c, S.features.ensure(std::max<uint64_t>(1, ntiles) * 5ull * kTileCap * 4));
-        CUDA_TRY(c, S.work.ensure(solo || chain ? 16 : std::max<uint64_t>(1, work) * 256));
+        CUDA_TRY(c, need(S.tile_out, std::max<uint64_t>(1, ntiles) * sizeof(TileOut)));
+        CUDA_TRY(c, need(S.features, std::max<uint64_t>(1, ntiles) * 5ull * kTileCap * 4));
+        bool chain = !ib && most_tiles >= kChainTiles && 2 * most_tiles >= ntiles && ntiles < kLkMaxTiles;
+        const size_t at_total = up(ntiles * 4), at_ends = at_total + up(g.count * 4);
+        if (chain && (S.links.ensure(ntiles * kTileCap * sizeof(uint4)) != cudaSuccess ||
+                      S.last_tab.ensure(nlinks * kLkTab * 4) != cudaSuccess || S.chain.ensure(at_ends + nfilters * 4) != cudaSuccess)) {
+            cudaGetLastError();
+            S.links.release();
+            S.last_tab.release();
+            chain = false;
+        }
+        CUDA_TRY(c, need(S.work, solo || chain ? 16 : std::max<uint64_t>(1, work) * 256));
+        if (chain && !S.links.p) {  // given back for the line above
+            chain = false;
+            CUDA_TRY(c, need(S.work, solo ? 16 : std::max<uint64_t>(1, work) * 256));
+        }
         CUDA_TRY(c, cudaMemcpyAsync(db, hb, table_bytes, cudaMemcpyHostToDevice, st));
         GenParams P{};
         P.data = gdata;
@@ -973,11 +996,13 @@ static int digest_block_group(sdbfg_ctx* c, const uint8_t* dev_base, const std::
         nitems += s.stretches[q];
     }
     first_item.push_back((uint32_t)nitems);
-    CUDA_TRY(c, c->d_chunks.ensure(nchunks * sizeof(GenChunk)));
+    // the tables, on the device and in their pinned copy: blocks | rank
+    // stretches | runs (| pieces, host copy only)
+    const size_t at_items = nchunks * sizeof(GenChunk), at_runs = at_items + nitems * sizeof(uint2);
+    const size_t table_bytes = at_runs + runs.size() * sizeof(GenChunk);
+    CUDA_TRY(c, c->d_chunks.ensure(table_bytes));
     bool pre = c->pre_ranks && dd % 8 == 0;
-    if (pre && (c->d_ranks.ensure(most8 * 16 + 256) != cudaSuccess ||
-                c->d_files.ensure(runs.size() * sizeof(GenChunk)) != cudaSuccess ||
-                c->d_tiles.ensure(nitems * sizeof(uint2)) != cudaSuccess)) {
+    if (pre && c->d_ranks.ensure(most8 * 16 + 256) != cudaSuccess) {
         cudaGetLastError();
         c->d_ranks.release();
         pre = false;
@@ -988,15 +1013,17 @@ static int digest_block_group(sdbfg_ctx* c, const uint8_t* dev_base, const std::
     P.nprobes = c->probe_counts;
     P.feats = c->feat_words;
     P.block_lmax = (lmax + 63) / 64 * 64;
-    // the tables' pinned copy: blocks | rank stretches | runs | pieces
     uint64_t npieces = 0;
     for (const GenChunk& R : runs) npieces += (R.n + kStagePiece - 1) / kStagePiece;
-    CUDA_TRY(c, c->h_block.ensure(nchunks * sizeof(GenChunk) + nitems * sizeof(uint2) + runs.size() * sizeof(GenChunk) +
-                                  npieces * sizeof(StagePiece)));
+    CUDA_TRY(c, c->h_block.ensure(table_bytes + npieces * sizeof(StagePiece)));
     GenChunk* chunks = static_cast<GenChunk*>(c->h_block.p);
     uint2* items = reinterpret_cast<uint2*>(chunks + nchunks);
     GenChunk* hruns = reinterpret_cast<GenChunk*>(items + nitems);
     StagePiece* pieces = reinterpret_cast<StagePiece*>(hruns + runs.size());
+    uint8_t* d_tables = c->d_chunks.as<uint8_t>();
+    P.chunks = c->d_chunks.as<GenChunk>();
+    GenParams R = P;  // the rank kernel's
+    R.chunks = reinterpret_cast<GenChunk*>(d_tables + at_runs);
     if (host_dev) {
         std::vector<uint32_t> first_piece;
         uint32_t np = 0;
@@ -1026,45 +1053,58 @@ static int digest_block_group(sdbfg_ctx* c, const uint8_t* dev_base, const std::
             CUDA_TRY(c, cudaEventRecord(c->ev_copy[k], c->copy_stream));
         }
     }
-    if (pre) {
-        memcpy(hruns, runs.data(), runs.size() * sizeof(GenChunk));
-        CUDA_TRY(c, cudaMemcpyAsync(c->d_files.p, hruns, runs.size() * sizeof(GenChunk), cudaMemcpyHostToDevice, st));
-        P.ranks = c->d_ranks.as<uint16_t>();
+    memcpy(hruns, runs.data(), runs.size() * sizeof(GenChunk));
+    const auto make_items = [&](size_t k) {
+        uint2* it = items + first_item[k];
+        for (uint32_t r = slabs[k].first_run; r < slabs[k].first_run + slabs[k].nruns; r++)
+            for (uint32_t s0 = 0; s0 < (runs[r].n + 7) / 8 * 8; s0 += rk_span(per[k])) *it++ = make_uint2(r, s0);
+    };
+    const auto make_chunks = [&](size_t k, GenChunk* ch) {
+        for (uint32_t r = slabs[k].first_run; r < slabs[k].first_run + slabs[k].nruns; r++) {
+            const GenChunk& u = runs[r];
+            for (uint32_t b = 0, q = 0; b < u.n; b += dd, q++) {
+                const uint32_t len = std::min(dd, u.n - b);
+                *ch++ = {u.data_off + b, len, u.file, 0, 0, u.filter + q, len < dd ? 1u : 0u, u.rank_off8 + b / 8};
+            }
+        }
+    };
+    const auto upload = [&](size_t at, size_t bytes) {
+        return cudaMemcpyAsync(d_tables + at, static_cast<uint8_t*>(c->h_block.p) + at, bytes, cudaMemcpyHostToDevice, st);
+    };
+    // few blocks: all tables in one copy; else a slab's block table is made
+    // while its ranks are computed and the slab before it runs
+    const bool small = slabs.size() == 1 && nchunks <= 4096;
+    if (small) {
+        make_chunks(0, chunks);
+        if (pre) make_items(0);
+        CUDA_TRY(c, upload(0, table_bytes));
+    } else if (pre) {
+        CUDA_TRY(c, upload(at_runs, runs.size() * sizeof(GenChunk)));
     }
-    // a slab's block table is made while the slab before it runs
+    if (pre) R.ranks = P.ranks = c->d_ranks.as<uint16_t>();
     uint64_t first = 0;
     for (size_t k = 0; k < slabs.size(); k++) {
-        const Slab& s = slabs[k];
         if (host_dev) CUDA_TRY(c, cudaStreamWaitEvent(st, c->ev_copy[k], 0));
         if (pre) {
-            uint2* it = items + first_item[k];
-            for (uint32_t r = s.first_run; r < s.first_run + s.nruns; r++)
-                for (uint32_t s0 = 0; s0 < (runs[r].n + 7) / 8 * 8; s0 += rk_span(per[k])) *it++ = make_uint2(r, s0);
-            GenParams R = P;
-            R.chunks = c->d_files.as<GenChunk>();
-            R.rk_items = c->d_tiles.as<uint2>() + first_item[k];
+            R.rk_items = reinterpret_cast<uint2*>(d_tables + at_items) + first_item[k];
             R.nrk_items = first_item[k + 1] - first_item[k];
             R.rk_per = per[k];
-            CUDA_TRY(c, cudaMemcpyAsync(c->d_tiles.as<uint2>() + first_item[k], items + first_item[k],
-                                        R.nrk_items * sizeof(uint2), cudaMemcpyHostToDevice, st));
+            if (!small) {
+                make_items(k);
+                CUDA_TRY(c, upload(at_items + first_item[k] * sizeof(uint2), R.nrk_items * sizeof(uint2)));
+            }
             TIMED_LAUNCH(c, "k_stream_ranks",
                          launch_stream_ranks(R, std::min<uint32_t>(R.nrk_items, (uint32_t)c->sms * 3 * 16), st));
         }
-        GenChunk* ch = chunks + first;
-        for (uint32_t r = s.first_run; r < s.first_run + s.nruns; r++) {
-            const GenChunk& R = runs[r];
-            for (uint32_t b = 0, q = 0; b < R.n; b += dd, q++) {
-                const uint32_t len = std::min(dd, R.n - b);
-                *ch++ = {R.data_off + b, len, R.file, 0, 0, R.filter + q, len < dd ? 1u : 0u, R.rank_off8 + b / 8};
-            }
-        }
         GenParams B = P;
-        B.chunks = c->d_chunks.as<GenChunk>() + first;
-        B.nchunks = s.nchunks;
-        CUDA_TRY(c, cudaMemcpyAsync(c->d_chunks.as<GenChunk>() + first, chunks + first, s.nchunks * sizeof(GenChunk),
-                                    cudaMemcpyHostToDevice, st));
+        B.chunks = P.chunks + first;
+        B.nchunks = slabs[k].nchunks;
+        if (!small) {
+            make_chunks(k, chunks + first);
+            CUDA_TRY(c, upload(first * sizeof(GenChunk), B.nchunks * sizeof(GenChunk)));
+        }
         TIMED_LAUNCH(c, "k_block_digest", launch_block(B, (uint32_t)c->sms, st));
-        first += s.nchunks;
+        first += B.nchunks;
     }
     // the tables are rewritten by the next call
     CUDA_TRY(c, cudaStreamSynchronize(st));

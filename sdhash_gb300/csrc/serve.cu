@@ -13,7 +13,7 @@
 //     order while their filters fit the slot's device memory (admission by
 //     memory), stages them, builds the batch's work units (every query
 //     against every target, orientation by the swap rule) and queues
-//     upload -> k_matrix -> finalize -> scores download on the slot stream;
+//     upload -> the matrix kernels -> scores download on the slot stream;
 //   * requests that arrive while batches are on the GPU wait only for the
 //     next free slot, so their work overlaps with the batches in flight.
 //
