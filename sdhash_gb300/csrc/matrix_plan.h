@@ -230,15 +230,21 @@ inline uint64_t cross_work(uint64_t q, uint64_t t, int variant) {
 // Unit budget for a job of `total` work (filter pairs; tensor-core units:
 // padded rows x target filters) on `slots` resident CTAs: the configured
 // budget, lowered for small jobs so that every CTA gets about four units
-// (no less than 2^16 filter pairs).  A tensor-core job of at most
-// 16 tiles per CTA is cut into one unit per CTA, of whole tiles: a unit's
-// start (rows fetched and widened, pipeline filled) costs about two tiles.
+// (no less than 2^16 filter pairs).  Tensor-core units are whole tiles, about
+// four per CTA, in jobs of at most 16 tiles per CTA about eight (one or two
+// tiles each): lists of uneven lengths leave more units than CTAs, and the
+// CTA that takes two of the large ones is what the job waits for, although a
+// unit's start (rows fetched and widened, pipeline filled) costs about two
+// tiles.  64 x 64 digests of 85 filters, 1,042 tiles: 101 us, with one unit
+// per CTA 140; 67 digests of 32 to 289: 135 and 163; one query of 1,024 filters
+// against four of 8,192: 127 and 144; 376 queries against one: 192 and 203.
+// Above, 120 digests of 20 to 400, 6,583 tiles: 360, with two-tile units 388.
 inline uint64_t effective_unit_budget(uint64_t configured, uint64_t total, uint64_t slots, int variant) {
     slots = std::max<uint64_t>(1, slots);
     if (variant == kMatVariantTc) {
         const uint64_t tile = (uint64_t)kMatVariantTable[variant].rows * kMatVariantTable[variant].tile;
         const uint64_t tiles = (total + tile - 1) / tile;
-        const uint64_t per = tiles <= 16 * slots ? (tiles + slots - 1) / slots : tiles / (4 * slots);
+        const uint64_t per = tiles <= 16 * slots ? tiles / (8 * slots) : tiles / (4 * slots);
         return std::min(configured, std::max<uint64_t>(1, per) * tile);
     }
     return std::min(configured, std::max<uint64_t>(1ull << 16, total / (4 * slots)));
