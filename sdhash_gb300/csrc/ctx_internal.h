@@ -183,9 +183,7 @@ struct sdbfg_ctx {
     // constant tables
     DevBuf d_rank, d_ent, d_cut, d_cut64;
     // generation buffers
-    DevBuf d_data, d_chunks, d_tiles, d_files, d_order, d_tile_out, d_features, d_work_filters, d_info, d_counters,
-        d_pack_src, d_pack_dst_off, d_out_filters, d_out_counts;
-    HostBuf h_stage;
+    DevBuf d_data, d_chunks, d_counters, d_out_filters, d_out_counts;
     HostBuf h_flags;  // small read-backs (pinned)
     // comparison buffers
     DevBuf d_pairs, d_scores;

@@ -60,9 +60,8 @@ extern "C" void sdbfg_ctx_destroy(sdbfg_ctx* c) {
     cudaSetDevice(c->device);
     for (MatPlan* p : c->plans) delete p;
     c->plans.clear();
-    for (DevBuf* b : {&c->d_rank, &c->d_ent, &c->d_cut, &c->d_cut64, &c->d_data, &c->d_chunks, &c->d_tiles, &c->d_files,
-                      &c->d_order, &c->d_tile_out, &c->d_features, &c->d_work_filters, &c->d_info,
-                      &c->d_counters, &c->d_pack_src, &c->d_pack_dst_off, &c->d_out_filters, &c->d_out_counts,
+    for (DevBuf* b : {&c->d_rank, &c->d_ent, &c->d_cut, &c->d_cut64, &c->d_data, &c->d_chunks, &c->d_counters,
+                      &c->d_out_filters, &c->d_out_counts,
                       &c->d_pairs, &c->d_scores, &c->d_result, &c->d_phase,
                       &c->d_match_counts, &c->d_match_offs, &c->d_matches, &c->d_mphase, &c->d_probes,
                       &c->d_nprobes, &c->d_hits, &c->d_index_tab, &c->d_feats, &c->d_idx_bits, &c->d_idx_first,
@@ -86,7 +85,6 @@ extern "C" void sdbfg_ctx_destroy(sdbfg_ctx* c) {
     c->h_stage_items.release();
     if (c->copy_stream) cudaStreamDestroy(c->copy_stream);
     if (c->ev_start) cudaEventDestroy(c->ev_start);
-    c->h_stage.release();
     c->h_flags.release();
     c->h_result.release();
     c->h_block.release();
@@ -204,19 +202,6 @@ extern "C" uint64_t sdbfg_digest_capacity(const uint64_t* lens, uint32_t n, uint
         s += dd ? block_count(lens[i], dd) : stream_cap(lens[i]);
     }
     return s;
-}
-
-// Packs each file's filters from the generation workspace to its final slot.
-__global__ void k_pack_filters(const uint32_t* __restrict__ src, uint32_t* __restrict__ dst,
-                               const uint64_t* __restrict__ src_off, const uint64_t* __restrict__ dst_off,
-                               const FileInfoDev* __restrict__ info, const uint32_t* __restrict__ ids, uint32_t n) {
-    for (uint32_t f = blockIdx.x; f < n; f += gridDim.x) {
-        const uint32_t id = ids[f];
-        const uint64_t words = (uint64_t)info[id].bf_count * 64;
-        const uint4* s = reinterpret_cast<const uint4*>(src + src_off[f] * 64);
-        uint4* d = reinterpret_cast<uint4*>(dst + dst_off[f] * 64);
-        for (uint64_t q = threadIdx.x; q < words / 4; q += blockDim.x) d[q] = s[q];
-    }
 }
 
 namespace {
