@@ -379,10 +379,11 @@ __global__ void __launch_bounds__(kGatherThreads) k_stage_gather(const StagePiec
 // host's page tables; null where neither holds.
 static const uint8_t* host_view(sdbfg_ctx* c, const uint8_t* p) {
     cudaPointerAttributes attr{};
-    const bool pinned = cudaPointerGetAttributes(&attr, p) == cudaSuccess && attr.type == cudaMemoryTypeHost &&
-                        attr.devicePointer != nullptr;
+    const bool known = cudaPointerGetAttributes(&attr, p) == cudaSuccess;
     cudaGetLastError();
-    if (pinned) return static_cast<const uint8_t*>(attr.devicePointer) + (p - static_cast<const uint8_t*>(attr.hostPointer));
+    if (known && attr.type == cudaMemoryTypeDevice) return nullptr;  // not host memory: left to the copies
+    if (known && attr.type == cudaMemoryTypeHost && attr.devicePointer)
+        return static_cast<const uint8_t*>(attr.devicePointer) + (p - static_cast<const uint8_t*>(attr.hostPointer));
     return c->reads_pageable ? p : nullptr;
 }
 

@@ -45,3 +45,17 @@ def test_block_slabs_from_host(ctx, shift, dd):
         assert (got[k] is None) == (one is None)
         if one is not None:
             assert np.array_equal(got[k].filters, one.filters) and np.array_equal(got[k].elem_counts, one.elem_counts)
+
+
+def test_file_backed_inputs(ctx, oracle, tmp_path):
+    """Inputs in a mapped file, as a caller that maps its files passes them."""
+    lens = [70_001, 513, 300_000]
+    offs = [7, 80_000, 100_003]
+    raw = synth.mixture_bytes(54, 0, 420_000)
+    raw.tofile(tmp_path / "in.bin")
+    buf = np.memmap(tmp_path / "in.bin", dtype=np.uint8, mode="r")
+    for dd in (0, 4096):
+        got = ctx.digest_packed(buf, np.array(offs), np.array(lens), dd, ["a", "b", "c"])
+        for k in range(3):
+            want = oracle.digest("abc"[k], raw[offs[k]:offs[k] + lens[k]].tobytes(), dd)
+            assert got[k].to_string() == want.to_string()
