@@ -27,8 +27,9 @@ constexpr uint64_t kFirstHostSlabBytes = 16ull << 20;  // first slab of a host-i
 // Stream batches (inputs sorted by size, largest first) in groups of this size:
 // a group's ordered commits, which one large file can draw out, run beside
 // the tiles of the groups behind it, and the last group's files are small.
-// 3.1 GB on the device: 21.2 ms, in groups of 2 GiB 22.2, of 128 MiB 25.4;
-// 0.9 GB from the host: 10.9 ms against 11.9 in groups of 512 MiB and more.
+// 3.1 GB on the device, with its tiles at 14.8 ms (13.0 now): 21.2 ms, in groups
+// of 2 GiB 22.2, of 128 MiB 25.4; 0.9 GB from the host: 10.9 ms against 11.9 in
+// groups of 512 MiB and more.
 constexpr uint64_t kStreamGroupBytes = 256ull << 20;
 // A long batch keeps the GPU busy whatever the groups' size, and many commits in
 // flight take the registers that the staging gather's CTAs need on an SM: groups
@@ -37,8 +38,8 @@ constexpr uint64_t kStreamGroupBytes = 256ull << 20;
 constexpr uint64_t kLongBatchBytes = 4ull << 30;
 constexpr uint64_t kLongGroupBytes = 1ull << 30;
 // First group of a host-input stream batch (each later one at most twice it):
-// its copy is the one nothing hides.  64 files of 1 MiB: 1.06 ms, with 16 MiB
-// 1.11, with 64 MiB (one group) 1.17.
+// its copy is the one nothing hides.  64 files of 1 MiB: 1.06 ms (1.02 now), with
+// 16 MiB 1.11, with 64 MiB (one group) 1.17.
 constexpr uint64_t kFirstHostGroupBytes = 32ull << 20;
 // A group with a file of this many tiles, and at least half of all, commits
 // through links (k_stream_chain): there the group waits for that one file's

@@ -2161,7 +2161,7 @@ __global__ void __launch_bounds__(256) k_stream_emit(GenParams P, const uint64_t
 // blocks on an SM.  Without (block sizes that are no multiple of 8, or no
 // room for the ranks) the whole block is ranked and walked at once, two
 // blocks to an SM.  A 1 GiB image at 16 KiB blocks: ranks 1.6 ms and this
-// kernel 5.1 ms; with the ranks in the tile it took 4.3 ms more than both,
+// kernel 4.45 ms; when the ranks left the tile the two went from 10.9 to 8.2 ms,
 // most of it the set-up of 96 threads' windows for 170 positions each.
 constexpr uint32_t kBlkL = 8192;
 static_assert(kBlkL / kSegs == 64 && kBlkL % 64 == 0, "a segment is one block of the full-rescan table");
@@ -2231,7 +2231,7 @@ __device__ inline TileSmem carve_block_pre(uint8_t* p) {
 // reaches 192.
 // (One warp that inserted 32 candidates at a time after the whole CTA had
 // counted all 16 K scores one by one and compacted them in two passes: 54 K
-// of a block's 119 K cycles, 6.6 ms for a 1 GiB image; now 5.1 ms.)
+// of a block's 119 K cycles; 6.6 ms for a 1 GiB image became 5.1.)
 constexpr uint32_t kBlkWarpList = ((kMaxBlockBytes / (kGenThreads / 32)) + 64) / 15 + 3;  // scores >= 15 in a warp's range
 
 // Index of the n-th (from 1) set bit of a mask of kGenThreads bits that has as many.
