@@ -226,8 +226,26 @@ static int upload_plan(sdbfg_ctx* c, MatPlan* p, UnitBuilder& ub, const std::vec
     put(at_targets, targets.data(), targets.size() * 4);
     put(at_refs, ub.refs.data(), ub.refs.size() * 4);
     put(at_split, ub.split.data(), ub.split.size() * sizeof(MatSplit));
-    if (at_redo) CUDA_TRY(c, cudaMemcpyAsync(d, p->tables.data(), at_redo, cudaMemcpyHostToDevice, c->stream));
+    if (at_redo) {
+        // queued only: runs on this stream come behind it, and a change of the
+        // stream waits for it (plan_tables_arrived)
+        CUDA_TRY(c, cudaMemcpyAsync(d, p->tables.data(), at_redo, cudaMemcpyHostToDevice, c->stream));
+        if (!c->ev_plan) CUDA_TRY(c, cudaEventCreateWithFlags(&c->ev_plan, cudaEventDisableTiming));
+        CUDA_TRY(c, cudaEventRecord(c->ev_plan, c->stream));
+        c->plan_tables_queued = true;
+    }
     return SDBFG_OK;
+}
+
+cudaError_t plan_tables_arrived(sdbfg_ctx* c) {
+    if (!c->plan_tables_queued) return cudaSuccess;
+    // (the caller may be capturing another stream)
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    const cudaError_t e = cudaEventSynchronize(c->ev_plan);
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    if (e == cudaSuccess) c->plan_tables_queued = false;
+    return e;
 }
 
 // All pairs i<j of one set.  Digests sorted by filter count: a digest is the
@@ -609,17 +627,18 @@ extern "C" int sdbfg_compare_autotune(sdbfg_ctx* c, const sdbfg_set* a, const sd
             int rc = get_plan(c, a, b, mode, &p);
             if (rc) return rc;
             // sampled unit list: every k-th unit (the plan is sorted largest first)
-            std::vector<MatUnit> units(p->nunits);
-            CUDA_TRY(c, cudaMemcpy(units.data(), p->d_units.p, units.size() * sizeof(MatUnit), cudaMemcpyDeviceToHost));
+            // (from the host's tables: their copy to the device may still be queued)
+            const MatUnit* units = reinterpret_cast<const MatUnit*>(p->tables.data());
+            const uint32_t* targets = reinterpret_cast<const uint32_t*>(
+                p->tables.data() + (static_cast<const uint8_t*>(p->d_targets.p) - p->d_all.as<uint8_t>()));
             const uint64_t avg = std::max<uint64_t>(1, p->filter_pairs / std::max<uint32_t>(1, p->nunits));
             const uint64_t want = std::max<uint64_t>(1, sample_pairs / avg);
-            const uint64_t step = std::max<uint64_t>(1, units.size() / want);
+            const uint64_t step = std::max<uint64_t>(1, p->nunits / want);
             std::vector<MatUnit> sample;
-            for (uint64_t k = 0; k < units.size(); k += step)
+            for (uint64_t k = 0; k < p->nunits; k += step)
                 if (!(units[k].flags & kUnitSplit)) sample.push_back(units[k]);
             if (sample.empty()) continue;
             uint64_t pairs = 0;
-            std::vector<uint32_t> tl;  // target list for work counting
             DevBuf d_sample;
             CUDA_TRY(c, d_sample.ensure(sample.size() * sizeof(MatUnit)));
             CUDA_TRY(c, cudaMemcpy(d_sample.p, sample.data(), sample.size() * sizeof(MatUnit), cudaMemcpyHostToDevice));
@@ -629,17 +648,10 @@ extern "C" int sdbfg_compare_autotune(sdbfg_ctx* c, const sdbfg_set* a, const sd
             P.nunits = (uint32_t)sample.size();
             P.nsplit = 0;
             {
-                std::vector<uint32_t> targets;
-                // count filter pairs of the sample from the target list on the host
+                // count filter pairs of the sample from the target list
                 const sdbfg_set* ts_all = b ? b : a;
-                size_t tn = 0;
-                for (const MatUnit& u : sample) tn = std::max<size_t>(tn, u.t1);
-                targets.resize(tn);
-                if (tn) CUDA_TRY(c, cudaMemcpy(targets.data(), p->d_targets.p, tn * 4, cudaMemcpyDeviceToHost));
                 for (const MatUnit& u : sample) {
-                    const sdbfg_set* rset = (u.flags & kUnitRefSide1) ? ts_all : a;
                     const sdbfg_set* tset = (u.flags & kUnitTgtSide1) ? ts_all : a;
-                    (void)rset;
                     for (uint32_t e = u.t0; e < u.t1; e++) pairs += (uint64_t)(u.r1 - u.r0) * tset->bf_count[targets[e]];
                 }
             }

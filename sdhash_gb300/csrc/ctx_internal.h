@@ -218,6 +218,8 @@ struct sdbfg_ctx {
     uint64_t mat_unit_work = 1ull << 22;
     bool mat_graphs = true;
     std::vector<struct MatPlan*> plans;
+    cudaEvent_t ev_plan = nullptr;      // behind the last copy of a plan's tables,
+    bool plan_tables_queued = false;    //   which may not have run yet
     DevBuf d_match_counts, d_match_offs, d_matches, d_mphase;
     // index search: per-slot probe words and counts of the group being
     // digested (set around a block-mode batch), the device index table
@@ -289,6 +291,10 @@ struct sdbfg_set {
 // Serial number of a new set (cached comparison plans are keyed by it).
 uint64_t next_set_serial();
 
+// Waits until the tables of the context's plans are on the device: before
+// work on another stream than the one their copies are queued on.
+cudaError_t plan_tables_arrived(sdbfg_ctx* c);
+
 // A comparison job prepared for the matrix engine: work units sorted by
 // size, the target list, split-pair table and slot array, and (once run) a
 // CUDA graph of its launches.
@@ -302,7 +308,7 @@ struct MatPlan {
     uint64_t filter_pairs = 0;  // sum over scored pairs of n_ref * n_tgt
     DevBuf d_all;  // one allocation: units, targets, refs, split | redo list | counters, slots
     DevView d_units, d_targets, d_refs, d_split, d_redo, d_counter;
-    std::vector<uint8_t> tables;  // the uploaded tables: alive for the copy, which nothing waits for
+    std::vector<uint8_t> tables;  // the uploaded tables: alive for their copy, which is only queued
     cudaGraphExec_t graph = nullptr;
     int32_t* graph_out = nullptr;  // output of the captured (or, before that, of the last) run
     uint64_t last_use = 0;

@@ -85,6 +85,7 @@ extern "C" void sdbfg_ctx_destroy(sdbfg_ctx* c) {
     c->h_stage_items.release();
     if (c->copy_stream) cudaStreamDestroy(c->copy_stream);
     if (c->ev_start) cudaEventDestroy(c->ev_start);
+    if (c->ev_plan) cudaEventDestroy(c->ev_plan);
     c->h_flags.release();
     c->h_result.release();
     c->h_block.release();
@@ -97,6 +98,7 @@ extern "C" const char* sdbfg_last_error(const sdbfg_ctx* c) { return c ? c->err.
 
 extern "C" int sdbfg_ctx_set_stream(sdbfg_ctx* c, void* s) {
     if (!c) return SDBFG_ERR_ARG;
+    CUDA_TRY(c, plan_tables_arrived(c));
     c->stream = s ? static_cast<cudaStream_t>(s) : c->own;
     return SDBFG_OK;
 }

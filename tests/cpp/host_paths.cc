@@ -1,0 +1,116 @@
+// Cases of the library's host code against fake_cuda.h: one per run, by name.
+// Exit status 0: the case holds.
+#include <cstdio>
+#include <cstdlib>
+#include <cstring>
+#include <map>
+#include <vector>
+
+#include "../../include/sdbf_gb300.h"
+#include "../../sdhash_gb300/csrc/compare_kernels.h"
+#include "fake_cuda.h"
+
+#define REQUIRE(c)                                                      \
+    do {                                                                \
+        if (!(c)) {                                                     \
+            fprintf(stderr, "%s:%d: %s\n", __FILE__, __LINE__, #c);     \
+            exit(1);                                                    \
+        }                                                               \
+    } while (0)
+
+namespace {
+
+sdbfg_ctx* context(int device = 0) {
+    sdbfg_ctx* c = nullptr;
+    REQUIRE(sdbfg_ctx_create(device, &c) == SDBFG_OK);
+    return c;
+}
+
+// n digests of 1, 2, 3, ... filters
+sdbfg_set* digests(sdbfg_ctx* c, uint32_t n) {
+    std::vector<uint8_t> filters(n * 256);
+    for (size_t i = 0; i < filters.size(); i++) filters[i] = (uint8_t)(i * 2654435761u >> 13);
+    std::vector<sdbfg_digest_desc> ds(n);
+    for (uint32_t i = 0; i < n; i++) {
+        ds[i] = {};
+        ds[i].name = "d";
+        ds[i].filters = filters.data();
+        ds[i].bf_count = i + 1;
+        ds[i].last_count = ds[i].max_elem = 160;
+        ds[i].orig_size = 4096;
+    }
+    sdbfg_set* s = nullptr;
+    REQUIRE(sdbfg_set_upload(c, ds.data(), n, &s) == SDBFG_OK);
+    return s;
+}
+
+template <class T>
+T* device_array(size_t n) {
+    void* p = nullptr;
+    REQUIRE(cudaMalloc(&p, n * sizeof(T)) == cudaSuccess);
+    return static_cast<T*>(p);
+}
+
+// every comparison kernel that runs has its units and targets
+int matrix_runs = 0;
+void expect_tables() {
+    fake::on_launch("k_matrix", [](void** args) {
+        const sdbfg::MatParams P = *static_cast<sdbfg::MatParams*>(args[0]);
+        return [P] {
+            matrix_runs++;
+            uint32_t poison;
+            memset(&poison, fake::kPoison, 4);
+            for (uint32_t u = 0; u < P.nunits; u++) {
+                REQUIRE(P.units[u].ref != poison && P.units[u].t1 != poison);
+                for (uint32_t t = P.units[u].t0; t < P.units[u].t1; t++) REQUIRE(P.targets[t] != poison);
+            }
+        };
+    });
+}
+
+// a plan's tables reach the device before a comparison on another stream than
+// the one it was made under
+void plan_other_stream(bool first_compared) {
+    sdbfg_ctx* c = context();
+    sdbfg_set* s = digests(c, 40);
+    int32_t* out = device_array<int32_t>(2 * 780);
+    expect_tables();
+    cudaStream_t a, b;
+    cudaStreamCreateWithFlags(&a, cudaStreamNonBlocking);
+    cudaStreamCreateWithFlags(&b, cudaStreamNonBlocking);
+    REQUIRE(sdbfg_ctx_set_stream(c, a) == SDBFG_OK);
+    if (first_compared) REQUIRE(sdbfg_compare_all_device(c, s, out) == SDBFG_OK);
+    else REQUIRE(sdbfg_compare_filter_pairs(c, s, nullptr) > 0);
+    REQUIRE(sdbfg_ctx_set_stream(c, b) == SDBFG_OK);
+    REQUIRE(sdbfg_compare_all_device(c, s, out + 780) == SDBFG_OK);
+    cudaStreamSynchronize(b);
+    REQUIRE(matrix_runs > 0);
+    sdbfg_set_free(s);
+    sdbfg_ctx_destroy(c);
+}
+
+// the tuner samples a plan's units as they are
+void autotune() {
+    sdbfg_ctx* c = context();
+    sdbfg_set* s = digests(c, 40);
+    expect_tables();
+    REQUIRE(sdbfg_compare_autotune(c, s, nullptr, 1 << 20, nullptr, nullptr, nullptr) == SDBFG_OK);
+    REQUIRE(matrix_runs > 0);
+    sdbfg_set_free(s);
+    sdbfg_ctx_destroy(c);
+}
+
+const std::map<std::string, std::function<void()>> kCases = {
+    {"plan_other_stream", [] { plan_other_stream(false); }},
+    {"plan_other_stream_compared", [] { plan_other_stream(true); }},
+    {"autotune", autotune},
+};
+
+}  // namespace
+
+int main(int argc, char** argv) {
+    const auto it = argc > 1 ? kCases.find(argv[1]) : kCases.end();
+    REQUIRE(it != kCases.end());
+    it->second();
+    return 0;
+}
