@@ -284,14 +284,17 @@ __global__ void k_scan_offsets(const FileInfoDev* __restrict__ info, uint64_t* _
     if (threadIdx.x == 0) *total = carry;
 }
 
+// Only slots below dst_cap are written: whether the batch fits is known to the
+// host when it is over.
 __global__ void k_pack_group(const uint32_t* __restrict__ work, const GenFile* __restrict__ files,
                              const FileInfoDev* __restrict__ info, const uint64_t* __restrict__ dst_off,
-                             uint32_t* __restrict__ dst, uint32_t n) {
+                             uint32_t* __restrict__ dst, uint64_t dst_cap, uint32_t n) {
     for (uint32_t f = blockIdx.x; f < n; f += gridDim.x) {
-        if (files[f].nchunks == 0) continue;
-        const uint64_t words = (uint64_t)info[f].bf_count * 64;
+        const uint64_t slot = dst_off[f];
+        if (files[f].nchunks == 0 || slot >= dst_cap) continue;
+        const uint64_t words = min((uint64_t)info[f].bf_count, dst_cap - slot) * 64;
         const uint4* s = reinterpret_cast<const uint4*>(work + files[f].filter_base * 64);
-        uint4* d = reinterpret_cast<uint4*>(dst + dst_off[f] * 64);
+        uint4* d = reinterpret_cast<uint4*>(dst + slot * 64);
         for (uint64_t q = threadIdx.x; q < words / 4; q += blockDim.x) d[q] = s[q];
     }
 }
@@ -892,7 +895,7 @@ static int digest_stream_pipelined(sdbfg_ctx* c, const uint8_t* host_data, const
         else
             TIMED_LAUNCH_ON(c, "k_pack_filters", st,
                             (k_pack_group<<<std::min<uint32_t>(g.count, (uint32_t)c->sms * 8), 256, 0, st>>>(
-                                 S.work.as<uint32_t>(), P.files, d_info + g.first, d_off + g.first, dev_out, g.count),
+                                 S.work.as<uint32_t>(), P.files, d_info + g.first, d_off + g.first, dev_out, out_cap, g.count),
                              cudaGetLastError()));
         CUDA_TRY(c, cudaEventRecord(S.done, st));
     }
