@@ -1160,9 +1160,14 @@ __device__ __forceinline__ void cp_async4(void* smem, const void* gmem) {
 }
 __device__ __forceinline__ void cp_async_wait_2() { asm volatile("cp.async.wait_group 2;\n" ::); }
 
-// The last filter is out; the chop of sdbf_core.cc:235-238 and the file's result.
+// The chop of sdbf_core.cc:235-238: a last filter of few elements is dropped.
+__device__ __forceinline__ bool commit_chops(uint32_t bf_count, uint32_t last_count) {
+    return bf_count > 1 && last_count < (uint32_t)kMaxElem / 8;
+}
+
+// The last filter is out: the file's result.
 __device__ __forceinline__ void commit_result(const GenParams& P, uint32_t file, uint32_t bf_count, uint32_t last_count) {
-    if (bf_count > 1 && last_count < (uint32_t)kMaxElem / 8) {
+    if (commit_chops(bf_count, last_count)) {
         bf_count--;
         last_count = kMaxElem;
     }
@@ -1495,9 +1500,10 @@ __device__ __forceinline__ void commit_files(const GenParams& P, uint8_t* smem) 
             if (bf_count - 1 <= Fd.filter_cap) out[(size_t)(bf_count - 2) * 64 + tid] = S.F[cur ^ 1u][tid];
             else if (tid == 0) atomicAdd(P.counters + 1, 1u);
         }
-        // emit the current (last) filter
+        // emit the current (last) filter, if it stays (out may be the caller's
+        // buffer, whose slots behind the result are not written)
         if (bf_count <= Fd.filter_cap) {
-            if (tid < 64) out[(size_t)(bf_count - 1) * 64 + tid] = S.F[cur][tid];
+            if (tid < 64 && !commit_chops(bf_count, last_count)) out[(size_t)(bf_count - 1) * 64 + tid] = S.F[cur][tid];
         } else if (tid == 0) {
             atomicAdd(P.counters + 1, 1u);
         }

@@ -53,3 +53,22 @@ def test_capacity_is_kept(ctx, sizes, room):
             [(r.bf_count, r.last_count, r.filter_offset) for r in full]
         assert np.array_equal(got[:need * 256], want[:need * 256])
     assert (got[cap * 256:] == SENTINEL).all()
+
+
+# mixture files whose last filter has fewer than 20 elements and is dropped
+@pytest.mark.parametrize("n", [60_000, 77_770, 97_317, 102_648, 106_202, 116_864, 129_303, 161_289])
+def test_dropped_last_filter_is_not_written(ctx, oracle, n):
+    import torch
+
+    raw = synth.mixture_bytes(72, n, n)
+    want = oracle.digest("f", raw.tobytes(), 0)
+    assert want.st.last_count == 160
+    data = torch.from_numpy(raw).cuda()
+    bound = ctx.capacity([n], 0)
+    dst = torch.full((bound * 256,), SENTINEL, dtype=torch.uint8, device="cuda")
+    torch.cuda.synchronize()
+    r = ctx.digest_device(data.data_ptr(), [0], [n], 0, dst.data_ptr(), bound)[0]
+    got = dst.cpu().numpy()
+    assert (r.bf_count, r.last_count) == (want.st.bf_count, want.st.last_count)
+    assert got[:r.bf_count * 256].tobytes() == bytes(want.filters())
+    assert (got[r.bf_count * 256:] == SENTINEL).all()
