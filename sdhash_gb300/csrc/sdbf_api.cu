@@ -740,8 +740,10 @@ static int digest_stream_pipelined(sdbfg_ctx* c, const uint8_t* host_data, const
             bool contiguous = true;
             for (uint32_t k = 0; k < g.count && contiguous; k++)
                 contiguous = offsets[g.first + k] - offsets[g.first] == doff[k];
-            if (contiguous) {
-                CUDA_TRY(c, cudaMemcpyAsync(S.data.p, host_data + offsets[g.first], bytes, cudaMemcpyHostToDevice, st));
+            if (contiguous) {  // one copy, exactly to the last input's end
+                const uint32_t last = g.count - 1;
+                CUDA_TRY(c, cudaMemcpyAsync(S.data.p, host_data + offsets[g.first], doff[last] + lens[g.first + last],
+                                            cudaMemcpyHostToDevice, st));
             } else {
                 for (uint32_t k = 0; k < g.count; k++) {
                     const uint32_t i = g.first + k;

@@ -100,10 +100,45 @@ void autotune() {
     sdbfg_ctx_destroy(c);
 }
 
+// a stream batch reads its inputs and nothing behind them
+void copies_end_with_the_input() {
+    sdbfg_ctx* c = context();
+    const std::vector<std::vector<uint64_t>> batches = {{1001}, {512}, {70'001}, {4096, 513}, {1040, 700, 1003}};
+    for (const bool page_locked : {false, true})
+        for (uint64_t shift = 0; shift < 16; shift += 3)
+            for (const auto& lens : batches) {
+                std::vector<uint64_t> offs;
+                uint64_t end = shift;
+                for (uint64_t n : lens) {  // each 16-byte aligned to the first: one contiguous range
+                    end = (end - shift + 15) / 16 * 16 + shift;
+                    offs.push_back(end);
+                    end += n;
+                }
+                void* p = nullptr;
+                if (page_locked) REQUIRE(cudaMallocHost(&p, end) == cudaSuccess);
+                else p = malloc(end);
+                const uint8_t* data = static_cast<uint8_t*>(p);
+                const uint64_t cap = sdbfg_digest_capacity(lens.data(), (uint32_t)lens.size(), 0);
+                std::vector<uint8_t> out(cap * 256);
+                std::vector<sdbfg_digest_result> res(lens.size());
+                fake::copies.clear();
+                REQUIRE(sdbfg_digest_batch(c, data, offs.data(), lens.data(), (uint32_t)lens.size(), 0, out.data(), cap,
+                                           nullptr, res.data()) == SDBFG_OK);
+                for (const fake::Copy& k : fake::copies) {
+                    const uint8_t* s = static_cast<const uint8_t*>(k.src);
+                    if (k.kind == cudaMemcpyHostToDevice && s >= data && s < data + end) REQUIRE(s + k.bytes <= data + end);
+                }
+                if (page_locked) cudaFreeHost(p);
+                else free(p);
+            }
+    sdbfg_ctx_destroy(c);
+}
+
 const std::map<std::string, std::function<void()>> kCases = {
     {"plan_other_stream", [] { plan_other_stream(false); }},
     {"plan_other_stream_compared", [] { plan_other_stream(true); }},
     {"autotune", autotune},
+    {"copies_end_with_the_input", copies_end_with_the_input},
 };
 
 }  // namespace
