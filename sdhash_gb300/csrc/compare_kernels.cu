@@ -17,6 +17,7 @@
 // The maximum over j is tracked exactly as the fraction (num, den) and
 // turned into one IEEE division at the end: division is correctly rounded
 // and monotone, so max_j fl(a_j/b_j) == fl(max_j a_j/b_j).
+#include <atomic>
 #include <cstdint>
 #include <cuda_runtime.h>
 
@@ -945,9 +946,15 @@ static int occupancy() {
     return n > 0 ? n : 1;
 }
 
+// (attributes and occupancy belong to a device: kept for each, contexts may
+// be used from several threads)
 int matrix_ctas_per_sm(int variant) {
-    static int cached[kMatVariants] = {0, 0, 0, 0, 0, 0};
-    if (variant >= 0 && variant < kMatVariants && cached[variant]) return cached[variant];
+    static std::atomic<int> cached[64][kMatVariants];
+    if (variant < 0 || variant >= kMatVariants) return 1;
+    int dev = 0;
+    cudaGetDevice(&dev);
+    const bool keep = dev >= 0 && dev < 64;
+    if (keep && cached[dev][variant]) return cached[dev][variant];
     int n = 1;
     switch (variant) {
         case 0: n = occupancy<128, 32>(); break;
@@ -958,7 +965,7 @@ int matrix_ctas_per_sm(int variant) {
         case kMatVariantTc: n = matrix_tc_ctas_per_sm(); break;
         default: return 1;
     }
-    cached[variant] = n;
+    if (keep) cached[dev][variant] = n;
     return n;
 }
 

@@ -35,6 +35,8 @@
 // rescan); a mismatch is re-walked from the neighbour's state.  The same
 // check links consecutive tiles of a chunk (k_stream_fails / k_stream_fix).
 #include <cstdint>
+#include <mutex>
+
 #include <cuda_runtime.h>
 
 #include "gen_kernels.h"
@@ -2450,9 +2452,9 @@ size_t stream_tile_smem() { return tile_smem_bytes(kTileL); }
 size_t stream_tile_smem_pre() { return tile_smem_bytes_pre(kTileL); }
 size_t block_smem(uint32_t lmax) { return tile_smem_bytes(lmax); }
 
-static void set_stream_attrs() {
-    static bool done = false;
-    if (done) return;
+// Attributes belong to a device: they are set once on each (contexts may be
+// used from several threads).
+static void set_stream_attrs_here() {
     const int sm = (int)stream_tile_smem(), smp = (int)stream_tile_smem_pre();
     cudaFuncSetAttribute(k_stream_tiles, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
     cudaFuncSetAttribute(k_stream_fix<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
@@ -2478,7 +2480,13 @@ static void set_stream_attrs() {
                           (const void*)k_feat_last, (const void*)k_feat_carry, (const void*)k_feat_links,
                           (const void*)k_stream_chain, (const void*)k_stream_emit})
         cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared);
-    done = true;
+}
+static void set_stream_attrs() {
+    static std::once_flag done[64];
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev >= 0 && dev < 64) std::call_once(done[dev], set_stream_attrs_here);
+    else set_stream_attrs_here();
 }
 
 int rk_choose(const uint64_t* stretches, uint32_t sms) {

@@ -134,11 +134,51 @@ void copies_end_with_the_input() {
     sdbfg_ctx_destroy(c);
 }
 
+// every kernel can be launched on each device of a process (fake_cuda refuses
+// more than 48 KB of dynamic shared memory on a device it was not asked for on)
+void second_device() {
+    std::vector<uint8_t> data(4 << 20), index(1 << 16);
+    for (size_t i = 0; i < data.size(); i++) data[i] = (uint8_t)(i * i >> 7);
+    for (int device = 0; device < 3; device++) {
+        sdbfg_ctx* c = context(device);
+        fake::launches.clear();
+        const std::vector<std::vector<uint64_t>> batches = {{4 << 20}, {1 << 20, 1 << 20, 70'000}};
+        for (const auto& lens : batches)
+            for (const uint32_t dd : {0u, 4096u, 1001u}) {
+                std::vector<uint64_t> offs(lens.size(), 0);
+                for (size_t i = 1; i < lens.size(); i++) offs[i] = offs[i - 1] + lens[i - 1];
+                const uint32_t n = (uint32_t)lens.size();
+                const uint64_t cap = sdbfg_digest_capacity(lens.data(), n, dd);
+                std::vector<uint8_t> out(cap * 256);
+                std::vector<uint16_t> counts(cap);
+                std::vector<sdbfg_digest_result> res(n);
+                uint64_t added = 0;
+                REQUIRE(sdbfg_digest_batch(c, data.data(), offs.data(), lens.data(), n, dd, out.data(), cap, counts.data(),
+                                           res.data()) == SDBFG_OK);
+                REQUIRE(sdbfg_digest_batch_index(c, data.data(), offs.data(), lens.data(), n, dd, out.data(), cap,
+                                                 counts.data(), res.data(), index.data(), index.size(), &added) == SDBFG_OK);
+            }
+        sdbfg_set* s = digests(c, 40);
+        std::vector<int32_t> scores(780);
+        for (int variant = 0; variant < 6; variant++) {
+            REQUIRE(sdbfg_ctx_set_compare_tuning(c, variant, 1 << 22, 1) == SDBFG_OK);
+            REQUIRE(sdbfg_compare_all(c, s, scores.data()) == SDBFG_OK);
+        }
+        REQUIRE(fake::launched("k_stream_chain(") && fake::launched("k_stream_commit(") &&
+                fake::launched("k_stream_commit_round(") && fake::launched("k_block_digest<true>") &&
+                fake::launched("k_block_digest<false>") && fake::launched("k_matrix_tc<false>"));
+        for (const fake::Launch& l : fake::launches) REQUIRE(l.device == device);
+        sdbfg_set_free(s);
+        sdbfg_ctx_destroy(c);
+    }
+}
+
 const std::map<std::string, std::function<void()>> kCases = {
     {"plan_other_stream", [] { plan_other_stream(false); }},
     {"plan_other_stream_compared", [] { plan_other_stream(true); }},
     {"autotune", autotune},
     {"copies_end_with_the_input", copies_end_with_the_input},
+    {"second_device", second_device},
 };
 
 }  // namespace
