@@ -634,7 +634,8 @@ static int digest_stream_pipelined(sdbfg_ctx* c, const uint8_t* host_data, const
     // parity: a group's rank kernel waits for the tile and fix kernels of the
     // group two back (the last readers of its half) and runs beside the
     // previous group's tile kernel.  Sized once for the largest group;
-    // without the room the tile kernels compute the ranks themselves.
+    // without the room, or with more ranks than GenChunk::rank_off8 can
+    // address (an input above 32 GiB), the tile kernels compute them themselves.
     bool pre_ranks = c->pre_ranks;
     if (pre_ranks) {
         uint64_t most = 0;
@@ -646,7 +647,9 @@ static int digest_stream_pipelined(sdbfg_ctx* c, const uint8_t* host_data, const
             }
             most = std::max(most, r8);
         }
-        if (c->d_ranks.ensure(2 * (most * 16 + 16)) != cudaSuccess) {
+        if (most >> 32) {
+            pre_ranks = false;
+        } else if (c->d_ranks.ensure(2 * (most * 16 + 16)) != cudaSuccess) {
             cudaGetLastError();
             c->d_ranks.release();
             pre_ranks = false;

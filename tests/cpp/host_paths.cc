@@ -8,6 +8,7 @@
 
 #include "../../include/sdbf_gb300.h"
 #include "../../sdhash_gb300/csrc/compare_kernels.h"
+#include "../../sdhash_gb300/csrc/gen_kernels.h"
 #include "fake_cuda.h"
 
 #define REQUIRE(c)                                                      \
@@ -173,12 +174,46 @@ void second_device() {
     }
 }
 
+// precomputed ranks are addressed in 32 bits of eight ranks: of an input
+// above 32 GiB they are not used
+void ranks_of_a_huge_input() {
+    for (const bool huge : {false, true}) {
+        sdbfg_ctx* c = context();
+        const std::vector<uint64_t> lens = huge ? std::vector<uint64_t>{(33ull << 30) + 5, 1 << 20} : std::vector<uint64_t>{31ull << 30, 1 << 20};
+        const std::vector<uint64_t> offs = {0, 34ull << 30};
+        uint8_t* data = device_array<uint8_t>(35ull << 30);
+        const uint64_t cap = sdbfg_digest_capacity(lens.data(), 2, 0);
+        uint8_t* out = device_array<uint8_t>(cap * 256);
+        sdbfg_digest_result res[2];
+        static uint64_t ranked, wrapped;
+        ranked = wrapped = 0;
+        fake::launches.clear();
+        fake::on_launch("k_stream_ranks", [](void** args) {
+            const sdbfg::GenParams P = *static_cast<sdbfg::GenParams*>(args[0]);
+            return [P] {  // every chunk's ranks lie behind those of the chunk before
+                for (uint32_t k = 1; k < P.nchunks; k++)
+                    wrapped += P.chunks[k].rank_off8 != P.chunks[k - 1].rank_off8 + (P.chunks[k - 1].n + 7) / 8 ||
+                               P.chunks[k].rank_off8 < P.chunks[k - 1].rank_off8;
+                ranked++;
+            };
+        });
+        REQUIRE(sdbfg_digest_batch_device(c, data, offs.data(), lens.data(), 2, 0, out, cap, nullptr, res) == SDBFG_OK);
+        REQUIRE(fake::launched("k_stream_tiles"));
+        REQUIRE(wrapped == 0);
+        REQUIRE(huge || ranked > 0);
+        sdbfg_ctx_destroy(c);
+        cudaFree(data);
+        cudaFree(out);
+    }
+}
+
 const std::map<std::string, std::function<void()>> kCases = {
     {"plan_other_stream", [] { plan_other_stream(false); }},
     {"plan_other_stream_compared", [] { plan_other_stream(true); }},
     {"autotune", autotune},
     {"copies_end_with_the_input", copies_end_with_the_input},
     {"second_device", second_device},
+    {"ranks_of_a_huge_input", ranks_of_a_huge_input},
 };
 
 }  // namespace
