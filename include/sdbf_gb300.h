@@ -30,6 +30,11 @@ extern "C" {
 #define SDBFG_ERR_FORMAT -4     /* malformed SDBF text */
 #define SDBFG_ERR_CAPACITY -5   /* output buffer too small */
 
+/* Every score of a comparison whose kernel gave up waiting for the tensor
+ * cores (each wait is bounded).  The calls that wait report it themselves;
+ * for the _device forms sdbfg_ctx_synchronize does. */
+#define SDBFG_SCORE_INVALID INT32_MIN
+
 /* Per-input digest status, mirroring the reference constructors' throws
  * (sdbf/sdbf_class.cc:37,81,117). */
 #define SDBFG_DIGEST_OK 0
@@ -48,6 +53,8 @@ void sdbfg_ctx_destroy(sdbfg_ctx *ctx);
 const char *sdbfg_last_error(const sdbfg_ctx *ctx);
 /* Launch on a caller-owned cudaStream_t (NULL = the context's own stream). */
 int sdbfg_ctx_set_stream(sdbfg_ctx *ctx, void *cuda_stream);
+/* Waits for the context's stream.  SDBFG_ERR_CUDA, once, when a comparison
+ * queued since the last call gave up (SDBFG_SCORE_INVALID). */
 int sdbfg_ctx_synchronize(sdbfg_ctx *ctx);
 /* Kernel launches issued on this context so far (instrumentation). */
 uint64_t sdbfg_ctx_launch_count(const sdbfg_ctx *ctx);

@@ -404,6 +404,7 @@ static MatParams plan_params(sdbfg_ctx* c, const MatPlan* p, const sdbfg_set* a,
     P.cutoffs64 = c->d_cut64.as<uint16_t>();
     P.redo = redo_list(p->d_redo.p, P.next_unit);
     P.error = p->d_counter.as<uint32_t>() + 1;
+    P.gave_up = c->gave_up();
     P.phase = c->profile ? c->d_mphase.as<unsigned long long>() : nullptr;
     return P;
 }
@@ -468,12 +469,14 @@ static int run_plan(sdbfg_ctx* c, MatPlan* p, const sdbfg_set* a, const sdbfg_se
 
 // Copies a run's scores to out, waits, and reports a bounded wait that gave up.
 static int fetch_scores(sdbfg_ctx* c, const MatPlan* p, int32_t* out) {
-    CUDA_TRY(c, c->h_flags.ensure(64));  // pinned: this copy does not block
-    uint32_t* err = static_cast<uint32_t*>(c->h_flags.p);
+    uint32_t* err = static_cast<uint32_t*>(c->h_flags.p);  // pinned: this copy does not block
     CUDA_TRY(c, cudaMemcpyAsync(err, p->d_counter.as<uint32_t>() + 1, 4, cudaMemcpyDeviceToHost, c->stream));
     if (out) CUDA_TRY(c, cudaMemcpyAsync(out, c->d_scores.p, p->nscores * 4, cudaMemcpyDeviceToHost, c->stream));
     CUDA_TRY(c, cudaStreamSynchronize(c->stream));
-    if (*err) return fail(c, SDBFG_ERR_CUDA, "comparison kernel: %u CTAs gave up waiting for the tensor cores", *err);
+    if (*err) {
+        *c->gave_up() = 0;  // reported here
+        return fail(c, SDBFG_ERR_CUDA, "comparison kernel: %u CTAs gave up waiting for the tensor cores", *err);
+    }
     return SDBFG_OK;
 }
 

@@ -21,6 +21,7 @@
 #include <cstdint>
 #include <cuda_runtime.h>
 
+#include "../../include/sdbf_gb300.h"
 #include "compare_device.cuh"
 #include "compare_kernels.h"
 #include "sdbf_device.cuh"
@@ -715,8 +716,9 @@ __device__ __forceinline__ void pair_of(uint64_t k, uint32_t mode, uint64_t n, u
     j = (uint32_t)(k - start(ii) + ii + 1);
 }
 
-// After the tensor-core kernel: the split pairs' scores from their row
-// maxima; every marked score goes to the redo list (k_matrix_redo), or, when
+// After the tensor-core kernel: where one of its waits gave up, no score holds
+// (unfinished units leave sums in the score array), and all are overwritten;
+// else the split pairs' scores from their row maxima; every marked score goes to the redo list (k_matrix_redo), or, when
 // the list is full, is scored here.  A block takes a split pair, then 128
 // scores at a time.
 __global__ void __launch_bounds__(kCmpThreads) k_matrix_finish(MatParams P) {
@@ -724,6 +726,12 @@ __global__ void __launch_bounds__(kCmpThreads) k_matrix_finish(MatParams P) {
     __shared__ unsigned long long total, place;
     __shared__ uint32_t hits[kCmpThreads], nhits;
     __shared__ int32_t mark;
+    if (*P.error) {
+        for (uint64_t k = (uint64_t)blockIdx.x * kCmpThreads + threadIdx.x; k < P.nscores; k += (uint64_t)gridDim.x * kCmpThreads)
+            P.scores[k] = SDBFG_SCORE_INVALID;
+        if (blockIdx.x == 0 && threadIdx.x == 0 && P.gave_up) *const_cast<volatile uint32_t*>(P.gave_up) = 1;
+        return;
+    }
     pair_tables(S, P.cutoffs, P.cutoffs64);
     const uint32_t* slots = reinterpret_cast<const uint32_t*>(P.slots);
     // all threads: the marked pair's score, now or later

@@ -147,7 +147,8 @@ struct MatParams {
     const uint16_t* cutoffs;   // CUTOFFS256
     const uint16_t* cutoffs64; // CUTOFFS64 (fast mode)
     RedoList redo;             // tensor-core kernel
-    uint32_t* error;           // tensor-core kernel: set when a bounded wait gave up
+    uint32_t* error;           // tensor-core kernel: set when a bounded wait gave up,
+    uint32_t* gave_up;         //   and then this (page-locked host memory), which no later run clears
     unsigned long long* phase; // tensor-core kernel: optional SM-cycle counters (kTcPh*), null = off
 };
 // phase counters of the tensor-core kernel: per role the busy cycles of its

@@ -185,7 +185,8 @@ struct sdbfg_ctx {
     DevBuf d_rank, d_ent, d_cut, d_cut64;
     // generation buffers
     DevBuf d_data, d_chunks, d_counters, d_out_filters, d_out_counts;
-    HostBuf h_flags;  // small read-backs (pinned)
+    HostBuf h_flags;  // pinned words: [0] small read-backs, [1] set when a comparison gave up
+    uint32_t* gave_up() const { return static_cast<uint32_t*>(h_flags.p) + 1; }
     // comparison buffers
     DevBuf d_pairs, d_scores;
     // stream-mode pipeline: two launch-group slots on their own streams

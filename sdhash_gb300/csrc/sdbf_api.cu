@@ -42,10 +42,11 @@ extern "C" int sdbfg_ctx_create(int device, sdbfg_ctx** out) {
     for (int i = 0; i < 65; i++) ent[i] = SDBF_ENTROPY64[i];
     if (c->d_rank.ensure(sizeof(SDBF_ENTR64_RANKS)) || c->d_ent.ensure(sizeof(ent)) ||
         c->d_cut.ensure(sizeof(SDBF_CUTOFFS256)) || c->d_cut64.ensure(sizeof(SDBF_CUTOFFS64)) ||
-        c->d_counters.ensure(64)) {
+        c->d_counters.ensure(64) || c->h_flags.ensure(64)) {
         sdbfg_ctx_destroy(c);
         return SDBFG_ERR_NOMEM;
     }
+    memset(c->h_flags.p, 0, 64);
     cudaMemcpy(c->d_rank.p, SDBF_ENTR64_RANKS, sizeof(SDBF_ENTR64_RANKS), cudaMemcpyHostToDevice);
     cudaMemcpy(c->d_ent.p, ent, sizeof(ent), cudaMemcpyHostToDevice);
     cudaMemcpy(c->d_cut.p, SDBF_CUTOFFS256, sizeof(SDBF_CUTOFFS256), cudaMemcpyHostToDevice);
@@ -106,6 +107,10 @@ extern "C" int sdbfg_ctx_set_stream(sdbfg_ctx* c, void* s) {
 extern "C" int sdbfg_ctx_synchronize(sdbfg_ctx* c) {
     if (!c) return SDBFG_ERR_ARG;
     CUDA_TRY(c, cudaStreamSynchronize(c->stream));
+    if (*const_cast<volatile uint32_t*>(c->gave_up())) {
+        *c->gave_up() = 0;
+        return fail(c, SDBFG_ERR_CUDA, "a comparison gave up waiting for the tensor cores: its scores are invalid");
+    }
     return SDBFG_OK;
 }
 

@@ -207,6 +207,41 @@ void ranks_of_a_huge_input() {
     }
 }
 
+// a comparison whose kernel gave up (an error word that the kernel sets) is
+// reported once: by the calls that wait, else by the next synchronisation
+void comparison_gave_up() {
+    sdbfg_ctx* c = context();
+    sdbfg_set* s = digests(c, 40);
+    int32_t* out = device_array<int32_t>(780);
+    std::vector<int32_t> scores(780);
+    static bool fails = true;
+    fake::on_launch("k_matrix_tc", [](void** args) {
+        const sdbfg::MatParams P = *static_cast<sdbfg::MatParams*>(args[0]);
+        return [P] { *P.error = fails; };
+    });
+    fake::on_launch("k_matrix_finish", [](void** args) {  // (the kernel's part of it: test_gpu_gave_up.py)
+        const sdbfg::MatParams P = *static_cast<sdbfg::MatParams*>(args[0]);
+        return [P] {
+            if (*P.error && P.gave_up) *P.gave_up = 1;
+        };
+    });
+    for (int k = 0; k < 3; k++) {  // launched, launched, from the graph
+        REQUIRE(sdbfg_compare_all_device(c, s, out) == SDBFG_OK);
+        REQUIRE(sdbfg_ctx_synchronize(c) == SDBFG_ERR_CUDA);
+        REQUIRE(sdbfg_ctx_synchronize(c) == SDBFG_OK);
+    }
+    REQUIRE(sdbfg_compare_to_device(c, s, s, device_array<int32_t>(1600)) == SDBFG_OK);
+    REQUIRE(sdbfg_ctx_synchronize(c) == SDBFG_ERR_CUDA);
+    REQUIRE(sdbfg_compare_all(c, s, scores.data()) == SDBFG_ERR_CUDA);
+    REQUIRE(sdbfg_ctx_synchronize(c) == SDBFG_OK);
+    fails = false;
+    REQUIRE(sdbfg_compare_all_device(c, s, out) == SDBFG_OK);
+    REQUIRE(sdbfg_ctx_synchronize(c) == SDBFG_OK);
+    REQUIRE(sdbfg_compare_all(c, s, scores.data()) == SDBFG_OK);
+    sdbfg_set_free(s);
+    sdbfg_ctx_destroy(c);
+}
+
 const std::map<std::string, std::function<void()>> kCases = {
     {"plan_other_stream", [] { plan_other_stream(false); }},
     {"plan_other_stream_compared", [] { plan_other_stream(true); }},
@@ -214,6 +249,7 @@ const std::map<std::string, std::function<void()>> kCases = {
     {"copies_end_with_the_input", copies_end_with_the_input},
     {"second_device", second_device},
     {"ranks_of_a_huge_input", ranks_of_a_huge_input},
+    {"comparison_gave_up", comparison_gave_up},
 };
 
 }  // namespace
