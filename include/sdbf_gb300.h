@@ -349,7 +349,7 @@ typedef struct {
 } sdbfg_server_config;
 typedef struct {
     uint64_t tag;                /* as submitted */
-    int32_t status;              /* SDBFG_OK */
+    int32_t status;              /* SDBFG_OK; SDBFG_ERR_CUDA: not scored (its scores are SDBFG_SCORE_INVALID) */
     int32_t best_score;          /* highest score over the targets (-1: none) */
     uint32_t best_target;        /* its index in the target set */
     uint32_t matches;            /* targets with score >= threshold */

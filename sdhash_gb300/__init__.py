@@ -728,7 +728,8 @@ class Server:
         self.ctx._check(lib().sdbfg_server_submit(self.h, C.byref(desc), tag))
 
     def poll(self, max_results: int = 1024, timeout_ms: int = 0, scores: bool = True):
-        """List of (result, score row or None)."""
+        """List of (result, score row or None).  A result's status is 0, or
+        negative for a query that could not be scored (submit it again)."""
         res = (ServerResult * max_results)()
         sc = np.zeros(max_results * self.nt if scores else 1, dtype=np.int32)
         n = C.c_uint32()

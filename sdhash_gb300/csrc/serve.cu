@@ -79,6 +79,7 @@ struct sdbfg_server {
         std::vector<Request> batch;
         uint32_t nunits = 0, nsplit = 0;
         HostBuf h_filters, h_meta, h_dig, h_units, h_targets, h_refs, h_split, h_scores;
+        HostBuf h_gave_up;  // one word, set by a batch whose kernel gave up (MatParams::gave_up)
         DevBuf d_filters, d_meta, d_dig, d_units, d_targets, d_refs, d_split, d_slots, d_scores, d_redo;  // slots behind the counters
         uint64_t cap_units = 0, cap_targets = 0, cap_refs = 0, cap_split = 0, cap_slots = 0;
     };
@@ -175,6 +176,8 @@ static cudaError_t launch_batch(sdbfg_server* sv, sdbfg_server::Slot& S) {
     P.cutoffs64 = sv->ctx->d_cut64.as<uint16_t>();
     P.redo = redo_list(S.d_redo.p, P.next_unit);
     P.error = P.next_unit + 1;
+    P.gave_up = S.h_gave_up.as<uint32_t>();
+    *P.gave_up = 0;
     uint64_t launched = 0;
     if ((e = run_matrix(P, variant, (uint32_t)ctas, (uint32_t)sv->ctx->sms, st, &launched))) return e;
     sv->launches += launched;
@@ -186,17 +189,18 @@ static void finish_batch(sdbfg_server* sv, sdbfg_server::Slot& S) {
     const uint32_t nt = sv->refs->n;
     const uint64_t t = now_ns();
     const int32_t* sc = S.h_scores.as<int32_t>();
+    const bool failed = *S.h_gave_up.as<volatile uint32_t>() != 0;  // every score is SDBFG_SCORE_INVALID then
     std::vector<Done> out(S.batch.size());
     for (size_t i = 0; i < S.batch.size(); i++) {
         Done& d = out[i];
         const int32_t* row = sc + i * nt;
         d.scores.assign(row, row + nt);
         d.r.tag = S.batch[i].tag;
-        d.r.status = 0;
+        d.r.status = failed ? SDBFG_ERR_CUDA : SDBFG_OK;
         d.r.best_score = -1;
         d.r.best_target = 0;
         d.r.matches = 0;
-        for (uint32_t j = 0; j < nt; j++) {
+        for (uint32_t j = 0; j < nt && !failed; j++) {
             if (row[j] > d.r.best_score) {
                 d.r.best_score = row[j];
                 d.r.best_target = j;
@@ -316,6 +320,7 @@ extern "C" int sdbfg_server_create(sdbfg_ctx* c, const sdbfg_set* refs, const sd
             if (e == cudaSuccess) e = dv->ensure(bytes);
             if (e == cudaSuccess) e = hv->ensure(bytes);
         }
+        if (e == cudaSuccess) e = S.h_gave_up.ensure(64);
         if (e == cudaSuccess) e = S.d_redo.ensure(kRedoBytes);
         if (e == cudaSuccess) e = grow(S.d_units, &S.h_units, S.cap_units, 1 << 16, sizeof(MatUnit));
         if (e == cudaSuccess)
@@ -415,7 +420,7 @@ extern "C" void sdbfg_server_destroy(sdbfg_server* sv) {
                           &S.d_slots, &S.d_scores, &S.d_redo})
             b->release();
         for (HostBuf* b : {&S.h_filters, &S.h_meta, &S.h_dig, &S.h_units, &S.h_targets, &S.h_refs, &S.h_split,
-                           &S.h_scores})
+                           &S.h_scores, &S.h_gave_up})
             b->release();
         if (S.st) cudaStreamDestroy(S.st);
         if (S.ev) cudaEventDestroy(S.ev);

@@ -242,6 +242,50 @@ void comparison_gave_up() {
     sdbfg_ctx_destroy(c);
 }
 
+// a served batch whose kernel gave up comes back with an error for each of
+// its queries, and the next one is served
+void server_batch_gave_up() {
+    sdbfg_ctx* c = context();
+    sdbfg_set* s = digests(c, 10);
+    static int runs = 0;
+    fake::on_launch("k_matrix_tc", [](void** args) {
+        const sdbfg::MatParams P = *static_cast<sdbfg::MatParams*>(args[0]);
+        return [P] { *P.error = runs++ < 1; };
+    });
+    fake::on_launch("k_matrix_finish", [](void** args) {  // (the kernel's part of it: test_gpu_gave_up.py)
+        const sdbfg::MatParams P = *static_cast<sdbfg::MatParams*>(args[0]);
+        return [P] {
+            if (*P.error && P.gave_up) *P.gave_up = 1;
+            const int32_t score = *P.error ? SDBFG_SCORE_INVALID : 7;
+            for (uint64_t k = 0; k < P.nscores; k++) P.scores[k] = score;
+        };
+    });
+    const sdbfg_server_config cfg{1, 4, 8ull << 20, 1, 0, 0};
+    sdbfg_server* srv = nullptr;
+    REQUIRE(sdbfg_server_create(c, s, &cfg, &srv) == SDBFG_OK);
+    const std::vector<uint8_t> filter(256, 0x11);
+    sdbfg_digest_desc q{};
+    q.name = "q";
+    q.filters = filter.data();
+    q.bf_count = 1;
+    q.last_count = q.max_elem = 160;
+    for (uint64_t tag = 0; tag < 2; tag++) {
+        REQUIRE(sdbfg_server_submit(srv, &q, tag) == SDBFG_OK);
+        sdbfg_server_result r{};
+        std::vector<int32_t> row(10);
+        uint32_t n = 0;
+        REQUIRE(sdbfg_server_poll(srv, &r, row.data(), 1, &n, 10'000) == SDBFG_OK);
+        REQUIRE(n == 1 && r.tag == tag);
+        REQUIRE(r.status == (tag ? SDBFG_OK : SDBFG_ERR_CUDA));
+        REQUIRE(r.best_score == (tag ? 7 : -1) && r.matches == (tag ? 10u : 0u));
+        for (int32_t v : row) REQUIRE(v == (tag ? 7 : SDBFG_SCORE_INVALID));
+    }
+    sdbfg_server_destroy(srv);
+    REQUIRE(sdbfg_ctx_synchronize(c) == SDBFG_OK);  // the server's runs are not the context's
+    sdbfg_set_free(s);
+    sdbfg_ctx_destroy(c);
+}
+
 const std::map<std::string, std::function<void()>> kCases = {
     {"plan_other_stream", [] { plan_other_stream(false); }},
     {"plan_other_stream_compared", [] { plan_other_stream(true); }},
@@ -250,6 +294,7 @@ const std::map<std::string, std::function<void()>> kCases = {
     {"second_device", second_device},
     {"ranks_of_a_huge_input", ranks_of_a_huge_input},
     {"comparison_gave_up", comparison_gave_up},
+    {"server_batch_gave_up", server_batch_gave_up},
 };
 
 }  // namespace
