@@ -135,8 +135,8 @@ static CmpPair orient(const sdbfg_set* a, uint32_t i, const sdbfg_set* b, uint32
 static int run_pairs(sdbfg_ctx* c, const sdbfg_set* a, const sdbfg_set* b, const std::vector<CmpPair>& pairs,
                      int32_t* out) {
     cudaStream_t st = c->stream;
-    CUDA_TRY(c, c->d_pairs.ensure(std::max<size_t>(1, pairs.size()) * sizeof(CmpPair)));
-    CUDA_TRY(c, c->d_scores.ensure(std::max<size_t>(1, pairs.size()) * 4));
+    CUDA_TRY(c, c->must(c->d_pairs, std::max<size_t>(1, pairs.size()) * sizeof(CmpPair)));
+    CUDA_TRY(c, c->must(c->d_scores, std::max<size_t>(1, pairs.size()) * 4));
     CUDA_TRY(c, cudaMemcpyAsync(c->d_pairs.p, pairs.data(), pairs.size() * sizeof(CmpPair), cudaMemcpyHostToDevice,
                                 st));
     CmpParams P{};
@@ -210,7 +210,7 @@ static int upload_plan(sdbfg_ctx* c, MatPlan* p, UnitBuilder& ub, const std::vec
     CUDA_TRY(c, cudaStreamIsCapturing(c->stream, &cap));
     if (cap != cudaStreamCaptureStatusNone)
         return fail(c, SDBFG_ERR_CUDA, "a comparison's first run cannot be captured");
-    CUDA_TRY(c, p->d_all.ensure(at_counter + kMatCounterBytes + std::max<uint64_t>(1, ub.slots) * 8));
+    CUDA_TRY(c, c->must(p->d_all, at_counter + kMatCounterBytes + std::max<uint64_t>(1, ub.slots) * 8));
     uint8_t* d = p->d_all.as<uint8_t>();
     p->d_units.p = d;
     p->d_targets.p = d + at_targets;
@@ -507,7 +507,7 @@ extern "C" int sdbfg_compare_all(sdbfg_ctx* c, const sdbfg_set* s, int32_t* out)
     MatPlan* p;
     int rc = get_plan(c, s, nullptr, kMatModeAll, &p);
     if (rc) return rc;
-    CUDA_TRY(c, c->d_scores.ensure(p->nscores * 4));
+    CUDA_TRY(c, c->must(c->d_scores, p->nscores * 4));
     rc = run_plan(c, p, s, nullptr, c->d_scores.as<int32_t>());
     if (rc) return rc;
     return fetch_scores(c, p, out);
@@ -520,7 +520,7 @@ extern "C" int sdbfg_compare_to(sdbfg_ctx* c, const sdbfg_set* q, const sdbfg_se
     MatPlan* p;
     int rc = get_plan(c, q, t, kMatModeCross, &p);
     if (rc) return rc;
-    CUDA_TRY(c, c->d_scores.ensure(p->nscores * 4));
+    CUDA_TRY(c, c->must(c->d_scores, p->nscores * 4));
     rc = run_plan(c, p, q, t, c->d_scores.as<int32_t>());
     if (rc) return rc;
     return fetch_scores(c, p, out);
@@ -531,8 +531,8 @@ static int collect_matches(sdbfg_ctx* c, uint64_t nscores, uint32_t mode, uint64
                            sdbfg_match* out, uint64_t cap, uint64_t* count) {
     cudaStream_t st = c->stream;
     const uint64_t nb = (nscores + kMatchBlockScores - 1) / kMatchBlockScores;
-    CUDA_TRY(c, c->d_match_counts.ensure(std::max<uint64_t>(1, nb) * 4));
-    CUDA_TRY(c, c->d_match_offs.ensure((nb + 1) * 8));
+    CUDA_TRY(c, c->must(c->d_match_counts, std::max<uint64_t>(1, nb) * 4));
+    CUDA_TRY(c, c->must(c->d_match_offs, (nb + 1) * 8));
     const int32_t* sc = c->d_scores.as<int32_t>();
     TIMED_LAUNCH_ON(c, "k_match_count", st, launch_match_count(sc, nscores, threshold, c->d_match_counts.as<uint32_t>(), st));
     TIMED_LAUNCH_ON(c, "k_match_scan", st, launch_match_scan(c->d_match_counts.as<uint32_t>(), nb,
@@ -544,7 +544,7 @@ static int collect_matches(sdbfg_ctx* c, uint64_t nscores, uint32_t mode, uint64
     if (total > cap) return fail(c, SDBFG_ERR_CAPACITY, "%llu matches, room for %llu", (unsigned long long)total,
                                  (unsigned long long)cap);
     if (!total) return SDBFG_OK;
-    CUDA_TRY(c, c->d_matches.ensure(total * sizeof(sdbfg_match)));
+    CUDA_TRY(c, c->must(c->d_matches, total * sizeof(sdbfg_match)));
     TIMED_LAUNCH_ON(c, "k_match_write", st, launch_match_write(sc, nscores, threshold, c->d_match_offs.as<uint64_t>(),
                                                                mode, dim, c->d_matches.as<uint32_t>(), total, st));
     CUDA_TRY(c, cudaMemcpyAsync(out, c->d_matches.p, total * sizeof(sdbfg_match), cudaMemcpyDeviceToHost, st));
@@ -561,7 +561,7 @@ extern "C" int sdbfg_compare_all_matches(sdbfg_ctx* c, const sdbfg_set* s, int32
     MatPlan* p;
     int rc = get_plan(c, s, nullptr, kMatModeAll, &p);
     if (rc) return rc;
-    CUDA_TRY(c, c->d_scores.ensure(p->nscores * 4));
+    CUDA_TRY(c, c->must(c->d_scores, p->nscores * 4));
     rc = run_plan(c, p, s, nullptr, c->d_scores.as<int32_t>());
     if (rc) return rc;
     if ((rc = fetch_scores(c, p, nullptr))) return rc;
@@ -577,7 +577,7 @@ extern "C" int sdbfg_compare_to_matches(sdbfg_ctx* c, const sdbfg_set* q, const 
     MatPlan* p;
     int rc = get_plan(c, q, t, kMatModeCross, &p);
     if (rc) return rc;
-    CUDA_TRY(c, c->d_scores.ensure(p->nscores * 4));
+    CUDA_TRY(c, c->must(c->d_scores, p->nscores * 4));
     rc = run_plan(c, p, q, t, c->d_scores.as<int32_t>());
     if (rc) return rc;
     if ((rc = fetch_scores(c, p, nullptr))) return rc;
@@ -643,9 +643,9 @@ extern "C" int sdbfg_compare_autotune(sdbfg_ctx* c, const sdbfg_set* a, const sd
             if (sample.empty()) continue;
             uint64_t pairs = 0;
             DevBuf d_sample;
-            CUDA_TRY(c, d_sample.ensure(sample.size() * sizeof(MatUnit)));
+            CUDA_TRY(c, c->must(d_sample, sample.size() * sizeof(MatUnit)));
             CUDA_TRY(c, cudaMemcpy(d_sample.p, sample.data(), sample.size() * sizeof(MatUnit), cudaMemcpyHostToDevice));
-            CUDA_TRY(c, c->d_scores.ensure(p->nscores * 4));
+            CUDA_TRY(c, c->must(c->d_scores, p->nscores * 4));
             MatParams P = plan_params(c, p, a, b, c->d_scores.as<int32_t>());
             P.units = d_sample.as<MatUnit>();
             P.nunits = (uint32_t)sample.size();

@@ -208,12 +208,28 @@ struct sdbfg_ctx {
     // host-input stream batches staged whole on the device: per-file copies
     // in launch-group order on their own stream, one event per group
     DevBuf d_stage_in, d_stage_items;
+    bool staging = false;  // a batch reads d_stage_in
     HostBuf h_stage_items;
     cudaStream_t copy_stream = nullptr;
     std::vector<cudaEvent_t> ev_copy;
     cudaEvent_t ev_scan[kSlots] = {};
     cudaEvent_t ev_tiles[kSlots] = {};  // a group's tile kernels done
     cudaEvent_t ev_start = nullptr;
+    // A buffer that a call cannot do without.  Where there is no room for it,
+    // what earlier calls left and later ones can do without or make again goes
+    // first: the linked commit's buffers (1.4 bytes per byte of a file) and the
+    // staging copy (cudaFree waits for their users).
+    cudaError_t must(DevBuf& b, size_t bytes) {
+        cudaError_t e = b.ensure(bytes);
+        if (e != cudaErrorMemoryAllocation) return e;
+        cudaGetLastError();
+        for (Slot& s : slot) {
+            s.links.release();
+            s.last_tab.release();
+        }
+        if (!staging) d_stage_in.release();
+        return b.ensure(bytes);
+    }
     // comparison engine: tuning and cached plans (work units + CUDA graph)
     int mat_variant = kMatVariantTc;  // tensor-core counting
     uint64_t mat_unit_work = 1ull << 22;
@@ -280,7 +296,7 @@ struct sdbfg_set {
     static uint64_t digests_at(uint64_t filters) { return meta_at(filters) + (filters * 4 + 255) / 256 * 256; }
     static uint64_t bytes(uint64_t filters, uint64_t digests) { return digests_at(filters) + (digests + 1) * sizeof(CmpDigest); }
     cudaError_t allocate(uint64_t filters, uint64_t digests) {
-        const cudaError_t e = d_all.ensure(bytes(filters, digests));
+        const cudaError_t e = ctx->must(d_all, bytes(filters, digests));
         if (e != cudaSuccess) return e;
         d_filters.p = d_all.p;
         d_meta.p = d_all.as<uint8_t>() + meta_at(filters);

@@ -220,7 +220,7 @@ int index_query(sdbfg_ctx* c, const uint32_t* d_probes, const uint8_t* d_nprobes
     std::vector<IndexDev> h(nidx);
     for (uint32_t i = 0; i < nidx; i++)
         h[i] = IndexDev{indexes[i]->d_bits.as<uint8_t>(), (uint32_t)indexes[i]->bit_mask, indexes[i]->hash_count};
-    CUDA_TRY(c, c->d_index_tab.ensure(nidx * sizeof(IndexDev)));
+    CUDA_TRY(c, c->must(c->d_index_tab, nidx * sizeof(IndexDev)));
     CUDA_TRY(c, cudaMemcpyAsync(c->d_index_tab.p, h.data(), nidx * sizeof(IndexDev), cudaMemcpyHostToDevice, st));
     const uint32_t grid = (uint32_t)std::min<uint64_t>((nslots + 7) / 8, (uint64_t)c->sms * 16);
     TIMED_LAUNCH_ON(c, "k_index_query", st,

@@ -460,13 +460,13 @@ static int commit_with_index(sdbfg_ctx* c, GenParams P, uint32_t cap_grid, cudaS
     const uint64_t nfeat = (uint64_t)P.ntiles * kTileCap;
     if (c->index_max_rounds && P.ntiles) {
         const uint64_t nwords = nfeat / 32 + 2, nbits = (uint64_t)P.index_mask + 1;
-        for (DevBuf* b : {&c->d_seen[0], &c->d_seen[1], &c->d_pred}) CUDA_TRY(c, b->ensure(nwords * 4));
-        CUDA_TRY(c, c->d_diff.ensure(8 + std::max<uint64_t>(1, P.nfiles)));
-        CUDA_TRY(c, c->d_from.ensure(std::max<uint64_t>(1, P.nfiles) * 4));
-        CUDA_TRY(c, c->d_ckpt.ensure(((uint64_t)P.ntiles / kCkptTiles + 1) * kCkptWords * 4));
+        for (DevBuf* b : {&c->d_seen[0], &c->d_seen[1], &c->d_pred}) CUDA_TRY(c, c->must(*b, nwords * 4));
+        CUDA_TRY(c, c->must(c->d_diff, 8 + std::max<uint64_t>(1, P.nfiles)));
+        CUDA_TRY(c, c->must(c->d_from, std::max<uint64_t>(1, P.nfiles) * 4));
+        CUDA_TRY(c, c->must(c->d_ckpt, ((uint64_t)P.ntiles / kCkptTiles + 1) * kCkptWords * 4));
         P.commit_ckpt = c->d_ckpt.as<uint32_t>();
         P.commit_from = c->d_from.as<uint32_t>();
-        CUDA_TRY(c, c->d_idx_first.ensure(nbits * 4));
+        CUDA_TRY(c, c->must(c->d_idx_first, nbits * 4));
         uint32_t* first = c->d_idx_first.as<uint32_t>();
         uint32_t* seen = c->d_seen[0].as<uint32_t>();
         uint32_t* pred[2] = {c->d_pred.as<uint32_t>(), c->d_seen[1].as<uint32_t>()};
@@ -550,11 +550,16 @@ static int digest_stream_pipelined(sdbfg_ctx* c, const uint8_t* host_data, const
         const bool gather = host_dev && (n > 1 || host_dev != host_data);
         if (gather && tot <= kStageMaxBytes && cudaMemGetInfo(&freeb, &totb) == cudaSuccess &&
             (c->d_stage_in.cap >= tot || tot <= freeb / 2)) {
-            CUDA_TRY(c, c->d_stage_in.ensure(std::max<uint64_t>(16, tot)));
+            CUDA_TRY(c, c->must(c->d_stage_in, std::max<uint64_t>(16, tot)));
             staged = true;
         }
         cudaGetLastError();
     }
+    struct InUse {  // until the batch is over, however it ends
+        bool& flag;
+        ~InUse() { flag = false; }
+    } in_use{c->staging};
+    c->staging = staged;
     std::vector<uint32_t> perm(n);
     std::iota(perm.begin(), perm.end(), 0u);
     if (!ib)
@@ -568,7 +573,7 @@ static int digest_stream_pipelined(sdbfg_ctx* c, const uint8_t* host_data, const
     const uint64_t* offsets = offs_v.data();
     // results: total | output slot per file | info per file, read back in one copy
     const size_t at_info = 64 + (size_t)n * sizeof(uint64_t), result_bytes = at_info + n * sizeof(FileInfoDev);
-    CUDA_TRY(c, c->d_result.ensure(result_bytes));
+    CUDA_TRY(c, c->must(c->d_result, result_bytes));
     const size_t at_fetch = (result_bytes + 64 + 255) / 256 * 256;  // the first `fetch` filters, with the results
     CUDA_TRY(c, c->h_result.ensure(at_fetch + fetch * 256));
     CUDA_TRY(c, cudaMemsetAsync(c->d_result.p, 0, result_bytes, c->stream));
@@ -610,7 +615,7 @@ static int digest_stream_pipelined(sdbfg_ctx* c, const uint8_t* host_data, const
         }
         first_item[groups.size()] = (uint32_t)nitems;
         CUDA_TRY(c, c->h_stage_items.ensure(std::max<uint64_t>(1, nitems) * sizeof(StagePiece)));
-        CUDA_TRY(c, c->d_stage_items.ensure(std::max<uint64_t>(1, nitems) * sizeof(StagePiece)));
+        CUDA_TRY(c, c->must(c->d_stage_items, std::max<uint64_t>(1, nitems) * sizeof(StagePiece)));
         // the previous batch's table copy has finished (its call synchronised
         // at its end); the host table may be rewritten
         StagePiece* it = reinterpret_cast<StagePiece*>(c->h_stage_items.p);
@@ -666,20 +671,6 @@ static int digest_stream_pipelined(sdbfg_ctx* c, const uint8_t* host_data, const
     const bool solo = n == 1 && !ib && lens[0] >= kMinFile && stream_cap(lens[0]) <= out_cap;
     cudaEvent_t prev_scan = c->ev_start, prev_tiles = c->ev_start, prev2_tiles = c->ev_start;
     const uint64_t rank_half = c->d_ranks.cap / 2 / 16 * 16;  // bytes per half, 16-byte aligned
-    // A buffer that must be had: without room the linked commit's, which need
-    // not, are given back first (cudaFree waits for their users).
-    const auto need = [&](DevBuf& b, size_t bytes) {
-        cudaError_t e = b.ensure(bytes);
-        if (e == cudaErrorMemoryAllocation) {
-            cudaGetLastError();
-            for (sdbfg_ctx::Slot& s : c->slot) {
-                s.links.release();
-                s.last_tab.release();
-            }
-            e = b.ensure(bytes);
-        }
-        return e;
-    };
     const int max_depth = c->depth == kSlots && long_batch ? 4 : kSlots;  // (a lower depth is taken as it is)
     for (size_t gi = 0; gi < groups.size(); gi++) {
         const Group& g = groups[gi];
@@ -718,7 +709,7 @@ static int digest_stream_pipelined(sdbfg_ctx* c, const uint8_t* host_data, const
         const size_t at_first = at_rk + up(pre ? nrk * sizeof(uint2) : 0);
         const size_t at_fix = at_first + up(g.count * 4), table_bytes = at_fix + 4;
         CUDA_TRY(c, S.h_tables.ensure(table_bytes));
-        CUDA_TRY(c, need(S.tables, table_bytes + ntiles * 4));
+        CUDA_TRY(c, c->must(S.tables, table_bytes + ntiles * 4));
         uint8_t* hb = static_cast<uint8_t*>(S.h_tables.p);
         uint8_t* db = S.tables.as<uint8_t>();
         GenChunk* hc = reinterpret_cast<GenChunk*>(hb);
@@ -738,7 +729,7 @@ static int digest_stream_pipelined(sdbfg_ctx* c, const uint8_t* host_data, const
             for (uint32_t k = 0; k < g.count; k++) doff[k] = stage_off[g.first + k];
             CUDA_TRY(c, cudaStreamWaitEvent(st, c->ev_copy[gi], 0));
         } else {
-            CUDA_TRY(c, need(S.data, std::max<uint64_t>(16, bytes)));
+            CUDA_TRY(c, c->must(S.data, std::max<uint64_t>(16, bytes)));
             gdata = S.data.as<uint8_t>();
             uint64_t b = 0;
             for (uint32_t k = 0; k < g.count; k++) {
@@ -791,8 +782,8 @@ static int digest_stream_pipelined(sdbfg_ctx* c, const uint8_t* host_data, const
         if (!ib)
             std::stable_sort(ho, ho + g.count,
                              [&](uint32_t a, uint32_t b) { return lens[g.first + a] > lens[g.first + b]; });
-        CUDA_TRY(c, need(S.tile_out, std::max<uint64_t>(1, ntiles) * sizeof(TileOut)));
-        CUDA_TRY(c, need(S.features, std::max<uint64_t>(1, ntiles) * 5ull * kTileCap * 4));
+        CUDA_TRY(c, c->must(S.tile_out, std::max<uint64_t>(1, ntiles) * sizeof(TileOut)));
+        CUDA_TRY(c, c->must(S.features, std::max<uint64_t>(1, ntiles) * 5ull * kTileCap * 4));
         bool chain = !ib && most_tiles >= kChainTiles && 2 * most_tiles >= ntiles && ntiles < kLkMaxTiles;
         const size_t at_total = up(ntiles * 4), at_ends = at_total + up(g.count * 4);
         if (chain && (S.links.ensure(ntiles * kTileCap * sizeof(uint4)) != cudaSuccess ||
@@ -802,10 +793,10 @@ static int digest_stream_pipelined(sdbfg_ctx* c, const uint8_t* host_data, const
             S.last_tab.release();
             chain = false;
         }
-        CUDA_TRY(c, need(S.work, solo || chain ? 16 : std::max<uint64_t>(1, work) * 256));
+        CUDA_TRY(c, c->must(S.work, solo || chain ? 16 : std::max<uint64_t>(1, work) * 256));
         if (chain && !S.links.p) {  // given back for the line above
             chain = false;
-            CUDA_TRY(c, need(S.work, solo ? 16 : std::max<uint64_t>(1, work) * 256));
+            CUDA_TRY(c, c->must(S.work, solo ? 16 : std::max<uint64_t>(1, work) * 256));
         }
         CUDA_TRY(c, cudaMemcpyAsync(db, hb, table_bytes, cudaMemcpyHostToDevice, st));
         GenParams P{};
@@ -1001,7 +992,7 @@ static int digest_block_group(sdbfg_ctx* c, const uint8_t* dev_base, const std::
     // stretches | runs (| pieces, host copy only)
     const size_t at_items = nchunks * sizeof(GenChunk), at_runs = at_items + nitems * sizeof(uint2);
     const size_t table_bytes = at_runs + runs.size() * sizeof(GenChunk);
-    CUDA_TRY(c, c->d_chunks.ensure(table_bytes));
+    CUDA_TRY(c, c->must(c->d_chunks, table_bytes));
     bool pre = c->pre_ranks && dd % 8 == 0;
     if (pre && c->d_ranks.ensure(most8 * 16 + 256) != cudaSuccess) {
         cudaGetLastError();
@@ -1040,7 +1031,7 @@ static int digest_block_group(sdbfg_ctx* c, const uint8_t* dev_base, const std::
         first_piece.push_back(np);
         const int rc = ensure_copy_stream(c, slabs.size());
         if (rc) return rc;
-        CUDA_TRY(c, c->d_stage_items.ensure(np * sizeof(StagePiece)));
+        CUDA_TRY(c, c->must(c->d_stage_items, np * sizeof(StagePiece)));
         CUDA_TRY(c, cudaMemcpyAsync(c->d_stage_items.p, pieces, np * sizeof(StagePiece), cudaMemcpyHostToDevice, st));
         CUDA_TRY(c, cudaEventRecord(c->ev_start, st));
         CUDA_TRY(c, cudaStreamWaitEvent(c->copy_stream, c->ev_start, 0));
@@ -1176,7 +1167,7 @@ static int digest_block_host(sdbfg_ctx* c, const uint8_t* host_data, const uint6
             off[k] = bytes;
             bytes += (lens[g.first + k] + 15) & ~15ull;
         }
-        CUDA_TRY(c, c->d_data.ensure(std::max<uint64_t>(bytes, 16)));
+        CUDA_TRY(c, c->must(c->d_data, std::max<uint64_t>(bytes, 16)));
         uint8_t* d = c->d_data.as<uint8_t>();
         // Small contiguous inputs: one copy (exactly to the last input's end).
         // Else the gather kernel brings them over slab by slab, where the
@@ -1209,17 +1200,17 @@ static int digest_block_host(sdbfg_ctx* c, const uint8_t* host_data, const uint6
             }
             group_slots = res[i].filter_offset + res[i].bf_count - group_first_slot;
         }
-        CUDA_TRY(c, c->d_out_filters.ensure(std::max<uint64_t>(1, group_slots) * 256));
-        CUDA_TRY(c, c->d_out_counts.ensure(std::max<uint64_t>(1, group_slots) * 2));
+        CUDA_TRY(c, c->must(c->d_out_filters, std::max<uint64_t>(1, group_slots) * 256));
+        CUDA_TRY(c, c->must(c->d_out_counts, std::max<uint64_t>(1, group_slots) * 2));
         if (nidx) {
-            CUDA_TRY(c, c->d_probes.ensure(std::max<uint64_t>(1, group_slots) * kProbeWords * 4));
-            CUDA_TRY(c, c->d_nprobes.ensure(std::max<uint64_t>(1, group_slots)));
-            CUDA_TRY(c, c->d_hits.ensure(std::max<uint64_t>(1, group_slots) * nidx));
+            CUDA_TRY(c, c->must(c->d_probes, std::max<uint64_t>(1, group_slots) * kProbeWords * 4));
+            CUDA_TRY(c, c->must(c->d_nprobes, std::max<uint64_t>(1, group_slots)));
+            CUDA_TRY(c, c->must(c->d_hits, std::max<uint64_t>(1, group_slots) * nidx));
             c->probe_words = c->d_probes.as<uint32_t>();
             c->probe_counts = c->d_nprobes.as<uint8_t>();
         }
         if (ib) {
-            CUDA_TRY(c, c->d_feats.ensure(std::max<uint64_t>(1, group_slots) * kFeatWords * 4));
+            CUDA_TRY(c, c->must(c->d_feats, std::max<uint64_t>(1, group_slots) * kFeatWords * 4));
             c->feat_words = c->d_feats.as<uint32_t>();
         }
         // shift slots into the group-local output buffer
@@ -1270,7 +1261,7 @@ extern "C" int sdbfg_digest_batch(sdbfg_ctx* c, const uint8_t* host_data, const 
         uint64_t cap_needed = 0;
         for (uint32_t i = 0; i < n; i++)
             if (lens[i] >= kMinFile) cap_needed += stream_cap(lens[i]);
-        CUDA_TRY(c, c->d_out_filters.ensure(std::max<uint64_t>(1, cap_needed) * 256));
+        CUDA_TRY(c, c->must(c->d_out_filters, std::max<uint64_t>(1, cap_needed) * 256));
         // a few filters come back with the results, as many as there can be,
         // instead of in a copy of their own behind a second wait (one 64 KiB
         // file: 104 us, 112 with them)
@@ -1309,8 +1300,8 @@ extern "C" int sdbfg_digest_batch_index(sdbfg_ctx* c, const uint8_t* host_data, 
     CUDA_TRY(c, cudaSetDevice(c->device));
     cudaStream_t st = c->stream;
     const uint64_t nbits = index_bytes * 8;
-    CUDA_TRY(c, c->d_idx_bits.ensure(index_bytes));
-    CUDA_TRY(c, c->d_idx_count.ensure(8));
+    CUDA_TRY(c, c->must(c->d_idx_bits, index_bytes));
+    CUDA_TRY(c, c->must(c->d_idx_count, 8));
     CUDA_TRY(c, cudaMemcpyAsync(c->d_idx_bits.p, index_bits, index_bytes, cudaMemcpyHostToDevice, st));
     CUDA_TRY(c, cudaMemsetAsync(c->d_idx_count.p, 0, 8, st));
     const IndexBuild ib{c->d_idx_bits.as<uint32_t>(), (uint32_t)(nbits - 1), c->d_idx_count.as<unsigned long long>()};
@@ -1318,7 +1309,7 @@ extern "C" int sdbfg_digest_batch_index(sdbfg_ctx* c, const uint8_t* host_data, 
         uint64_t cap_needed = 0;
         for (uint32_t i = 0; i < n; i++)
             if (lens[i] >= kMinFile) cap_needed += stream_cap(lens[i]);
-        CUDA_TRY(c, c->d_out_filters.ensure(std::max<uint64_t>(1, cap_needed) * 256));
+        CUDA_TRY(c, c->must(c->d_out_filters, std::max<uint64_t>(1, cap_needed) * 256));
         uint64_t total = 0;
         rc = digest_stream_pipelined(c, host_data, nullptr, offsets, lens, n, c->d_out_filters.as<uint32_t>(),
                                      std::min(cap_needed, out_cap), res, &total, &ib);
@@ -1330,7 +1321,7 @@ extern "C" int sdbfg_digest_batch_index(sdbfg_ctx* c, const uint8_t* host_data, 
             return fail(c, SDBFG_ERR_CAPACITY, "need %llu filter slots", (unsigned long long)total_slots);
         if (total_slots && !out_counts) return fail(c, SDBFG_ERR_ARG, "block mode needs element-count output");
         if ((total_slots + 1) >> 24) return fail(c, SDBFG_ERR_ARG, "index build: more than 2^24 blocks in one batch");
-        CUDA_TRY(c, c->d_idx_first.ensure(nbits * 4));
+        CUDA_TRY(c, c->must(c->d_idx_first, nbits * 4));
         rc = index_first_init(c, ib.bits, c->d_idx_first.as<uint32_t>(), nbits, st);
         if (rc) return rc;
         rc = digest_block_host(c, host_data, offsets, lens, n, dd, out_filters, out_counts, res, nullptr, 0, nullptr,

@@ -416,8 +416,8 @@ extern "C" int sdbfg_set_load_text(sdbfg_ctx* c, const char* text, uint64_t len,
         d_flags.release();
         d_recs.release();
     };
-    if (s->allocate(total, nl) || d_text.ensure(std::max<uint64_t>(16, text_used + 16)) ||
-        d_lines.ensure(std::max<uint32_t>(1, nl) * sizeof(TextLine)) || d_flags.ensure(std::max<uint32_t>(1, nl) * 4)) {
+    if (s->allocate(total, nl) || c->must(d_text, std::max<uint64_t>(16, text_used + 16)) ||
+        c->must(d_lines, std::max<uint32_t>(1, nl) * sizeof(TextLine)) || c->must(d_flags, std::max<uint32_t>(1, nl) * 4)) {
         release_scratch();
         cudaGetLastError();
         return cleanup(fail(c, SDBFG_ERR_NOMEM, "set load: out of device memory"));
@@ -461,7 +461,7 @@ extern "C" int sdbfg_set_load_text(sdbfg_ctx* c, const char* text, uint64_t len,
             }
         }
         if (!recs.empty()) {
-            if (d_recs.ensure(recs.size() * sizeof(TextRecord))) {
+            if (c->must(d_recs, recs.size() * sizeof(TextRecord))) {
                 cudaGetLastError();
                 rc = fail(c, SDBFG_ERR_NOMEM, "set load: out of device memory");
                 break;

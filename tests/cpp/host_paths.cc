@@ -1,5 +1,7 @@
 // Cases of the library's host code against fake_cuda.h: one per run, by name.
 // Exit status 0: the case holds.
+#include <sys/mman.h>
+
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -50,6 +52,12 @@ T* device_array(size_t n) {
     void* p = nullptr;
     REQUIRE(cudaMalloc(&p, n * sizeof(T)) == cudaSuccess);
     return static_cast<T*>(p);
+}
+
+uint8_t* host_array(size_t n) {  // (never touched as a whole)
+    void* p = mmap(nullptr, n, PROT_READ | PROT_WRITE, MAP_PRIVATE | MAP_ANONYMOUS | MAP_NORESERVE, -1, 0);
+    REQUIRE(p != MAP_FAILED);
+    return static_cast<uint8_t*>(p);
 }
 
 // every comparison kernel that runs has its units and targets
@@ -286,6 +294,61 @@ void server_batch_gave_up() {
     sdbfg_ctx_destroy(c);
 }
 
+// where device memory is short, what earlier calls left for later ones (the
+// links of a large file, the staging copy of a pageable batch) makes room
+void room_is_made() {
+    const auto limit_to = [](uint64_t more) {
+        size_t free_ = 0, total = 0;
+        fake::memory_limit = 1ull << 40;
+        cudaMemGetInfo(&free_, &total);
+        fake::memory_limit = total - free_ + more;
+    };
+    constexpr uint64_t kGiB = 1ull << 30, kMiB = 1ull << 20;
+    fake::reads_pageable = true;
+    const uint64_t len = kGiB, off = 0, cap = sdbfg_digest_capacity(&len, 1, 0);
+    uint8_t* file = device_array<uint8_t>(len);
+    uint8_t* filters = device_array<uint8_t>(cap * 256);
+    uint8_t* data = host_array(3 * kGiB);
+    uint8_t* out = host_array(cap * 3 * 256);
+    std::vector<uint16_t> counts(3 * kGiB / 4096);
+    std::vector<int32_t> scores(499'500);
+    const std::vector<uint64_t> lens(12, kGiB / 4);
+    std::vector<uint64_t> offs(12);
+    for (size_t i = 0; i < offs.size(); i++) offs[i] = i * (kGiB / 4);
+    std::vector<sdbfg_digest_result> res(12);
+    for (const bool staging : {false, true}) {
+        // each call on a context of its own, which the call before filled
+        for (int call = 0; call < 4; call++) {
+            fake::memory_limit = 1ull << 40;
+            sdbfg_ctx* c = context();
+            sdbfg_set* s = call == 2 ? digests(c, 1000) : nullptr;
+            if (staging)
+                REQUIRE(sdbfg_digest_batch(c, data, offs.data(), lens.data(), 12, 0, out, 3 * cap, nullptr, res.data()) == SDBFG_OK);
+            else
+                REQUIRE(sdbfg_digest_batch_device(c, file, &off, &len, 1, 0, filters, cap, nullptr, res.data()) == SDBFG_OK);
+            REQUIRE(fake::launched(staging ? "k_stage_gather" : "k_stream_chain"));
+            limit_to(call == 2 ? 1 * kMiB : 64 * kMiB);
+            if (call == 0) s = digests(c, 1000);  // 128 MB of filters
+            if (call == 1)
+                REQUIRE(sdbfg_digest_batch(c, data, &off, &len, 1, 4096, out, cap, counts.data(), res.data()) == SDBFG_OK);
+            if (call == 2) REQUIRE(sdbfg_compare_all(c, s, scores.data()) == SDBFG_OK);
+            if (call == 3) {
+                const std::vector<uint64_t> small(1000, 300'000);
+                std::vector<uint64_t> at(1000);
+                for (size_t i = 0; i < at.size(); i++) at[i] = i * 300'000;
+                std::vector<sdbfg_digest_result> r(1000);
+                const uint64_t room = sdbfg_digest_capacity(small.data(), 1000, 0);
+                std::vector<uint8_t> f(room * 256), bits(16 << 20);
+                uint64_t added = 0;
+                REQUIRE(sdbfg_digest_batch_index(c, data, at.data(), small.data(), 1000, 0, f.data(), room, nullptr, r.data(),
+                                                 bits.data(), bits.size(), &added) == SDBFG_OK);
+            }
+            if (s) sdbfg_set_free(s);
+            sdbfg_ctx_destroy(c);
+        }
+    }
+}
+
 const std::map<std::string, std::function<void()>> kCases = {
     {"plan_other_stream", [] { plan_other_stream(false); }},
     {"plan_other_stream_compared", [] { plan_other_stream(true); }},
@@ -295,6 +358,7 @@ const std::map<std::string, std::function<void()>> kCases = {
     {"ranks_of_a_huge_input", ranks_of_a_huge_input},
     {"comparison_gave_up", comparison_gave_up},
     {"server_batch_gave_up", server_batch_gave_up},
+    {"room_is_made", room_is_made},
 };
 
 }  // namespace
