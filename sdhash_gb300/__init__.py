@@ -475,20 +475,25 @@ class Context:
                                       out_filters.ctypes.data, cap, counts.ctypes.data if dd_block_size else None,
                                       res)
         self._check(rc)
-        # one pass over the results as an array; a batch's digests view one
-        # array of filters and one of counts (768 digests: 2.2 ms through the
-        # result structures one field at a time, 0.6 ms for a copy per digest),
-        # those of a batch with more than _SHARED_FILTERS filters parts of them
-        r = np.frombuffer(res, dtype=_RESULT_DTYPE, count=n)
-        ok = r["status"] == 0
-        if not own:
+        # one pass over the results, of more than a few as arrays; a batch's
+        # digests view one array of filters and one of counts (768 digests: 2.2
+        # ms through the result structures one field at a time, 0.6 ms for a
+        # copy per digest), those of a batch with more than _SHARED_FILTERS
+        # filters parts of them
+        if n <= 4:
+            rows = [(x.status == 0, x.filter_offset, x.bf_count, x.last_count, length) for x, length in zip(res, lens.tolist())]
+            used = max((o + k for good, o, k, _, _ in rows if good), default=0)
+        else:
+            r = np.frombuffer(res, dtype=_RESULT_DTYPE, count=n)
+            ok = r["status"] == 0
             used = int((r["filter_offset"] + r["bf_count"])[ok].max(initial=0))
+            rows = zip(ok.tolist(), r["filter_offset"].tolist(), r["bf_count"].tolist(), r["last_count"].tolist(), lens.tolist())
+        if not own:
             split = used > _SHARED_FILTERS
             if not split:
                 out_filters = np.array(out_filters[:used * 256], dtype=np.uint8)
         out = []
-        for i, (good, o, k, last, length) in enumerate(zip(ok.tolist(), r["filter_offset"].tolist(), r["bf_count"].tolist(),
-                                                           r["last_count"].tolist(), lens.tolist())):
+        for i, (good, o, k, last, length) in enumerate(rows):
             if not good:
                 out.append(None)
                 continue
@@ -499,7 +504,7 @@ class Context:
             else:
                 out.append(Digest._of(name, length, k, last, STREAM_MAX_ELEM, 0, filt, None))
         if not own and split:
-            _copy_in_parts(out, r["filter_offset"], out_filters, counts if dd_block_size else None)
+            _copy_in_parts(out, [x.filter_offset for x in res], out_filters, counts if dd_block_size else None)
         return out
 
     def load_index(self, path: str) -> Index:

@@ -8,7 +8,7 @@ import pytest
 
 
 @pytest.mark.parametrize("dd", [0, 16384])
-@pytest.mark.parametrize("count", [1, 40, 3000])
+@pytest.mark.parametrize("count", [1, 3, 40, 3000])
 def test_digest_keeps_a_bounded_array(native, monkeypatch, dd, count):
     import sdhash_gb300 as g
 
