@@ -945,8 +945,8 @@ static int digest_block_group(sdbfg_ctx* c, const uint8_t* dev_base, const std::
     P.counters = c->d_counters.as<uint32_t>();
     P.lead = c->lead;
     // Ranks ahead of the block kernel (2 bytes per input byte, in runs of
-    // whole blocks) where a block's ranks start 16-byte aligned; slabs
-    // bound their buffer.
+    // whole blocks) where a block's ranks start 16-byte aligned and there are
+    // enough blocks; slabs bound their buffer.
     struct Slab {
         uint32_t first_run, nruns, nchunks;
         uint64_t r8, stretches[kRkChoices];
@@ -993,7 +993,11 @@ static int digest_block_group(sdbfg_ctx* c, const uint8_t* dev_base, const std::
     const size_t at_items = nchunks * sizeof(GenChunk), at_runs = at_items + nitems * sizeof(uint2);
     const size_t table_bytes = at_runs + runs.size() * sizeof(GenChunk);
     CUDA_TRY(c, c->must(c->d_chunks, table_bytes));
-    bool pre = c->pre_ranks && dd % 8 == 0;
+    // Up to two blocks per SM run at once with their ranks computed in the
+    // kernel, and a rank kernel ahead of it is one launch more to wait for: 8
+    // blocks of 512 bytes 31 us and 35 with it, 300 of 16 KiB 65 and 72; 600 of
+    // 16 KiB 102 and 96 (of 4 KiB 49 and 55), 2,400 of 512 bytes 76 and 74.
+    bool pre = c->pre_ranks && dd % 8 == 0 && nchunks > 2 * (uint64_t)c->sms;
     if (pre && c->d_ranks.ensure(most8 * 16 + 256) != cudaSuccess) {
         cudaGetLastError();
         c->d_ranks.release();
