@@ -79,9 +79,11 @@ int sdbfg_ctx_kernel_time(sdbfg_ctx *ctx, const char *kernel, double *total_ms, 
  * lead-ins only make the re-walk path run more often; tests use this to
  * exercise it.  No counterpart in the reference (its walk is sequential). */
 int sdbfg_ctx_set_lead(sdbfg_ctx *ctx, uint32_t steps);
-/* Stream-mode launch groups (<= 256 MiB of input each, or one larger input)
- * kept in flight on separate streams, 1..8 (default 8: up to eight, four of
- * 1 GiB in batches of more than 4 GiB): the ordered commit of one group
+/* Stream-mode launch groups (<= 256 MiB of input each, or one larger input;
+ * 1 GiB in batches of more than 4 GiB) kept in flight on separate streams,
+ * 1..8.  8 (the default) is four in batches of more than 4 GiB, where eight
+ * are slower (28.4 GB from the host: 99 against 141 GB/s); 1..7 hold for every
+ * batch.  The ordered commit of one group
  * overlaps the next groups' tile kernels.  Depth 1 runs groups one after
  * another (used to time kernels without overlap).  Tuning knob without a
  * counterpart in the reference. */

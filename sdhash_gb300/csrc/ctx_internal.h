@@ -22,44 +22,58 @@ namespace sdbfg_host {
 
 constexpr uint32_t kMaxTilesPerLaunch = 1u << 18;  // 2 GiB of stream input per launch group
 constexpr uint64_t kMaxBytesPerLaunch = 2ull << 30;
-constexpr uint64_t kBlockSlabBytes = 256ull << 20;  // block-mode input whose ranks are held at once (512 MiB of them)
-constexpr uint64_t kFirstHostSlabBytes = 16ull << 20;  // first slab of a host-input block batch (each later one at most twice it)
+// Block-mode input whose ranks are held at once (512 MiB of them).  On the
+// device 1 GiB in blocks of 16 KiB: 6.13 ms, with 128 MiB 6.29, with 512 MiB
+// 6.03; 400 uneven files in blocks of 4 KiB: 5.32, 5.40 and 5.27.
+constexpr uint64_t kBlockSlabBytes = 256ull << 20;
+// First slab of a host-input block batch (each later one at most twice it).
+// 768 fragments of 140 MB: 2.40 ms, with 8 MiB 2.54, with 32 MiB 2.40; 100
+// files of 600 KiB: 1.61, 1.65 and 1.67; four of 128 MiB: 4.81, 4.64 and 4.86.
+constexpr uint64_t kFirstHostSlabBytes = 16ull << 20;
 // Stream batches (inputs sorted by size, largest first) in groups of this size:
 // a group's ordered commits, which one large file can draw out, run beside
 // the tiles of the groups behind it, and the last group's files are small.
-// 3.1 GB on the device, with its tiles at 14.8 ms (13.0 now): 21.2 ms, in groups
-// of 2 GiB 22.2, of 128 MiB 25.4; 0.9 GB from the host: 10.9 ms against 11.9 in
-// groups of 512 MiB and more.
+// On the device 64 files of 40 MiB: 18.6 ms, in groups of 128 MiB 19.1, of 512
+// MiB 18.5; 1,000 of 1 MiB: 6.20, 6.31 and 6.21.  From the host 300 uneven files
+// of up to 16 MiB: 7.85, 7.46 and 8.10; 400 of 1 MiB: 4.24, 4.18 and 4.27.
 constexpr uint64_t kStreamGroupBytes = 256ull << 20;
 // A long batch keeps the GPU busy whatever the groups' size, and many commits in
 // flight take the registers that the staging gather's CTAs need on an SM: groups
 // of 1 GiB, four in flight.  28.4 GB: 160 ms on the device and 201 from the
-// host; 256 MiB, eight in flight: 164 and 303; 2 GiB, four: 160 and 200.
+// host (eight in flight: 160 and 287); groups of 256 MiB, eight in flight: 164
+// and 303.  1,500 files of 4 MiB: 35.8 and 54.2, in groups of 256 MiB 36.1 and
+// 71.9; 2,500 from the host 88.0, in groups of 512 MiB 89.0, of 2 GiB 91.5.  The
+// line is not sharp: 2.4 GiB from the host take 23.2 ms either way, 3.7 GiB
+// 41.3 and with the long batches' groups 35.4.
 constexpr uint64_t kLongBatchBytes = 4ull << 30;
 constexpr uint64_t kLongGroupBytes = 1ull << 30;
 // First group of a host-input stream batch (each later one at most twice it):
-// its copy is the one nothing hides.  64 files of 1 MiB: 1.06 ms (1.02 now), with
-// 16 MiB 1.11, with 64 MiB (one group) 1.17.
+// its copy is the one nothing hides.  64 files of 1 MiB: 1.06 ms, with 16 MiB
+// 1.11, with 64 MiB (one group) 1.17; 200 of 200 KiB: 0.86, 0.78 and 0.85; 600 of
+// 1 MiB: 6.23, 6.28 and 6.27; 160 uneven ones of 0.86 GB: 9.68, 9.52 and 9.70.
 constexpr uint64_t kFirstHostGroupBytes = 32ull << 20;
 // A group with a file of this many tiles, and at least half of all, commits
 // through links (k_stream_chain): there the group waits for that one file's
 // chain.  One file of 2, 3, 8 and 32 MiB on the device: 209, 267, 537 and 1,698
-// us, through k_stream_commit 191, 289, 717 and 2,646.  Where many files'
+// us, through k_stream_commit 191, 289, 717 and 2,646; of 5 and 100 MiB 380 and
+// 5,110 against 464 and 8,280; two files of 4 MiB 384 against 440.  Where many files'
 // commits run beside tiles anyway, the links are only more work: 3.1 GB of
 // uneven files 22.9 ms against 21.2.
 constexpr uint32_t kChainTiles = 384;
 constexpr uint64_t kFirstIndexGroupBytes = 256ull << 20;  // with an index being built (groups one after another)
-constexpr uint64_t kFetchFilters = 512;  // output filters (128 KiB) that a host batch reads back with its results
+// Output filters (128 KiB) that a host batch reads back with its results: one
+// file of 200 and 900 KiB 113 and 164 us, without 118 and 171.
+constexpr uint64_t kFetchFilters = 512;
 constexpr uint32_t kMinFile = 512;                 // MIN_FILE_SIZE (sdbf_defines.h:56)
 constexpr uint64_t kPairsPerLaunch = 1ull << 22;
 constexpr int kSlots = 8;  // stream-mode launch groups in flight (at most)
-// pinned host-input stream batches up to this size (and half the free
-// device memory) are staged whole on the device
+// host-input stream batches up to this size (and half the free device
+// memory) are staged whole on the device, where it can read the host's memory
 constexpr uint64_t kStageMaxBytes = 64ull << 30;
 constexpr uint64_t kStagePiece = 1ull << 20;  // work item of the staging gather
 struct StagePiece {
     uint64_t dst;  // staging offset (16-byte aligned)
-    uint64_t src;  // device address of the pinned host bytes
+    uint64_t src;  // the host bytes as the device addresses them
     uint64_t len;
 };
 
@@ -189,7 +203,7 @@ struct sdbfg_ctx {
     uint32_t* gave_up() const { return static_cast<uint32_t*>(h_flags.p) + 1; }
     // comparison buffers
     DevBuf d_pairs, d_scores;
-    // stream-mode pipeline: two launch-group slots on their own streams
+    // stream-mode pipeline: launch-group slots on their own streams
     struct Slot {
         cudaStream_t stream = nullptr;
         cudaEvent_t done = nullptr;

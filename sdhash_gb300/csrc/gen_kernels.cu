@@ -2166,8 +2166,8 @@ __global__ void __launch_bounds__(256) k_stream_emit(GenParams P, const uint64_t
 // know about blocks; only a block's last 64 positions have rank 0), and the
 // block is walked as one or two tiles of kBlkL steps, the second entered
 // with the first one's exit state.  55 KB of shared memory then hold four
-// blocks on an SM.  Without (block sizes that are no multiple of 8, or no
-// room for the ranks) the whole block is ranked and walked at once, two
+// blocks on an SM.  Without (block sizes that are no multiple of 8, few blocks,
+// or no room for the ranks) the whole block is ranked and walked at once, two
 // blocks to an SM.  A 1 GiB image at 16 KiB blocks: ranks 1.6 ms and this
 // kernel 4.45 ms; when the ranks left the tile the two went from 10.9 to 8.2 ms,
 // most of it the set-up of 96 threads' windows for 170 positions each.

@@ -239,6 +239,9 @@ inline uint64_t cross_work(uint64_t q, uint64_t t, int variant) {
 // per CTA 140; 67 digests of 32 to 289: 135 and 163; one query of 1,024 filters
 // against four of 8,192: 127 and 144; 376 queries against one: 192 and 203.
 // Above, 120 digests of 20 to 400, 6,583 tiles: 360, with two-tile units 388.
+// The line is not sharp: of 13 other jobs of 4 to 96 tiles per CTA one of 23
+// would be 13 % slower in eight units per CTA, but one of 11 and one of 14 are 6
+// and 12 % faster in four (154 and 182 us); the rest are the same either way.
 inline uint64_t effective_unit_budget(uint64_t configured, uint64_t total, uint64_t slots, int variant) {
     slots = std::max<uint64_t>(1, slots);
     if (variant == kMatVariantTc) {

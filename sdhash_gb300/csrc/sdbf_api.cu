@@ -291,7 +291,7 @@ __global__ void k_scan_offsets(const FileInfoDev* __restrict__ info, uint64_t* _
 
 // Only slots below dst_cap are written: whether the batch fits is known to the
 // host when it is over.
-__global__ void k_pack_group(const uint32_t* __restrict__ work, const GenFile* __restrict__ files,
+__global__ void k_pack_filters(const uint32_t* __restrict__ work, const GenFile* __restrict__ files,
                              const FileInfoDev* __restrict__ info, const uint64_t* __restrict__ dst_off,
                              uint32_t* __restrict__ dst, uint64_t dst_cap, uint32_t n) {
     for (uint32_t f = blockIdx.x; f < n; f += gridDim.x) {
@@ -427,7 +427,7 @@ static int ensure_pipeline(sdbfg_ctx* c) {
     if (!c->ev_start) CUDA_TRY(c, cudaEventCreateWithFlags(&c->ev_start, cudaEventDisableTiming));
     // the pipeline's small kernels take the tile kernels' shared-memory / L1
     // split, so their CTAs can share an SM with them
-    for (const void* f : {(const void*)k_scan_offsets, (const void*)k_pack_group})
+    for (const void* f : {(const void*)k_scan_offsets, (const void*)k_pack_filters})
         cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared);
     cudaGetLastError();
     return SDBFG_OK;
@@ -437,9 +437,10 @@ static int ensure_pipeline(sdbfg_ctx* c) {
 // (dev_data + offsets[i], 16-byte aligned) or in host memory (host_data +
 // offsets[i]) and copied per launch group.  Filters are packed in input
 // order into dev_out (device); results[] gets counts and slots.  Launch
-// groups alternate between two streams with their own workspaces, so the
-// commit of one group overlaps the tiles (and the input copy) of the next;
-// the host synchronises once, at the end.
+// groups take turns on up to eight streams with their own workspaces, so the
+// commit of one group overlaps the tiles (and the input copies) of the next
+// ones; the host waits for a stream when it comes round again and once at the
+// end.
 // An index being built alongside (sdhash --index): device bits, bit mask,
 // counter of inserts that set a new bit.
 struct IndexBuild {
@@ -895,12 +896,12 @@ static int digest_stream_pipelined(sdbfg_ctx* c, const uint8_t* host_data, const
                             launch_stream_emit(P, d_off + g.first, dev_out, out_cap, (uint32_t)c->sms, st));
         else
             TIMED_LAUNCH_ON(c, "k_pack_filters", st,
-                            (k_pack_group<<<std::min<uint32_t>(g.count, (uint32_t)c->sms * 8), 256, 0, st>>>(
+                            (k_pack_filters<<<std::min<uint32_t>(g.count, (uint32_t)c->sms * 8), 256, 0, st>>>(
                                  S.work.as<uint32_t>(), P.files, d_info + g.first, d_off + g.first, dev_out, out_cap, g.count),
                              cudaGetLastError()));
         CUDA_TRY(c, cudaEventRecord(S.done, st));
     }
-    // join: the caller's stream waits for both slots, then results come back
+    // join: the caller's stream waits for the slots, then results come back
     for (int k = 0; k < kSlots; k++)
         if (c->slot[k].used) CUDA_TRY(c, cudaStreamWaitEvent(c->stream, c->slot[k].done, 0));
     uint8_t* hr = static_cast<uint8_t*>(c->h_result.p);
