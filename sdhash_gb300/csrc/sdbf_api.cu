@@ -547,7 +547,7 @@ static int digest_stream_pipelined(sdbfg_ctx* c, const uint8_t* host_data, const
         uint64_t tot = 0;
         for (uint32_t i = 0; i < n; i++) tot += (lens_in[i] + 15) & ~15ull;
         size_t freeb = 0, totb = 0;
-        // (one pageable input: a plain copy of it)
+        // (one input: a plain copy of it, where the device has no address of its own for it)
         const bool gather = host_dev && (n > 1 || host_dev != host_data);
         if (gather && tot <= kStageMaxBytes && cudaMemGetInfo(&freeb, &totb) == cudaSuccess &&
             (c->d_stage_in.cap >= tot || tot <= freeb / 2)) {
