@@ -600,7 +600,7 @@ extern "C" int sdbfg_ctx_get_compare_tuning(const sdbfg_ctx* c, int* variant, ui
 }
 
 extern "C" uint64_t sdbfg_compare_filter_pairs(sdbfg_ctx* c, const sdbfg_set* a, const sdbfg_set* b) {
-    if (!c || !a) return 0;
+    if (!c || !a || cudaSetDevice(c->device) != cudaSuccess) return 0;
     MatPlan* p;
     if (get_plan(c, a, b, b ? kMatModeCross : kMatModeAll, &p)) return 0;
     return p->filter_pairs;

@@ -118,6 +118,7 @@ extern "C" uint64_t sdbfg_ctx_launch_count(const sdbfg_ctx* c) { return c ? c->l
 
 extern "C" int sdbfg_ctx_profile(sdbfg_ctx* c, int enable) {
     if (!c) return SDBFG_ERR_ARG;
+    CUDA_TRY(c, cudaSetDevice(c->device));
     timer_collect(c);
     c->profile = enable != 0;
     if (enable) {

@@ -44,6 +44,7 @@ namespace {
 std::recursive_mutex mu;
 std::set<CUstream_st*> streams;
 std::map<uintptr_t, size_t> device_mem, pinned;
+std::map<uintptr_t, int> devices;  // of the allocations
 uint64_t used = 0;
 thread_local int current = 0;
 thread_local cudaError_t last = cudaSuccess;
@@ -133,6 +134,11 @@ bool launched(const char* kernel) {
     for (const Launch& x : launches)
         if (x.kernel.find(kernel) != std::string::npos) return true;
     return false;
+}
+int device_of(const void* p) {
+    Lock l;
+    if (!room(device_mem, p)) return -1;
+    return std::prev(devices.upper_bound((uintptr_t)p))->second;
 }
 }  // namespace fake
 
@@ -237,6 +243,7 @@ cudaError_t cudaMalloc(void** p, size_t n) {
     if (a == MAP_FAILED) return ret(cudaErrorMemoryAllocation);
     if (n <= (64u << 20)) memset(a, fake::kPoison, n);
     device_mem[(uintptr_t)a] = n;
+    devices[(uintptr_t)a] = current;
     used += n;
     *p = a;
     return cudaSuccess;
@@ -249,6 +256,7 @@ cudaError_t cudaFree(void* p) {
     if (it == device_mem.end()) return ret(cudaErrorInvalidValue);
     used -= it->second;
     munmap(p, it->second + 4096);
+    devices.erase(it->first);
     device_mem.erase(it);
     return cudaSuccess;
 }

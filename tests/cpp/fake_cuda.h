@@ -34,6 +34,7 @@ extern bool reads_pageable;           // the device reads pageable memory
 // the arguments, returns what runs when the stream gets there
 void on_launch(const char* kernel, std::function<std::function<void()>(void**)> f);
 bool launched(const char* kernel);    // a kernel whose name contains this
+int device_of(const void* p);         // the device that was current when this allocation was made
 
 constexpr uint8_t kPoison = 0xCD;     // fresh device memory (allocations of up to 64 MiB)
 

@@ -349,6 +349,33 @@ void room_is_made() {
     }
 }
 
+// a context's memory is on its own device, whichever device is current when it
+// is called
+void other_device_current() {
+    sdbfg_ctx* c = context(1);
+    sdbfg_set* s = digests(c, 40);
+    int32_t* out = device_array<int32_t>(780);
+    static int runs = 0;
+    fake::on_launch("k_matrix", [](void** args) {
+        const sdbfg::MatParams P = *static_cast<sdbfg::MatParams*>(args[0]);
+        return [P] {
+            runs++;
+            REQUIRE(fake::device_of(P.units) == 1 && fake::device_of(P.filters[0]) == 1);
+            REQUIRE(!P.phase || fake::device_of(P.phase) == 1);
+        };
+    });
+    cudaSetDevice(0);
+    REQUIRE(sdbfg_compare_filter_pairs(c, s, nullptr) > 0);
+    REQUIRE(sdbfg_compare_all_device(c, s, out) == SDBFG_OK);
+    cudaSetDevice(0);
+    REQUIRE(sdbfg_ctx_profile(c, 1) == SDBFG_OK);
+    REQUIRE(sdbfg_compare_all_device(c, s, out) == SDBFG_OK);
+    REQUIRE(sdbfg_ctx_synchronize(c) == SDBFG_OK);
+    REQUIRE(runs > 0);
+    sdbfg_set_free(s);
+    sdbfg_ctx_destroy(c);
+}
+
 const std::map<std::string, std::function<void()>> kCases = {
     {"plan_other_stream", [] { plan_other_stream(false); }},
     {"plan_other_stream_compared", [] { plan_other_stream(true); }},
@@ -359,6 +386,7 @@ const std::map<std::string, std::function<void()>> kCases = {
     {"comparison_gave_up", comparison_gave_up},
     {"server_batch_gave_up", server_batch_gave_up},
     {"room_is_made", room_is_made},
+    {"other_device_current", other_device_current},
 };
 
 }  // namespace
